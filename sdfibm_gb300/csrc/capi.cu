@@ -314,12 +314,6 @@ static cudaError_t dalloc(T** p, size_t n) {
 }
 
 // ---- explicit polyMesh (unstructured) contexts: helpers ----------------------------------------------------------
-__global__ void poly_ft_kernel(const double* ftacc, double* ft, int S, double rho_f) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    for (int r = 0; r < 6; ++r) ft[6 * s + r] = ftacc[6 * s + r] * rho_f;  // force *= m_rhof (solidcloud.cpp:423)
-}
-
 template <typename T>
 static cudaError_t poly_alloc(sdfibm_ctx::Poly& P, T** p, size_t n) {
     const cudaError_t e = cudaMalloc((void**)p, std::max<size_t>(1, n) * sizeof(T));
@@ -1709,16 +1703,41 @@ int sdfibm_cuda_create_polymesh(const double* points, int64_t npoints, const int
         poly_upload(P, &k.cf, hm.cell_faces) && poly_upload(P, &k.cp_off, hm.cell_pts_off) &&
         poly_upload(P, &k.cp, hm.cell_pts) && poly_upload(P, &k.cc_off, hm.cell_cells_off) &&
         poly_upload(P, &k.ccl, hm.cell_cells) && poly_upload(P, &k.Cf, hm.Cf) && poly_upload(P, &k.Sf, hm.Sf) &&
-        poly_upload(P, &k.Cc, hm.Cc) && poly_upload(P, &k.Vc, hm.Vc);
+        poly_upload(P, &k.Cc, hm.Cc) && poly_upload(P, &k.Vc, hm.Vc) &&
+        poly_upload(P, &k.cfv_off, hm.cfv_off) && poly_upload(P, &k.cfv, hm.cfv);
+    k.nblocks = (int32_t)((N + POLY_BLOCK - 1) / POLY_BLOCK);
+    k.uniform_np = hm.uniform_np ? 1 : 0;
+    float4 *pt32 = nullptr, *cell32 = nullptr;
+    double* mSf = nullptr;
+    float* blk = nullptr;
+    const bool ok_set = ok_up && poly_alloc(P, &pt32, 2 * (size_t)hm.npoints) == cudaSuccess &&
+                        poly_alloc(P, &cell32, (size_t)N) == cudaSuccess &&
+                        poly_alloc(P, &mSf, (size_t)hm.nfaces) == cudaSuccess &&
+                        poly_alloc(P, &blk, 12 * (size_t)k.nblocks) == cudaSuccess;
+    if (ok_set) poly_setup_kernel<<<ctx->num_sms * 4, 256, 0, ctx->stream>>>(k, pt32, cell32, mSf, blk);
+    k.pt32 = pt32; k.cell32 = cell32; k.mSf = mSf; k.blk = blk;
     PolyWork& w = P.w;
     w.words = (N + 31) / 32;
     w.qcap = N;
-    const bool ok = ok_up && poly_alloc(P, &w.visited, (size_t)(S * w.words)) == cudaSuccess &&
+    const bool ok = ok_set && poly_alloc(P, &w.visited, (size_t)(S * w.words)) == cudaSuccess &&
          poly_alloc(P, &w.queue, (size_t)(S * w.qcap)) == cudaSuccess &&
          poly_alloc(P, &w.qtype, (size_t)(S * w.qcap)) == cudaSuccess &&
          poly_alloc(P, &w.count, (size_t)S) == cudaSuccess && poly_alloc(P, &w.acc, (size_t)(5 * N)) == cudaSuccess &&
-         poly_alloc(P, &w.claim, (size_t)N) == cudaSuccess &&
-         cudaMemset(w.count, 0, sizeof(int32_t) * S) == cudaSuccess;
+         poly_alloc(P, &w.claim, (size_t)N) == cudaSuccess && poly_alloc(P, &w.nitems, 1) == cudaSuccess &&
+         (!k.uniform_np ||
+          (poly_alloc(P, &w.plan, (size_t)S) == cudaSuccess &&
+           poly_alloc(P, &w.items, (size_t)(S * k.nblocks)) == cudaSuccess &&
+           poly_alloc(P, &w.parent, (size_t)(S * w.qcap)) == cudaSuccess &&
+           poly_alloc(P, &w.clist, (size_t)(S * w.qcap)) == cudaSuccess &&
+           poly_alloc(P, &w.ctype, (size_t)(S * w.qcap)) == cudaSuccess &&
+           poly_alloc(P, &w.ccount, (size_t)S) == cudaSuccess && poly_alloc(P, &w.seed, (size_t)S) == cudaSuccess &&
+           poly_alloc(P, &w.mincand, (size_t)S) == cudaSuccess)) &&
+         cudaMemset(w.count, 0, sizeof(int32_t) * S) == cudaSuccess &&
+         // poly_finalize_kernel leaves these as they are here
+         cudaMemset(w.acc, 0, sizeof(double) * 5 * N) == cudaSuccess &&
+         cudaMemset(w.claim, 0xff, sizeof(int32_t) * N) == cudaSuccess &&
+         cudaMemset(w.nitems, 0, sizeof(int32_t)) == cudaSuccess && cudaGetLastError() == cudaSuccess &&
+         cudaStreamSynchronize(ctx->stream) == cudaSuccess;
     w.err = &ctx->d_cnt->error;
     if (!ok) {
         ctx->err = "polyMesh: device allocation failed";
@@ -1737,32 +1756,36 @@ static int poly_interact(sdfibm_ctx* ctx, double time, double dt, const float* U
     cudaStream_t st = ctx->stream;
     int launches = 0;
     mark_begin(ctx);
-    set_step_kernel<<<1, 1, 0, st>>>(ctx->d_step, time, dt, 1, 0.0);
-    // SolidCloud::interact zeroes the four fields over the whole mesh (solidcloud.cpp:438-441)
-    CK(cudaMemsetAsync(As, 0, sizeof(float) * N, st));
-    CK(cudaMemsetAsync(Fs, 0, sizeof(float) * 3 * N, st));
-    CK(cudaMemsetAsync(Ts, 0, sizeof(float) * N, st));
-    CK(cudaMemsetAsync(Ct, 0, sizeof(int32_t) * N, st));
-    CK(cudaMemsetAsync(P.w.acc, 0, sizeof(double) * 5 * N, st));
-    CK(cudaMemsetAsync(P.w.claim, 0xff, sizeof(int32_t) * N, st));
-    launches = 1;
     if (S > 0) {
-        CK(cudaMemsetAsync(P.w.visited, 0, sizeof(uint32_t) * P.w.words * S, st));
-        CK(cudaMemsetAsync(ctx->d_ftacc, 0, sizeof(double) * 6 * S, st));
-        poly_enum_kernel<<<S, 256, 0, st>>>(P.k, ctx->d_sk, ctx->d_st, P.w);
-        mark(ctx, "poly_enum_kernel");
-        poly_couple_kernel<<<dim3(8, S), 256, 0, st>>>(P.k, ctx->d_sk, ctx->d_st, P.w, U, ctx->d_ftacc, ctx->d_step);
+        // CTAs per solid of the kernels that walk a solid's blocks or list: four per SM over all solids
+        const int per = std::max(1, std::min(64, (4 * ctx->num_sms + S - 1) / S));
+        if (P.k.uniform_np) {
+            const int pb = std::max(1, std::min(per, (P.k.nblocks + 255) / 256));
+            poly_plan_kernel<<<dim3(S, pb), 256, 0, st>>>(P.k, ctx->d_sk, ctx->d_st, P.w, ctx->d_ftacc);
+            mark(ctx, "poly_plan_kernel");
+            poly_classify_kernel<<<S + 4 * ctx->num_sms, 256, 0, st>>>(P.k, ctx->d_sk, ctx->d_st, P.w, S);
+            mark(ctx, "poly_classify_kernel");
+            poly_link_kernel<<<dim3(S, per), 256, 0, st>>>(P.k, P.w);
+            mark(ctx, "poly_link_kernel");
+            poly_couple_kernel<<<dim3(S, per), 256, 0, st>>>(P.k, ctx->d_sk, ctx->d_st, P.w, U, ctx->d_ftacc,
+                                                               1.0 / dt, 1);
+            launches += 4;
+        } else {
+            CK(cudaMemsetAsync(P.w.visited, 0, sizeof(uint32_t) * P.w.words * S, st));
+            CK(cudaMemsetAsync(ctx->d_ftacc, 0, sizeof(double) * 6 * S, st));
+            poly_enum_kernel<<<S, 256, 0, st>>>(P.k, ctx->d_sk, ctx->d_st, P.w);
+            mark(ctx, "poly_enum_kernel");
+            poly_couple_kernel<<<dim3(S, per), 256, 0, st>>>(P.k, ctx->d_sk, ctx->d_st, P.w, U, ctx->d_ftacc,
+                                                               1.0 / dt, 0);
+            launches += 2;
+        }
         mark(ctx, "poly_couple_kernel");
-        launches += 2;
     }
-    poly_finalize_kernel<<<ctx->num_sms * 4, 256, 0, st>>>(P.w, (int32_t)N, As, Fs, Ts, Ct);
+    // SolidCloud::interact zeroes the four fields over the whole mesh (solidcloud.cpp:438-441): written whole here
+    poly_finalize_kernel<<<ctx->num_sms * 4, 256, 0, st>>>(P.w, (int32_t)N, As, Fs, Ts, Ct, S, ctx->d_ftacc, ctx->d_ft,
+                                                           ctx->opt.rho_f, ctx->d_st);
     mark(ctx, "poly_finalize_kernel");
     ++launches;
-    if (S > 0) {
-        poly_ft_kernel<<<(S + 127) / 128, 128, 0, st>>>(ctx->d_ftacc, ctx->d_ft, S, ctx->opt.rho_f);
-        ft_to_state_kernel<<<(S + 127) / 128, 128, 0, st>>>(ctx->d_ft, ctx->d_st, S);
-        launches += 2;
-    }
     CK(cudaGetLastError());
     ctx->launches_last = launches;
     ctx->interacted = true;

@@ -131,23 +131,38 @@ bool build_polymesh(const double* points, int64_t npoints, const int32_t* face_o
         m.Cc[3 * c] = x.x; m.Cc[3 * c + 1] = x.y; m.Cc[3 * c + 2] = x.z;
         m.Vc[c] = vc[c] * (1.0 / 3.0);
     }
-    // cell -> points in ascending label order (cellPoints), cell -> face neighbours (cellCells)
+    // cell -> points in ascending label order (cellPoints), the position of every face vertex among them; cell -> face
+    // neighbours (cellCells)
     m.cell_pts_off.assign(nc + 1, 0);
+    m.cell_pts.reserve(8 * nc);
+    m.cfv_off.reserve(m.cell_faces.size() + 1);
+    m.cfv.reserve(4 * m.cell_faces.size());
     std::vector<int32_t> pts;
-    std::vector<std::vector<int32_t>> cp(nc);
     for (int64_t c = 0; c < nc; ++c) {
         pts.clear();
         for (int32_t q = m.cell_faces_off[c]; q < m.cell_faces_off[c + 1]; ++q) {
             const int32_t f = m.cell_faces[q];
-            for (int32_t r = face_off[f]; r < face_off[f + 1]; ++r) pts.push_back(face_lab[r]);
+            for (int32_t r = face_off[f]; r < face_off[f + 1]; ++r) {  // insertion: a cell has few points
+                const int32_t l = face_lab[r];
+                size_t at = pts.size();
+                while (at > 0 && pts[at - 1] > l) --at;
+                if (at == 0 || pts[at - 1] != l) pts.insert(pts.begin() + at, l);
+            }
         }
-        std::sort(pts.begin(), pts.end());
-        pts.erase(std::unique(pts.begin(), pts.end()), pts.end());
-        cp[c] = pts;
-        m.cell_pts_off[c + 1] = m.cell_pts_off[c] + (int32_t)pts.size();
+        m.cell_pts.insert(m.cell_pts.end(), pts.begin(), pts.end());
+        m.cell_pts_off[c + 1] = (int32_t)m.cell_pts.size();
+        for (int32_t q = m.cell_faces_off[c]; q < m.cell_faces_off[c + 1]; ++q) {
+            const int32_t f = m.cell_faces[q];
+            m.cfv_off.push_back((int32_t)m.cfv.size());
+            for (int32_t r = face_off[f]; r < face_off[f + 1]; ++r) {
+                size_t at = 0;
+                while (pts[at] != face_lab[r]) ++at;
+                m.cfv.push_back((uint8_t)std::min<size_t>(at, 255));
+            }
+        }
+        if (c > 0 && m.cell_pts_off[c + 1] - m.cell_pts_off[c] != m.cell_pts_off[1]) m.uniform_np = false;
     }
-    m.cell_pts.reserve(m.cell_pts_off[nc]);
-    for (int64_t c = 0; c < nc; ++c) m.cell_pts.insert(m.cell_pts.end(), cp[c].begin(), cp[c].end());
+    m.cfv_off.push_back((int32_t)m.cfv.size());
     std::vector<int32_t> ncc(nc + 1, 0);
     for (int64_t f = 0; f < ninternal; ++f) { ++ncc[owner[f] + 1]; ++ncc[neighbour[f] + 1]; }
     m.cell_cells_off.assign(nc + 1, 0);

@@ -20,6 +20,10 @@ struct PolyHostMesh {
     std::vector<int32_t> cell_cells_off, cell_cells;  // cell -> face neighbours (cellCells)
     std::vector<double> Cf, Sf, Cc, Vc;             // [nfaces][3], [nfaces][3], [ncells][3], [ncells]
     double bmin[3] = {0, 0, 0}, bmax[3] = {0, 0, 0};  // bounding box of the points
+    // what the kernels read beside it
+    std::vector<int32_t> cfv_off;                   // entry of cell_faces -> its vertices in cfv
+    std::vector<uint8_t> cfv;                       // position of each face vertex in the cell's point list
+    bool uniform_np = true;                         // every cell has the same number of points
 };
 
 // Builds the mesh from OpenFOAM's polyMesh lists: points [npoints][3], faces as a compact list (face f has the

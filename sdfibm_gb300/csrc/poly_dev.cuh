@@ -23,6 +23,28 @@ struct PolyK {
     const double* Sf;         // [nfaces][3] face area vectors
     const double* Cc;         // [ncells][3] cell centres
     const double* Vc;         // [ncells] cell volumes
+    const float4* pt32;       // [npoints][2]: points as FP32 pairs (hi.x, hi.y, hi.z, lo.x), (lo.y, lo.z, -, -)
+    const int32_t* cfv_off;   // entry of cf -> its vertices' slots in cfv
+    const uint8_t* cfv;       // position of each face vertex in the cell's point list (255: beyond the 255th)
+    const float4* cell32;     // [ncells]: centre and a radius that holds the cell's points (FP32, widened)
+    const double* mSf;        // [nfaces] |Sf|
+    const float* blk;         // [nblocks][12]: boxes of the points and of the centres of POLY_BLOCK consecutive cells
+    int32_t nblocks;          //   (lo, hi, lo, hi; widened)
+    int32_t uniform_np;       // 1: every cell has the same number of points
+};
+constexpr int POLY_BLOCK = 128;  // cells per block: four bitmap words
+
+// Per-call record of a solid (poly_plan_kernel): FP32 map to the local frame and the region its inside points lie in.
+struct PolySolid {
+    float M[9];        // |q|^2 R^T
+    float xh[3], xl[3];  // solid centre as FP32 pairs
+    float mn;          // bound of the row sums of |M|
+    float xabs;        // |centre|_1
+    float pad;
+    double R[9];       // the map in FP64 (distances)
+    float c[3], r;     // bounding sphere (2-D shapes: the axis point and the radius), widened
+    float axis[3];     // 2-D shapes: direction of the prism
+    int32_t kind;      // 0 sphere, 1 prism along z, 2 prism, 3 half space
 };
 
 struct PolyWork {
@@ -35,12 +57,27 @@ struct PolyWork {
     double* acc;        // [N][5]: sums over the solids of As, Ts, Fs.x, Fs.y, Fs.z
     int32_t* claim;     // [N]: largest 4 * solid + type over the solids touching the cell (-1: none)
     int32_t* err;       // first device error (DeviceError)
+    // meshes whose cells all have the same point count: cells with an inside vertex and their connected sets
+    PolySolid* plan;    // [S]
+    int2* items;        // (solid, block) pairs whose boxes meet the solid
+    int32_t* nitems;    // their count (left zero by poly_finalize_kernel)
+    int32_t* parent;    // [S][qcap], by cell: union-find forest (parent label <= own label)
+    int32_t* clist;     // [S][qcap]: cells with an inside vertex
+    int8_t* ctype;      // [S][qcap]: their types
+    int32_t* ccount;    // [S]: how many
+    int32_t* seed;      // [S]: nearest cell
+    int32_t* mincand;   // [S]: lowest label of the cells with an inside vertex
 };
 
 __global__ void poly_enum_kernel(PolyK m, const SolidK* sk, const sdfibm_solid_state* st, PolyWork w);
+__global__ void poly_setup_kernel(PolyK m, float4* pt32, float4* cell32, double* mSf, float* blk);
+__global__ void poly_plan_kernel(PolyK m, const SolidK* sk, const sdfibm_solid_state* st, PolyWork w, double* ftacc);
+__global__ void poly_classify_kernel(PolyK m, const SolidK* sk, const sdfibm_solid_state* st, PolyWork w, int S);
+__global__ void poly_link_kernel(PolyK m, PolyWork w);
 __global__ void poly_couple_kernel(PolyK m, const SolidK* sk, const sdfibm_solid_state* st, PolyWork w, const float* U,
-                                   double* ftacc, const StepParams* step);
-__global__ void poly_finalize_kernel(PolyWork w, int32_t N, float* As, float* Fs, float* Ts, int32_t* Ct);
+                                   double* ftacc, double dtINV, int linked);
+__global__ void poly_finalize_kernel(PolyWork w, int32_t N, float* As, float* Fs, float* Ts, int32_t* Ct, int S,
+                                     const double* ftacc, double* ft, double rho_f, sdfibm_solid_state* st);
 __global__ void poly_fix_kernel(PolyK m, const sdfibm_solid_state* st, int S, const int32_t* Ct, float* U);
 
 }  // namespace sdfibm_dev
