@@ -55,7 +55,7 @@ __global__ void claim_kernel(const int32_t* in_cell, const int32_t* in_solid, co
                              const int32_t* cut_solid, int32_t* Ct, Counters* cnt, int64_t N, uint32_t* cbits,
                              uint32_t* sbits);
 __global__ void ft_kernel(const double* ftacc, double* ft, int S, const StepParams* step);
-__global__ void set_step_kernel(StepParams* p, double time, double dt, int nsub, double rho_V);
+__global__ void set_step_kernel(StepParams* p, double time, double dt, int nsub, double rho_V, EvolveCtrl* ctrl);
 int export_chunk_cells();
 __global__ void mark_export_kernel(const int32_t* in_cell, const int32_t* cut_cell, const int32_t* prev_in_cell,
                                    const int32_t* prev_cut_cell, const Counters* cnt, int64_t N, uint32_t* dirty);
@@ -91,6 +91,12 @@ __global__ void grid_scatter_kernel(const int64_t* hashes, int32_t* cursor, int3
 __global__ void collide_kernel(const SolidK* sk, sdfibm_solid_state* st, int S, GridK gk, const int64_t* hashes,
                                const int32_t* start, const int32_t* list, int mode, FineGridK fg, const int32_t* fstart,
                                const int32_t* flist, const int32_t* planes, int nplanes, const CollRec* recs);
+__global__ void evolve_contacts_kernel(const SolidK* sk, sdfibm_solid_state* st, int S, int per, int nsub,
+                                       const StepParams* step, double rho_f, D3 g, GridK gk, FineGridK fg, int mode,
+                                       const int32_t* planes, int nplanes, float skin, EvolveWork w, Counters* cnt);
+int evolve_contacts_threads();
+int evolve_contacts_list();
+int evolve_contacts_hot();
 __global__ void move_kernel(const SolidK* sk, sdfibm_solid_state* st, int S, const StepParams* step);
 __global__ void store_old_kernel(sdfibm_solid_state* st, int S);
 __global__ void ft_to_state_kernel(const double* ft, sdfibm_solid_state* st, int S);
@@ -175,6 +181,10 @@ struct sdfibm_ctx {
     int32_t *d_fcount = nullptr, *d_fstart = nullptr, *d_fcursor = nullptr, *d_flist = nullptr, *d_planes = nullptr;
     int32_t *d_fsums = nullptr, *d_fsums_excl = nullptr;  // block sums of the multi-block scans of the two grids
     int nplanes = 0;
+    // all sub-steps in one cooperative launch: solids per CTA (0: one launch per stage), see evolve_limit
+    int ev_per = 0;
+    float ev_skin = 0.f;
+    EvolveWork evw{};
     // fields seen by the last interact (sparse reset is only valid on the same buffers)
     const void* last_fields[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     bool interacted = false;
@@ -262,6 +272,13 @@ struct sdfibm_ctx {
     };
     Poly* poly = nullptr;
 };
+
+// Most solids of the one-launch evolve.  Each CTA (one per SM) tests its solids' pairs a warp at a time, so its sub-step grows
+// with the solids per SM, where the launch-per-stage path keeps its launches' cost: 20 sub-steps of free spheres took (one
+// launch / launch per stage) 0.19 / 0.88 ms at 2000 solids, 0.55 / 1.13 at 8000, 1.83 / 1.45 at 16 384, 4.75 / 2.45 at
+// 38 000.  More plane-like solids than EV_MAX_PLANES (each tests every sphere) take the launches too.
+static int evolve_limit(int num_sms) { return 64 * num_sms; }
+constexpr int EV_MAX_PLANES = 64;
 
 // event bracketing of each launch when timing is on: mark(ctx, name) after a launch records its end
 static void mark_begin(sdfibm_ctx* ctx) {
@@ -561,6 +578,13 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
                     cap += e;
                 }
                 f.cap = std::max<int64_t>(1, cap);
+                double rsum = 0.0;
+                for (int s = 0; s < nsolids; ++s) rsum += std::max(0.0, solids[s].shape.radiusB);
+                if (nsolids <= evolve_limit(ctx->num_sms) && ctx->nplanes <= EV_MAX_PLANES) {
+                    ctx->ev_per = std::max(8, (nsolids + ctx->num_sms - 1) / ctx->num_sms);
+                    // a quarter of the mean radius: far beyond a CFL-bound step's motion, few listed neighbours more
+                    ctx->ev_skin = (float)(0.25 * rsum / std::max(1, nsolids));
+                }
                 if (dalloc(&ctx->d_planes, planes.size()) ||
                     (planes.size() && cudaMemcpy(ctx->d_planes, planes.data(), sizeof(int32_t) * planes.size(),
                                                  cudaMemcpyHostToDevice) != cudaSuccess) ||
@@ -597,6 +621,15 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
         cudaMallocHost((void**)&ctx->h_ft, std::max<size_t>(1, 6 * (size_t)nsolids) * sizeof(double)) != cudaSuccess) {
         ctx->err = "device allocation failed";
         return bail(SDFIBM_ERR_CUDA);
+    }
+    if (ctx->ev_per > 0) {
+        EvolveWork& e = ctx->evw;
+        const size_t S2 = 2 * (size_t)nsolids, P2 = 2 * (size_t)std::max(1, ctx->nplanes);
+        if (dalloc(&e.x, 4 * S2) || dalloc(&e.rec, S2) || dalloc(&e.key, S2) || dalloc(&e.pn, P2) ||
+            dalloc(&e.pq, 8 * P2) || dalloc(&e.hot, (size_t)evolve_contacts_hot()) || dalloc(&e.list, (size_t)nsolids * evolve_contacts_list()) || dalloc(&e.ctrl, 1)) {
+            ctx->err = "device allocation failed (contacts)";
+            return bail(SDFIBM_ERR_CUDA);
+        }
     }
     if (ctx->grid_active) {
         if (dalloc(&ctx->d_hash, nsolids) || dalloc(&ctx->d_recs, nsolids) || dalloc(&ctx->d_gcount, ctx->gk.ncell) ||
@@ -668,6 +701,7 @@ static int check_device_error(sdfibm_ctx* ctx) {
         case DERR_BBOX: return fail(ctx, SDFIBM_ERR_CAPACITY, "a 2-D shape tilted out of its reserved bounding box");
         case DERR_FLOOD_LIMIT: return fail(ctx, SDFIBM_ERR_TIMEOUT, "flood fill did not converge within its bound");
         case DERR_SHARED_TABLE: return fail(ctx, SDFIBM_ERR_CAPACITY, "shared-cell table full");
+        case DERR_EVOLVE_TIMEOUT: return fail(ctx, SDFIBM_ERR_TIMEOUT, "evolve: a grid barrier timed out");
         case DERR_MMA_TIMEOUT: return fail(ctx, SDFIBM_ERR_TIMEOUT, "learned fraction: tensor-core wait timed out");
         default: return fail(ctx, SDFIBM_ERR_CUDA, "device error " + std::to_string(e));
     }
@@ -685,7 +719,7 @@ static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float
     const int64_t N = ctx->mesh.ncells;
     const int S = ctx->S;
     cudaStream_t st = ctx->stream;
-    set_step_kernel<<<1, 1, 0, st>>>(ctx->d_step, time, dt, 1, ctx->opt.rho_f * ctx->mesh.V);
+    set_step_kernel<<<1, 1, 0, st>>>(ctx->d_step, time, dt, 1, ctx->opt.rho_f * ctx->mesh.V, nullptr);
     ++launches;
     begin_kernel<<<1, 1, 0, st>>>(ctx->d_cnt);
     ++launches;
@@ -876,7 +910,7 @@ static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float
 // arguments of its set_step_kernel node.  Returns a status, or -1 when capture is not possible (the caller then
 // launches directly).
 static int run_graph(sdfibm_ctx* ctx, sdfibm_ctx::Graph& g, bool key_changed, const std::function<int()>& enqueue,
-                     StepParams* step, double time, double dt, int nsub, double rho_V) {
+                     StepParams* step, double time, double dt, int nsub, double rho_V, EvolveCtrl* ctrl) {
     cudaStream_t st = ctx->stream;
     if (!g.valid || key_changed) {
         if (g.valid) {
@@ -919,7 +953,7 @@ static int run_graph(sdfibm_ctx* ctx, sdfibm_ctx::Graph& g, bool key_changed, co
         ctx->graphs_keep.push_back(graph);
         g.valid = true;
     }
-    void* args[5] = {&step, &time, &dt, &nsub, &rho_V};
+    void* args[6] = {&step, &time, &dt, &nsub, &rho_V, &ctrl};
     cudaKernelNodeParams kp = g.step_params;
     kp.kernelParams = args;
     kp.extra = nullptr;
@@ -965,7 +999,7 @@ int sdfibm_cuda_interact(sdfibm_ctx* ctx, double time, double dt, const float* U
                            counted = 0;
                            return enqueue_interact(ctx, time, dt, U, As, Fs, Ts, Ct, dense, counted);
                        },
-                       ctx->d_step, time, dt, 1, ctx->opt.rho_f * ctx->mesh.V);
+                       ctx->d_step, time, dt, 1, ctx->opt.rho_f * ctx->mesh.V, nullptr);
         if (rc == -1) {
             ctx->graphs_failed = true;
         } else {
@@ -1234,9 +1268,21 @@ static int enqueue_evolve(sdfibm_ctx* ctx, double time, double dt) {
     const D3 g{ctx->opt.gravity[0], ctx->opt.gravity[1], ctx->opt.gravity[2]};
     // thread-per-solid kernels are FP64-pipe bound: small blocks spread a few thousand solids over every SM
     const int B = S <= ctx->num_sms * 4 * 64 ? 32 : 128, G = (S + B - 1) / B;
-    set_step_kernel<<<1, 1, 0, st>>>(step, time, dt, nsub, 0.0);
+    set_step_kernel<<<1, 1, 0, st>>>(step, time, dt, nsub, 0.0, ctx->evw.ctrl);
     if (!ctx->grid_active) {
         evolve_independent_kernel<<<G, B, 0, st>>>(ctx->d_sk, ctx->d_st, S, nsub, step, ctx->opt.rho_f, g);
+    } else if (ctx->ev_per > 0) {
+        const int per = ctx->ev_per;
+        const SolidK* sk = ctx->d_sk;
+        const StepParams* stp = step;
+        const int32_t* planes = ctx->d_planes;
+        double rho_f = ctx->opt.rho_f;
+        D3 gg = g;
+        int mode = ctx->opt.collision_mode, S_ = S, per_ = per, nsub_ = nsub;
+        void* args[] = {&sk, &ctx->d_st, &S_, &per_, &nsub_, &stp, &rho_f, &gg, &ctx->gk, &ctx->fg, &mode, &planes, &ctx->nplanes,
+                        &ctx->ev_skin, &ctx->evw, &ctx->d_cnt};
+        CK(cudaLaunchCooperativeKernel((const void*)evolve_contacts_kernel, dim3((S + per - 1) / per),
+                                       dim3(evolve_contacts_threads()), args, 0, st));
     } else {
         const GridK& gk = ctx->gk;
         const FineGridK& fg = ctx->fg;
@@ -1272,7 +1318,7 @@ int sdfibm_cuda_evolve(sdfibm_ctx* ctx, double time, double dt) {
     if (ctx->S == 0) return SDFIBM_OK;
     if (graphs_on(ctx)) {
         const int rc = run_graph(ctx, ctx->egraph, false, [&] { return enqueue_evolve(ctx, time, dt); },
-                                 ctx->d_step + 1, time, dt, ctx->nsub, 0.0);
+                                 ctx->d_step + 1, time, dt, ctx->nsub, 0.0, ctx->evw.ctrl);
         if (rc != -1) return rc;
         ctx->graphs_failed = true;
     }
@@ -1625,6 +1671,9 @@ void sdfibm_cuda_destroy(sdfibm_ctx* ctx) {
     if (ctx->d_sbits) cudaFree(ctx->d_sbits);
     if (ctx->d_shent) cudaFree(ctx->d_shent);
     if (ctx->d_f64) cudaFree(ctx->d_f64);
+    for (void* p : {(void*)ctx->evw.x, (void*)ctx->evw.rec, (void*)ctx->evw.key, (void*)ctx->evw.pn, (void*)ctx->evw.pq,
+                    (void*)ctx->evw.list, (void*)ctx->evw.hot, (void*)ctx->evw.ctrl})
+        if (p) cudaFree(p);
     if (ctx->poly) {
         for (void* p : ctx->poly->allocs)
             if (p) cudaFree(p);

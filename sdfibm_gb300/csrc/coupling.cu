@@ -1032,7 +1032,8 @@ __global__ void ft_kernel(const double* __restrict__ ftacc, double* __restrict__
     for (int r = 0; r < 6; ++r) ft[6 * s + r] = ftacc[6 * s + r] * scale;
 }
 
-__global__ void set_step_kernel(StepParams* p, double time, double dt, int nsub, double rho_V) {
+__global__ void set_step_kernel(StepParams* p, double time, double dt, int nsub, double rho_V, EvolveCtrl* ctrl) {
+    if (ctrl) *ctrl = EvolveCtrl{};
     p->time = time;
     p->dt = dt;
     p->dt_sub = dt / nsub;

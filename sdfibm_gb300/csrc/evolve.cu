@@ -5,8 +5,9 @@
 // src/libcollision/ugrid.cpp:5-77, collision.cpp:7-57).
 //
 // Without collisions every solid is independent, so one thread runs all sub-steps of one solid in a single launch.
-// With collisions each sub-step is: forces + grid hash, counting sort of solid ids by grid cell, pair forces
-// (each solid sums its own side of every pair: no atomics, the pair law is evaluated once per side), move.
+// With collisions up to 64 solids per SM run all sub-steps in one cooperative launch (evolve_contacts_kernel); for more, each
+// sub-step is: forces + grid hash, counting sort of solid ids by grid cell, pair forces (each solid sums its own side of
+// every pair: no atomics, the pair law is evaluated once per side), move.
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -105,11 +106,9 @@ __device__ inline void pre_forces(const SolidK& k, sdfibm_solid_state& s, double
     st3(s.torque, torque);
 }
 
-// Solid::move
-__device__ inline void move_solid(const SolidK& k, sdfibm_solid_state& s, double time, double dt) {
-    const D3 velocity_old = ld3(s.vel), omega_old = ld3(s.omega);
-    D3 vel = velocity_old + ld3(s.force) * k.mass_inv * dt;
-    const Q4 q{s.quat[0], D3{s.quat[1], s.quat[2], s.quat[3]}};
+// Solid::move, its rotation half (which needs no force): the new angular velocity and orientation
+__device__ inline void move_rotation(const SolidK& k, const Q4& q, const D3& omega_old, const D3& T, double time, double dt,
+                                     D3& om, Q4& qn) {
     const double w2 = q.w * q.w, x2 = q.v.x * q.v.x, y2 = q.v.y * q.v.y, z2 = q.v.z * q.v.z;
     const double txy = 2 * q.v.x * q.v.y, twz = 2 * q.w * q.v.z, txz = 2 * q.v.x * q.v.z;
     const double twy = 2 * q.w * q.v.y, tyz = 2 * q.v.y * q.v.z, twx = 2 * q.w * q.v.x;
@@ -121,21 +120,40 @@ __device__ inline void move_solid(const SolidK& k, sdfibm_solid_state& s, double
         for (int c = 0; c < 3; ++c) RI[3 * r + c] = R[3 * r] * I[c] + R[3 * r + 1] * I[3 + c] + R[3 * r + 2] * I[6 + c];
     for (int r = 0; r < 3; ++r)  // (R & I) & R^T
         for (int c = 0; c < 3; ++c) W[3 * r + c] = RI[3 * r] * R[3 * c] + RI[3 * r + 1] * R[3 * c + 1] + RI[3 * r + 2] * R[3 * c + 2];
-    const D3 T = ld3(s.torque);
     const D3 WT{W[0] * T.x + W[1] * T.y + W[2] * T.z, W[3] * T.x + W[4] * T.y + W[5] * T.z,
                 W[6] * T.x + W[7] * T.y + W[8] * T.z};
-    D3 om = omega_old + WT * dt;
-    if (k.motion_type != SDFIBM_MOTION_FREE) motion_constraint(k, time, vel, om);
-    const D3 c = ld3(s.pos) + 0.5 * (vel + velocity_old) * dt;
+    om = omega_old + WT * dt;
+    if (k.motion_type != SDFIBM_MOTION_FREE) {
+        D3 unused{0, 0, 0};
+        motion_constraint(k, time, unused, om);
+    }
     const Q4 h{0.5 * 0.0, 0.5 * (0.5 * (om + omega_old))};
     const Q4 dq0 = qmul(h, q);
     const Q4 dq{dq0.w * dt, dq0.v * dt};
-    Q4 qn{q.w + dq.w, q.v + dq.v};
+    qn = Q4{q.w + dq.w, q.v + dq.v};
     const double mq = sqrt(qn.w * qn.w + magSqr(qn.v));
     qn = Q4{qn.w / mq, qn.v / mq};
+}
+
+// its translation half: velocity and position
+__device__ inline void move_translation(const SolidK& k, const D3& force, double time, double dt, D3& vel, D3& pos) {
+    const D3 velocity_old = vel;
+    vel = velocity_old + force * k.mass_inv * dt;
+    if (k.motion_type != SDFIBM_MOTION_FREE) {
+        D3 unused{0, 0, 0};
+        motion_constraint(k, time, vel, unused);
+    }
+    pos = pos + 0.5 * (vel + velocity_old) * dt;
+}
+
+__device__ inline void move_solid(const SolidK& k, sdfibm_solid_state& s, double time, double dt) {
+    D3 om, vel = ld3(s.vel), pos = ld3(s.pos);
+    Q4 qn;
+    move_rotation(k, Q4{s.quat[0], D3{s.quat[1], s.quat[2], s.quat[3]}}, ld3(s.omega), ld3(s.torque), time, dt, om, qn);
+    move_translation(k, ld3(s.force), time, dt, vel, pos);
     st3(s.vel, vel);
     st3(s.omega, om);
-    st3(s.pos, c);
+    st3(s.pos, pos);
     s.quat[0] = qn.w; s.quat[1] = qn.v.x; s.quat[2] = qn.v.y; s.quat[3] = qn.v.z;
 }
 
@@ -461,6 +479,474 @@ __global__ void collide_kernel(const SolidK* __restrict__ sk, sdfibm_solid_state
         st[p].force[0] += fsum.x;
         st[p].force[1] += fsum.y;
         st[p].force[2] += fsum.z;
+    }
+}
+
+// ---- all sub-steps of a cloud with contacts in one cooperative launch --------------------------------------------------
+// The sub-steps are short chains of dependent FP64 work (a solid's move is about 250 operations) with a search between
+// them; as six launches each (forces, counts, scan, scatter, pairs) they took 1.26 ms for 104 solids and 1.4 ms for 1800,
+// launch and memory latency.  Here CTA b keeps solids [b per, (b + 1) per): a thread per solid holds its state in
+// registers over all sub-steps, the other warps test its pairs meanwhile, and one grid barrier a sub-step publishes the
+// new positions (two buffers).  The pairs come from lists built once, by testing all solids in FP32, of the solids nearer
+// than the contact distance plus a skin.  A solid that has moved half the skin is hot from then on: it tests every solid, the others test
+// the hot ones beside their lists (a solid that left its stable step size does not make everybody search again); past
+// EV_HOT of them every CTA builds its lists again.  Pairs go through the FP32 screen, the reference's 27-cell rule on the UGrid keys and the FP64 contact law, as in collide_kernel, so the contacts are
+// the same.  The rotation half of a move needs no pair and runs in warps of its own beside the barrier and the pairs.  Plane-like solids (law 0) test every sphere, spheres every plane: for up to EV_MAX_PLANES.
+// Bound by latency: 9 us a sub-step (barrier, two dependent L2 reads, the FP64 chains of a contact and a move).  Measured
+// (GB300): 104 solids 1.26 -> 0.20 ms, 1800 solids 1.4 -> 0.19 ms.
+constexpr int EV_THREADS = 256, EV_WARPS = EV_THREADS / 32;
+constexpr int EV_LIST = 128;              // listed neighbours of a solid; more: it tests every solid every sub-step
+constexpr int EV_HOT = 256;               // solids beyond half the skin before the lists are made again
+int evolve_contacts_threads() { return EV_THREADS; }
+int evolve_contacts_list() { return EV_LIST; }
+int evolve_contacts_hot() { return EV_HOT; }
+constexpr long long EV_WAIT_CYCLES = 4000000000LL;  // about two seconds
+
+// Grid barrier in two halves: one thread arrives after a __syncthreads, one waits.  The wait gives up after its limit.
+__device__ inline void ev_arrive(EvolveWork w) {
+    __threadfence();
+    atomicAdd(&w.ctrl->arrived, 1u);
+}
+__device__ inline bool ev_wait(EvolveWork w, unsigned target) {
+    const long long t0 = clock64();
+    volatile unsigned* a = &w.ctrl->arrived;
+    while (*a < target)
+        if (clock64() - t0 > EV_WAIT_CYCLES) return false;
+    __threadfence();
+    return true;
+}
+__device__ inline void ev_bar(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+// Position record of a solid for the pair tests: x, y, z and the radius, signed by the contact law (1: positive, 2:
+// negative, others: NaN), so that two records have a sphere law when the product of their radii is positive.
+__device__ inline float4 ev_record(const D3& x, int id, double rB) {
+    const float r = (float)rB;
+    return make_float4((float)x.x, (float)x.y, (float)x.z, id == 1 ? r : (id == 2 ? -r : NAN));
+}
+
+// the UGrid key of a position, decomposed as its neighbour loops do; w = 1 when it is on the grid
+__device__ inline int4 ev_key(const GridK& gk, const D3& x) {
+    const int i = (int)floor((x.x - gk.low[0]) * gk.dINV), j = (int)floor((x.y - gk.low[1]) * gk.dINV),
+              k = (int)floor((x.z - gk.low[2]) * gk.dINV);
+    if (i >= 0 && i < gk.nx && j >= 0 && j < gk.ny && k >= 0 && k < gk.nz) return make_int4(i, j, k, 1);
+    const int64_t h = (int64_t)i * gk.nynz + (int64_t)j * gk.nz + k;
+    if (h < 0 || h >= gk.ncell) return make_int4(0, 0, 0, 0);
+    return make_int4((int)(h / gk.nynz), (int)((h / gk.nz) % gk.ny), (int)(h % gk.nz), 1);
+}
+__device__ inline bool ev_neighbours(const int4& a, const int4& b) {
+    return a.w && b.w && abs(a.x - b.x) <= 1 && abs(a.y - b.y) <= 1 && abs(a.z - b.z) <= 1;
+}
+
+__device__ inline D3 ev_pos(const EvolveWork& w, int buf, int S, int q) {
+    const double2* p = reinterpret_cast<const double2*>(w.x + 4 * ((int64_t)buf * S + q));
+    const double2 a = __ldcg(p), b = __ldcg(p + 1);
+    return D3{a.x, a.y, b.x};
+}
+
+// FP32 screens: false only when the FP64 contact depth is certainly negative (margins of 2^-16 of the magnitudes)
+__device__ inline bool ev_sphere_near(const float4& a, const float4& b, float skin) {
+    const float dx = b.x - a.x, dy = b.y - a.y, dz = b.z - a.z;
+    const float mag = fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fabsf(a.z)) + fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fabsf(b.z));
+    const float rr = fabsf(a.w) + fabsf(b.w);
+    const float reach = rr + skin + 1.52587890625e-5f * (mag + rr);
+    return a.w * b.w > 0.f && dx * dx + dy * dy + dz * dz <= reach * reach;
+}
+__device__ inline bool ev_plane_near(const float4& n, const float4& xp, const float4& xs) {
+    const float d = n.x * (xs.x - xp.x) + n.y * (xs.y - xp.y) + n.z * (xs.z - xp.z), r = fabsf(xs.w);
+    const float mag = fabsf(xs.x) + fabsf(xs.y) + fabsf(xs.z) + fabsf(xp.x) + fabsf(xp.y) + fabsf(xp.z);
+    return xs.w == xs.w && !(r - d < -1.52587890625e-5f * (mag + r));  // a position that is not finite goes to the law
+}
+
+// force on solid p of its contact with q, and of a plane-like solid's contact on the sphere (collision.cpp:7-35)
+__device__ inline D3 ev_sphere_force(const D3& xp, const D3& xq, double rp, double rq) {
+    const D3 d = xp - xq;
+    const double m = mag(d);
+    const D3 cN = m < 1e-150 ? D3{0, 0, 0} : d / m;
+    const double cd = rp + rq - m;
+    return cd < 0 ? D3{0, 0, 0} : 1e4 * cd * cN;
+}
+// record of a plane-like solid: orientation, then the normal qtransform(q, (0, 1, 0))
+__device__ inline D3 ev_plane_force(const double* rec, const D3& xp, const D3& xs, double rB_s) {
+    const double2* r = reinterpret_cast<const double2*>(rec);
+    const double2 a = __ldcg(r), b = __ldcg(r + 1), c = __ldcg(r + 2), d = __ldcg(r + 3);
+    const D3 l = qtransform(qconj(Q4{a.x, D3{a.y, b.x, b.y}}), xs - xp);
+    const double cd = rB_s - l.y;
+    return cd < 0 ? D3{0, 0, 0} : 1e4 * cd * D3{c.x, c.y, d.x};
+}
+
+// move_rotation by four lanes: lane r of the group computes row r of R I R^T and component r of the products (3: the scalar
+// part of the quaternion).  The same operations in the same order, about 120 instructions a lane instead of 290.
+// All lanes of the warp call it; w receives component r of the quaternion (x, y, z, w), o of the angular velocity.
+__device__ inline void move_rotation4(const SolidK& k, const double* q4, const double* o3, const double* T, double time,
+                                      double dt, double& o, double& qn) {
+    const unsigned FULL = 0xffffffffu;
+    const int r = threadIdx.x & 3;
+    const Q4 q{q4[0], D3{q4[1], q4[2], q4[3]}};
+    const D3 oo{o3[0], o3[1], o3[2]};
+    const double w2 = q.w * q.w, x2 = q.v.x * q.v.x, y2 = q.v.y * q.v.y, z2 = q.v.z * q.v.z;
+    const double txy = 2 * q.v.x * q.v.y, twz = 2 * q.w * q.v.z, txz = 2 * q.v.x * q.v.z;
+    const double twy = 2 * q.w * q.v.y, tyz = 2 * q.v.y * q.v.z, twx = 2 * q.w * q.v.x;
+    const double R[9] = {w2 + x2 - y2 - z2, txy - twz, txz + twy, txy + twz, w2 - x2 + y2 - z2,
+                         tyz - twx, txz - twy, tyz + twx, w2 - x2 - y2 + z2};
+    double row[3], RI[3], W[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) row[c] = r == 0 ? R[c] : (r == 1 ? R[3 + c] : R[6 + c]);
+    const double* I = k.moi_inv;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) RI[c] = row[0] * I[c] + row[1] * I[3 + c] + row[2] * I[6 + c];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) W[c] = RI[0] * R[3 * c] + RI[1] * R[3 * c + 1] + RI[2] * R[3 * c + 2];
+    o = (r == 0 ? oo.x : (r == 1 ? oo.y : oo.z)) + (W[0] * T[0] + W[1] * T[1] + W[2] * T[2]) * dt;
+    D3 om{__shfl_sync(FULL, o, 0, 4), __shfl_sync(FULL, o, 1, 4), __shfl_sync(FULL, o, 2, 4)};
+    if (k.motion_type != SDFIBM_MOTION_FREE) {
+        D3 unused{0, 0, 0};
+        motion_constraint(k, time, unused, om);
+        o = r == 0 ? om.x : (r == 1 ? om.y : om.z);
+    }
+    const Q4 h{0.5 * 0.0, 0.5 * (0.5 * (om + oo))};
+    double d;
+    if (r == 3) {
+        d = h.w * q.w - dot(h.v, q.v);
+    } else {
+        // component r of h.w q.v + q.w h.v + h.v x q.v: the cross product from the two cyclically next components
+        const double hr = r == 0 ? h.v.x : (r == 1 ? h.v.y : h.v.z), qr = r == 0 ? q.v.x : (r == 1 ? q.v.y : q.v.z);
+        const double h1 = r == 0 ? h.v.y : (r == 1 ? h.v.z : h.v.x), q1 = r == 0 ? q.v.y : (r == 1 ? q.v.z : q.v.x);
+        const double h2 = r == 0 ? h.v.z : (r == 1 ? h.v.x : h.v.y), q2 = r == 0 ? q.v.z : (r == 1 ? q.v.x : q.v.y);
+        d = h.w * qr + q.w * hr + (h1 * q2 - h2 * q1);
+    }
+    const double e = (r == 3 ? q.w : (r == 0 ? q.v.x : (r == 1 ? q.v.y : q.v.z))) + d * dt;
+    const double ex = __shfl_sync(FULL, e, 0, 4), ey = __shfl_sync(FULL, e, 1, 4), ez = __shfl_sync(FULL, e, 2, 4),
+                 ew = __shfl_sync(FULL, e, 3, 4);
+    qn = e / sqrt(ew * ew + magSqr(D3{ex, ey, ez}));
+}
+
+// Sum of the sphere contacts q[0..n) of solid p over the warp (result on every lane): a lane per contact.  Up to two commute;
+// more are added as collide_kernel adds them (lane and order by the pair's home cell in the fine grid), so that both paths
+// give the same bits.
+__device__ inline D3 ev_contact_sum(const EvolveWork& w, const SolidK* sk, int buf, int S, const FineGridK& fg, int p, int n,
+                                    const int32_t* q, double (*fc)[3], int32_t* home) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    D3 f{0, 0, 0};
+    const D3 xp = ev_pos(w, buf, S, p);
+    if (lane < n) f = ev_sphere_force(xp, ev_pos(w, buf, S, q[lane]), sk[p].radiusB, sk[q[lane]].radiusB);
+    if (n > 2) {
+        if (lane < n) {
+            int lp[3], hp[3], lq[3], hq[3];
+            fine_range(fg, xp, sk[p].radiusB, lp, hp);
+            fine_range(fg, ev_pos(w, buf, S, q[lane]), sk[q[lane]].radiusB, lq, hq);
+            const int nx = hp[0] - lp[0] + 1, ny = hp[1] - lp[1] + 1;
+            home[lane] = (max(lp[0], lq[0]) - lp[0]) +
+                         nx * ((max(lp[1], lq[1]) - lp[1]) + ny * (max(lp[2], lq[2]) - lp[2]));
+            fc[lane][0] = f.x; fc[lane][1] = f.y; fc[lane][2] = f.z;
+        }
+        __syncwarp();
+        f = D3{0, 0, 0};
+        int64_t done = -1;  // cell and solid last added
+        for (int t = 0; t < n; ++t) {
+            int at = -1;
+            int64_t next = INT64_MAX;
+            for (int i = 0; i < n; ++i) {
+                const int64_t key = ((int64_t)home[i] << 32) | (uint32_t)q[i];
+                if ((home[i] & 31) == lane && key > done && key < next) { next = key; at = i; }
+            }
+            if (at < 0) break;
+            f = f + D3{fc[at][0], fc[at][1], fc[at][2]};
+            done = next;
+        }
+        __syncwarp();
+    }
+    return f;
+}
+
+__global__ void __launch_bounds__(EV_THREADS, 1) evolve_contacts_kernel(const SolidK* __restrict__ sk,
+                                                                        sdfibm_solid_state* st, int S, int per, int nsub,
+                                                                        const StepParams* step, double rho_f, D3 g,
+                                                                        GridK gk, FineGridK fg, int mode,
+                                                                        const int32_t* __restrict__ planes, int nplanes,
+                                                                        float skin, EvolveWork w, Counters* cnt) {
+    __shared__ double s_f[EV_THREADS][3];
+    __shared__ double s_q[32][4], s_om[32][3], s_T[32][3], s_qn[32][4], s_omn[32][3];  // four lanes a solid
+    __shared__ double s_fc[EV_WARPS][32][3];
+    __shared__ int32_t s_cq[EV_WARPS][32], s_ce[EV_WARPS][32], s_cn[EV_WARPS];
+    __shared__ int32_t s_n[EV_THREADS];   // listed neighbours, -1: more than the list holds
+    __shared__ int s_hot[EV_THREADS];
+    __shared__ int s_ok, s_move, s_build;
+    const unsigned FULL = 0xffffffffu;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int s0 = blockIdx.x * per, own = min(per, S - s0);  // >= 1
+    const double time = step->time, dt = step->dt_sub;
+    unsigned arrive = 0;
+    // warps 0 .. nrot - 1 do the rotations (four lanes a solid up to 32 solids, else a thread each) while the others wait
+    // for the barrier and test the pairs; with more than 128 solids every warp does both
+    const bool quad = own <= 32;
+    const int nrot = quad ? (own + 7) >> 3 : (own + 31) >> 5;
+    const int cw0 = nrot <= EV_WARPS / 2 ? nrot : 0, ncw = EV_WARPS - cw0, bar = cw0 > 0 ? 1 : 0;
+    // this thread's solid
+    const int s = s0 + tid;
+    const bool mine = tid < own;
+    D3 pos{0, 0, 0}, vel{0, 0, 0}, om{0, 0, 0}, force{0, 0, 0}, torque{0, 0, 0}, at{0, 0, 0};
+    Q4 q{1, D3{0, 0, 0}};
+    int id = -1, plane = -1;
+    double rB = 0.0;
+    auto publish = [&](int buf) {  // true when the solid is on the grid
+        double2* xo = reinterpret_cast<double2*>(w.x + 4 * ((int64_t)buf * S + s));
+        __stcg(xo, make_double2(pos.x, pos.y));
+        __stcg(xo + 1, make_double2(pos.z, 0.0));
+        __stcg(w.rec + (int64_t)buf * S + s, ev_record(pos, id, rB));
+        const int4 key = ev_key(gk, pos);
+        __stcg(w.key + (int64_t)buf * S + s, key);
+        if (plane >= 0) {
+            const D3 n = qtransform(q, D3{0, 1, 0});
+            __stcg(w.pn + buf * nplanes + plane, make_float4((float)n.x, (float)n.y, (float)n.z, 0.f));
+            double2* qo = reinterpret_cast<double2*>(w.pq + 8 * ((int64_t)buf * nplanes + plane));
+            __stcg(qo, make_double2(q.w, q.v.x));
+            __stcg(qo + 1, make_double2(q.v.y, q.v.z));
+            __stcg(qo + 2, make_double2(n.x, n.y));
+            __stcg(qo + 3, make_double2(n.z, 0.0));
+        }
+        if (quad) {
+            s_q[tid][0] = q.w; s_q[tid][1] = q.v.x; s_q[tid][2] = q.v.y; s_q[tid][3] = q.v.z;
+            s_om[tid][0] = om.x; s_om[tid][1] = om.y; s_om[tid][2] = om.z;
+        }
+        return key.w != 0;
+    };
+    if (mine) {
+        const SolidK& k = sk[s];
+        const sdfibm_solid_state& x = st[s];
+        pos = ld3(x.pos); vel = ld3(x.vel); om = ld3(x.omega);
+        q = state_quat(x);
+        id = coll_id(k, mode);
+        rB = k.radiusB;
+        if (id == 0)
+            for (int i = 0; i < nplanes; ++i)
+                if (planes[i] == s) plane = i;
+        publish(0);
+    }
+    s_hot[tid] = 0;
+    if (blockIdx.x == 0 && tid < EV_HOT) __stcg(w.hot + tid, make_int2(0, 0x7fffffff));
+    // the forces that need no pair (clearForceAndTorque, applyForcer, addMidFluidForceAndTorque, addMidEnvironment: the
+    // same in every sub-step without a forcer) and the rotation half of the move
+    D3 om_new{0, 0, 0};
+    Q4 q_new{1, D3{0, 0, 0}};
+    auto rotate = [&](bool first) {
+        if (mine) {
+            const SolidK& k = sk[s];
+            if (first || k.forcer_type != SDFIBM_FORCER_NONE) {
+                sdfibm_solid_state& x = st[s];
+                if (!first) {  // the forcers look at the pose
+                    st3(x.pos, pos);
+                    x.quat[0] = q.w; x.quat[1] = q.v.x; x.quat[2] = q.v.y; x.quat[3] = q.v.z;
+                }
+                pre_forces(k, x, time, rho_f, g);
+                force = ld3(x.force);
+                torque = ld3(x.torque);
+                if (quad) { s_T[tid][0] = torque.x; s_T[tid][1] = torque.y; s_T[tid][2] = torque.z; }
+            }
+        }
+        if (quad) {
+            ev_bar(2, 32 * nrot);
+            const int i = min(tid >> 2, own - 1), r = tid & 3;
+            double o, e;
+            move_rotation4(sk[s0 + i], s_q[i], s_om[i], s_T[i], time, dt, o, e);
+            if ((tid >> 2) < own) {
+                s_qn[i][(r + 1) & 3] = e;
+                if (r < 3) s_omn[i][r] = o;
+            }
+        } else if (mine) {
+            move_rotation(sk[s], q, om, torque, time, dt, om_new, q_new);
+        }
+    };
+    if (tid == 0) { s_build = 1; s_move = 0; }
+    __syncthreads();
+    if (tid == 0) ev_arrive(w);
+    for (int it = 0; it < nsub; ++it) {
+        const int buf = it & 1;
+        const float4* rec = w.rec + (int64_t)buf * S;
+        const int4* key = w.key + (int64_t)buf * S;
+        ++arrive;
+        if (wid < nrot) rotate(it == 0);
+        if (wid >= cw0) {
+            if (tid == 32 * cw0) {
+                s_ok = ev_wait(w, gridDim.x * arrive) ? 1 : 0;
+                if (it > 0) s_build = __ldcg(&w.ctrl->rebuild[(it - 1) & 1]) == it;
+            }
+            ev_bar(bar, 32 * ncw);
+            if (s_ok && s_build) {  // lists of the CTA's solids, four of them per pass over the records
+                for (int i0 = (wid - cw0) * 4; i0 < own; i0 += ncw * 4) {
+                    float4 a[4];
+                    int n[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        a[u] = i0 + u < own ? __ldcg(rec + s0 + i0 + u) : make_float4(0.f, 0.f, 0.f, NAN);
+                        n[u] = 0;
+                    }
+                    for (int q0 = 0; q0 < S; q0 += 32) {
+                        const int qq = q0 + lane;
+                        const float4 b = qq < S ? __ldcg(rec + qq) : make_float4(0.f, 0.f, 0.f, NAN);
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const bool hit = ev_sphere_near(a[u], b, skin) && qq != s0 + i0 + u;
+                            const unsigned bal = __ballot_sync(FULL, hit);
+                            if (bal) {
+                                const int to = n[u] + __popc(bal & ((1u << lane) - 1u));
+                                if (hit && to < EV_LIST) w.list[(int64_t)(s0 + i0 + u) * EV_LIST + to] = qq;
+                                n[u] += __popc(bal);
+                            }
+                        }
+                    }
+                    if (lane == 0)
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (i0 + u < own) s_n[i0 + u] = n[u] <= EV_LIST ? n[u] : -1;
+                }
+                ev_bar(bar, 32 * ncw);
+            }
+            // pair forces, a warp per solid; entries of the hot list hold the step they count from (a CTA ahead of this one
+            // may add to it meanwhile)
+            const int nhot = s_ok ? min(__ldcg(&w.ctrl->nhot), EV_HOT) : 0;
+            for (int i = wid - cw0; i < (s_ok ? own : 0); i += ncw) {
+                const int p = s0 + i;
+                const int4 kp = __ldcg(key + p);
+                const float4 rp = __ldcg(rec + p);
+                D3 f{0, 0, 0};
+                bool any = false;
+                if (kp.w) {
+                    if (rp.w == rp.w) {  // a sphere law
+                        const int n = s_n[i];
+                        const int32_t* list = w.list + (int64_t)p * EV_LIST;
+                        const bool all = n < 0 || s_hot[i];
+                        if (lane == 0) s_cn[wid] = 0;
+                        __syncwarp();
+                        auto near = [&](int qq) {
+                            return qq != p && ev_sphere_near(rp, __ldcg(rec + qq), 0.f) && ev_neighbours(kp, __ldcg(key + qq));
+                        };
+                        auto is_hot = [&](int qq) {
+                            for (int h = 0; h < nhot; ++h) {
+                                const int2 hs = __ldcg(w.hot + h);
+                                if (hs.x == qq && hs.y <= it) return true;
+                            }
+                            return false;
+                        };
+                        auto add = [&](int qq) {
+                            const int slot = atomicAdd(&s_cn[wid], 1);
+                            if (slot < 32) s_cq[wid][slot] = qq;
+                        };
+                        for (int e = lane; e < (all ? S : n); e += 32) {
+                            const int qq = all ? e : list[e];
+                            if (near(qq) && (all || !is_hot(qq))) add(qq);
+                        }
+                        if (!all)
+                            for (int h = lane; h < nhot; h += 32) {
+                                const int2 hs = __ldcg(w.hot + h);
+                                if (hs.y <= it && near(hs.x)) add(hs.x);
+                            }
+                        __syncwarp();
+                        const int nc = s_cn[wid];
+                        if (nc > 32) {  // a crowd: no room, summed as found
+                            auto sum = [&](int qq) {
+                                f = f + ev_sphere_force(ev_pos(w, buf, S, p), ev_pos(w, buf, S, qq), sk[p].radiusB,
+                                                        sk[qq].radiusB);
+                            };
+                            for (int e = lane; e < (all ? S : n); e += 32) {
+                                const int qq = all ? e : list[e];
+                                if (near(qq) && (all || !is_hot(qq))) sum(qq);
+                            }
+                            if (!all)
+                                for (int h = lane; h < nhot; h += 32) {
+                                    const int2 hs = __ldcg(w.hot + h);
+                                    if (hs.y <= it && near(hs.x)) sum(hs.x);
+                                }
+                            any = true;
+                        } else if (nc > 0) {
+                            f = ev_contact_sum(w, sk, buf, S, fg, p, nc, s_cq[wid], s_fc[wid], s_ce[wid]);
+                            any = true;
+                        }
+                        for (int e = lane; e < nplanes; e += 32) {
+                            const int qq = planes[e];
+                            if (!ev_plane_near(__ldcg(w.pn + buf * nplanes + e), __ldcg(rec + qq), rp) ||
+                                !ev_neighbours(kp, __ldcg(key + qq)))
+                                continue;
+                            const D3 fp = ev_plane_force(w.pq + 8 * ((int64_t)buf * nplanes + e), ev_pos(w, buf, S, qq),
+                                                         ev_pos(w, buf, S, p), sk[p].radiusB);
+                            f = p < qq ? f + (-fp) : f + fp;
+                            any = true;
+                        }
+                    } else if (coll_id(sk[p], mode) == 0) {
+                        int e = 0;
+                        while (e < nplanes && planes[e] != p) ++e;
+                        const float4 n = __ldcg(w.pn + buf * nplanes + e);
+                        for (int qq = lane; qq < S; qq += 32) {
+                            if (!ev_plane_near(n, rp, __ldcg(rec + qq)) || !ev_neighbours(kp, __ldcg(key + qq))) continue;
+                            const D3 fp = ev_plane_force(w.pq + 8 * ((int64_t)buf * nplanes + e), ev_pos(w, buf, S, p),
+                                                         ev_pos(w, buf, S, qq), sk[qq].radiusB);
+                            f = p < qq ? f + (-fp) : f + fp;
+                            any = true;
+                        }
+                    }
+                }
+                if (__any_sync(FULL, any)) {
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        f.x += __shfl_xor_sync(FULL, f.x, o);
+                        f.y += __shfl_xor_sync(FULL, f.y, o);
+                        f.z += __shfl_xor_sync(FULL, f.z, o);
+                    }
+                }
+                if (lane == 0) { s_f[i][0] = f.x; s_f[i][1] = f.y; s_f[i][2] = f.z; }
+            }
+        }
+        __syncthreads();
+        if (!s_ok) {
+            if (tid == 0) set_error(cnt, DERR_EVOLVE_TIMEOUT);
+            return;
+        }
+        const bool last = it + 1 == nsub;
+        if (mine) {
+            const SolidK& k = sk[s];
+            if (s_build) at = pos;
+            const D3 ft{force.x + s_f[tid][0], force.y + s_f[tid][1], force.z + s_f[tid][2]};
+            move_translation(k, ft, time, dt, vel, pos);
+            if (quad) {
+                om = D3{s_omn[tid][0], s_omn[tid][1], s_omn[tid][2]};
+                q = Q4{s_qn[tid][0], D3{s_qn[tid][1], s_qn[tid][2], s_qn[tid][3]}};
+            } else {
+                om = om_new;
+                q = q_new;
+            }
+            if (last) {
+                sdfibm_solid_state& x = st[s];
+                st3(x.force, ft);
+                st3(x.vel, vel);
+                st3(x.omega, om);
+                st3(x.pos, pos);
+                x.quat[0] = q.w; x.quat[1] = q.v.x; x.quat[2] = q.v.y; x.quat[3] = q.v.z;
+                store_old(x);
+            } else {
+                const bool on = publish(buf ^ 1);
+                const D3 d = pos - at;
+                // beyond half the skin, with room.  Off the grid, or not finite, a solid has no sphere pair; back on the grid
+                // it counts from then on
+                if (on && !s_hot[tid] && magSqr(d) > 0.24 * (double)skin * (double)skin) {
+                    const int slot = atomicAdd(&w.ctrl->nhot, 1);
+                    if (slot < EV_HOT) {
+                        __stcg(w.hot + slot, make_int2(s, it + 1));
+                        s_hot[tid] = 1;
+                    } else {
+                        s_move = 1;
+                    }
+                }
+            }
+        }
+        if (last) break;
+        __syncthreads();
+        if (tid == 0) {
+            // no room among the hot ones: every CTA lists again.  Two slots by step, since a CTA ahead of this one may
+            // already ask for the next step (but not for the one after it)
+            if (s_move) atomicMax(&w.ctrl->rebuild[it & 1], it + 1);
+            s_move = 0;
+            ev_arrive(w);
+        }
     }
 }
 

@@ -280,6 +280,24 @@ struct alignas(16) CollRec {
     float x, y, z, r;  // centre and bounding radius rounded to FP32 (the screen of sphere pairs)
 };
 
+// Work space of evolve_contacts_kernel: published positions (two buffers), the plane-like solids' normals and
+// orientations, neighbour lists and the grid barrier.
+struct EvolveCtrl {
+    unsigned arrived;
+    int32_t rebuild[2];   // last step (counted from 1) of each parity that asked for new lists
+    int32_t nhot;         // solids that have moved beyond half the skin
+};
+struct EvolveWork {
+    double* x;      // [2][S][4]
+    float4* rec;    // [2][S]: position and signed radius
+    int4* key;      // [2][S]: UGrid key, decomposed
+    float4* pn;     // [2][planes]: normal
+    double* pq;     // [2][planes][8]: orientation, normal
+    int32_t* list;  // [S][EV_LIST]
+    int2* hot;      // [EV_HOT]: solid, step it is hot from
+    EvolveCtrl* ctrl;  // zeroed by set_step_kernel
+};
+
 // list entry word: solid index in bits 0..29, cell type (1 all inside, 2 centre inside, 3 centre outside) in 30..31
 constexpr int LIST_TYPE_SHIFT = 30;
 constexpr int32_t LIST_SOLID_MASK = (1 << LIST_TYPE_SHIFT) - 1;
@@ -294,6 +312,7 @@ enum DeviceError : int32_t {
     DERR_BBOX = 2,         // a solid's region left its static bbox (tilted 2-D shape)
     DERR_FLOOD_LIMIT = 3,  // flood fill hit its iteration bound
     DERR_SHARED_TABLE = 4, // the shared-cell table is full
+    DERR_EVOLVE_TIMEOUT = 5,  // a CTA of evolve_contacts_kernel did not reach the grid barrier in time
     DERR_MMA_TIMEOUT = 7   // a tensor-core completion was not observed in time (SDFIBM_MLP_ERR_TIMEOUT)
 };
 
