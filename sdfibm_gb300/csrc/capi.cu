@@ -36,7 +36,7 @@ __global__ void recheck_kernel(MeshK m, const SolidK* sk, const sdfibm_solid_sta
                                const Recheck* rq, int64_t cap, Counters* cnt, float* alpha);
 __global__ void connect_kernel(MeshK m, const SolidK* sk, SolidPlan* plan, const uint8_t* scratch, uint32_t* gbitmaps,
                                int32_t* in_cell, int32_t* in_solid, int32_t* cut_cell, int32_t* cut_solid,
-                               int64_t cap_in, int64_t cap_cut, Counters* cnt, int smem_words, const int32_t* solids);
+                               int64_t cap_in, int64_t cap_cut, Counters* cnt, const int32_t* solids);
 __global__ void connect_small_kernel(MeshK m, const SolidK* sk, SolidPlan* plan, const uint8_t* scratch,
                                      int32_t* in_cell, int32_t* in_solid, int32_t* cut_cell, int32_t* cut_solid,
                                      int64_t cap_in, int64_t cap_cut, Counters* cnt, const int32_t* solids,
@@ -420,7 +420,7 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
     int max_smem_words = 0;
     // the flood fill's bitmaps stay in shared memory up to this size (every CTA of the launch reserves the largest, so
     // the cap keeps two 512-thread CTAs per SM); larger ones live in global memory
-    const int SMEM_CAP_BYTES = 96 * 1024;
+    constexpr int SMEM_CAP_BYTES = 96 * 1024;
     for (int s = 0; s < nsolids; ++s) {
         const sdfibm_solid_desc& d = solids[s];
         SolidK& k = ctx->hk[s];
@@ -470,8 +470,10 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
         bbox_total += std::min<int64_t>(cells, N);
         // connect_kernel: four bitmaps (candidates, reached, inside, centre inside) of ext[1] * ext[2] rows
         const int64_t words = 4 * (int64_t)k.ext[1] * k.ext[2] * ((k.ext[0] + 31) / 32);
-        if (words / 4 <= 256) {
-            small_solids.push_back(s);  // warp-per-solid flood fill (connect_small_kernel)
+        if (words / 4 <= (nsolids >= 8 * ctx->num_sms ? 256 : 32)) {
+            // a warp per solid (connect_small_kernel): small bitmaps, and medium ones when there are solids enough to fill
+            // the GPU that way (100 circles of 200 words: 65 us as warps, under 19 us as CTAs)
+            small_solids.push_back(s);
         } else if (words * 4 > SMEM_CAP_BYTES) {
             k.bitmap_global = 1;
             k.bitmap_off = gwords;
@@ -489,6 +491,13 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
         for (int i = 0; i < 9; ++i) k.moi_inv[i] = d.moi_inv[i];
         for (int i = 0; i < 8; ++i) { k.motion_p[i] = d.motion_p[i]; k.forcer_p[i] = d.forcer_p[i]; }
     }
+    // the largest bitmaps first: a CTA per solid, and the last one to start decides when the launch ends
+    auto larger = [&](int32_t a, int32_t b) {
+        const SolidK &ka = ctx->hk[a], &kb = ctx->hk[b];
+        return (int64_t)ka.ext[0] * ka.ext[1] * ka.ext[2] > (int64_t)kb.ext[0] * kb.ext[1] * kb.ext[2];
+    };
+    std::stable_sort(big_solids.begin(), big_solids.end(), larger);
+    std::stable_sort(small_solids.begin(), small_solids.end(), larger);
     if (tiles >= ((int64_t)1 << 31)) { ctx->err = "too many bbox tiles"; return bail(SDFIBM_ERR_CAPACITY); }
     ctx->total_tiles = (int)tiles;
     ctx->chunks_cap = tiles;
@@ -667,9 +676,11 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
         ctx->err = "upload failed";
         return bail(SDFIBM_ERR_CUDA);
     }
-    if (ctx->connect_smem_bytes > 48 * 1024) {
-        if (cudaFuncSetAttribute(connect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 ctx->connect_smem_bytes) != cudaSuccess) {
+    if (ctx->connect_smem_bytes > 32 * 1024) {  // beside its static part: 48 KB need no attribute
+        // the attribute is the process's, not the context's: always the cap, or a context with smaller bitmaps would lower
+        // it under another's launches
+        if (cudaFuncSetAttribute(connect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP_BYTES) !=
+            cudaSuccess) {
             ctx->err = "cannot reserve shared memory for the flood fill";
             return bail(SDFIBM_ERR_CUDA);
         }
@@ -779,8 +790,7 @@ static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float
         if (ctx->n_big > 0)
             connect_kernel<<<ctx->n_big, 512, ctx->connect_smem_bytes, sb>>>(
                 ctx->mesh, ctx->d_sk, ctx->d_plan, ctx->d_scratch, ctx->d_gbitmaps, ctx->in_cell(), ctx->in_solid(),
-                ctx->cut_cell(), ctx->cut_solid(), ctx->cap, ctx->cap, ctx->d_cnt, ctx->connect_smem_bytes / 4,
-                ctx->d_big);
+                ctx->cut_cell(), ctx->cut_solid(), ctx->cap, ctx->cap, ctx->d_cnt, ctx->d_big);
         mark(ctx, "connect_kernel");
         claim_kernel<<<ctx->num_sms * 8, 256, 0, sb>>>(ctx->in_cell(), ctx->in_solid(), ctx->cut_cell(),
                                                         ctx->cut_solid(), Ct, ctx->d_cnt, N, ctx->d_cbits,

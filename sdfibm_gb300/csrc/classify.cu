@@ -905,10 +905,12 @@ __device__ __forceinline__ void classify_body(const ClassifyArgs& A) {
                 return (int64_t)(tx * TX + a) + (int64_t)k.ext[0] * ((ty * TY + b) + (int64_t)k.ext[1] * (tz * TZ + c));
             };
             // whole tile outside the mesh or outside the solid's oriented bounding box: no cell has an inside vertex
-            bool cull = pl.err != 0 || I0 + cx <= 0 || J0 + cy <= 0 || K0 + cz <= 0 || I0 >= m.nx ||
-                        J0 >= m.ny || K0 >= m.nz || I0 + cx < vlo0 || I0 > vhi0 || J0 + cy < vlo1 ||
-                        J0 > vhi1 || K0 + cz < vlo2 || K0 > vhi2;
-            if (!cull && pl.cull_box) {
+            // (nobody reads the class bytes of such a tile)
+            if (pl.err != 0 || I0 + cx <= 0 || J0 + cy <= 0 || K0 + cz <= 0 || I0 >= m.nx || J0 >= m.ny || K0 >= m.nz ||
+                I0 + cx < vlo0 || I0 > vhi0 || J0 + cy < vlo1 || J0 > vhi1 || K0 + cz < vlo2 || K0 > vhi2)
+                continue;
+            bool cull = false;
+            if (pl.cull_box) {
                 // separating axes of the solid's local box: the tile's centre and half extents seen in the local
                 // frame (FP32 with a relative margin of 1e-4 on both sides of every comparison)
                 const float hx = 0.5f * (float)cx * m.h32[0], hy = 0.5f * (float)cy * m.h32[1],

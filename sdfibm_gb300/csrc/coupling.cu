@@ -63,6 +63,23 @@ __global__ void plan_kernel(MeshK m, const SolidK* __restrict__ sk, const sdfibm
     for (int a = 0; a < 3; ++a) { p.vlo[a] = 0; p.vhi[a] = n3v(m, a); }
     if (k.infinite) {
         p.lo[0] = p.lo[1] = p.lo[2] = 0;
+        // the half space n . (v - x) < 0 over the mesh box bounds the inside vertices along every axis its normal has a
+        // component of (a wall along an axis: one layer of cells), widened far beyond the rounding of the inside test
+        const D3 nw = qtransform(q, D3{0, 1, 0});
+        const double nv[3] = {nw.x, nw.y, nw.z}, xv[3] = {x.x, x.y, x.z};
+        double low = 0.0, mag = 0.0, term[3];
+        for (int a = 0; a < 3; ++a) {
+            const double l = m.o[a], u = mesh_coord(m, a, n[a]);
+            term[a] = dmin(nv[a] * (l - xv[a]), nv[a] * (u - xv[a]));
+            low += term[a];
+            mag += fabs(nv[a]) * (fabs(l) + fabs(u) + fabs(xv[a]));
+        }
+        for (int a = 0; a < 3; ++a) {
+            if (nv[a] == 0.0) continue;
+            const double bound = xv[a] - (low - term[a]) / nv[a], tol = 1e-12 * (mag / fabs(nv[a])) + 1e-12 * fabs(xv[a]);
+            if (nv[a] > 0.0) p.vhi[a] = (int32_t)dmin(dmax(floor((bound + tol - m.o[a]) / m.h[a]) + 1, -1.0), (double)n[a]);
+            else p.vlo[a] = (int32_t)dmin(dmax(ceil((bound - tol - m.o[a]) / m.h[a]) - 1, 0.0), (double)n[a] + 1);
+        }
     } else {
         D3 cl{-k.shape.com[0], -k.shape.com[1], -k.shape.com[2]};
         if (k.shape.type == SDFIBM_SHAPE_ELLIPSOID) cl = D3{0, 0, 0};
@@ -244,59 +261,320 @@ __device__ inline int32_t decode_claim(uint32_t w) {
     return code == 1 ? s + 4 : code;
 }
 
-// ---- connect: bit-parallel flood fill --------------------------------------------------------------------------------
+// ---- connect: the connected set of the seed, bit-parallel --------------------------------------------------------------------------------
 constexpr int CON_THREADS = 512;
 
 // fill upward (towards higher bits) inside runs of c starting from seeds s (s subset of c)
 __device__ inline uint32_t fill_up(uint32_t c, uint32_t s) { return (((c + s) ^ c) & c) | s; }
 __device__ inline uint32_t fill_down(uint32_t c, uint32_t s) { return __brev(fill_up(__brev(c), __brev(s))); }
 
-__device__ inline int block_excl_scan(int v, int* warp_sums, int& total) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
+// The cells that can have an inside vertex: the bbox cells of the mesh next to the plan's vertex box (the classify pass
+// writes class bytes for these only).  c0: lowest cell, n: cells per axis (0 on some axis: none).
+struct ActiveBox {
+    int c0[3], n[3];
+};
+__device__ inline ActiveBox active_box(const MeshK& m, const SolidK& k, const SolidPlan& pl) {
+    const int nm[3] = {m.nx, m.ny, m.nz};
+    ActiveBox b;
+    for (int a = 0; a < 3; ++a) {
+        const int lo = max(max(pl.vlo[a] - 1, 0), pl.lo[a]);
+        const int64_t top = (int64_t)pl.lo[a] + k.ext[a] - 1;
+        const int hi = (int)min((int64_t)min(pl.vhi[a], nm[a] - 1), top);
+        b.c0[a] = lo;
+        b.n[a] = max(0, hi - lo + 1);
     }
-    if (lane == 31) warp_sums[wid] = x;
-    __syncthreads();
-    if (wid == 0) {
-        int w = lane < nw ? warp_sums[lane] : 0;
+    return b;
+}
+
+// bit index (row * sx + x) of the flood-fill seed in the active box: the nearest cell when it has an inside vertex, else the
+// lowest-label cell that has one (the seed fallback scan of cellenumerator.cpp:52-63); -1 when the solid touches no cell
+__device__ inline int64_t seed_bit(const MeshK& m, const SolidK& k, const SolidPlan& pl, const ActiveBox& b,
+                                   const uint8_t* cls) {
+    auto at = [&](int64_t i, int64_t j, int64_t kk) -> int64_t {
+        const int64_t x = i - b.c0[0], y = j - b.c0[1], z = kk - b.c0[2];
+        if (x < 0 || y < 0 || z < 0 || x >= b.n[0] || y >= b.n[1] || z >= b.n[2]) return -1;
+        return x + (int64_t)b.n[0] * (y + (int64_t)b.n[1] * z);
+    };
+    const int i = pl.seed_ijk[0], j = pl.seed_ijk[1], kk = pl.seed_ijk[2];
+    const int64_t sl = at(i, j, kk);
+    if (sl >= 0 && cls[(i - pl.lo[0]) + (int64_t)k.ext[0] * ((j - pl.lo[1]) + (int64_t)k.ext[1] * (kk - pl.lo[2]))])
+        return sl;
+    if (pl.min_cand == ~0ull) return -1;
+    int gi, gj, gk;
+    cell_ijk(m, (int64_t)pl.min_cand, gi, gj, gk);
+    return at(gi, gj, gk);
+}
+
+// The reached cells of one solid by a group of NT threads (a CTA, or a warp): bitmaps of the active box, rows along x of W
+// words, C (an inside vertex), I (all inside) and T (centre inside) from the class bytes, then the connected set of the
+// seed, then the lists in ascending label order.
+//
+// Nearly every set is connected, and that can be seen in one parallel pass: every row of candidates is one run, every
+// non-empty row but the first of its layer shares a column with the row before it, and every non-empty layer but the
+// first has such a pair with the layer below.  Then C is the answer.  Only sets that fail this (plates thinner than a
+// cell, concave shapes) are flooded from the seed, in sweeps that carry serial chains along y and z.  Bound by latency and
+// by the launch's tail (one CTA per solid, the largest first).  Measured (GB300): 0.69 -> 0.45 ms at 512^3 and 16 384 solids,
+// 0.18 -> 0.11 at 256^3 and 4096, 0.69 -> 0.02 for the four walls of a 1024^2 box (which the plan's vertex box reduces to
+// the cells beside the walls).
+__device__ inline FastDiv device_fastdiv(uint32_t d) {  // make_fastdiv for d < 2^31
+    const uint32_t l = d <= 1 ? 0 : 32 - __clz(d - 1);
+    return FastDiv{((1ull << (32 + l)) + d - 1) / d, 32 + l, d};
+}
+struct ConnectShared {
+    int bad, starts, base_in, base_cut;
+    int64_t seed;
+    FastDiv div_sy, div_w;   // by the rows per layer and by the words per row
+    int cnt[16][2];          // reached cells of each warp's words
+};
+template <int NT>
+__device__ __forceinline__ void group_sync() {
+    if (NT == 32) __syncwarp();
+    else __syncthreads();
+}
+template <int NT>
+__device__ __forceinline__ void connect_body(const MeshK& m, const SolidK& k, SolidPlan& pl, const uint8_t* cls, int s,
+                                             uint32_t* bitmaps, ConnectShared& sh, uint32_t* layers, int max_layers,
+                                             int tid, int32_t* in_cell, int32_t* in_solid, int32_t* cut_cell,
+                                             int32_t* cut_solid, int64_t cap_in, int64_t cap_cut, Counters* cnt) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = tid & 31, wid = tid >> 5;
+    constexpr int NW = NT / 32;
+    const ActiveBox b = active_box(m, k, pl);
+    const int sx = b.n[0], sy = b.n[1], sz = b.n[2];
+    if (tid == 0) {
+        sh.seed = pl.err || sx == 0 || sy == 0 || sz == 0 ? -1 : seed_bit(m, k, pl, b, cls);
+        sh.bad = 0;
+        sh.starts = 0;
+        sh.div_sy = device_fastdiv((uint32_t)max(1, sy));
+        sh.div_w = device_fastdiv((uint32_t)max(1, (sx + 31) >> 5));
+    }
+    const bool proof = sz <= max_layers;
+    const int lw = (sz + 31) >> 5;  // words per layer bitmap: non-empty layers, then layers joined to the one below
+    if (proof)
+        for (int i = tid; i < 2 * lw; i += NT) layers[i] = 0u;
+    group_sync<NT>();
+    if (sh.seed < 0) {
+        if (tid == 0) { pl.n_inside = 0; pl.n_cut = 0; }
+        return;
+    }
+    const int W = (sx + 31) >> 5, rows = sy * sz, nwords = rows * W;
+    uint32_t* C = bitmaps;
+    uint32_t* I = C + nwords;
+    uint32_t* T = I + nwords;
+    uint32_t* R = T + nwords;
+    const FastDiv dsy = sh.div_sy, dw = sh.div_w;
+    const int ox = b.c0[0] - pl.lo[0], oy = b.c0[1] - pl.lo[1], oz = b.c0[2] - pl.lo[2];
+    auto row_bytes = [&](int row) {
+        const int kk = (int)fdiv((uint32_t)row, dsy), jj = row - kk * sy;
+        return cls + ox + (int64_t)k.ext[0] * ((jj + oy) + (int64_t)k.ext[1] * (kk + oz));
+    };
+    // bitmaps: coalesced byte loads and ballots, several loads in flight; narrow boxes take two or four rows at once
+    {
+        constexpr int GW = 8;
+        const int lg = sx <= 8 ? 3 : (sx <= 16 ? 4 : 5), rpl = 32 >> lg;
+        const int sub = lane >> lg, col = lane & ((1 << lg) - 1);
+        const uint32_t msk = lg == 5 ? FULL : (1u << (1 << lg)) - 1u;
+        const int units = W == 1 ? (rows + rpl - 1) / rpl : nwords;  // loads
+        for (int u0 = wid * GW; u0 < units; u0 += NW * GW) {
+            uint8_t v[GW];
+#pragma unroll
+            for (int u = 0; u < GW; ++u) {
+                int row, x;
+                if (W == 1) { row = (u0 + u) * rpl + sub; x = col; }
+                else { row = (int)fdiv((uint32_t)(u0 + u), dw); x = ((u0 + u - row * W) << 5) + lane; }
+                v[u] = (u0 + u < units && row < rows && x < sx) ? row_bytes(row)[x] : (uint8_t)0;
+            }
+#pragma unroll
+            for (int u = 0; u < GW; ++u) {
+                const uint32_t bc = __ballot_sync(FULL, v[u] != 0), bi = __ballot_sync(FULL, v[u] == 1),
+                               bt = __ballot_sync(FULL, v[u] == 2);
+                const int w = W == 1 ? (u0 + u) * rpl + lane : u0 + u;
+                if (u0 + u < units && lane < (W == 1 ? rpl : 1) && w < nwords) {
+                    const int sft = W == 1 ? lane << lg : 0;
+                    C[w] = (bc >> sft) & msk;
+                    I[w] = (bi >> sft) & msk;
+                    T[w] = (bt >> sft) & msk;
+                }
+            }
+        }
+    }
+    group_sync<NT>();
+    bool connected = false;
+    if (proof) {
+        int bad = 0, starts = 0;
+        for (int row = tid; row < rows; row += NT) {
+            const uint32_t* c = C + row * W;
+            const int kk = (int)fdiv((uint32_t)row, dsy), jj = row - kk * sy;
+            int first = -1, last = -1, pop = 0;
+            uint32_t along = 0, below = 0;
+            for (int w = 0; w < W; ++w) {
+                const uint32_t x = c[w];
+                if (!x) continue;
+                pop += __popc(x);
+                if (first < 0) first = (w << 5) + __ffs(x) - 1;
+                last = (w << 5) + 31 - __clz(x);
+                if (jj > 0) along |= x & c[w - W];
+                if (kk > 0) below |= x & c[w - W * sy];
+            }
+            if (pop == 0) continue;
+            if (last - first + 1 != pop) ++bad;
+            if (!along) ++starts;
+            atomicOr(layers + (kk >> 5), 1u << (kk & 31));
+            if (below) atomicOr(layers + lw + (kk >> 5), 1u << (kk & 31));
+        }
+        bad = __reduce_add_sync(FULL, bad);
+        starts = __reduce_add_sync(FULL, starts);
+        if (lane == 0) {
+            if (bad) atomicAdd(&sh.bad, bad);
+            if (starts) atomicAdd(&sh.starts, starts);
+        }
+        group_sync<NT>();
+        int nl = 0, links = 0;
+        for (int i = 0; i < lw; ++i) {
+            nl += __popc(layers[i]);
+            links += __popc(layers[lw + i]);
+        }
+        connected = sh.bad == 0 && sh.starts == nl && links == nl - 1;
+    }
+    if (!connected) {
+        for (int w = tid; w < nwords; w += NT) R[w] = 0u;
+        group_sync<NT>();
+        if (tid == 0) {
+            const int srow = (int)(sh.seed / sx), x = (int)(sh.seed - (int64_t)srow * sx);
+            R[srow * W + (x >> 5)] = 1u << (x & 31);
+        }
+        group_sync<NT>();
+        // directional sweeps until nothing changes
+        const int max_rounds = 8 + 2 * (sx + sy + sz);
+        for (int round = 0;; ++round) {
+            int changed = 0;
+            // x: carry fill along each row
+            for (int row = tid; row < rows; row += NT) {
+                uint32_t* r = R + row * W;
+                const uint32_t* c = C + row * W;
+                uint32_t carry = 0;
+                for (int w = 0; w < W; ++w) {
+                    const uint32_t seeds = (r[w] | (carry & 1u)) & c[w];
+                    const uint32_t f = fill_up(c[w], seeds);
+                    if (f != r[w]) { changed = 1; r[w] = f; }
+                    carry = f >> 31;
+                }
+                carry = 0;
+                for (int w = W - 1; w >= 0; --w) {
+                    const uint32_t seeds = (r[w] | (carry << 31)) & c[w];
+                    const uint32_t f = fill_down(c[w], seeds);
+                    if (f != r[w]) { changed = 1; r[w] = f; }
+                    carry = f & 1u;
+                }
+            }
+            group_sync<NT>();
+            // y, then z: forward and backward scans along each column of words (the running value in a register)
+            for (int axis = 1; axis < 3; ++axis) {
+                const int len = axis == 1 ? sy : sz, ncol = axis == 1 ? sz * W : sy * W, stride = axis == 1 ? W : sy * W;
+                for (int col = tid; col < ncol; col += NT) {
+                    const int u = col / W, w = col - u * W;
+                    const int o = axis == 1 ? u * sy * W + w : u * W + w;
+                    uint32_t* r = R + o;
+                    const uint32_t* c = C + o;
+                    uint32_t prev = r[0];
+                    for (int j = 1; j < len; ++j) {
+                        const uint32_t cur = r[j * stride], f = cur | (prev & c[j * stride]);
+                        if (f != cur) { changed = 1; r[j * stride] = f; }
+                        prev = f;
+                    }
+                    for (int j = len - 2; j >= 0; --j) {
+                        const uint32_t cur = r[j * stride], f = cur | (prev & c[j * stride]);
+                        if (f != cur) { changed = 1; r[j * stride] = f; }
+                        prev = f;
+                    }
+                }
+                group_sync<NT>();
+            }
+            changed = NT == 32 ? __any_sync(FULL, changed) : __syncthreads_or(changed);
+            if (!changed) break;
+            if (round >= max_rounds) {
+                if (tid == 0) set_error(cnt, DERR_FLOOD_LIMIT);
+                break;
+            }
+        }
+        C = R;
+    }
+    // the lists: warp w takes the words [w0, w1), a lane counting a word, then a lane storing a cell
+    const int per = (((nwords + NW - 1) / NW) + 31) & ~31;
+    const int w0 = min(nwords, wid * per), w1 = min(nwords, w0 + per);
+    int nin = 0, ncut = 0;
+    for (int w = w0 + lane; w < w1; w += 32) {
+        const uint32_t bits = C[w], in = I[w];
+        nin += __popc(bits & in);
+        ncut += __popc(bits & ~in);
+    }
+    nin = __reduce_add_sync(FULL, nin);
+    ncut = __reduce_add_sync(FULL, ncut);
+    if (lane == 0) { sh.cnt[wid][0] = nin; sh.cnt[wid][1] = ncut; }
+    group_sync<NT>();
+    int before_in = 0, before_cut = 0, tot_in = 0, tot_cut = 0;
+#pragma unroll
+    for (int i = 0; i < NW; ++i) {
+        const int a = sh.cnt[i][0], c = sh.cnt[i][1];
+        if (i < wid) { before_in += a; before_cut += c; }
+        tot_in += a;
+        tot_cut += c;
+    }
+    if (tid == 0) {
+        sh.base_in = atomicAdd(&cnt->n_inside, tot_in);
+        sh.base_cut = atomicAdd(&cnt->n_cut, tot_cut);
+        pl.n_inside = tot_in;
+        pl.n_cut = tot_cut;
+    }
+    group_sync<NT>();
+    if ((int64_t)sh.base_in + tot_in > cap_in || (int64_t)sh.base_cut + tot_cut > cap_cut) {
+        if (tid == 0) set_error(cnt, DERR_CAPACITY);
+        return;
+    }
+    int64_t pin = (int64_t)sh.base_in + before_in, pcut = (int64_t)sh.base_cut + before_cut;
+    const uint32_t below = (1u << lane) - 1u;
+    for (int wb = w0; wb < w1; wb += 32) {
+        const int w = wb + lane;
+        uint32_t bits = 0, in = 0, ci = 0;
+        int label = 0;
+        if (w < w1) {
+            bits = C[w]; in = I[w]; ci = T[w];
+            const int row = (int)fdiv((uint32_t)w, dw), kk = (int)fdiv((uint32_t)row, dsy), jj = row - kk * sy;
+            label = (b.c0[0] + ((w - row * W) << 5)) + m.nx * ((b.c0[1] + jj) + m.ny * (b.c0[2] + kk));
+        }
+        const int a = __popc(bits & in), c = __popc(bits & ~in);
+        int xa = a, xc = c;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            int y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += y;
+            const int ya = __shfl_up_sync(FULL, xa, o), yc = __shfl_up_sync(FULL, xc, o);
+            if (lane >= o) { xa += ya; xc += yc; }
         }
-        if (lane < nw) warp_sums[lane] = w;  // inclusive
+        uint32_t some = __ballot_sync(FULL, bits != 0);
+        while (some) {
+            const int src = __ffs(some) - 1;
+            some &= some - 1;
+            const uint32_t bb = __shfl_sync(FULL, bits, src), ii = __shfl_sync(FULL, in, src), tt = __shfl_sync(FULL, ci, src);
+            const int cell = __shfl_sync(FULL, label, src) + lane, oi = __shfl_sync(FULL, xa - a, src),
+                      oc = __shfl_sync(FULL, xc - c, src);
+            if ((bb >> lane) & 1u) {
+                if ((ii >> lane) & 1u) {
+                    const int64_t p = pin + oi + __popc(bb & ii & below);
+                    in_cell[p] = cell;
+                    in_solid[p] = list_word(s, 1);
+                } else {
+                    const int64_t p = pcut + oc + __popc(bb & ~ii & below);
+                    cut_cell[p] = cell;
+                    cut_solid[p] = list_word(s, ((tt >> lane) & 1u) ? 2 : 3);
+                }
+            }
+        }
+        pin += __shfl_sync(FULL, xa, 31);
+        pcut += __shfl_sync(FULL, xc, 31);
     }
-    __syncthreads();
-    total = warp_sums[nw - 1];
-    const int before = (wid > 0 ? warp_sums[wid - 1] : 0) + x - v;
-    __syncthreads();
-    return before;
 }
 
-// local cell index of the flood-fill seed: the nearest cell when it has an inside vertex, else the lowest-label cell
-// that has one (the seed fallback scan of cellenumerator.cpp:52-63); -1 when the solid touches no cell
-__device__ inline int seed_local(const MeshK& m, const SolidPlan& pl, const uint8_t* cls, int ex, int ey, int ez) {
-    int sl = -1;
-    const int64_t seed = pl.seed;
-    const int64_t si = seed % m.nx, sj = (seed / m.nx) % m.ny, sk2 = seed / ((int64_t)m.nx * m.ny);
-    const int64_t a = si - pl.lo[0], b = sj - pl.lo[1], c = sk2 - pl.lo[2];
-    if (a >= 0 && b >= 0 && c >= 0 && a < ex && b < ey && c < ez) {
-        const int li = (int)(a + (int64_t)ex * (b + (int64_t)ey * c));
-        if (cls[li]) sl = li;
-    }
-    if (sl < 0 && pl.min_cand != ~0ull) {
-        const int64_t g = (int64_t)pl.min_cand;
-        const int64_t gi = g % m.nx, gj = (g / m.nx) % m.ny, gk = g / ((int64_t)m.nx * m.ny);
-        sl = (int)((gi - pl.lo[0]) + (int64_t)ex * ((gj - pl.lo[1]) + (int64_t)ey * (gk - pl.lo[2])));
-    }
-    if (sl >= ex * ey * ez) sl = -1;
-    return sl;
-}
-
+// a CTA per solid; bitmaps in shared memory, or in global memory above a size (bitmap_global)
+constexpr int CON_MAX_LAYERS = 2048;
 __global__ void __launch_bounds__(CON_THREADS, 2) connect_kernel(MeshK m, const SolidK* __restrict__ sk,
                                                               SolidPlan* __restrict__ plan,
                                                               const uint8_t* __restrict__ scratch,
@@ -304,352 +582,34 @@ __global__ void __launch_bounds__(CON_THREADS, 2) connect_kernel(MeshK m, const 
                                                               int32_t* __restrict__ in_cell, int32_t* __restrict__ in_solid,
                                                               int32_t* __restrict__ cut_cell, int32_t* __restrict__ cut_solid,
                                                               int64_t cap_in, int64_t cap_cut, Counters* cnt,
-                                                              int smem_words, const int32_t* __restrict__ solids) {
+                                                              const int32_t* __restrict__ solids) {
     extern __shared__ uint32_t dsm[];
-    __shared__ int s_seed;  // local cell index of the seed, -1: none
-    __shared__ int warp_sums[32];
-    __shared__ int s_base_in, s_base_cut;
+    __shared__ ConnectShared sh;
+    __shared__ uint32_t layers[2 * (CON_MAX_LAYERS / 32)];
     const int s = solids ? solids[blockIdx.x] : blockIdx.x;
-    const int tid = threadIdx.x;
     const SolidK& k = sk[s];
-    SolidPlan& pl = plan[s];
-    const int ex = k.ext[0], ey = k.ext[1], ez = k.ext[2];
-    const int W = (ex + 31) >> 5;
-    const int rows = ey * ez;
-    const int nwords = rows * W;
-    uint32_t* C = k.bitmap_global ? gbitmaps + k.bitmap_off : dsm;  // candidates (class != 0)
-    uint32_t* R = C + nwords;                                        // reached
-    uint32_t* I = R + nwords;                                        // class 1 (all inside)
-    uint32_t* T = I + nwords;                                        // class 2 (centre inside)
-    const uint8_t* cls = scratch + k.scratch_off;
-    if (pl.err) {
-        if (tid == 0) { pl.n_inside = 0; pl.n_cut = 0; }
-        return;
-    }
-    // seed: nearest cell when it has an inside vertex, else the lowest-label cell that has one
-    if (tid == 0) {
-        s_seed = seed_local(m, pl, cls, ex, ey, ez);
-    }
-    __syncthreads();
-    if (s_seed < 0) {
-        if (tid == 0) { pl.n_inside = 0; pl.n_cut = 0; }
-        return;
-    }
-    // the bitmaps from the class bytes: a warp per group of 16 words (16 independent loads in flight per lane),
-    // each word one coalesced 32-byte load and three ballots (the emission below then reads no class byte again)
-    {
-        const int lane = tid & 31;
-        constexpr int GW = 16;
-        for (int w0 = (tid >> 5) * GW; w0 < nwords; w0 += CON_THREADS / 32 * GW) {
-            uint8_t v[GW];
-#pragma unroll
-            for (int u = 0; u < GW; ++u) {
-                const int w = w0 + u;
-                const int row = w / W, xx = ((w - row * W) << 5) + lane;
-                v[u] = (w < nwords && xx < ex) ? cls[(int64_t)row * ex + xx] : (uint8_t)0;
-            }
-#pragma unroll
-            for (int u = 0; u < GW; ++u) {
-                const uint32_t bc = __ballot_sync(0xffffffffu, v[u] != 0), bi = __ballot_sync(0xffffffffu, v[u] == 1),
-                               bt = __ballot_sync(0xffffffffu, v[u] == 2);
-                if (lane == 0 && w0 + u < nwords) {
-                    C[w0 + u] = bc;
-                    I[w0 + u] = bi;
-                    T[w0 + u] = bt;
-                    R[w0 + u] = 0;
-                }
-            }
-        }
-    }
-    __syncthreads();
-    if (tid == 0) {
-        const int sx = s_seed % ex, srow = s_seed / ex;
-        R[srow * W + (sx >> 5)] |= 1u << (sx & 31);
-    }
-    __syncthreads();
-    // directional sweeps until nothing changes
-    const int max_rounds = 8 + 2 * (ex + ey + ez);
-    int round = 0;
-    for (;; ++round) {
-        int changed = 0;
-        // x: carry fill along each row
-        for (int row = tid; row < rows; row += CON_THREADS) {
-            uint32_t* r = R + row * W;
-            const uint32_t* c = C + row * W;
-            uint32_t carry = 0;
-            for (int w = 0; w < W; ++w) {
-                const uint32_t seeds = (r[w] | (carry & 1u)) & c[w];
-                const uint32_t f = fill_up(c[w], seeds);
-                if (f != r[w]) { changed = 1; r[w] = f; }
-                carry = f >> 31;
-            }
-            carry = 0;
-            for (int w = W - 1; w >= 0; --w) {
-                const uint32_t seeds = (r[w] | (carry << 31)) & c[w];
-                const uint32_t f = fill_down(c[w], seeds);
-                if (f != r[w]) { changed = 1; r[w] = f; }
-                carry = f & 1u;
-            }
-        }
-        __syncthreads();
-        // y: forward and backward scans along j for every (k, word)
-        for (int col = tid; col < ez * W; col += CON_THREADS) {
-            const int kk = col / W, w = col - kk * W;
-            uint32_t* r = R + (kk * ey) * W + w;
-            const uint32_t* c = C + (kk * ey) * W + w;
-            // the running value stays in a register: the loads of r and c do not depend on the previous step
-            uint32_t prev = r[0];
-            for (int j = 1; j < ey; ++j) {
-                const uint32_t cur = r[j * W], f = cur | (prev & c[j * W]);
-                if (f != cur) { changed = 1; r[j * W] = f; }
-                prev = f;
-            }
-            for (int j = ey - 2; j >= 0; --j) {
-                const uint32_t cur = r[j * W], f = cur | (prev & c[j * W]);
-                if (f != cur) { changed = 1; r[j * W] = f; }
-                prev = f;
-            }
-        }
-        __syncthreads();
-        // z: forward and backward scans along k for every (j, word)
-        if (ez > 1) {
-            for (int col = tid; col < ey * W; col += CON_THREADS) {
-                const int jj = col / W, w = col - jj * W;
-                uint32_t* r = R + jj * W + w;
-                const uint32_t* c = C + jj * W + w;
-                const int stride = ey * W;
-                uint32_t prev = r[0];
-                for (int kk = 1; kk < ez; ++kk) {
-                    const uint32_t cur = r[kk * stride], f = cur | (prev & c[kk * stride]);
-                    if (f != cur) { changed = 1; r[kk * stride] = f; }
-                    prev = f;
-                }
-                for (int kk = ez - 2; kk >= 0; --kk) {
-                    const uint32_t cur = r[kk * stride], f = cur | (prev & c[kk * stride]);
-                    if (f != cur) { changed = 1; r[kk * stride] = f; }
-                    prev = f;
-                }
-            }
-        }
-        changed = __syncthreads_or(changed);
-        if (!changed) break;
-        if (round >= max_rounds) {
-            if (tid == 0) set_error(cnt, DERR_FLOOD_LIMIT);
-            break;
-        }
-    }
-    // emit the reached cells in ascending label order: thread t owns rows [t*rpt, (t+1)*rpt)
-    const int rpt = (rows + CON_THREADS - 1) / CON_THREADS;
-    const int r0 = min(rows, tid * rpt), r1 = min(rows, r0 + rpt);
-    int nin = 0, ncut = 0;
-    for (int row = r0; row < r1; ++row)
-        for (int w = 0; w < W; ++w) {
-            const uint32_t bits = R[row * W + w], in = I[row * W + w];
-            nin += __popc(bits & in);
-            ncut += __popc(bits & ~in);
-        }
-    int tot_in, tot_cut;
-    const int off_in = block_excl_scan(nin, warp_sums, tot_in);
-    const int off_cut = block_excl_scan(ncut, warp_sums, tot_cut);
-    if (tid == 0) {
-        s_base_in = atomicAdd(&cnt->n_inside, tot_in);
-        s_base_cut = atomicAdd(&cnt->n_cut, tot_cut);
-        pl.n_inside = tot_in;
-        pl.n_cut = tot_cut;
-    }
-    __syncthreads();
-    const int64_t bin = s_base_in, bcut = s_base_cut;
-    if (bin + tot_in > cap_in || bcut + tot_cut > cap_cut) {
-        if (tid == 0) set_error(cnt, DERR_CAPACITY);
-        return;
-    }
-    int64_t pin = bin + off_in, pcut = bcut + off_cut;
-    for (int row = r0; row < r1; ++row) {
-        const int jj = row % ey, kk = row / ey;
-        for (int w = 0; w < W; ++w) {
-            uint32_t bits = R[row * W + w];
-            const uint32_t in = I[row * W + w], ci = T[row * W + w];
-            while (bits) {
-                const int b = __ffs(bits) - 1;
-                bits &= bits - 1;
-                const int xx = (w << 5) + b;
-                const uint8_t cc = ((in >> b) & 1u) ? 1 : (((ci >> b) & 1u) ? 2 : 3);
-                const int64_t gi = pl.lo[0] + xx, gj = pl.lo[1] + jj, gk = pl.lo[2] + kk;
-                const int32_t cell = (int32_t)(gi + (int64_t)m.nx * (gj + (int64_t)m.ny * gk));
-                if (cc == 1) { in_cell[pin] = cell; in_solid[pin] = list_word(s, 1); ++pin; }
-                else { cut_cell[pcut] = cell; cut_solid[pcut] = list_word(s, cc); ++pcut; }
-            }
-        }
-    }
+    connect_body<CON_THREADS>(m, k, plan[s], scratch + k.scratch_off, s, k.bitmap_global ? gbitmaps + k.bitmap_off : dsm, sh,
+                              layers, CON_MAX_LAYERS, threadIdx.x, in_cell, in_solid, cut_cell, cut_solid, cap_in, cap_cut,
+                              cnt);
 }
 
-// The same connected component for solids whose bbox bitmap has at most CON_SMALL_WORDS words: one warp per solid,
-// eight solids per CTA, bitmaps in shared memory, warp-synchronous sweeps.
+// a warp per solid for the solids whose bbox bitmap has at most CON_SMALL_WORDS words
 constexpr int CON_SMALL_WORDS = 256;
 constexpr int CON_SMALL_WARPS = 8;
-
 __global__ void __launch_bounds__(CON_SMALL_WARPS * 32) connect_small_kernel(
     MeshK m, const SolidK* __restrict__ sk, SolidPlan* __restrict__ plan, const uint8_t* __restrict__ scratch,
     int32_t* __restrict__ in_cell, int32_t* __restrict__ in_solid, int32_t* __restrict__ cut_cell,
     int32_t* __restrict__ cut_solid, int64_t cap_in, int64_t cap_cut, Counters* cnt, const int32_t* __restrict__ solids,
     int nsolids) {
-    __shared__ uint32_t s_bits[CON_SMALL_WARPS][2 * CON_SMALL_WORDS];
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int item = blockIdx.x * CON_SMALL_WARPS + wid;
+    __shared__ uint32_t s_bits[CON_SMALL_WARPS][4 * CON_SMALL_WORDS];
+    __shared__ ConnectShared sh[CON_SMALL_WARPS];
+    __shared__ uint32_t layers[CON_SMALL_WARPS][2 * (CON_SMALL_WORDS / 32)];
+    const int wid = threadIdx.x >> 5, item = blockIdx.x * CON_SMALL_WARPS + wid;
     if (item >= nsolids) return;
     const int s = solids[item];
     const SolidK& k = sk[s];
-    SolidPlan& pl = plan[s];
-    const int ex = k.ext[0], ey = k.ext[1], ez = k.ext[2];
-    const int W = (ex + 31) >> 5;
-    const int rows = ey * ez;
-    const int nwords = rows * W;
-    uint32_t* C = s_bits[wid];
-    uint32_t* R = C + CON_SMALL_WORDS;
-    const uint8_t* cls = scratch + k.scratch_off;
-    if (pl.err) {
-        if (lane == 0) { pl.n_inside = 0; pl.n_cut = 0; }
-        return;
-    }
-    int sl = 0;
-    if (lane == 0) sl = seed_local(m, pl, cls, ex, ey, ez);
-    sl = __shfl_sync(FULL, sl, 0);
-    if (sl < 0) {
-        if (lane == 0) { pl.n_inside = 0; pl.n_cut = 0; }
-        return;
-    }
-    for (int w = lane; w < nwords; w += 32) {
-        const int row = w / W, wi = w - row * W;
-        const uint8_t* rp = cls + (int64_t)row * ex;
-        uint32_t bits = 0;
-        const int x0 = wi << 5, x1 = min(ex, x0 + 32);
-        for (int xx = x0; xx < x1; ++xx) bits |= (rp[xx] ? 1u : 0u) << (xx - x0);
-        C[w] = bits;
-        R[w] = 0;
-    }
-    __syncwarp();
-    if (lane == 0) {
-        const int sx = sl % ex, srow = sl / ex;
-        R[srow * W + (sx >> 5)] |= 1u << (sx & 31);
-    }
-    __syncwarp();
-    const int max_rounds = 8 + 2 * (ex + ey + ez);
-    for (int round = 0;; ++round) {
-        int changed = 0;
-        for (int row = lane; row < rows; row += 32) {
-            uint32_t* r = R + row * W;
-            const uint32_t* c = C + row * W;
-            uint32_t carry = 0;
-            for (int w = 0; w < W; ++w) {
-                const uint32_t seeds = (r[w] | (carry & 1u)) & c[w];
-                const uint32_t f = fill_up(c[w], seeds);
-                if (f != r[w]) { changed = 1; r[w] = f; }
-                carry = f >> 31;
-            }
-            carry = 0;
-            for (int w = W - 1; w >= 0; --w) {
-                const uint32_t seeds = (r[w] | (carry << 31)) & c[w];
-                const uint32_t f = fill_down(c[w], seeds);
-                if (f != r[w]) { changed = 1; r[w] = f; }
-                carry = f & 1u;
-            }
-        }
-        __syncwarp();
-        for (int col = lane; col < ez * W; col += 32) {
-            const int kk = col / W, w = col - kk * W;
-            uint32_t* r = R + (kk * ey) * W + w;
-            const uint32_t* c = C + (kk * ey) * W + w;
-            // the running value stays in a register: the loads of r and c do not depend on the previous step
-            uint32_t prev = r[0];
-            for (int j = 1; j < ey; ++j) {
-                const uint32_t cur = r[j * W], f = cur | (prev & c[j * W]);
-                if (f != cur) { changed = 1; r[j * W] = f; }
-                prev = f;
-            }
-            for (int j = ey - 2; j >= 0; --j) {
-                const uint32_t cur = r[j * W], f = cur | (prev & c[j * W]);
-                if (f != cur) { changed = 1; r[j * W] = f; }
-                prev = f;
-            }
-        }
-        __syncwarp();
-        if (ez > 1) {
-            for (int col = lane; col < ey * W; col += 32) {
-                const int jj = col / W, w = col - jj * W;
-                uint32_t* r = R + jj * W + w;
-                const uint32_t* c = C + jj * W + w;
-                const int stride = ey * W;
-                uint32_t prev = r[0];
-                for (int kk = 1; kk < ez; ++kk) {
-                    const uint32_t cur = r[kk * stride], f = cur | (prev & c[kk * stride]);
-                    if (f != cur) { changed = 1; r[kk * stride] = f; }
-                    prev = f;
-                }
-                for (int kk = ez - 2; kk >= 0; --kk) {
-                    const uint32_t cur = r[kk * stride], f = cur | (prev & c[kk * stride]);
-                    if (f != cur) { changed = 1; r[kk * stride] = f; }
-                    prev = f;
-                }
-            }
-        }
-        __syncwarp();
-        if (!__any_sync(FULL, changed)) break;
-        if (round >= max_rounds) {
-            if (lane == 0) set_error(cnt, DERR_FLOOD_LIMIT);
-            break;
-        }
-    }
-    // emit in ascending label order: lane t owns rows [t*rpt, (t+1)*rpt)
-    const int rpt = (rows + 31) / 32;
-    const int r0 = min(rows, lane * rpt), r1 = min(rows, r0 + rpt);
-    int nin = 0, ncut = 0;
-    for (int row = r0; row < r1; ++row)
-        for (int w = 0; w < W; ++w) {
-            uint32_t bits = R[row * W + w];
-            while (bits) {
-                const int b = __ffs(bits) - 1;
-                bits &= bits - 1;
-                if (cls[(int64_t)row * ex + (w << 5) + b] == 1) ++nin; else ++ncut;
-            }
-        }
-    int xin = nin, xcut = ncut;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int a = __shfl_up_sync(FULL, xin, o), b = __shfl_up_sync(FULL, xcut, o);
-        if (lane >= o) { xin += a; xcut += b; }
-    }
-    const int tot_in = __shfl_sync(FULL, xin, 31), tot_cut = __shfl_sync(FULL, xcut, 31);
-    int bin = 0, bcut = 0;
-    if (lane == 0) {
-        bin = atomicAdd(&cnt->n_inside, tot_in);
-        bcut = atomicAdd(&cnt->n_cut, tot_cut);
-        pl.n_inside = tot_in;
-        pl.n_cut = tot_cut;
-    }
-    bin = __shfl_sync(FULL, bin, 0);
-    bcut = __shfl_sync(FULL, bcut, 0);
-    if ((int64_t)bin + tot_in > cap_in || (int64_t)bcut + tot_cut > cap_cut) {
-        if (lane == 0) set_error(cnt, DERR_CAPACITY);
-        return;
-    }
-    int64_t pin = (int64_t)bin + xin - nin, pcut = (int64_t)bcut + xcut - ncut;
-    for (int row = r0; row < r1; ++row) {
-        const int jj = row % ey, kk = row / ey;
-        for (int w = 0; w < W; ++w) {
-            uint32_t bits = R[row * W + w];
-            while (bits) {
-                const int b = __ffs(bits) - 1;
-                bits &= bits - 1;
-                const int xx = (w << 5) + b;
-                const uint8_t cc = cls[(int64_t)row * ex + xx];
-                const int64_t gi = pl.lo[0] + xx, gj = pl.lo[1] + jj, gk = pl.lo[2] + kk;
-                const int32_t cell = (int32_t)(gi + (int64_t)m.nx * (gj + (int64_t)m.ny * gk));
-                if (cc == 1) { in_cell[pin] = cell; in_solid[pin] = list_word(s, 1); ++pin; }
-                else { cut_cell[pcut] = cell; cut_solid[pcut] = list_word(s, cc); ++pcut; }
-            }
-        }
-    }
+    connect_body<32>(m, k, plan[s], scratch + k.scratch_off, s, s_bits[wid], sh[wid], layers[wid], CON_SMALL_WORDS,
+                     threadIdx.x & 31, in_cell, in_solid, cut_cell, cut_solid, cap_in, cap_cut, cnt);
 }
 
 // ---- shared cells -----------------------------------------------------------------------------------------------------

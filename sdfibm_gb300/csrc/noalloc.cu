@@ -37,7 +37,7 @@ void launch_classify(const ClassifyArgs& A, bool flat, int grid, cudaStream_t st
 int classify_occupancy(int method, bool flat);
 __global__ void connect_kernel(MeshK m, const SolidK* sk, SolidPlan* plan, const uint8_t* scratch, uint32_t* gbitmaps,
                                int32_t* in_cell, int32_t* in_solid, int32_t* cut_cell, int32_t* cut_solid,
-                               int64_t cap_in, int64_t cap_cut, Counters* cnt, int smem_words, const int32_t* solids);
+                               int64_t cap_in, int64_t cap_cut, Counters* cnt, const int32_t* solids);
 }  // namespace sdfibm_dev
 
 using namespace sdfibm_dev;
@@ -45,7 +45,7 @@ using namespace sdfibm_dev;
 namespace {
 
 constexpr int64_t NA_MAX_BBOX_CELLS = 1 << 19;    // 524288 cells, e.g. an 80 x 80 x 80 box
-constexpr int64_t NA_MAX_BITMAP_WORDS = 1 << 18;  // candidate + reached bitmaps, 32 cells per word
+constexpr int64_t NA_MAX_BITMAP_WORDS = 1 << 18;  // two of the four bitmaps, 32 cells per word
 
 constexpr size_t na_align(size_t x) { return (x + 255) & ~(size_t)255; }
 constexpr size_t OFF_SK = 0;
@@ -57,7 +57,7 @@ constexpr size_t OFF_CHUNKS = OFF_CNT + na_align(sizeof(Counters));
 constexpr size_t OFF_CLS = OFF_CHUNKS + na_align(sizeof(int2) * NA_MAX_CHUNKS);
 constexpr size_t OFF_BITMAP = OFF_CLS + na_align(NA_MAX_BBOX_CELLS);
 constexpr size_t LIST_BYTES = na_align(4 * NA_MAX_BBOX_CELLS);
-constexpr size_t OFF_IN_CELL = OFF_BITMAP + na_align(4 * NA_MAX_BITMAP_WORDS);
+constexpr size_t OFF_IN_CELL = OFF_BITMAP + na_align(2 * 4 * NA_MAX_BITMAP_WORDS);
 constexpr size_t OFF_IN_SOLID = OFF_IN_CELL + LIST_BYTES;
 constexpr size_t OFF_CUT_CELL = OFF_IN_SOLID + LIST_BYTES;
 constexpr size_t OFF_CUT_SOLID = OFF_CUT_CELL + LIST_BYTES;
@@ -303,7 +303,7 @@ extern "C" int sdfibm_cuda_touched_noalloc(const sdfibm_mesh_desc* mesh, const s
     connect_kernel<<<1, 512, 0, st>>>(m, d_sk, d_plan, b + OFF_CLS, reinterpret_cast<uint32_t*>(b + OFF_BITMAP),
                                       reinterpret_cast<int32_t*>(b + OFF_IN_CELL), reinterpret_cast<int32_t*>(b + OFF_IN_SOLID),
                                       reinterpret_cast<int32_t*>(b + OFF_CUT_CELL), reinterpret_cast<int32_t*>(b + OFF_CUT_SOLID),
-                                      NA_MAX_BBOX_CELLS, NA_MAX_BBOX_CELLS, d_cnt, 0, nullptr);
+                                      NA_MAX_BBOX_CELLS, NA_MAX_BBOX_CELLS, d_cnt, nullptr);
     noalloc_order_kernel<<<1, 1024, 0, st>>>(cells, types, capacity, n_device);
     return cudaGetLastError() == cudaSuccess ? SDFIBM_OK : SDFIBM_ERR_CUDA;
 }
