@@ -25,6 +25,7 @@ __global__ void plan_kernel(MeshK m, const SolidK* sk, const sdfibm_solid_state*
                             Counters* cnt);
 void launch_classify(const ClassifyArgs& A, bool flat, int grid, cudaStream_t st);
 int classify_occupancy(int method, bool flat);
+int classify_kind(int shape_type, bool flat);
 __global__ void subsample_cells_kernel(FallbackArgs A);
 __global__ void recount_kernel(FallbackArgs A);
 __global__ void learned_stencil_kernel(StencilArgs A);
@@ -131,6 +132,7 @@ struct sdfibm_ctx {
     SolidPlan* d_plan = nullptr;
     int2* d_chunks = nullptr;  // classify work items: (solid, first tile)
     int total_chunks = 0;
+    int fast_chunks = 0;       // leading chunks of the shapes classify_kernel may take
     int chunk_tiles = CHUNK_TILES;
     int64_t chunks_cap = 0;    // entries reserved in d_chunks
     int total_tiles = 0;
@@ -311,16 +313,22 @@ static int fail(sdfibm_ctx* ctx, int code, const std::string& msg) {
 // classify work items: chunks of up to chunk_tiles consecutive tiles of each solid, the solids grouped by shape type
 // (stable): the cut-cell lists then come out grouped by type too, so that the warps of the per-cell kernels mostly
 // run one shape's distance code (the learned stencil: 11 % faster at 256^3 than with the types interleaved)
-static std::vector<int2> make_chunks(const std::vector<SolidK>& hk, int chunk_tiles) {
+static std::vector<int2> make_chunks(const std::vector<SolidK>& hk, int chunk_tiles, bool flat, int* fast_chunks) {
     std::vector<int2> chunks;
+    *fast_chunks = 0;
     std::vector<size_t> order(hk.size());
     for (size_t s = 0; s < hk.size(); ++s) order[s] = s;
     std::stable_sort(order.begin(), order.end(),
-                     [&](size_t a, size_t b) { return hk[a].shape.type < hk[b].shape.type; });
+                     [&](size_t a, size_t b) {
+                         const int ta = hk[a].shape.type, tb = hk[b].shape.type;
+                         const int ka = classify_kind(ta, flat), kb = classify_kind(tb, flat);
+                         return ka != kb ? ka < kb : ta < tb;
+                     });
     for (size_t s : order) {
         const SolidK& k = hk[s];
         const int nt = k.ntile[0] * k.ntile[1] * k.ntile[2];
         for (int t0 = 0; t0 < nt; t0 += chunk_tiles) chunks.push_back(make_int2((int)s, t0));
+        if (classify_kind(k.shape.type, flat) == 0) *fast_chunks = (int)chunks.size();
     }
     return chunks;
 }
@@ -520,12 +528,18 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
         ctx->sh_mask = (int32_t)(t - 1);
         ctx->shent_cap = 2 * t;  // a shared cell has two or more entries
     }
-    ctx->chunk_tiles = CHUNK_TILES;
+    // work items of CHUNK_TILES tiles, fewer where they would leave warps of the launch without one (about 24 warps an SM;
+    // half spaces do not count, nearly all of their tiles are skipped): one cylinder's 9 tiles took 36 us in two items and
+    // 12 in nine
+    int64_t finite_tiles = 0;
+    for (const SolidK& k : ctx->hk)
+        if (!k.infinite) finite_tiles += (int64_t)k.ntile[0] * k.ntile[1] * k.ntile[2];
+    ctx->chunk_tiles = (int)std::max<int64_t>(1, std::min<int64_t>(CHUNK_TILES, finite_tiles / (24 * (int64_t)ctx->num_sms)));
     if (ctx->opt.tile_cells > 0) {
         const int cells_per_tile = mesh->nz <= 2 ? 8 * 8 * 2 : 4 * 4 * 4;
         ctx->chunk_tiles = std::max(1, std::min(255, ctx->opt.tile_cells / cells_per_tile));
     }
-    std::vector<int2> chunks = make_chunks(ctx->hk, ctx->chunk_tiles);
+    std::vector<int2> chunks = make_chunks(ctx->hk, ctx->chunk_tiles, mesh->nz <= 2, &ctx->fast_chunks);
     ctx->total_chunks = (int)chunks.size();
 
     // collision grid (UGrid(bbox of the mesh, 2*max radiusB))
@@ -753,6 +767,9 @@ static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float
         CA.m = ctx->mesh; CA.sk = ctx->d_sk; CA.st = ctx->d_st; CA.plan = ctx->d_plan; CA.chunks = ctx->d_chunks;
         CA.total_chunks = ctx->total_chunks; CA.cls = ctx->d_scratch; CA.alpha = ctx->d_alpha; CA.cnt = ctx->d_cnt;
         CA.chunk_tiles = ctx->chunk_tiles;
+        CA.fast_chunks = ctx->fast_chunks;
+        CA.any_first = ctx->mesh.nz <= 2 ? 0 : ctx->fast_chunks;
+        CA.any_grid = std::min(2 * ctx->num_sms, (ctx->total_chunks - CA.any_first + 7) / 8);
         CA.method = ctx->opt.fraction_method; CA.subsample_n = ctx->opt.subsample_n;
         const bool learned = ctx->opt.fraction_method == SDFIBM_FRACTION_LEARNED;
         const bool subsample = ctx->opt.fraction_method == SDFIBM_FRACTION_SUBSAMPLE;
@@ -773,7 +790,7 @@ static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float
             CA.feat_cap = ctx->feat_cap; CA.fref_solid = ctx->d_fref_solid; CA.fref_index = ctx->d_fref_index;
             CA.rho_min = ctx->rho_min;
         }
-        launch_classify(CA, ctx->mesh.nz <= 2, ctx->classify_grid, st);
+        launch_classify(CA, ctx->mesh.nz <= 2, std::min(ctx->classify_grid, (ctx->fast_chunks + 7) / 8), st);
         mark(ctx, "classify_kernel");
         // the component pass needs only the class bytes and the seeds: on the side stream, beside the fraction
         // kernels below (one stream while timing, so that every kernel has its own events)
@@ -1472,11 +1489,13 @@ static std::string tune_key(const sdfibm_ctx* ctx) {
 }
 
 static int apply_tuning(sdfibm_ctx* ctx, const Tuning& t) {
-    std::vector<int2> ch = make_chunks(ctx->hk, t.chunk_tiles);
+    int fast = 0;
+    std::vector<int2> ch = make_chunks(ctx->hk, t.chunk_tiles, ctx->mesh.nz <= 2, &fast);
     if ((int64_t)ch.size() > ctx->chunks_cap) return fail(ctx, SDFIBM_ERR_CAPACITY, "chunk table too small");
     CK(cudaMemcpy(ctx->d_chunks, ch.data(), sizeof(int2) * ch.size(), cudaMemcpyHostToDevice));
     ctx->chunk_tiles = t.chunk_tiles;
     ctx->total_chunks = (int)ch.size();
+    ctx->fast_chunks = fast;
     ctx->opt.tile_cells = t.chunk_tiles * (ctx->mesh.nz <= 2 ? 8 * 8 * 2 : 4 * 4 * 4);
     ctx->classify_grid = t.classify_grid;
     ctx->subsample_grid = t.subsample_grid;
@@ -1553,7 +1572,8 @@ int sdfibm_cuda_autotune(sdfibm_ctx* ctx, double dt, const float* U, float* As, 
     for (int tc : tiles_cand) {
         Tuning t = best;
         t.chunk_tiles = tc;
-        if ((int64_t)make_chunks(ctx->hk, tc).size() > ctx->chunks_cap) continue;
+        int fast = 0;
+        if ((int64_t)make_chunks(ctx->hk, tc, ctx->mesh.nz <= 2, &fast).size() > ctx->chunks_cap) continue;
         std::map<std::string, float> ms;
         if ((rc = measure(t, ms))) break;
         if (ms.count("classify_kernel") && ms["classify_kernel"] < best_cls) {

@@ -203,7 +203,6 @@ __global__ void plan_kernel(MeshK m, const SolidK* __restrict__ sk, const sdfibm
                                  fabs(x.y) + fabs(x.z)));
         p.pad2 = 0.f;
     }
-    p.min_cand = ~0ull;
     p.n_inside = p.n_cut = 0;
     plan[s] = p;
 }
@@ -286,23 +285,11 @@ __device__ inline ActiveBox active_box(const MeshK& m, const SolidK& k, const So
     return b;
 }
 
-// bit index (row * sx + x) of the flood-fill seed in the active box: the nearest cell when it has an inside vertex, else the
-// lowest-label cell that has one (the seed fallback scan of cellenumerator.cpp:52-63); -1 when the solid touches no cell
-__device__ inline int64_t seed_bit(const MeshK& m, const SolidK& k, const SolidPlan& pl, const ActiveBox& b,
-                                   const uint8_t* cls) {
-    auto at = [&](int64_t i, int64_t j, int64_t kk) -> int64_t {
-        const int64_t x = i - b.c0[0], y = j - b.c0[1], z = kk - b.c0[2];
-        if (x < 0 || y < 0 || z < 0 || x >= b.n[0] || y >= b.n[1] || z >= b.n[2]) return -1;
-        return x + (int64_t)b.n[0] * (y + (int64_t)b.n[1] * z);
-    };
-    const int i = pl.seed_ijk[0], j = pl.seed_ijk[1], kk = pl.seed_ijk[2];
-    const int64_t sl = at(i, j, kk);
-    if (sl >= 0 && cls[(i - pl.lo[0]) + (int64_t)k.ext[0] * ((j - pl.lo[1]) + (int64_t)k.ext[1] * (kk - pl.lo[2]))])
-        return sl;
-    if (pl.min_cand == ~0ull) return -1;
-    int gi, gj, gk;
-    cell_ijk(m, (int64_t)pl.min_cand, gi, gj, gk);
-    return at(gi, gj, gk);
+// bit index (row * sx + x) in the active box of the solid's nearest cell; -1 outside it
+__device__ inline int64_t seed_bit(const SolidPlan& pl, const ActiveBox& b) {
+    const int64_t x = pl.seed_ijk[0] - b.c0[0], y = pl.seed_ijk[1] - b.c0[1], z = pl.seed_ijk[2] - b.c0[2];
+    if (x < 0 || y < 0 || z < 0 || x >= b.n[0] || y >= b.n[1] || z >= b.n[2]) return -1;
+    return x + (int64_t)b.n[0] * (y + (int64_t)b.n[1] * z);
 }
 
 // The reached cells of one solid by a group of NT threads (a CTA, or a warp): bitmaps of the active box, rows along x of W
@@ -322,7 +309,7 @@ __device__ inline FastDiv device_fastdiv(uint32_t d) {  // make_fastdiv for d < 
 }
 struct ConnectShared {
     int bad, starts, base_in, base_cut;
-    int64_t seed;
+    unsigned first;          // lowest word of C with a bit
     FastDiv div_sy, div_w;   // by the rows per layer and by the words per row
     int cnt[16][2];          // reached cells of each warp's words
 };
@@ -342,7 +329,7 @@ __device__ __forceinline__ void connect_body(const MeshK& m, const SolidK& k, So
     const ActiveBox b = active_box(m, k, pl);
     const int sx = b.n[0], sy = b.n[1], sz = b.n[2];
     if (tid == 0) {
-        sh.seed = pl.err || sx == 0 || sy == 0 || sz == 0 ? -1 : seed_bit(m, k, pl, b, cls);
+        sh.first = ~0u;
         sh.bad = 0;
         sh.starts = 0;
         sh.div_sy = device_fastdiv((uint32_t)max(1, sy));
@@ -353,7 +340,7 @@ __device__ __forceinline__ void connect_body(const MeshK& m, const SolidK& k, So
     if (proof)
         for (int i = tid; i < 2 * lw; i += NT) layers[i] = 0u;
     group_sync<NT>();
-    if (sh.seed < 0) {
+    if (pl.err || sx == 0 || sy == 0 || sz == 0) {
         if (tid == 0) { pl.n_inside = 0; pl.n_cut = 0; }
         return;
     }
@@ -434,14 +421,32 @@ __device__ __forceinline__ void connect_body(const MeshK& m, const SolidK& k, So
             nl += __popc(layers[i]);
             links += __popc(layers[lw + i]);
         }
-        connected = sh.bad == 0 && sh.starts == nl && links == nl - 1;
+        connected = nl > 0 && sh.bad == 0 && sh.starts == nl && links == nl - 1;
     }
     if (!connected) {
-        for (int w = tid; w < nwords; w += NT) R[w] = 0u;
+        unsigned first = ~0u;
+        for (int w = tid; w < nwords; w += NT) {
+            R[w] = 0u;
+            if (C[w]) first = min(first, (unsigned)w);
+        }
+        first = __reduce_min_sync(FULL, first);
+        if (lane == 0 && first != ~0u) atomicMin(&sh.first, first);
         group_sync<NT>();
+        if (sh.first == ~0u) {  // no cell has an inside vertex
+            if (tid == 0) { pl.n_inside = 0; pl.n_cut = 0; }
+            return;
+        }
+        // the flood's seed: the nearest cell when it has an inside vertex, else the lowest-label cell that has one (the seed
+        // fallback scan of cellenumerator.cpp:52-63; rows are in label order)
         if (tid == 0) {
-            const int srow = (int)(sh.seed / sx), x = (int)(sh.seed - (int64_t)srow * sx);
-            R[srow * W + (x >> 5)] = 1u << (x & 31);
+            const int64_t sb = seed_bit(pl, b);
+            int w = (int)sh.first;
+            uint32_t bit = C[w] & (0u - C[w]);
+            if (sb >= 0) {
+                const int srow = (int)(sb / sx), x = (int)(sb - (int64_t)srow * sx);
+                if ((C[srow * W + (x >> 5)] >> (x & 31)) & 1u) { w = srow * W + (x >> 5); bit = 1u << (x & 31); }
+            }
+            R[w] = bit;
         }
         group_sync<NT>();
         // directional sweeps until nothing changes
@@ -977,7 +982,7 @@ __global__ void finalize_kernel(float* __restrict__ As, float* __restrict__ Ts, 
 __global__ void begin_kernel(Counters* cnt) {
     cnt->prev_n_inside = cnt->n_inside;
     cnt->prev_n_cut = cnt->n_cut;
-    cnt->classify_next = 0; cnt->couple_next = 0; cnt->finalize_next = 0;
+    cnt->classify_next = 0; cnt->classify_any_next = 0;
     cnt->n_inside = 0; cnt->n_cut = 0; cnt->n_shared = 0; cnt->shared_marks = 0;
     cnt->exact_rechecks = 0; cnt->bbox_cells = 0;
     cnt->n_feat = 0; cnt->n_fb = 0; cnt->n_recheck = 0; cnt->n_ovf = 0; cnt->n_shent = 0;

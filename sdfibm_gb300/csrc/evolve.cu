@@ -625,7 +625,6 @@ __device__ inline void move_rotation4(const SolidK& k, const double* q4, const d
 // give the same bits.
 __device__ inline D3 ev_contact_sum(const EvolveWork& w, const SolidK* sk, int buf, int S, const FineGridK& fg, int p, int n,
                                     const int32_t* q, double (*fc)[3], int32_t* home) {
-    const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     D3 f{0, 0, 0};
     const D3 xp = ev_pos(w, buf, S, p);

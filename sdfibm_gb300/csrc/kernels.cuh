@@ -69,7 +69,6 @@ struct SolidPlan {
     int32_t lo[3];            // bbox lower cell index (may lie outside the mesh)
     int32_t err;              // nonzero: bbox too small for the current pose
     int64_t seed;             // meshSearch::findNearestCell result
-    unsigned long long min_cand;  // lowest cell label with an inside vertex (atomicMin), ~0 when none
     float M[9];               // FP32 world->local matrix (|q|^2 R^T)
     int32_t n_inside, n_cut;  // touched cells by kind
     int32_t seed_ijk[3];      // cell indices of the seed cell
@@ -99,8 +98,8 @@ struct SolidPlan {
 // Global counters / flags (one record per context, device memory).
 struct Counters {
     int32_t classify_next;
-    int32_t couple_next;
-    int32_t finalize_next;
+    int32_t classify_any_next;
+    int32_t pad1;
     int32_t n_inside;         // entries in the ALL_INSIDE list of this call
     int32_t n_cut;            // entries in the cut-cell list of this call
     int32_t n_shared;         // cells touched by two or more solids this call (slots used in the shared table)
@@ -195,6 +194,9 @@ struct ClassifyArgs {
     const int2* chunks;  // (solid, first tile)
     int total_chunks;
     int chunk_tiles;     // tiles per work item
+    int fast_chunks;     // leading chunks whose shapes classify_kernel may take
+    int any_first;       // first chunk classify_any_kernel looks at
+    int any_grid;        // its CTAs
     uint8_t* cls;      // class byte per bbox cell
     float* alpha;      // solid fraction per bbox cell (cut candidates only)
     Counters* cnt;

@@ -33,6 +33,7 @@
 namespace sdfibm_dev {
 __global__ void plan_kernel(MeshK m, const SolidK* sk, const sdfibm_solid_state* st, SolidPlan* plan, int S,
                             Counters* cnt);
+int classify_kind(int shape_type, bool flat);
 void launch_classify(const ClassifyArgs& A, bool flat, int grid, cudaStream_t st);
 int classify_occupancy(int method, bool flat);
 __global__ void connect_kernel(MeshK m, const SolidK* sk, SolidPlan* plan, const uint8_t* scratch, uint32_t* gbitmaps,
@@ -299,6 +300,10 @@ extern "C" int sdfibm_cuda_touched_noalloc(const sdfibm_mesh_desc* mesh, const s
     ClassifyArgs CA{};
     CA.m = m; CA.sk = d_sk; CA.st = d_st; CA.plan = d_plan; CA.chunks = d_chunks; CA.total_chunks = nchunks; CA.chunk_tiles = CHUNK_TILES;
     CA.cls = b + OFF_CLS; CA.alpha = nullptr; CA.cnt = d_cnt; CA.method = -1; CA.subsample_n = 0;
+    const int kind = classify_kind(solid->shape.type, m.nz <= 2);
+    CA.fast_chunks = kind == 0 ? nchunks : 0;
+    CA.any_first = kind == 0 && m.nz > 2 ? nchunks : 0;
+    CA.any_grid = grid;
     launch_classify(CA, m.nz <= 2, grid, st);
     connect_kernel<<<1, 512, 0, st>>>(m, d_sk, d_plan, b + OFF_CLS, reinterpret_cast<uint32_t*>(b + OFF_BITMAP),
                                       reinterpret_cast<int32_t*>(b + OFF_IN_CELL), reinterpret_cast<int32_t*>(b + OFF_IN_SOLID),

@@ -37,13 +37,20 @@ def _case(name, rng):
     if name == "bitmaps":  # 7, 30 and 90 cells across
         n = (96, 96, 96)
         return n, 0, [(S("Sphere", radius=r), (48.3, 47.9, 48.1), (0, 0, 0)) for r in (2.0, 3.4, 13.0, 25.0, 44.0)]
+    if name in ("flat1", "flat2"):  # one- and two-layer meshes: shapes that turn about z, and tilted ones
+        n = (30, 26, int(name[4]))
+        return n, 0, [(S("Circle", radius=5.2), (14.3, 12.1, 0.4), (0, 0, 20)), (S("Ellipse", radiusa=2.0, radiusb=7.5), (15, 13, 0), (0, 0, 33)),
+                      (S("Rectangle", radiusa=6.0, radiusb=1.5), (15, 13, 0), (0, 0, 45)), (S("Circle", radius=1.1), (3, 3, 0), (0, 0, 0)),
+                      (S("Plane"), (15, 13, 0), (0, 0, 37)), (S("Plane"), (15, 26, 0), (0, 0, 180)), (S("Plane"), (0, 13, 0), (0, 0, -90)),
+                      (S("Circle", radius=4.0), (15, 13, 0.5), (10, 5, 0)), (S("Sphere", radius=4.0), (15, 13, 0.5), (0, 0, 0)),
+                      (S("Plane"), (15, 13, 0.7), (60, 20, 10))]
     n = (60, 50, 1)  # "concave": 2-D tails, and one circle of a cell
     return n, 1, [(S("Circle_Tail", radius=4.0, ratio=3.0, thickness=0.4), (20, 20, 0), (0, 0, 25)),
                   (S("Circle_TwoTail", radius=4.0, ratio=3.0, thickness=0.8), (35, 30, 0), (0, 0, 70)),
                   (S("Rectangle", radiusa=15.0, radiusb=0.3), (30, 25, 0), (0, 0, 13)), (S("Circle", radius=0.8), (50, 8, 0), (0, 0, 0))]
 
 
-@pytest.mark.parametrize("name", ["plates", "rows", "planes", "boundary", "bitmaps", "concave"])
+@pytest.mark.parametrize("name", ["plates", "rows", "planes", "boundary", "bitmaps", "concave", "flat1", "flat2"])
 def test_touched_sets_match_the_oracle(cuda_lib, torch_cuda, name):
     rng = np.random.default_rng(len(name))
     n, twod, shapes = _case(name, rng)
