@@ -43,10 +43,12 @@ __global__ void connect_small_kernel(MeshK m, const SolidK* sk, SolidPlan* plan,
                                      int64_t cap_in, int64_t cap_cut, Counters* cnt, const int32_t* solids,
                                      int nsolids);
 
-__global__ void couple_shared_kernel(CoupleArgs A);
+void launch_couple_shared(const CoupleArgs& A, bool exact, int grid, cudaStream_t st);
 __global__ void shared_scan_kernel(const int32_t* in_cell, const int32_t* cut_cell, const int32_t* Ct, Counters* cnt,
                                    int64_t N, const uint32_t* sbits, uint32_t* shent, int64_t shent_cap);
-__global__ void couple_chunks_kernel(CoupleArgs A);
+void launch_couple_chunks(const CoupleArgs& A, bool exact, int grid, cudaStream_t st);
+int couple_occupancy(bool exact);
+__global__ void centres_kernel(MeshK m, double* out);
 __global__ void apply_forcing_kernel(int64_t N, const uint32_t* cbits, double dt, const float* As, const float* Fs,
                                      const float* Ts, float* U, float* T);
 __global__ void finalize_kernel(float* As, float* Ts, float* Fs, int32_t* Ct, const Counters* cnt, int64_t N,
@@ -142,6 +144,7 @@ struct sdfibm_ctx {
     uint32_t* d_gbitmaps = nullptr;
     // chunked coupling: one bit per 8-cell chunk holding a claimed cell / a cell claimed twice (cleared as used)
     uint32_t *d_cbits = nullptr, *d_sbits = nullptr;
+    double* d_centres = nullptr;  // FP64 cell centres per axis
     uint32_t* d_shent = nullptr;  // list entries on shared cells, compacted by shared_scan_kernel
     int64_t shent_cap = 0;
     int64_t gbitmap_words = 0;
@@ -635,6 +638,7 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
         dalloc(&ctx->d_sh_used, (size_t)ctx->sh_mask + 1) || dalloc(&ctx->d_step, 2) ||
         dalloc(&ctx->d_cbits, (size_t)(ctx->mesh.ncells + 255) / 256) ||
         dalloc(&ctx->d_sbits, (size_t)(ctx->mesh.ncells + 255) / 256) || dalloc(&ctx->d_shent, (size_t)ctx->shent_cap) ||
+        dalloc(&ctx->d_centres, (size_t)mesh->nx + mesh->ny + mesh->nz) ||
         dalloc(&ctx->d_small, small_solids.size()) || dalloc(&ctx->d_big, big_solids.size()) ||
         dalloc(&ctx->d_rq, (size_t)ctx->rq_cap) || dalloc(&ctx->d_ovf, (size_t)ctx->ovf_cap) ||
         (cell_list &&
@@ -699,12 +703,17 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
             return bail(SDFIBM_ERR_CUDA);
         }
     }
+    centres_kernel<<<32, 256>>>(c->mesh, c->d_centres);
+    if (cudaDeviceSynchronize() != cudaSuccess) {
+        ctx->err = "set-up kernel failed";
+        return bail(SDFIBM_ERR_CUDA);
+    }
     int occ = 0;
     occ = classify_occupancy(ctx->opt.fraction_method, mesh->nz <= 2);
     ctx->classify_grid = std::max(1, occ) * ctx->num_sms;
     ctx->classify_occ = std::max(1, occ);
     occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, couple_chunks_kernel, 256, 0);
+    occ = couple_occupancy(ctx->opt.exact_forcing != 0);
     ctx->couple_grid = std::max(1, occ) * ctx->num_sms;
     ctx->couple_occ = std::max(1, occ);
     ctx->subsample_grid = 8 * ctx->num_sms;
@@ -904,10 +913,9 @@ static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float
         CoupleArgs A{};
         A.m = ctx->mesh; A.sk = ctx->d_sk; A.st = ctx->d_st; A.plan = ctx->d_plan;
         A.in_cell = ctx->in_cell(); A.in_solid = ctx->in_solid(); A.cut_cell = ctx->cut_cell();
-        A.cut_solid = ctx->cut_solid(); A.alpha = ctx->d_alpha; A.U = U; A.As = As; A.Fs = Fs; A.Ts = Ts; A.Ct = Ct;
+        A.cut_solid = ctx->cut_solid(); A.alpha = ctx->d_alpha; A.centres = ctx->d_centres; A.U = U; A.As = As; A.Fs = Fs; A.Ts = Ts; A.Ct = Ct;
         A.ftacc = ctx->d_ftacc; A.cnt = ctx->d_cnt; A.step = ctx->d_step;
         A.method = ctx->opt.fraction_method; A.subsample_n = ctx->opt.subsample_n;
-        A.exact_forcing = ctx->opt.exact_forcing;
         {
             const int nc = ctx->opt.fraction_method == SDFIBM_FRACTION_LEARNED
                                ? (ctx->opt.learned_fallback_n > 0 ? ctx->opt.learned_fallback_n : 16)
@@ -917,9 +925,9 @@ static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float
         A.sh_keys = ctx->d_sh_keys; A.sh_vals = ctx->d_sh_vals; A.sh_used = ctx->d_sh_used; A.sh_mask = ctx->sh_mask;
         A.cbits = ctx->d_cbits; A.sbits = ctx->d_sbits; A.shent = ctx->d_shent; A.shent_cap = ctx->shent_cap;
         // the compacted entries on shared cells (their FP64 sums), then every cell of the marked chunks
-        couple_shared_kernel<<<ctx->num_sms, 256, 0, st>>>(A);
+        launch_couple_shared(A, ctx->opt.exact_forcing != 0, ctx->num_sms, st);
         mark(ctx, "couple_shared_kernel");
-        couple_chunks_kernel<<<ctx->couple_grid, 256, 0, st>>>(A);
+        launch_couple_chunks(A, ctx->opt.exact_forcing != 0, ctx->couple_grid, st);
         mark(ctx, "couple_chunks_kernel");
         finalize_kernel<<<ctx->num_sms, 256, 0, st>>>(As, Ts, Fs, Ct, ctx->d_cnt, N, ctx->d_sh_keys, ctx->d_sh_vals,
                                                        ctx->d_sh_used, ctx->sh_mask);
@@ -1700,6 +1708,7 @@ void sdfibm_cuda_destroy(sdfibm_ctx* ctx) {
     if (ctx->d_cbits) cudaFree(ctx->d_cbits);
     if (ctx->d_sbits) cudaFree(ctx->d_sbits);
     if (ctx->d_shent) cudaFree(ctx->d_shent);
+    if (ctx->d_centres) cudaFree(ctx->d_centres);
     if (ctx->d_f64) cudaFree(ctx->d_f64);
     for (void* p : {(void*)ctx->evw.x, (void*)ctx->evw.rec, (void*)ctx->evw.key, (void*)ctx->evw.pn, (void*)ctx->evw.pq,
                     (void*)ctx->evw.list, (void*)ctx->evw.hot, (void*)ctx->evw.ctrl})

@@ -1079,14 +1079,15 @@ __device__ __forceinline__ void classify_any(const ClassifyArgs& A, const int2 c
 // meshes circles, ellipses, rectangles and half spaces that turn about z.  One error bound covers every vertex of the solid's bounding box,
 // so a vertex costs a few multiply-adds and two comparisons; a tile's answers are ballots, and cells are read off them with
 // shifts.  Tiles are culled 32 at a time, a lane each.  Bound by instruction issue.  Measured against a test per vertex with
-// its own bound (GB300, 512^3, 16 384 solids): LEARNED 1.13 -> 0.50 ms, REF-GEO (half of it now the vertex distances)
-// 1.63 -> 1.02 ms.
+// its own bound (GB300, 512^3, 16 384 solids): LEARNED 1.13 -> 0.43 ms, REF-GEO (half of it now the vertex distances)
+// 1.63 -> 0.92 ms.
 //
 // The bound.  A local coordinate is M (b + v h) + com from FP32 roundings of the base b (bbox corner minus centre), M, h and
 // com, added in a chain of at most 12 roundings of partial sums no larger than A = max|M| (|b|_1 + sum_a ext_a h_a) + |com|_1:
 // 16 u A, plus the FP64 reference's own rounding e64, holds its error (E).  For the inside function the bounds are those of
 // the sampling kernels (SampleFrame::Eg, and 64 units of roundoff of the magnitudes where a column's polynomial is used), with
-// the largest coordinates of the whole box.  Values within the bound go to the FP64 test, so the classes are the reference's.
+// the largest coordinates of the whole box.  Values within the bound go to the point's own bound and then to the FP64 test,
+// so the classes are the reference's.
 struct FastFrame {
     float px, py, pz;  // local coordinates of the bbox corner (com added)
     float sxx, sxy, sxz, syx, syy, syz, szx, szy, szz;  // local images of the cell edges
@@ -1152,10 +1153,21 @@ __device__ __forceinline__ float fast_g(const FastFrame& f, float X, float Y, fl
     if (f.half_space) return Y;
     return fmaxf(fmaxf(fabsf(X) - f.k0, fabsf(Y) - f.k1), fabsf(Z) - f.k2);
 }
-// the FP64 answer for a value the bound does not decide
-static __device__ __noinline__ bool fast_exact(const MeshK& m, const SolidK& k, const sdfibm_solid_state& st, int I, int J,
-                                               int K, int centre) {
-    return exact_inside_point(k.shape, m, I, J, K, centre, state_pos(st), state_quat(st)) != 0;
+// the answer for a value the box's bound does not decide: the point's own bound (a few times tighter), then FP64
+static __device__ __noinline__ bool fast_exact(const MeshK& m, const SolidK& k, const SolidPlan& pl,
+                                               const sdfibm_solid_state& st, int I, int J, int K, int centre,
+                                               unsigned& rechecks) {
+    const float half = centre ? 0.5f : 0.f;
+    TileFrame tf;
+    tf.bx = pl.base32[0]; tf.by = pl.base32[1]; tf.bz = pl.base32[2];
+    tf.babs = fabsf(tf.bx) + fabsf(tf.by) + fabsf(tf.bz);
+    tf.e64 = pl.e64;
+    unsigned long long n = 0;
+    const int in = classify_point(k.shape, pl.M, tf, ((float)(I - pl.lo[0]) + half) * m.h32[0],
+                                  ((float)(J - pl.lo[1]) + half) * m.h32[1], ((float)(K - pl.lo[2]) + half) * m.h32[2], m, I, J,
+                                  K, centre, state_pos(st), state_quat(st), &n);
+    rechecks += (unsigned)n;
+    return in != 0;
 }
 
 // vertex distances of a tile for REF-GEO (see classify_any): u-th needed vertex v = (a, b, c) of the tile at (x0, y0, z0)
@@ -1281,10 +1293,8 @@ __device__ __forceinline__ void classify_fast(const ClassifyArgs& A, const int2 
                     const float g = fast_g(f, __fmaf_rn(fva, f.sxx, __fmaf_rn(fb, f.syx, Lx)),
                                            __fmaf_rn(fva, f.sxy, __fmaf_rn(fb, f.syy, Ly)), Lz);
                     bool in = g < -f.Eg;
-                    if (lane < 27 && !in && !(g > f.Eg)) {
-                        ++rechecks;
-                        in = fast_exact(m, k, st, I0 + va, J0 + vb + 3 * l, K0, 0);
-                    }
+                    if (lane < 27 && !in && !(g > f.Eg))
+                        in = fast_exact(m, k, pl, st, I0 + va, J0 + vb + 3 * l, K0, 0, rechecks);
                     bits[l] = __ballot_sync(FULL, in) & 0x7ffffffu;
                 }
             } else {
@@ -1305,10 +1315,8 @@ __device__ __forceinline__ void classify_fast(const ClassifyArgs& A, const int2 
                     if (f.quadric) g = __fmaf_rn(__fmaf_rn(f.A2, c, B2), c, C0);
                     else g = fast_g(f, __fmaf_rn(c, f.szx, wx), __fmaf_rn(c, f.szy, wy), __fmaf_rn(c, f.szz, wz));
                     bool in = g < -f.Eg;
-                    if (lane < 25 && !in && !(g > f.Eg)) {
-                        ++rechecks;
-                        in = fast_exact(m, k, st, I0 + va, J0 + vb, K0 + l, 0);
-                    }
+                    if (lane < 25 && !in && !(g > f.Eg))
+                        in = fast_exact(m, k, pl, st, I0 + va, J0 + vb, K0 + l, 0, rechecks);
                     bits[l] = __ballot_sync(FULL, in) & 0x1ffffffu;
                 }
             }
@@ -1366,10 +1374,7 @@ __device__ __forceinline__ void classify_fast(const ClassifyArgs& A, const int2 
                                                __fmaf_rn(fa, f.sxy, __fmaf_rn(fb, f.syy, __fmaf_rn(fc, f.szy, Ly))),
                                                __fmaf_rn(fa, f.sxz, __fmaf_rn(fb, f.syz, __fmaf_rn(fc, f.szz, Lz))));
                         bool in = g < -f.Eg;
-                        if (!in && !(g > f.Eg)) {
-                            ++rechecks;
-                            in = fast_exact(m, k, st, I0 + ca, J0 + b, K0 + c, 1);
-                        }
+                        if (!in && !(g > f.Eg)) in = fast_exact(m, k, pl, st, I0 + ca, J0 + b, K0 + c, 1, rechecks);
                         cls[p] = in ? 2 : 3;
                     }
                     ncut += __popc(cut_b[p]);

@@ -700,6 +700,7 @@ __device__ __forceinline__ float ff_u_minus_us(float U, float u0h, float u0l, fl
 // Per-cell forcing of solid s on cell c with fluid velocity U (pcHydrodynamicInteraction, solidcloud.cpp:384-390):
 // alpha, the FP32 Fs and the cell's contributions to the force/torque sums (:411-421), FP64 in f6 (exact mode) or
 // FP32 in g6.
+template <bool EXACT>
 __device__ __forceinline__ float cell_forcing(const CoupleArgs& A, int64_t c, int s, int type, float dtINV32,
                                               double dtINV, float fs[3], double f6[8], float g6[8], float Ux,
                                               float Uy, float Uz) {
@@ -716,11 +717,12 @@ __device__ __forceinline__ float cell_forcing(const CoupleArgs& A, int64_t c, in
         // a SUBSAMPLE count whose undecided points were rechecked on full warps
         if (alpha < 0.f) alpha = __fdiv_rn(-alpha - 1.f, (float)A.count_samples);
     }
-    if (A.exact_forcing) {
+    if (EXACT) {
         // the reference's FP64 sequence
         const sdfibm_solid_state& st = A.st[s];
         const D3 x = state_pos(st);
-        const D3 cc = mesh_C(m, i, j, k);
+        // mesh_C from its per-axis tables: the FP64 pipe also converts the indices, twelve of its instructions a cell
+        const D3 cc{A.centres[i], A.centres[m.nx + j], A.centres[m.nx + m.ny + k]};
         const D3 vel{st.vel[0], st.vel[1], st.vel[2]}, om{st.omega[0], st.omega[1], st.omega[2]};
         const D3 uf{(double)Ux, (double)Uy, (double)Uz};
         const D3 us = vel + cross(om, cc - x);
@@ -786,6 +788,7 @@ __global__ void shared_scan_kernel(const int32_t* __restrict__ in_cell, const in
 // Shared pass, second half (after the fraction kernels): every compacted entry adds its solid's As / Ts / Fs to the
 // cell's FP64 sums in the shared table (finalize_kernel writes them) and its force/torque contribution to the solid's
 // sums.
+template <bool EXACT>
 __global__ void __launch_bounds__(CPL_THREADS) couple_shared_kernel(CoupleArgs A) {
     const int64_t N = A.m.ncells;
     const int64_t n = min((int64_t)A.cnt->n_shent, A.shent_cap);
@@ -802,16 +805,20 @@ __global__ void __launch_bounds__(CPL_THREADS) couple_shared_kernel(CoupleArgs A
         double f6[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         float g6[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         float fs[3];
-        const float alpha = cell_forcing(A, c, s, list_type(sw), dtINV32, dtINV, fs, f6, g6, A.U[c], A.U[N + c],
-                                         A.U[2 * N + c]);
+        const float alpha = cell_forcing<EXACT>(A, c, s, list_type(sw), dtINV32, dtINV, fs, f6, g6, A.U[c],
+                                                A.U[N + c], A.U[2 * N + c]);
         add_shared(A, c, alpha, fs);
-        for (int r = 0; r < 6; ++r) atomicAdd(A.ftacc + 6 * s + r, A.exact_forcing ? f6[r] : (double)g6[r]);
+        for (int r = 0; r < 6; ++r) atomicAdd(A.ftacc + 6 * s + r, EXACT ? f6[r] : (double)g6[r]);
     }
+}
+void launch_couple_shared(const CoupleArgs& A, bool exact, int grid, cudaStream_t st) {
+    if (exact) couple_shared_kernel<true><<<grid, CPL_THREADS, 0, st>>>(A);
+    else couple_shared_kernel<false><<<grid, CPL_THREADS, 0, st>>>(A);
 }
 
 // Chunked coupling.  The claim pass marks in cbits every chunk of 8 consecutive cells that holds a claimed cell (and
-// in sbits the chunks of cells claimed more than once).  This kernel runs over the marked chunks in memory order, a
-// warp per bitmap word (256 cells), four chunks at a time with 8 lanes each, and writes the four fields of every
+// in sbits the chunks of cells claimed more than once).  This kernel runs over the marked chunks, a warp per 64 bits of the bitmap
+// (in the order given below), four chunks at a time with 8 lanes each, and writes the four fields of every
 // cell of a marked chunk: zero for an unclaimed cell (a cell that no solid touches, or one the previous call touched:
 // the sparse reset inside these chunks), zero As / Ts / Fs and the claim word kept in Ct for a shared cell
 // (finalize_kernel writes its sums and decodes its Ct), and for a cell claimed once the forcing of its solid.  The
@@ -824,6 +831,7 @@ __global__ void __launch_bounds__(CPL_THREADS) couple_shared_kernel(CoupleArgs A
 constexpr int CPL_WARPS = CPL_THREADS / 32;
 
 // forcing of the first `count` queued cells (lane l takes entry l), written to the fields, F/T summed per solid
+template <bool EXACT>
 __device__ __forceinline__ void couple_queued(const CoupleArgs& A, const int32_t* qc, const uint32_t* qk, int count,
                                               float dtINV32, double dtINV) {
     const int lane = threadIdx.x & 31;
@@ -837,8 +845,8 @@ __device__ __forceinline__ void couple_queued(const CoupleArgs& A, const int32_t
         s = (int)(key >> 2);
         const int type = (int)(key & 3u);
         float fs[3];
-        const float alpha = cell_forcing(A, c, s, type, dtINV32, dtINV, fs, f6, g6, A.U[c], A.U[N + c],
-                                         A.U[2 * N + c]);
+        const float alpha = cell_forcing<EXACT>(A, c, s, type, dtINV32, dtINV, fs, f6, g6, A.U[c], A.U[N + c],
+                                                A.U[2 * N + c]);
         A.As[c] = fminf(alpha, 1.0f);
         A.Ts[c] = alpha;
         A.Fs[c] = fs[0];
@@ -852,7 +860,7 @@ __device__ __forceinline__ void couple_queued(const CoupleArgs& A, const int32_t
         const bool mine = s == sl;
         pend &= ~__ballot_sync(0xffffffffu, mine);
         double v;
-        if (A.exact_forcing) {
+        if (EXACT) {
             double t[8];
 #pragma unroll
             for (int r = 0; r < 8; ++r) t[r] = mine ? f6[r] : 0.0;
@@ -868,42 +876,71 @@ __device__ __forceinline__ void couple_queued(const CoupleArgs& A, const int32_t
     }
 }
 
+// Order of the marked chunks.  Memory order for the FP32 forcing, whose time goes to memory latency.  The FP64 forcing is
+// bound by the FP64 pipe (1/64 of the FP32 rate), where every distinct solid of a batch costs a reduction of nine additions:
+// there an item is 64 consecutive cells (a byte of the bitmap) on each of 8 rows, whose distance is the row length in whole
+// bytes, its chunks taken column by column, so that a batch of 32 queued cells covers about 8 x 8 cells of one or two solids
+// instead of a row's five (the mesh rows need not be multiples of 64 cells: any partition of the bytes gives the same fields).
+// Measured (GB300): FP64 at 256^3 and 4096 solids, 2.2 M cells, 0.51 -> 0.34 ms (0.37 and 0.35 with 2 and 4 rows, 0.46 in
+// memory order); FP32 at 512^3, 10.5 M cells, 0.56 ms in memory order and 0.62 with 4 rows.
+template <bool EXACT>
 __global__ void __launch_bounds__(CPL_THREADS) couple_chunks_kernel(CoupleArgs A) {
     __shared__ int32_t s_qc[CPL_WARPS][64];   // per warp: queued cells claimed once, and their claim words
     __shared__ uint32_t s_qk[CPL_WARPS][64];
+    const unsigned FULL = 0xffffffffu;
     const int64_t N = A.m.ncells;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, grp = lane >> 3, sub = lane & 7;
     int32_t* qc = s_qc[wib];
     uint32_t* qk = s_qk[wib];
-    const int64_t words = (N + 255) >> 8;
+    const int64_t nbytes = (N + 63) >> 6;
+    const int rs = max(1, (A.m.nx + 32) >> 6);  // row length in bytes
+    const int64_t items = EXACT ? (nbytes + 8 * rs - 1) / (8 * rs) * rs : (nbytes + 7) >> 3;
     const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
     const double dtINV = A.step->dtINV;
     const float dtINV32 = (float)dtINV;
     const uint32_t* C = reinterpret_cast<const uint32_t*>(A.Ct);
+    const uint8_t* marks = reinterpret_cast<const uint8_t*>(A.cbits);
     int nq = 0;  // warp-uniform
-    for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < words; w += nw) {
-        uint32_t rem = A.cbits[w];
-        while (rem) {  // warp-uniform: four marked chunks per pass
-            uint32_t x = rem;
-            for (int q = 0; q < grp; ++q) x &= x - 1;  // this group's chunk: the grp-th lowest mark left
+    for (int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < items; t += nw) {
+        int64_t b0;        // first byte
+        uint64_t rem = 0;  // EXACT: bit 8 chunk + row; else bit = chunk
+        if (EXACT) {
+            const int64_t blk = t / rs;
+            b0 = blk * 8 * rs + (t - blk * rs);
+            unsigned byte = 0;
+            if (lane < 8 && b0 + (int64_t)lane * rs < nbytes) byte = marks[b0 + (int64_t)lane * rs];
+            if (!__any_sync(FULL, byte != 0)) continue;
+#pragma unroll
+            for (int bit = 0; bit < 8; ++bit) rem |= (uint64_t)__ballot_sync(FULL, (byte >> bit) & 1u) << (8 * bit);
+        } else {
+            b0 = t * 8;
+            rem = A.cbits[2 * t];
+            if (b0 + 4 < nbytes) rem |= (uint64_t)A.cbits[2 * t + 1] << 32;
+        }
+        auto cell_of = [&](uint64_t left) {  // this lane's cell of the next four chunks of `left`, -1: none
+            for (int q = 0; q < grp; ++q) left &= left - 1;
+            const int at = __ffsll((long long)left) - 1;
+            if (at < 0) return (int64_t)-1;
+            const int64_t c = EXACT ? ((b0 + (int64_t)(at & 7) * rs) << 6) + (at & ~7) + sub : (b0 << 6) + (at << 3) + sub;
+            return c < N ? c : (int64_t)-1;
+        };
+        int64_t c = cell_of(rem);
+        uint32_t claim = c >= 0 ? C[c] : 0u;
+        while (rem) {  // warp-uniform: four marked chunks per pass, the claims of the next pass loaded ahead
 #pragma unroll
             for (int q = 0; q < 4; ++q) rem &= rem - 1;
-            const int64_t c = (((w << 5) + (__ffs(x) - 1)) << 3) + sub;
-            bool single = false;
-            uint32_t claim = 0;
-            if (x != 0 && c < N) {
-                claim = C[c];
-                single = claim >= CT_KEY_BASE && !(claim & CT_SHARED);
-                if (!single) {
-                    A.As[c] = 0.f;
-                    A.Ts[c] = 0.f;
-                    A.Fs[c] = 0.f;
-                    A.Fs[N + c] = 0.f;
-                    A.Fs[2 * N + c] = 0.f;
-                    A.Ct[c] = (claim & CT_SHARED) ? (int32_t)claim : 0;
-                }
+            const int64_t c_next = cell_of(rem);
+            const uint32_t claim_next = c_next >= 0 ? C[c_next] : 0u;
+            const bool single = claim >= CT_KEY_BASE && !(claim & CT_SHARED);
+            if (c >= 0 && !single) {
+                A.As[c] = 0.f;
+                A.Ts[c] = 0.f;
+                A.Fs[c] = 0.f;
+                A.Fs[N + c] = 0.f;
+                A.Fs[2 * N + c] = 0.f;
+                A.Ct[c] = (claim & CT_SHARED) ? (int32_t)claim : 0;
             }
-            const uint32_t m = __ballot_sync(0xffffffffu, single);
+            const uint32_t m = __ballot_sync(FULL, single);
             if (single) {
                 const int pos = nq + __popc(m & ((1u << lane) - 1u));
                 qc[pos] = (int32_t)c;
@@ -912,7 +949,7 @@ __global__ void __launch_bounds__(CPL_THREADS) couple_chunks_kernel(CoupleArgs A
             nq += __popc(m);
             __syncwarp();
             if (nq >= 32) {
-                couple_queued(A, qc, qk, 32, dtINV32, dtINV);
+                couple_queued<EXACT>(A, qc, qk, 32, dtINV32, dtINV);
                 __syncwarp();
                 if (lane < nq - 32) {
                     qc[lane] = qc[32 + lane];
@@ -921,9 +958,29 @@ __global__ void __launch_bounds__(CPL_THREADS) couple_chunks_kernel(CoupleArgs A
                 nq -= 32;
                 __syncwarp();
             }
+            c = c_next;
+            claim = claim_next;
         }
     }
-    if (nq > 0) couple_queued(A, qc, qk, nq, dtINV32, dtINV);
+    if (nq > 0) couple_queued<EXACT>(A, qc, qk, nq, dtINV32, dtINV);
+}
+void launch_couple_chunks(const CoupleArgs& A, bool exact, int grid, cudaStream_t st) {
+    if (exact) couple_chunks_kernel<true><<<grid, CPL_THREADS, 0, st>>>(A);
+    else couple_chunks_kernel<false><<<grid, CPL_THREADS, 0, st>>>(A);
+}
+int couple_occupancy(bool exact) {  // resident CTAs per SM
+    int occ = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &occ, exact ? (const void*)couple_chunks_kernel<true> : (const void*)couple_chunks_kernel<false>, CPL_THREADS, 0);
+    return occ;
+}
+
+// FP64 cell centres per axis, x then y then z (mesh_C), once per context
+__global__ void centres_kernel(MeshK m, double* __restrict__ out) {
+    const int64_t n = (int64_t)m.nx + m.ny + m.nz;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = i < m.nx ? mesh_centre(m, 0, i)
+                          : (i < (int64_t)m.nx + m.ny ? mesh_centre(m, 1, i - m.nx) : mesh_centre(m, 2, i - m.nx - m.ny));
 }
 
 // Forcing applied to a GPU-resident fluid (main.cpp:70-77, its cell fields): U = U - Fs dt and T = (1 - As) T + Ts,

@@ -153,6 +153,7 @@ struct CoupleArgs {
     const int32_t* cut_cell;
     const int32_t* cut_solid;
     const float* alpha;  // per bbox cell, from the classify pass
+    const double* centres;  // per-axis FP64 cell centres, x then y then z
     const float* U;
     float* As;
     float* Fs;
@@ -164,7 +165,6 @@ struct CoupleArgs {
     int count_samples;   // a negative alpha is -(1 + inside count) out of this many SUBSAMPLE points
     int method;
     int subsample_n;
-    int exact_forcing;
     // FP64 accumulation of the cells shared by several solids (open addressing, key -1 = empty)
     int32_t* sh_keys;
     double* sh_vals;   // [slot][5]: As, Ts, Fs.x, Fs.y, Fs.z
