@@ -21,8 +21,7 @@
 
 namespace sdfibm_dev {
 // coupling.cu
-__global__ void plan_kernel(MeshK m, const SolidK* sk, const sdfibm_solid_state* st, SolidPlan* plan, int S,
-                            Counters* cnt);
+__global__ void plan_kernel(PrepArgs A);
 void launch_classify(const ClassifyArgs& A, bool flat, int grid, cudaStream_t st);
 int classify_occupancy(int method, bool flat);
 int classify_kind(int shape_type, bool flat);
@@ -43,22 +42,23 @@ __global__ void connect_small_kernel(MeshK m, const SolidK* sk, SolidPlan* plan,
                                      int64_t cap_in, int64_t cap_cut, Counters* cnt, const int32_t* solids,
                                      int nsolids);
 
-void launch_couple_shared(const CoupleArgs& A, bool exact, int grid, cudaStream_t st);
-__global__ void shared_scan_kernel(const int32_t* in_cell, const int32_t* cut_cell, const int32_t* Ct, Counters* cnt,
-                                   int64_t N, const uint32_t* sbits, uint32_t* shent, int64_t shent_cap);
+__global__ void scan_reset_kernel(const int32_t* in_cell, const int32_t* cut_cell, Counters* cnt, int64_t N,
+                                  const uint32_t* sbits, uint32_t* shent, int64_t shent_cap, const int32_t* prev_in_cell,
+                                  const int32_t* prev_cut_cell, float* As, float* Fs, float* Ts, int32_t* Ct,
+                                  const uint32_t* cbits);
 void launch_couple_chunks(const CoupleArgs& A, bool exact, int grid, cudaStream_t st);
 int couple_occupancy(bool exact);
 __global__ void centres_kernel(MeshK m, double* out);
 __global__ void apply_forcing_kernel(int64_t N, const uint32_t* cbits, double dt, const float* As, const float* Fs,
                                      const float* Ts, float* U, float* T);
 __global__ void finalize_kernel(float* As, float* Ts, float* Fs, int32_t* Ct, const Counters* cnt, int64_t N,
-                                int32_t* sh_keys, double* sh_vals, const int32_t* sh_used, int32_t sh_mask);
-__global__ void begin_kernel(Counters* cnt);
+                                int32_t* sh_keys, double* sh_vals, const int32_t* sh_used, int32_t sh_mask,
+                                const double* ftacc, double* ft, int S, const StepParams* step, sdfibm_solid_state* st);
+__global__ void export_ft_kernel(const double* ft, int64_t n, const Counters* cnt, double* h_ft, Counters* h_cnt);
 __global__ void claim_kernel(const int32_t* in_cell, const int32_t* in_solid, const int32_t* cut_cell,
                              const int32_t* cut_solid, int32_t* Ct, Counters* cnt, int64_t N, uint32_t* cbits,
                              uint32_t* sbits);
-__global__ void ft_kernel(const double* ftacc, double* ft, int S, const StepParams* step);
-__global__ void set_step_kernel(StepParams* p, double time, double dt, int nsub, double rho_V, EvolveCtrl* ctrl);
+__global__ void set_step_kernel(StepParams* p, StepParams v, EvolveCtrl* ctrl);
 int export_chunk_cells();
 __global__ void mark_export_kernel(const int32_t* in_cell, const int32_t* cut_cell, const int32_t* prev_in_cell,
                                    const int32_t* prev_cut_cell, const Counters* cnt, int64_t N, uint32_t* dirty);
@@ -73,14 +73,12 @@ __global__ void export64_kernel(Counters* cnt, int64_t N, uint32_t* dirty, const
 __global__ void u64_to_planes_kernel(const double* U64, int64_t N, float* U);
 __global__ void fields_to_f64_kernel(int64_t N, const float* As, const float* Fs, const float* Ts, const int32_t* Ct,
                                      double* out);
-__global__ void reset_kernel(const int32_t* in_cell, const int32_t* cut_cell, const Counters* cnt, int64_t N,
-                             float* As, float* Fs, float* Ts, int32_t* Ct, const uint32_t* cbits);
 __global__ void fix_internal_kernel(MeshK m, const sdfibm_solid_state* st, const int32_t* in_cell,
                                     const int32_t* in_solid, const int32_t* Ct, float* U, const Counters* cnt);
 // evolve.cu
 
 __global__ void evolve_independent_kernel(const SolidK* sk, sdfibm_solid_state* st, int S, int nsub,
-                                          const StepParams* step, double rho_f, D3 g);
+                                          StepParams step, double rho_f, D3 g);
 __global__ void evolve_pre_kernel(const SolidK* sk, sdfibm_solid_state* st, int S, const StepParams* step, double rho_f, D3 g,
                                   GridK gk, int64_t* hashes, int32_t* counts, FineGridK fg, int32_t* fcounts, int mode,
                                   int coarse_needed, CollRec* recs, int move_first);
@@ -102,22 +100,9 @@ int evolve_contacts_list();
 int evolve_contacts_hot();
 __global__ void move_kernel(const SolidK* sk, sdfibm_solid_state* st, int S, const StepParams* step);
 __global__ void store_old_kernel(sdfibm_solid_state* st, int S);
-__global__ void ft_to_state_kernel(const double* ft, sdfibm_solid_state* st, int S);
 }  // namespace sdfibm_dev
 
 using namespace sdfibm_dev;
-
-// copies this call's fluid force and torque into the solid state (Solid::setFluidForceAndTorque)
-namespace sdfibm_dev {
-__global__ void ft_to_state_kernel(const double* ft, sdfibm_solid_state* st, int S) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    for (int a = 0; a < 3; ++a) {
-        st[s].fluid_force[a] = ft[6 * s + a];
-        st[s].fluid_torque[a] = ft[6 * s + 3 + a];
-    }
-}
-}  // namespace sdfibm_dev
 
 struct sdfibm_ctx {
     cudaStream_t stream = nullptr;
@@ -145,7 +130,7 @@ struct sdfibm_ctx {
     // chunked coupling: one bit per 8-cell chunk holding a claimed cell / a cell claimed twice (cleared as used)
     uint32_t *d_cbits = nullptr, *d_sbits = nullptr;
     double* d_centres = nullptr;  // FP64 cell centres per axis
-    uint32_t* d_shent = nullptr;  // list entries on shared cells, compacted by shared_scan_kernel
+    uint32_t* d_shent = nullptr;  // list entries on shared cells, compacted by scan_reset_kernel
     int64_t shent_cap = 0;
     int64_t gbitmap_words = 0;
     int connect_smem_bytes = 0;
@@ -747,16 +732,42 @@ static int sync_counters(sdfibm_ctx* ctx) {
     return check_device_error(ctx);
 }
 
+// the last interact's forces (into h_ft) and counters, on the host
+static int sync_forces(sdfibm_ctx* ctx) {
+    const int64_t n = 6 * (int64_t)ctx->S;
+    export_ft_kernel<<<(unsigned)std::min<int64_t>(ctx->num_sms, n / 256 + 1), 256, 0, ctx->stream>>>(ctx->d_ft, n, ctx->d_cnt,
+                                                                                                   ctx->h_ft, ctx->h_cnt);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(ctx->stream));
+    return check_device_error(ctx);
+}
+
+static PrepArgs prep_args(sdfibm_ctx* ctx, double time, double dt) {
+    PrepArgs a{};
+    a.m = ctx->mesh; a.sk = ctx->d_sk; a.st = ctx->d_st; a.plan = ctx->d_plan; a.S = ctx->S;
+    a.plan_ctas = std::max(1, (ctx->S + 31) / 32);
+    a.cnt = ctx->d_cnt; a.new_call = 1; a.step = ctx->d_step;
+    a.sp = step_params(time, dt, 1, ctx->opt.rho_f * ctx->mesh.V);
+    a.ftacc = ctx->d_ftacc;
+    // chunk marks of this call's claims (they stay after the call for sdfibm_cuda_apply_forcing)
+    a.cbits = ctx->d_cbits; a.sbits = ctx->d_sbits; a.words = (ctx->mesh.ncells + 255) / 256;
+    return a;
+}
+// CTAs of plan_kernel that clear the chunk marks: about 16 words a thread, up to four per SM
+static int clear_ctas(const sdfibm_ctx* ctx) {
+    return (int)std::min<int64_t>(4 * ctx->num_sms, (ctx->mesh.ncells + 255) / 256 / (96 * 16) + 1);
+}
+
 // The device work of one interact on the context's stream: what a captured graph holds.
 static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float* U, float* As, float* Fs, float* Ts,
                             int32_t* Ct, bool dense, int& launches) {
     const int64_t N = ctx->mesh.ncells;
     const int S = ctx->S;
     cudaStream_t st = ctx->stream;
-    set_step_kernel<<<1, 1, 0, st>>>(ctx->d_step, time, dt, 1, ctx->opt.rho_f * ctx->mesh.V, nullptr);
+    const PrepArgs pa = prep_args(ctx, time, dt);
+    plan_kernel<<<pa.plan_ctas + clear_ctas(ctx), 96, 0, st>>>(pa);
     ++launches;
-    begin_kernel<<<1, 1, 0, st>>>(ctx->d_cnt);
-    ++launches;
+    mark(ctx, "plan_kernel");
     if (dense) {
         // SolidCloud::interact zeroes the four fields over the whole mesh (solidcloud.cpp:438-441)
         CK(cudaMemsetAsync(As, 0, sizeof(float) * N, st));
@@ -766,12 +777,6 @@ static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float
         mark(ctx, "dense_reset");
     }
     if (S > 0) {
-        CK(cudaMemsetAsync(ctx->d_ftacc, 0, sizeof(double) * 6 * S, st));
-        // chunk marks of this call's claims (they stay after the call for sdfibm_cuda_apply_forcing)
-        CK(cudaMemsetAsync(ctx->d_cbits, 0, sizeof(uint32_t) * (size_t)((N + 255) / 256), st));
-        CK(cudaMemsetAsync(ctx->d_sbits, 0, sizeof(uint32_t) * (size_t)((N + 255) / 256), st));
-        plan_kernel<<<(S + 127) / 128, 128, 0, st>>>(ctx->mesh, ctx->d_sk, ctx->d_st, ctx->d_plan, S, ctx->d_cnt);
-        mark(ctx, "plan_kernel");
         ClassifyArgs CA{};
         CA.m = ctx->mesh; CA.sk = ctx->d_sk; CA.st = ctx->d_st; CA.plan = ctx->d_plan; CA.chunks = ctx->d_chunks;
         CA.total_chunks = ctx->total_chunks; CA.cls = ctx->d_scratch; CA.alpha = ctx->d_alpha; CA.cnt = ctx->d_cnt;
@@ -822,21 +827,16 @@ static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float
                                                         ctx->cut_solid(), Ct, ctx->d_cnt, N, ctx->d_cbits,
                                                         ctx->d_sbits);
         mark(ctx, "claim_kernel");
-        shared_scan_kernel<<<ctx->num_sms * 8, 256, 0, sb>>>(ctx->in_cell(), ctx->cut_cell(), Ct, ctx->d_cnt, N,
-                                                              ctx->d_sbits, ctx->d_shent, ctx->shent_cap);
-        mark(ctx, "shared_scan_kernel");
-        launches += 5;
+        const int prev = ctx->cur ^ 1;
+        scan_reset_kernel<<<ctx->num_sms * 8, 256, 0, sb>>>(
+            ctx->in_cell(), ctx->cut_cell(), ctx->d_cnt, N, ctx->d_sbits, ctx->d_shent, ctx->shent_cap,
+            dense ? nullptr : ctx->d_lists[prev][0], ctx->d_lists[prev][2], As, Fs, Ts, Ct, ctx->d_cbits);
+        mark(ctx, "scan_reset_kernel");
+        launches += 4;
         if (ctx->u64_dev) {  // interact_host64: U read at the coupling cells from the page-locked FP64 field
             gather_u64_kernel<<<ctx->num_sms * 8, 256, 0, sb>>>(ctx->in_cell(), ctx->cut_cell(), ctx->d_cnt, N,
                                                                  ctx->u64_dev, const_cast<float*>(U));
             mark(ctx, "gather_u64_kernel");
-            ++launches;
-        }
-        if (!dense) {
-            const int p = ctx->cur ^ 1;
-            reset_kernel<<<ctx->num_sms * 4, 256, 0, sb>>>(ctx->d_lists[p][0], ctx->d_lists[p][2], ctx->d_cnt, N, As,
-                                                            Fs, Ts, Ct, ctx->d_cbits);
-            mark(ctx, "reset_kernel");
             ++launches;
         }
         if (refgeo) {
@@ -901,8 +901,9 @@ static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float
         }
     } else if (!dense) {
         const int p = ctx->cur ^ 1;
-        reset_kernel<<<ctx->num_sms * 4, 256, 0, st>>>(ctx->d_lists[p][0], ctx->d_lists[p][2], ctx->d_cnt, N, As, Fs,
-                                                        Ts, Ct, ctx->d_cbits);
+        scan_reset_kernel<<<ctx->num_sms * 4, 256, 0, st>>>(
+            ctx->in_cell(), ctx->cut_cell(), ctx->d_cnt, N, ctx->d_sbits, ctx->d_shent, ctx->shent_cap, ctx->d_lists[p][0],
+            ctx->d_lists[p][2], As, Fs, Ts, Ct, ctx->d_cbits);
         ++launches;
     }
     if (ctx->u_wait) {  // U staged on a copy stream (interact_host)
@@ -925,27 +926,23 @@ static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float
         A.sh_keys = ctx->d_sh_keys; A.sh_vals = ctx->d_sh_vals; A.sh_used = ctx->d_sh_used; A.sh_mask = ctx->sh_mask;
         A.cbits = ctx->d_cbits; A.sbits = ctx->d_sbits; A.shent = ctx->d_shent; A.shent_cap = ctx->shent_cap;
         // the compacted entries on shared cells (their FP64 sums), then every cell of the marked chunks
-        launch_couple_shared(A, ctx->opt.exact_forcing != 0, ctx->num_sms, st);
-        mark(ctx, "couple_shared_kernel");
         launch_couple_chunks(A, ctx->opt.exact_forcing != 0, ctx->couple_grid, st);
         mark(ctx, "couple_chunks_kernel");
         finalize_kernel<<<ctx->num_sms, 256, 0, st>>>(As, Ts, Fs, Ct, ctx->d_cnt, N, ctx->d_sh_keys, ctx->d_sh_vals,
-                                                       ctx->d_sh_used, ctx->sh_mask);
+                                                       ctx->d_sh_used, ctx->sh_mask, ctx->d_ftacc, ctx->d_ft, S, ctx->d_step,
+                                                       ctx->d_st);
         mark(ctx, "finalize_kernel");
-        ft_kernel<<<(S + 127) / 128, 128, 0, st>>>(ctx->d_ftacc, ctx->d_ft, S, ctx->d_step);
-        ft_to_state_kernel<<<(S + 127) / 128, 128, 0, st>>>(ctx->d_ft, ctx->d_st, S);
-        mark(ctx, "ft_kernel");
-        launches += 5;
+        launches += 2;
     }
     CK(cudaGetLastError());
     return SDFIBM_OK;
 }
 
 // Runs `enqueue` as a CUDA graph: captured on first use (or when `key_changed`), then replayed after updating the
-// arguments of its set_step_kernel node.  Returns a status, or -1 when capture is not possible (the caller then
-// launches directly).
+// arguments of the node of kernel `func` (the one that takes the time step).  Returns a status, or -1 when capture is not
+// possible (the caller then launches directly).
 static int run_graph(sdfibm_ctx* ctx, sdfibm_ctx::Graph& g, bool key_changed, const std::function<int()>& enqueue,
-                     StepParams* step, double time, double dt, int nsub, double rho_V, EvolveCtrl* ctrl) {
+                     void* func, void** args) {
     cudaStream_t st = ctx->stream;
     if (!g.valid || key_changed) {
         if (g.valid) {
@@ -973,7 +970,7 @@ static int run_graph(sdfibm_ctx* ctx, sdfibm_ctx::Graph& g, bool key_changed, co
             cudaGraphNodeType t;
             if (cudaGraphNodeGetType(nd, &t) != cudaSuccess || t != cudaGraphNodeTypeKernel) continue;
             cudaKernelNodeParams kp;
-            if (cudaGraphKernelNodeGetParams(nd, &kp) == cudaSuccess && kp.func == (void*)set_step_kernel) {
+            if (cudaGraphKernelNodeGetParams(nd, &kp) == cudaSuccess && kp.func == func) {
                 g.step_node = nd;
                 g.step_params = kp;
                 break;
@@ -988,7 +985,6 @@ static int run_graph(sdfibm_ctx* ctx, sdfibm_ctx::Graph& g, bool key_changed, co
         ctx->graphs_keep.push_back(graph);
         g.valid = true;
     }
-    void* args[6] = {&step, &time, &dt, &nsub, &rho_V, &ctrl};
     cudaKernelNodeParams kp = g.step_params;
     kp.kernelParams = args;
     kp.extra = nullptr;
@@ -1011,7 +1007,6 @@ int sdfibm_cuda_interact(sdfibm_ctx* ctx, double time, double dt, const float* U
     if (!(dt != 0.0)) return fail(ctx, SDFIBM_ERR_ARG, "dt must be nonzero");
     if (ctx->poly) return poly_interact(ctx, time, dt, U, As, Fs, Ts, Ct, FT);
     const int S = ctx->S;
-    cudaStream_t st = ctx->stream;
     int launches = 0;
     mark_begin(ctx);
     const void* f5[5] = {U, As, Fs, Ts, Ct};
@@ -1029,12 +1024,14 @@ int sdfibm_cuda_interact(sdfibm_ctx* ctx, double time, double dt, const float* U
         bool changed = g.cur != ctx->cur || g.dense != (int)dense || g.u64 != ctx->u64_dev;
         for (int i = 0; i < 5; ++i) changed = changed || g.fields[i] != f5[i];
         int counted = 0;
+        PrepArgs pa = prep_args(ctx, time, dt);
+        void* args[] = {&pa};
         rc = run_graph(ctx, g, changed,
                        [&] {
                            counted = 0;
                            return enqueue_interact(ctx, time, dt, U, As, Fs, Ts, Ct, dense, counted);
                        },
-                       ctx->d_step, time, dt, 1, ctx->opt.rho_f * ctx->mesh.V, nullptr);
+                       (void*)plan_kernel, args);
         if (rc == -1) {
             ctx->graphs_failed = true;
         } else {
@@ -1051,8 +1048,7 @@ int sdfibm_cuda_interact(sdfibm_ctx* ctx, double time, double dt, const float* U
     ctx->launches_last = launches;
     ctx->interacted = true;
     if (FT) {
-        if (S > 0) CK(cudaMemcpyAsync(ctx->h_ft, ctx->d_ft, sizeof(double) * 6 * S, cudaMemcpyDeviceToHost, st));
-        const int rs = sync_counters(ctx);
+        const int rs = sync_forces(ctx);
         if (rs) return rs;
         std::memcpy(FT, ctx->h_ft, sizeof(double) * 6 * S);
     }
@@ -1126,9 +1122,7 @@ int sdfibm_cuda_interact_host64(sdfibm_ctx* ctx, double time, double dt, const d
             static_cast<double*>(hp[1]), static_cast<double*>(hp[2]), static_cast<double*>(hp[3]));
         CK(cudaGetLastError());
         mark(ctx, "export64_kernel");
-        if (ctx->S > 0)
-            CK(cudaMemcpyAsync(ctx->h_ft, ctx->d_ft, sizeof(double) * 6 * ctx->S, cudaMemcpyDeviceToHost, st));
-        rc = sync_counters(ctx);
+        rc = sync_forces(ctx);
         if (rc) return rc;
         const Counters& c = *ctx->h_cnt;
         ctx->host_h2d = 24 * ((int64_t)clamp_len(c.n_inside, c.list_cap) + clamp_len(c.n_cut, c.list_cap));
@@ -1153,8 +1147,7 @@ int sdfibm_cuda_interact_host64(sdfibm_ctx* ctx, double time, double dt, const d
     CK(cudaMemcpyAsync(Fs, out + N, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(Ts, out + 4 * N, sizeof(double) * N, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(Ct, out + 5 * N, sizeof(double) * N, cudaMemcpyDeviceToHost, st));
-    if (ctx->S > 0) CK(cudaMemcpyAsync(ctx->h_ft, ctx->d_ft, sizeof(double) * 6 * ctx->S, cudaMemcpyDeviceToHost, st));
-    rc = sync_counters(ctx);
+    rc = sync_forces(ctx);
     if (rc) return rc;
     ctx->host_h2d = 24 * N;
     ctx->host_d2h = 48 * N + 48 * ctx->S;
@@ -1240,9 +1233,7 @@ int sdfibm_cuda_interact_host(sdfibm_ctx* ctx, double time, double dt, const flo
             CK(cudaMemcpyAsync(Ct, ctx->d_Ct, sizeof(int32_t) * N, cudaMemcpyDeviceToHost, st));
             mark(ctx, "host_copies");
         }
-        if (ctx->S > 0)
-            CK(cudaMemcpyAsync(ctx->h_ft, ctx->d_ft, sizeof(double) * 6 * ctx->S, cudaMemcpyDeviceToHost, st));
-        rc = sync_counters(ctx);
+        rc = sync_forces(ctx);
         if (rc) return rc;
         const Counters& c = *ctx->h_cnt;
         ctx->host_h2d = u_host ? 12 * ((int64_t)c.n_inside + c.n_cut) : 12 * N;
@@ -1268,8 +1259,7 @@ int sdfibm_cuda_interact_host(sdfibm_ctx* ctx, double time, double dt, const flo
         CK(cudaStreamWaitEvent(ctx->copy_st[i], ctx->ev_done, 0));
         CK(cudaMemcpyAsync(dst[i], src[i], bytes[i], cudaMemcpyDeviceToHost, ctx->copy_st[i]));
     }
-    if (ctx->S > 0) CK(cudaMemcpyAsync(ctx->h_ft, ctx->d_ft, sizeof(double) * 6 * ctx->S, cudaMemcpyDeviceToHost, st));
-    rc = sync_counters(ctx);
+    rc = sync_forces(ctx);
     for (auto& c : ctx->copy_st) CK(cudaStreamSynchronize(c));
     if (rc) return rc;
     ctx->host_h2d = u_host ? 12 * ((int64_t)ctx->h_cnt->n_inside + ctx->h_cnt->n_cut) : 12 * N;
@@ -1303,9 +1293,10 @@ static int enqueue_evolve(sdfibm_ctx* ctx, double time, double dt) {
     const D3 g{ctx->opt.gravity[0], ctx->opt.gravity[1], ctx->opt.gravity[2]};
     // thread-per-solid kernels are FP64-pipe bound: small blocks spread a few thousand solids over every SM
     const int B = S <= ctx->num_sms * 4 * 64 ? 32 : 128, G = (S + B - 1) / B;
-    set_step_kernel<<<1, 1, 0, st>>>(step, time, dt, nsub, 0.0, ctx->evw.ctrl);
+    const StepParams sp = step_params(time, dt, nsub, 0.0);
+    if (ctx->grid_active) set_step_kernel<<<1, 1, 0, st>>>(step, sp, ctx->evw.ctrl);
     if (!ctx->grid_active) {
-        evolve_independent_kernel<<<G, B, 0, st>>>(ctx->d_sk, ctx->d_st, S, nsub, step, ctx->opt.rho_f, g);
+        evolve_independent_kernel<<<G, B, 0, st>>>(ctx->d_sk, ctx->d_st, S, nsub, sp, ctx->opt.rho_f, g);
     } else if (ctx->ev_per > 0) {
         const int per = ctx->ev_per;
         const SolidK* sk = ctx->d_sk;
@@ -1352,8 +1343,15 @@ int sdfibm_cuda_evolve(sdfibm_ctx* ctx, double time, double dt) {
     if (!ctx) return SDFIBM_ERR_ARG;
     if (ctx->S == 0) return SDFIBM_OK;
     if (graphs_on(ctx)) {
+        StepParams sp = step_params(time, dt, ctx->nsub, 0.0);
+        StepParams* step = ctx->d_step + 1;
+        EvolveCtrl* ctrl = ctx->evw.ctrl;
+        D3 g{ctx->opt.gravity[0], ctx->opt.gravity[1], ctx->opt.gravity[2]};
+        void* args_c[] = {&step, &sp, &ctrl};
+        void* args_i[] = {&ctx->d_sk, &ctx->d_st, &ctx->S, &ctx->nsub, &sp, &ctx->opt.rho_f, &g};
+        const bool grid = ctx->grid_active;
         const int rc = run_graph(ctx, ctx->egraph, false, [&] { return enqueue_evolve(ctx, time, dt); },
-                                 ctx->d_step + 1, time, dt, ctx->nsub, 0.0, ctx->evw.ctrl);
+                                 grid ? (void*)set_step_kernel : (void*)evolve_independent_kernel, grid ? args_c : args_i);
         if (rc != -1) return rc;
         ctx->graphs_failed = true;
     }
@@ -1878,8 +1876,7 @@ static int poly_interact(sdfibm_ctx* ctx, double time, double dt, const float* U
     ctx->launches_last = launches;
     ctx->interacted = true;
     if (FT) {
-        if (S > 0) CK(cudaMemcpyAsync(ctx->h_ft, ctx->d_ft, sizeof(double) * 6 * S, cudaMemcpyDeviceToHost, st));
-        const int rs = sync_counters(ctx);
+        const int rs = sync_forces(ctx);
         if (rs) return rs;
         std::memcpy(FT, ctx->h_ft, sizeof(double) * 6 * S);
     }
@@ -1918,8 +1915,7 @@ static int poly_interact_host(sdfibm_ctx* ctx, double time, double dt, const voi
         CK(cudaMemcpyAsync(Ts, P.dTs, sizeof(float) * N, cudaMemcpyDeviceToHost, st));
         CK(cudaMemcpyAsync(Ct, P.dCt, sizeof(int32_t) * N, cudaMemcpyDeviceToHost, st));
     }
-    if (ctx->S > 0) CK(cudaMemcpyAsync(ctx->h_ft, ctx->d_ft, sizeof(double) * 6 * ctx->S, cudaMemcpyDeviceToHost, st));
-    rc = sync_counters(ctx);
+    rc = sync_forces(ctx);
     if (rc) return rc;
     ctx->host_h2d = (f64 ? 24 : 12) * N;
     ctx->host_d2h = (f64 ? 48 : 24) * N + 48 * ctx->S;

@@ -28,41 +28,13 @@ namespace sdfibm_dev {
 
 
 // ---- plan ---------------------------------------------------------------------------------------------------------
-__device__ inline int32_t n3v(const MeshK& m, int a) { return a == 0 ? m.nx : (a == 1 ? m.ny : m.nz); }
-
-__global__ void plan_kernel(MeshK m, const SolidK* __restrict__ sk, const sdfibm_solid_state* __restrict__ st,
-                            SolidPlan* __restrict__ plan, int S, Counters* cnt) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    const SolidK& k = sk[s];
-    const Q4 q = state_quat(st[s]);
-    const D3 x = state_pos(st[s]);
-    SolidPlan p;
-    local_matrix32(q, p.M);  // |q|^2 R(q)^T: the linear map of world2local
-    p.err = 0;
-    // local box holding the inside region (widened far beyond FP32 rounding): tiles of the classify pass that lie
-    // outside it hold no inside vertex
-    p.cull_box = 0;
-    p.radius_cells = (float)k.radiusB * (1.f / m.h32[0]);
-    if (!k.shape.prism && !k.infinite &&
-        (k.shape.type == SDFIBM_SHAPE_SPHERE || k.shape.type == SDFIBM_SHAPE_ELLIPSOID ||
-         k.shape.type == SDFIBM_SHAPE_BOX)) {
-        const double* sp = k.shape.p;
-        const bool ell = k.shape.type == SDFIBM_SHAPE_ELLIPSOID;  // ignores com
-        const bool sph = k.shape.type == SDFIBM_SHAPE_SPHERE;
-        for (int a = 0; a < 3; ++a) {
-            const double half = sph ? sp[0] : sp[a];
-            p.lbox_c[a] = ell ? 0.f : (float)(-k.shape.com[a]);
-            p.lbox_s[a] = (float)(half * (1.0 + 1e-4) + 1e-4 * fabs(k.shape.com[a]) + 1e-30);
-        }
-        p.cull_box = 1;
-    }
+// bounding region and bbox origin (warp 0 of a plan CTA)
+__device__ inline void plan_box(const MeshK& m, const SolidK& k, const Q4& q, const D3& x, SolidPlan& p, Counters* cnt) {
+    int err = 0;
     const int32_t n[3] = {m.nx, m.ny, m.nz};
-    p.cw[0] = p.cw[1] = p.cw[2] = 0.0;
-    p.rcull = 0.0;
-    for (int a = 0; a < 3; ++a) { p.vlo[a] = 0; p.vhi[a] = n3v(m, a); }
+    int32_t vlo[3] = {0, 0, 0}, vhi[3] = {m.nx, m.ny, m.nz}, lo3[3] = {0, 0, 0};
+    const double inv[3] = {1.0 / m.h[0], 1.0 / m.h[1], 1.0 / m.h[2]};
     if (k.infinite) {
-        p.lo[0] = p.lo[1] = p.lo[2] = 0;
         // the half space n . (v - x) < 0 over the mesh box bounds the inside vertices along every axis its normal has a
         // component of (a wall along an axis: one layer of cells), widened far beyond the rounding of the inside test
         const D3 nw = qtransform(q, D3{0, 1, 0});
@@ -77,134 +49,207 @@ __global__ void plan_kernel(MeshK m, const SolidK* __restrict__ sk, const sdfibm
         for (int a = 0; a < 3; ++a) {
             if (nv[a] == 0.0) continue;
             const double bound = xv[a] - (low - term[a]) / nv[a], tol = 1e-12 * (mag / fabs(nv[a])) + 1e-12 * fabs(xv[a]);
-            if (nv[a] > 0.0) p.vhi[a] = (int32_t)dmin(dmax(floor((bound + tol - m.o[a]) / m.h[a]) + 1, -1.0), (double)n[a]);
-            else p.vlo[a] = (int32_t)dmin(dmax(ceil((bound - tol - m.o[a]) / m.h[a]) - 1, 0.0), (double)n[a] + 1);
+            if (nv[a] > 0.0) vhi[a] = (int32_t)dmin(dmax(floor((bound + tol - m.o[a]) / m.h[a]) + 1, -1.0), (double)n[a]);
+            else vlo[a] = (int32_t)dmin(dmax(ceil((bound - tol - m.o[a]) / m.h[a]) - 1, 0.0), (double)n[a] + 1);
         }
     } else {
         D3 cl{-k.shape.com[0], -k.shape.com[1], -k.shape.com[2]};
         if (k.shape.type == SDFIBM_SHAPE_ELLIPSOID) cl = D3{0, 0, 0};
         if (k.shape.prism) cl.z = 0.0;
-        const D3 cw = x + qtransform(q, cl);
+        D3 cw = x;
+        if (cl.x != 0.0 || cl.y != 0.0 || cl.z != 0.0) cw = x + qtransform(q, cl);
         const double r = k.shape.bound_r * (1.0 + 1e-9) + 1e-12;
         double rad[3] = {r, r, r};
-        if (k.shape.prism) {
+        if (k.shape.prism && !(q.v.x == 0.0 && q.v.y == 0.0)) {
             // the inside region is a prism along the local z axis a; clip it to the mesh slab in z
             const double qq = q.w * q.w + magSqr(q.v);
             const D3 a = qtransform(q, D3{0, 0, 1}) / qq;
             const double sxy = sqrt(a.x * a.x + a.y * a.y), az = fabs(a.z);
-            if (az < 0.3 && (k.ext[0] < n[0] + 2 || k.ext[1] < n[1] + 2)) p.err = DERR_BBOX;
+            if (az < 0.3 && (k.ext[0] < n[0] + 2 || k.ext[1] < n[1] + 2)) err = DERR_BBOX;
             const double zlo = m.o[2], zhi = mesh_coord(m, 2, m.nz);
             const double zspan = dmax(fabs(zhi - cw.z), fabs(zlo - cw.z));
             const double rxy = (sxy > 0) ? r + (zspan + r * sxy) / dmax(az, 0.3) * sxy : r;
             rad[0] = rad[1] = rxy * (1.0 + 1e-9);
         }
-        p.cw[0] = cw.x; p.cw[1] = cw.y; p.cw[2] = cw.z;
-        p.rcull = rad[0];
-        // oriented bounding box of the inside region: half extents along the world axes
-        {
-            const double qq = q.w * q.w + magSqr(q.v);
-            const D3 ex = qtransform(q, D3{1, 0, 0}) / qq, ey = qtransform(q, D3{0, 1, 0}) / qq,
-                     ez = qtransform(q, D3{0, 0, 1}) / qq;  // columns of the unit rotation
-            const double Rm[3][3] = {{ex.x, ey.x, ez.x}, {ex.y, ey.y, ez.y}, {ex.z, ey.z, ez.z}};
-            double e[3] = {rad[0], rad[1], rad[2]};
-            const double* sp = k.shape.p;
-            if (k.shape.type == SDFIBM_SHAPE_ELLIPSOID) {
-                for (int a = 0; a < 3; ++a)
-                    e[a] = sqrt(Rm[a][0] * Rm[a][0] * sp[0] * sp[0] + Rm[a][1] * Rm[a][1] * sp[1] * sp[1] +
-                                Rm[a][2] * Rm[a][2] * sp[2] * sp[2]);
-            } else if (k.shape.type == SDFIBM_SHAPE_BOX) {
-                for (int a = 0; a < 3; ++a) e[a] = fabs(Rm[a][0]) * sp[0] + fabs(Rm[a][1]) * sp[1] + fabs(Rm[a][2]) * sp[2];
-            }
-            const double c3v[3] = {cw.x, cw.y, cw.z};
+        // half extents of the oriented bounding box of the inside region along the world axes; FP32, widened
+        float e[3] = {INFINITY, INFINITY, INFINITY};
+        if (k.shape.type == SDFIBM_SHAPE_ELLIPSOID || k.shape.type == SDFIBM_SHAPE_BOX) {
+            const float w = (float)q.w, qx = (float)q.v.x, qy = (float)q.v.y, qz = (float)q.v.z;
+            const float qq = w * w + qx * qx + qy * qy + qz * qz, iq = 1.f / qq;
+            const float size = (float)k.shape.bound_r, isize = 1.f / size;  // squares of the sizes stay in range
+            const float Rm[3][3] = {{w * w + qx * qx - qy * qy - qz * qz, 2.f * (qx * qy - w * qz), 2.f * (qx * qz + w * qy)},
+                                    {2.f * (qx * qy + w * qz), w * w - qx * qx + qy * qy - qz * qz, 2.f * (qy * qz - w * qx)},
+                                    {2.f * (qx * qz - w * qy), 2.f * (qy * qz + w * qx), w * w - qx * qx - qy * qy + qz * qz}};
+            const float* sp = k.shape.p32;
+            const bool ell = k.shape.type == SDFIBM_SHAPE_ELLIPSOID;
             for (int a = 0; a < 3; ++a) {
-                if (k.shape.prism && a == 2) continue;  // all layers
-                const double ea = dmin(e[a], rad[a]) * (1.0 + 1e-9) + 1e-12;
-                const double l = ceil((c3v[a] - ea - m.o[a]) / m.h[a]) - 1, u = floor((c3v[a] + ea - m.o[a]) / m.h[a]) + 1;
-                p.vlo[a] = (int32_t)dmin(dmax(l, -1.0), (double)n3v(m, a) + 1);
-                p.vhi[a] = (int32_t)dmin(dmax(u, -1.0), (double)n3v(m, a) + 1);
+                float t = 0.f;
+                for (int c = 0; c < 3; ++c) {
+                    const float v = fabsf(Rm[a][c]) * iq * (sp[c] * isize);
+                    t += ell ? v * v : v;
+                }
+                // FP32 errors of R are relative to 1, not to the entry
+                if (qq > 1e-6f && qq < 1e6f) e[a] = size * ((ell ? sqrtf(t) : t) + 3e-5f);
             }
         }
         const double c3[3] = {cw.x, cw.y, cw.z};
         for (int a = 0; a < 3; ++a) {
-            if (k.shape.prism && a == 2) { p.lo[2] = 0; continue; }
-            if (k.ext[a] >= n[a] + 2) { p.lo[a] = -1; continue; }  // the window spans the whole axis
-            const double lo = floor((c3[a] - rad[a] - m.o[a]) / m.h[a]) - 1;
-            const double hi = floor((c3[a] + rad[a] - m.o[a]) / m.h[a]) + 1;
+            if (k.shape.prism && a == 2) continue;  // all layers
+            const double ea = dmin(rad[a], (double)e[a]) * (1.0 + 1e-9) + 1e-12;
+            const double l = ceil((c3[a] - ea - m.o[a]) * inv[a]) - 1, u = floor((c3[a] + ea - m.o[a]) * inv[a]) + 1;
+            vlo[a] = (int32_t)dmin(dmax(l, -1.0), (double)n[a] + 1);
+            vhi[a] = (int32_t)dmin(dmax(u, -1.0), (double)n[a] + 1);
+            if (k.ext[a] >= n[a] + 2) { lo3[a] = -1; continue; }  // the window spans the whole axis
+            const double lo = floor((c3[a] - rad[a] - m.o[a]) * inv[a]) - 1, hi = floor((c3[a] + rad[a] - m.o[a]) * inv[a]) + 1;
             // only cells 0..n-1 matter: start the window no lower than -1 (this also keeps the int conversion
             // defined for solids far outside the mesh)
             const double lo_c = dmin(dmax(lo, -1.0), 1e9), hi_c = dmin(hi, (double)n[a]);
-            p.lo[a] = (int32_t)lo_c;
-            if (hi_c >= lo_c && hi_c - lo_c + 1 > (double)k.ext[a]) p.err = DERR_BBOX;
+            lo3[a] = (int32_t)lo_c;
+            if (hi_c >= lo_c && hi_c - lo_c + 1 > (double)k.ext[a]) err = DERR_BBOX;
         }
     }
-    if (p.err) set_error(cnt, p.err);
-    // meshSearch::findNearestCell: nearest cell centre, ties to the lowest cell label
-    {
-        const double pc[3] = {x.x, x.y, x.z};
-        int64_t lo[3], hi[3];
-        for (int a = 0; a < 3; ++a) {
-            double t = floor((pc[a] - m.o[a]) / m.h[a]);
-            int64_t e = t < 0 ? 0 : (t > (double)(n[a] - 1) ? n[a] - 1 : (int64_t)t);
-            lo[a] = e > 0 ? e - 1 : 0;
-            hi[a] = e + 1 < n[a] ? e + 1 : n[a] - 1;
+    for (int a = 0; a < 3; ++a) { p.lo[a] = lo3[a]; p.vlo[a] = vlo[a]; p.vhi[a] = vhi[a]; }
+    p.err = err;
+    if (err) set_error(cnt, err);
+    // FP64 origin of the tile frames and the local map (world2local of the bbox corner plus the images of the cell edge
+    // vectors), so tiles build their frames without per-tile FP64 work
+    const D3 p0 = mesh_point(m, lo3[0], lo3[1], lo3[2]);
+    const D3 b = p0 - x;
+    p.base32[0] = (float)b.x; p.base32[1] = (float)b.y; p.base32[2] = (float)b.z;
+    double L[9];
+    local_matrix(q, L);
+    double l12[12];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        l12[r] = L[3 * r] * b.x + L[3 * r + 1] * b.y + L[3 * r + 2] * b.z;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) l12[3 + 3 * a + r] = L[3 * r + a] * m.h[a];
+    }
+#pragma unroll
+    for (int r = 0; r < 12; ++r) {
+        p.lmap[r] = l12[r];
+        p.lmap_hi[r] = (float)l12[r];
+        p.lmap_lo[r] = (float)(l12[r] - (double)p.lmap_hi[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < 9; ++r) p.M[r] = (float)L[r];  // |q|^2 R(q)^T: the linear map of world2local
+    float mag = 0.f;
+    const float o3[3] = {(float)m.o[0], (float)m.o[1], (float)m.o[2]}, x3[3] = {(float)x.x, (float)x.y, (float)x.z};
+    for (int a = 0; a < 3; ++a)
+        mag += fabsf(o3[a] + (float)lo3[a] * m.h32[a]) + fabsf(o3[a] + (float)(lo3[a] + k.ext[a]) * m.h32[a]) + fabsf(x3[a]) +
+               1e-6f * fabsf(o3[a]);
+    p.e64 = 4.1e-15f * mag;
+}
+
+// nearest cell (warp 1): meshSearch::findNearestCell, ties to the lowest label, and the rigid-body velocity there.  The
+// squared distance is (dx^2 + dy^2) + dz^2 with each sum rounded, which never falls when a term grows, so the minimum over
+// the neighbourhood is at the axes' minima; the lowest label among equals is found axis by axis.
+__device__ inline void plan_nearest(const MeshK& m, const Q4& q, const D3& x, const sdfibm_solid_state& st, SolidPlan& p) {
+    const double pc[3] = {x.x, x.y, x.z};
+    const int32_t n[3] = {m.nx, m.ny, m.nz};
+    int lo[3], cnt3[3];
+    double d[3][3], sq[3][3], least[3];
+    for (int a = 0; a < 3; ++a) {
+        const double t = floor((pc[a] - m.o[a]) / m.h[a]);
+        const int e = !(t >= 0.0) ? 0 : (t > (double)(n[a] - 1) ? n[a] - 1 : (int)t);
+        lo[a] = e > 0 ? e - 1 : 0;
+        cnt3[a] = (e + 1 < n[a] ? e + 1 : n[a] - 1) - lo[a] + 1;
+        for (int i = 0; i < 3; ++i) {
+            d[a][i] = mesh_centre(m, a, lo[a] + i) - pc[a];
+            sq[a][i] = i < cnt3[a] ? d[a][i] * d[a][i] : INFINITY;
         }
-        int64_t best = -1;
-        double bd = 0;
-        for (int64_t kk = lo[2]; kk <= hi[2]; ++kk)
-            for (int64_t jj = lo[1]; jj <= hi[1]; ++jj)
-                for (int64_t ii = lo[0]; ii <= hi[0]; ++ii) {
-                    const int64_t c = ii + (int64_t)m.nx * (jj + (int64_t)m.ny * kk);
-                    const double d = magSqr(mesh_C(m, ii, jj, kk) - x);
-                    if (best < 0 || d < bd || (d == bd && c < best)) { bd = d; best = c; }
-                }
-        p.seed = best;
-        const int64_t si = best % m.nx, sj = (best / m.nx) % m.ny, sk3 = best / ((int64_t)m.nx * m.ny);
-        p.seed_ijk[0] = (int32_t)si; p.seed_ijk[1] = (int32_t)sj; p.seed_ijk[2] = (int32_t)sk3;
-        p.pad1 = 0;
-        const D3 cb = mesh_C(m, si, sj, sk3) - x;
-        p.cbase[0] = cb.x; p.cbase[1] = cb.y; p.cbase[2] = cb.z;
-        // us at a cell (i, j, k) = us0 + omega x ((i, j, k) - seed) h: us0 and the six per-step terms, split into
-        // FP32 pairs (the couple kernel evaluates U - us in two-float arithmetic)
-        const D3 vel{st[s].vel[0], st[s].vel[1], st[s].vel[2]}, om{st[s].omega[0], st[s].omega[1], st[s].omega[2]};
-        const D3 us0 = vel + cross(om, cb);
-        const double u3[3] = {us0.x, us0.y, us0.z};
-        const double d6[6] = {-om.z * m.h[1], om.y * m.h[2], om.z * m.h[0], -om.x * m.h[2], -om.y * m.h[0],
-                              om.x * m.h[1]};
-        for (int a = 0; a < 3; ++a) {
-            p.us_hi[a] = (float)u3[a];
-            p.us_lo[a] = (float)(u3[a] - (double)p.us_hi[a]);
-            p.cb32[a] = (float)p.cbase[a];
+        least[a] = sq[a][0];
+        for (int i = 1; i < 3; ++i) least[a] = sq[a][i] < least[a] ? sq[a][i] : least[a];
+    }
+    const double best = least[0] + least[1] + least[2];
+    int at[3] = {0, 0, 0};
+    for (int i = 2; i >= 0; --i) at[2] = least[0] + least[1] + sq[2][i] == best ? i : at[2];
+    const double dz2 = at[2] == 0 ? sq[2][0] : (at[2] == 1 ? sq[2][1] : sq[2][2]);
+    for (int i = 2; i >= 0; --i) at[1] = least[0] + sq[1][i] + dz2 == best ? i : at[1];
+    const double dy2 = at[1] == 0 ? sq[1][0] : (at[1] == 1 ? sq[1][1] : sq[1][2]);
+    for (int i = 2; i >= 0; --i) at[0] = sq[0][i] + dy2 + dz2 == best ? i : at[0];
+    double cb[3];
+    for (int a = 0; a < 3; ++a) {
+        p.seed_ijk[a] = lo[a] + at[a];
+        cb[a] = at[a] == 0 ? d[a][0] : (at[a] == 1 ? d[a][1] : d[a][2]);
+        p.cb32[a] = (float)cb[a];
+    }
+    // us at a cell (i, j, k) = us0 + omega x ((i, j, k) - seed) h: us0 and the six per-step terms, split into
+    // FP32 pairs (the couple kernel evaluates U - us in two-float arithmetic)
+    const D3 vel{st.vel[0], st.vel[1], st.vel[2]}, om{st.omega[0], st.omega[1], st.omega[2]};
+    const D3 us0 = vel + cross(om, D3{cb[0], cb[1], cb[2]});
+    const double u3[3] = {us0.x, us0.y, us0.z};
+    const double d6[6] = {-om.z * m.h[1], om.y * m.h[2], om.z * m.h[0], -om.x * m.h[2], -om.y * m.h[0], om.x * m.h[1]};
+    for (int a = 0; a < 3; ++a) {
+        p.us_hi[a] = (float)u3[a];
+        p.us_lo[a] = (float)(u3[a] - (double)p.us_hi[a]);
+    }
+    for (int r = 0; r < 6; ++r) {
+        p.ds_hi[r] = (float)d6[r];
+        p.ds_lo[r] = (float)(d6[r] - (double)p.ds_hi[r]);
+    }
+}
+
+// Head of an interact: the time-step block, the counters, the cleared sums and chunk marks, and the plan of every solid.  A
+// CTA plans 32 solids, warp 0 their boxes, warp 1 their nearest cells, warp 2 the rest; the CTAs after those clear the marks.
+// Bound by FP64 latency (one chain per solid): one thread a solid with the 27-cell search written out took 46 us for one
+// solid and 55 for 4096, with two launches and three fills before it; this takes 12 and 15 (GB300).
+__global__ void __launch_bounds__(96) plan_kernel(PrepArgs A) {
+    const MeshK& m = A.m;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if ((int)blockIdx.x >= A.plan_ctas) {
+        const int64_t t = (int64_t)(blockIdx.x - A.plan_ctas) * 96 + threadIdx.x, nt = (int64_t)(gridDim.x - A.plan_ctas) * 96;
+        for (int64_t i = t; i < A.words; i += nt) {
+            A.cbits[i] = 0u;
+            A.sbits[i] = 0u;
         }
-        for (int r = 0; r < 6; ++r) {
-            p.ds_hi[r] = (float)d6[r];
-            p.ds_lo[r] = (float)(d6[r] - (double)p.ds_hi[r]);
+        return;
+    }
+    if (blockIdx.x == 0 && wid == 2 && lane == 0) {
+        if (A.step) *A.step = A.sp;
+        Counters* cnt = A.cnt;
+        if (A.new_call) {  // the previous lengths are kept for the sparse reset
+            cnt->prev_n_inside = cnt->n_inside;
+            cnt->prev_n_cut = cnt->n_cut;
+            cnt->classify_next = 0; cnt->classify_any_next = 0;
+            cnt->n_inside = 0; cnt->n_cut = 0; cnt->n_shared = 0; cnt->shared_marks = 0;
+            cnt->exact_rechecks = 0; cnt->bbox_cells = 0;
+            cnt->n_feat = 0; cnt->n_fb = 0; cnt->n_recheck = 0; cnt->n_ovf = 0; cnt->n_shent = 0;
+            cnt->n_inband = 0; cnt->n_small = 0;
         }
     }
-    // FP64 origin of the tile frames and the local map (world2local of the bbox corner plus the images of the cell
-    // edge vectors), so tiles build their frames without per-tile FP64 work
-    {
-        const D3 p0 = mesh_point(m, p.lo[0], p.lo[1], p.lo[2]);
-        const D3 b = p0 - x;
-        p.base[0] = b.x; p.base[1] = b.y; p.base[2] = b.z;
-        p.base32[0] = (float)b.x; p.base32[1] = (float)b.y; p.base32[2] = (float)b.z;
-        p.pad4 = 0.f;
-        const D3 cl = world2local(p0, x, q);
-        const Q4 qc = qconj(q);
-        const D3 lx = qtransform(qc, D3{m.h[0], 0, 0}), ly = qtransform(qc, D3{0, m.h[1], 0}),
-                 lz = qtransform(qc, D3{0, 0, m.h[2]});
-        const double l12[12] = {cl.x, cl.y, cl.z, lx.x, lx.y, lx.z, ly.x, ly.y, ly.z, lz.x, lz.y, lz.z};
-        for (int r = 0; r < 12; ++r) {
-            p.lmap[r] = l12[r];
-            p.lmap_hi[r] = (float)l12[r];
-            p.lmap_lo[r] = (float)(l12[r] - (double)p.lmap_hi[r]);
+    const int s = blockIdx.x * 32 + lane;
+    if (s >= A.S) return;
+    const SolidK& k = A.sk[s];
+    SolidPlan& p = A.plan[s];
+    const Q4 q = state_quat(A.st[s]);
+    const D3 x = state_pos(A.st[s]);
+    if (wid == 0) {
+        plan_box(m, k, q, x, p, A.cnt);
+    } else if (wid == 1) {
+        plan_nearest(m, q, x, A.st[s], p);
+    } else {
+        // local box holding the inside region (widened far beyond FP32 rounding): tiles of the classify pass that lie
+        // outside it hold no inside vertex
+        p.cull_box = 0;
+        p.radius_cells = (float)k.radiusB * (1.f / m.h32[0]);
+        if (!k.shape.prism && !k.infinite &&
+            (k.shape.type == SDFIBM_SHAPE_SPHERE || k.shape.type == SDFIBM_SHAPE_ELLIPSOID ||
+             k.shape.type == SDFIBM_SHAPE_BOX)) {
+            const double* sp = k.shape.p;
+            const bool ell = k.shape.type == SDFIBM_SHAPE_ELLIPSOID;  // ignores com
+            const bool sph = k.shape.type == SDFIBM_SHAPE_SPHERE;
+            for (int a = 0; a < 3; ++a) {
+                const double half = sph ? sp[0] : sp[a];
+                p.lbox_c[a] = ell ? 0.f : (float)(-k.shape.com[a]);
+                p.lbox_s[a] = (float)(half * (1.0 + 1e-4) + 1e-4 * fabs(k.shape.com[a]) + 1e-30);
+            }
+            p.cull_box = 1;
         }
-        const D3 pf = mesh_point(m, (int64_t)p.lo[0] + k.ext[0], (int64_t)p.lo[1] + k.ext[1], (int64_t)p.lo[2] + k.ext[2]);
-        p.e64 = (float)(2e-15 * (fabs(p0.x) + fabs(p0.y) + fabs(p0.z) + fabs(pf.x) + fabs(pf.y) + fabs(pf.z) + fabs(x.x) +
-                                 fabs(x.y) + fabs(x.z)));
-        p.pad2 = 0.f;
+        p.n_inside = p.n_cut = 0;
+        if (A.ftacc)
+            for (int r = 0; r < 6; ++r) A.ftacc[6 * (int64_t)s + r] = 0.0;
     }
-    p.n_inside = p.n_cut = 0;
-    plan[s] = p;
 }
 
 // ---- claims ----------------------------------------------------------------------------------------------------------
@@ -764,35 +809,48 @@ __device__ __forceinline__ void add_shared(const CoupleArgs& A, int64_t c, float
     }
 }
 
-// Shared pass of the coupling, first half (on the side stream after the claims, beside the fraction kernels): the list
-// entries on cells that several solids claimed, compacted into shent (entry index into the in list then the cut list).
-// Only the chunks marked in sbits are looked at; the kernel returns at once when no cell was claimed twice.
-__global__ void shared_scan_kernel(const int32_t* __restrict__ in_cell, const int32_t* __restrict__ cut_cell,
-                                   const int32_t* __restrict__ Ct, Counters* cnt, int64_t N,
-                                   const uint32_t* __restrict__ sbits, uint32_t* __restrict__ shent,
-                                   int64_t shent_cap) {
-    if (cnt->shared_marks == 0) return;
-    const int64_t n_in = clamp_len(cnt->n_inside, cnt->list_cap), n_cut = clamp_len(cnt->n_cut, cnt->list_cap);
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n_in + n_cut;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t c = e < n_in ? in_cell[e] : cut_cell[e - n_in];
-        if (c < 0 || c >= N) continue;
-        if (!((sbits[c >> 8] >> ((c >> 3) & 31)) & 1u)) continue;  // no cell of this chunk is shared
-        if (!(reinterpret_cast<const uint32_t*>(Ct)[c] & CT_SHARED)) continue;
-        const int32_t slot = atomicAdd(&cnt->n_shent, 1);
-        if (slot < shent_cap) shent[slot] = (uint32_t)e;
-        else set_error(cnt, DERR_SHARED_TABLE);
+// After the claims, on the side stream beside the fraction kernels.
+// Shared cells: the list entries on cells that several solids claimed, compacted into shent (entry index into the in list
+// then the cut list).  Only the chunks marked in sbits are looked at; nothing when no cell was claimed twice.
+// Sparse reset (prev_in_cell not null): the cells the previous call touched and this call does not go back to zero -- the
+// sparse form of solidcloud.cpp:438-441.  Cells in the chunks marked in cbits are left to couple_chunks_kernel, which writes
+// every cell of those chunks.
+__global__ void scan_reset_kernel(const int32_t* __restrict__ in_cell, const int32_t* __restrict__ cut_cell, Counters* cnt,
+                                  int64_t N, const uint32_t* __restrict__ sbits, uint32_t* __restrict__ shent,
+                                  int64_t shent_cap, const int32_t* __restrict__ prev_in_cell,
+                                  const int32_t* __restrict__ prev_cut_cell, float* As, float* Fs, float* Ts, int32_t* Ct,
+                                  const uint32_t* __restrict__ cbits) {
+    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    if (cnt->shared_marks != 0) {
+        const int64_t n_in = clamp_len(cnt->n_inside, cnt->list_cap), n_cut = clamp_len(cnt->n_cut, cnt->list_cap);
+        for (int64_t e = t0; e < n_in + n_cut; e += nt) {
+            const int32_t c = e < n_in ? in_cell[e] : cut_cell[e - n_in];
+            if (c < 0 || c >= N) continue;
+            if (!((sbits[c >> 8] >> ((c >> 3) & 31)) & 1u)) continue;  // no cell of this chunk is shared
+            if (!(reinterpret_cast<const uint32_t*>(Ct)[c] & CT_SHARED)) continue;
+            const int32_t slot = atomicAdd(&cnt->n_shent, 1);
+            if (slot < shent_cap) shent[slot] = (uint32_t)e;
+            else set_error(cnt, DERR_SHARED_TABLE);
+        }
+    }
+    if (prev_in_cell) {
+        const int64_t n_in = clamp_len(cnt->prev_n_inside, cnt->list_cap), n_cut = clamp_len(cnt->prev_n_cut, cnt->list_cap);
+        for (int64_t e = t0; e < n_in + n_cut; e += nt) {
+            const int64_t c = e < n_in ? prev_in_cell[e] : prev_cut_cell[e - n_in];
+            if (c < 0 || c >= N) continue;
+            if ((cbits[c >> 8] >> ((c >> 3) & 31)) & 1u) continue;  // written by the chunked coupling
+            if (reinterpret_cast<const uint32_t*>(Ct)[c] >= CT_KEY_BASE) continue;
+            As[c] = 0.f; Ts[c] = 0.f; Ct[c] = 0;
+            Fs[c] = 0.f; Fs[N + c] = 0.f; Fs[2 * N + c] = 0.f;
+        }
     }
 }
 
-// Shared pass, second half (after the fraction kernels): every compacted entry adds its solid's As / Ts / Fs to the
-// cell's FP64 sums in the shared table (finalize_kernel writes them) and its force/torque contribution to the solid's
-// sums.
+// Shared cells, second half (after the fraction kernels): every compacted entry adds its solid's As / Ts / Fs to the
+// cell's FP64 sums in the shared table (finalize_kernel writes them) and its force/torque contribution to the solid's sums.
 template <bool EXACT>
-__global__ void __launch_bounds__(CPL_THREADS) couple_shared_kernel(CoupleArgs A) {
+__device__ __noinline__ void couple_shared(const CoupleArgs& A, int64_t n) {
     const int64_t N = A.m.ncells;
-    const int64_t n = min((int64_t)A.cnt->n_shent, A.shent_cap);
-    if (n == 0) return;
     const int64_t n_in = clamp_len(A.cnt->n_inside, A.cnt->list_cap);
     const double dtINV = A.step->dtINV;
     const float dtINV32 = (float)dtINV;
@@ -810,10 +868,6 @@ __global__ void __launch_bounds__(CPL_THREADS) couple_shared_kernel(CoupleArgs A
         add_shared(A, c, alpha, fs);
         for (int r = 0; r < 6; ++r) atomicAdd(A.ftacc + 6 * s + r, EXACT ? f6[r] : (double)g6[r]);
     }
-}
-void launch_couple_shared(const CoupleArgs& A, bool exact, int grid, cudaStream_t st) {
-    if (exact) couple_shared_kernel<true><<<grid, CPL_THREADS, 0, st>>>(A);
-    else couple_shared_kernel<false><<<grid, CPL_THREADS, 0, st>>>(A);
 }
 
 // Chunked coupling.  The claim pass marks in cbits every chunk of 8 consecutive cells that holds a claimed cell (and
@@ -900,6 +954,8 @@ __global__ void __launch_bounds__(CPL_THREADS) couple_chunks_kernel(CoupleArgs A
     const float dtINV32 = (float)dtINV;
     const uint32_t* C = reinterpret_cast<const uint32_t*>(A.Ct);
     const uint8_t* marks = reinterpret_cast<const uint8_t*>(A.cbits);
+    const int64_t n_shared = min((int64_t)A.cnt->n_shent, A.shent_cap);
+    if (n_shared > 0) couple_shared<EXACT>(A, n_shared);
     int nq = 0;  // warp-uniform
     for (int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < items; t += nw) {
         int64_t b0;        // first byte
@@ -1010,15 +1066,27 @@ __global__ void apply_forcing_kernel(int64_t N, const uint32_t* __restrict__ cbi
     }
 }
 
-// ---- finalize: cells shared by several solids ---------------------------------------------------------------------------
+// ---- finalize: cells shared by several solids, forces ------------------------------------------------------------------
 // FP64 sums rounded once to the FP32 fields, Ct decoded from the largest claim, As = min(As, 1) (checkAlpha); the slot
-// is cleared for the next call.
+// is cleared for the next call.  F = rho_f * V / dt * sum f, T = rho_f * V / dt * sum (C - x) x f  (solidcloud.cpp:411-421),
+// into ft and the solid's state (Solid::setFluidForceAndTorque).
 __global__ void finalize_kernel(float* __restrict__ As, float* __restrict__ Ts, float* __restrict__ Fs,
                                 int32_t* __restrict__ Ct, const Counters* cnt, int64_t N, int32_t* __restrict__ sh_keys,
-                                double* __restrict__ sh_vals, const int32_t* __restrict__ sh_used, int32_t sh_mask) {
+                                double* __restrict__ sh_vals, const int32_t* __restrict__ sh_used, int32_t sh_mask,
+                                const double* __restrict__ ftacc, double* __restrict__ ft, int S, const StepParams* step,
+                                sdfibm_solid_state* __restrict__ st) {
+    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    const double scale = step->ft_scale;
+    for (int64_t e = t0; e < 6 * (int64_t)S; e += nt) {
+        const int64_t s = e / 6, r = e - 6 * s;
+        const double y = ftacc[e] * scale;
+        ft[e] = y;
+        if (r < 3) st[s].fluid_force[r] = y;
+        else st[s].fluid_torque[r - 3] = y;
+    }
     const int n_sh = min(cnt->n_shared, sh_mask + 1);
     uint32_t* C = reinterpret_cast<uint32_t*>(Ct);
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n_sh; e += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t e = t0; e < n_sh; e += nt) {
         const int slot = sh_used[e];
         const int32_t c = sh_keys[slot];
         double* v = sh_vals + 5 * (int64_t)slot;
@@ -1035,50 +1103,19 @@ __global__ void finalize_kernel(float* __restrict__ As, float* __restrict__ Ts, 
     }
 }
 
-// per-call counters: the previous lengths are kept for the sparse reset
-__global__ void begin_kernel(Counters* cnt) {
-    cnt->prev_n_inside = cnt->n_inside;
-    cnt->prev_n_cut = cnt->n_cut;
-    cnt->classify_next = 0; cnt->classify_any_next = 0;
-    cnt->n_inside = 0; cnt->n_cut = 0; cnt->n_shared = 0; cnt->shared_marks = 0;
-    cnt->exact_rechecks = 0; cnt->bbox_cells = 0;
-    cnt->n_feat = 0; cnt->n_fb = 0; cnt->n_recheck = 0; cnt->n_ovf = 0; cnt->n_shent = 0;
-    cnt->n_inband = 0; cnt->n_small = 0;
+// forces and counters into page-locked host memory (read after the stream is synchronised): one launch instead of two copies
+__global__ void export_ft_kernel(const double* __restrict__ ft, int64_t n, const Counters* __restrict__ cnt,
+                                 double* __restrict__ h_ft, Counters* __restrict__ h_cnt) {
+    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t e = t0; e < n; e += nt) h_ft[e] = ft[e];
+    const uint32_t* a = reinterpret_cast<const uint32_t*>(cnt);
+    uint32_t* b = reinterpret_cast<uint32_t*>(h_cnt);
+    if (t0 < (int64_t)(sizeof(Counters) / 4)) b[t0] = a[t0];
 }
 
-// F = rho_f * V / dt * sum f, T = rho_f * V / dt * sum (C - x) x f  (solidcloud.cpp:411-421)
-__global__ void ft_kernel(const double* __restrict__ ftacc, double* __restrict__ ft, int S, const StepParams* step) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    const double scale = step->ft_scale;
-    for (int r = 0; r < 6; ++r) ft[6 * s + r] = ftacc[6 * s + r] * scale;
-}
-
-__global__ void set_step_kernel(StepParams* p, double time, double dt, int nsub, double rho_V, EvolveCtrl* ctrl) {
+__global__ void set_step_kernel(StepParams* p, StepParams v, EvolveCtrl* ctrl) {
     if (ctrl) *ctrl = EvolveCtrl{};
-    p->time = time;
-    p->dt = dt;
-    p->dt_sub = dt / nsub;
-    p->dtINV = 1.0 / dt;
-    p->ft_scale = rho_V / dt;
-}
-
-// sparse reset: the cells the previous call touched and this call does not (after this call's claims) go back to
-// zero -- the sparse form of solidcloud.cpp:438-441.  Cells in the chunks marked in cbits are left to
-// couple_chunks_kernel, which writes every cell of those chunks.
-__global__ void reset_kernel(const int32_t* __restrict__ prev_in_cell, const int32_t* __restrict__ prev_cut_cell,
-                             const Counters* cnt, int64_t N, float* As, float* Fs, float* Ts, int32_t* Ct,
-                             const uint32_t* __restrict__ cbits) {
-    const int n_in = clamp_len(cnt->prev_n_inside, cnt->list_cap), n_cut = clamp_len(cnt->prev_n_cut, cnt->list_cap);
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)n_in + n_cut;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t c = e < n_in ? prev_in_cell[e] : prev_cut_cell[e - n_in];
-        if (c < 0 || c >= N) continue;
-        if ((cbits[c >> 8] >> ((c >> 3) & 31)) & 1u) continue;  // written by the chunked coupling
-        if (reinterpret_cast<const uint32_t*>(Ct)[c] >= CT_KEY_BASE) continue;
-        As[c] = 0.f; Ts[c] = 0.f; Ct[c] = 0;
-        Fs[c] = 0.f; Fs[N + c] = 0.f; Fs[2 * N + c] = 0.f;
-    }
+    *p = v;
 }
 
 // interact_host on page-locked host fields.  The host fields held the previous call's values; the cells this call or

@@ -168,10 +168,10 @@ __device__ inline void store_old(sdfibm_solid_state& s) {
 
 // all sub-steps of one solid (no solid-solid interaction)
 __global__ void evolve_independent_kernel(const SolidK* __restrict__ sk, sdfibm_solid_state* st, int S, int nsub,
-                                          const StepParams* step, double rho_f, D3 g) {
+                                          StepParams step, double rho_f, D3 g) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= S) return;
-    const double time = step->time, dt_sub = step->dt_sub;
+    const double time = step.time, dt_sub = step.dt_sub;
     const SolidK& k = sk[s];
     sdfibm_solid_state x = st[s];
     for (int it = 0; it < nsub; ++it) {

@@ -68,25 +68,20 @@ struct SolidK {
 struct SolidPlan {
     int32_t lo[3];            // bbox lower cell index (may lie outside the mesh)
     int32_t err;              // nonzero: bbox too small for the current pose
-    int64_t seed;             // meshSearch::findNearestCell result
     float M[9];               // FP32 world->local matrix (|q|^2 R^T)
     int32_t n_inside, n_cut;  // touched cells by kind
     int32_t seed_ijk[3];      // cell indices of the seed cell
     int32_t pad1;
-    double cbase[3];          // centre of the seed cell minus the solid centre (FP64), origin of FP32 cell offsets
-    double base[3];           // mesh point (lo) minus the solid centre: FP64 origin of the FP32 tile frames
-    float base32[3];          // base rounded to FP32 (the frames' origin)
+    float base32[3];          // mesh point (lo) minus the solid centre, rounded to FP32: origin of the FP32 tile frames
     float pad4;
     double lmap[12];          // world2local of mesh point (lo), then the local images of h_x e_x, h_y e_y, h_z e_z
     float lmap_hi[12], lmap_lo[12];  // the same as FP32 pairs hi + lo (two-float vertex distances)
     float e64;                // bound of the FP64 rounding of point coordinates (see TileFrame)
     float pad2;
-    double cw[3];             // centre of the bounding sphere (2-D shapes: of the bounding disc)
-    double rcull;             // its radius
     int32_t vlo[3], vhi[3];   // mesh-vertex index box of the solid's oriented bounding box: vertices outside it are
                               // outside the solid (vlo > vhi on some axis: no vertex can be inside)
     // mixed forcing: the rigid-body velocity at the seed cell centre and its change per cell step (components
-    // x: dj, dk; y: di, dk; z: di, dj) as FP32 pairs hi + lo, and cbase rounded to FP32
+    // x: dj, dk; y: di, dk; z: di, dj) as FP32 pairs hi + lo, and the seed cell's centre minus the solid's in FP32
     float us_hi[3], us_lo[3];
     float ds_hi[6], ds_lo[6];
     float cb32[3];
@@ -116,7 +111,7 @@ struct Counters {
     int32_t n_fb;             // LEARNED: of those, cells outside the model's band (SUBSAMPLE fallback)
     int32_t n_recheck;        // SUBSAMPLE points left to recheck_kernel this call
     int32_t n_ovf;            // LEARNED: fallback cells whose points overflowed the recheck list (recount_kernel)
-    int32_t n_shent;          // list entries on cells several solids claimed (shared_scan_kernel)
+    int32_t n_shent;          // list entries on cells several solids claimed (scan_reset_kernel)
     int32_t n_inband;         // LEARNED: listed cut cells inside the band, compacted for the network
     int32_t n_small;          // LEARNED: cut cells of solids under rho_min, listed from the back (fallback)
     int32_t pad2;
@@ -133,7 +128,7 @@ struct Recheck {
     uint32_t sample;
 };
 
-// Time-step parameters the kernels read from device memory; set_step_kernel writes them at the head of a call, so a
+// Time-step parameters the kernels read from device memory; plan_kernel and set_step_kernel write them at the head of a call, so a
 // captured graph replays with new values after one kernel-node update.
 struct StepParams {
     double time;
@@ -141,6 +136,27 @@ struct StepParams {
     double dt_sub;    // evolve: dt / sub-steps
     double dtINV;     // interact: 1 / dt
     double ft_scale;  // interact: rho_f * V / dt
+};
+
+inline StepParams step_params(double time, double dt, int nsub, double rho_V) {
+    return StepParams{time, dt, dt / nsub, 1.0 / dt, rho_V / dt};
+}
+
+// plan_kernel: the head of an interact
+struct PrepArgs {
+    MeshK m;
+    const SolidK* sk;
+    const sdfibm_solid_state* st;
+    SolidPlan* plan;
+    int S;
+    int plan_ctas;       // CTAs that plan 32 solids each (at least one); the others clear the marks
+    Counters* cnt;
+    int new_call;        // 1: begin a call's counters
+    StepParams* step;    // receives sp (nullptr: not)
+    StepParams sp;
+    double* ftacc;       // cleared (nullptr: not)
+    uint32_t *cbits, *sbits;
+    int64_t words;
 };
 
 struct CoupleArgs {
@@ -173,7 +189,7 @@ struct CoupleArgs {
     // chunked coupling: marks of the 8-cell chunks with claimed cells / with shared cells (one bit per chunk)
     uint32_t* cbits;
     uint32_t* sbits;
-    const uint32_t* shent;  // list entries on shared cells (shared_scan_kernel)
+    const uint32_t* shent;  // list entries on shared cells (scan_reset_kernel)
     int64_t shent_cap;
 };
 

@@ -31,8 +31,7 @@
 #include "kernels.cuh"
 
 namespace sdfibm_dev {
-__global__ void plan_kernel(MeshK m, const SolidK* sk, const sdfibm_solid_state* st, SolidPlan* plan, int S,
-                            Counters* cnt);
+__global__ void plan_kernel(PrepArgs A);
 int classify_kind(int shape_type, bool flat);
 void launch_classify(const ClassifyArgs& A, bool flat, int grid, cudaStream_t st);
 int classify_occupancy(int method, bool flat);
@@ -292,7 +291,9 @@ extern "C" int sdfibm_cuda_touched_noalloc(const sdfibm_mesh_desc* mesh, const s
     int2* d_chunks = reinterpret_cast<int2*>(b + OFF_CHUNKS);
     // the records travel as kernel arguments (counters start from zero on every call)
     noalloc_init_kernel<<<(nchunks + 255) / 256, 256, 0, st>>>(k, x, NA_MAX_BBOX_CELLS, nchunks);
-    plan_kernel<<<1, 32, 0, st>>>(m, d_sk, d_st, d_plan, 1, d_cnt);
+    PrepArgs pa{};
+    pa.m = m; pa.sk = d_sk; pa.st = d_st; pa.plan = d_plan; pa.S = 1; pa.plan_ctas = 1; pa.cnt = d_cnt;
+    plan_kernel<<<1, 96, 0, st>>>(pa);
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return SDFIBM_ERR_CUDA;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
