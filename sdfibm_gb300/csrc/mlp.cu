@@ -3,8 +3,8 @@
 //
 // Model output: a = sigmoid(prior + network), the prior logit(P4) of the sub-cell planar reconstruction (row 16 of the
 // feature buffer, see cell_stencil in mlp.cuh).
-// One CTA of 128 threads works on tiles of 128 cells; thread t owns cell t of the tile, row t of every M = 128
-// operand and lane t of tensor memory.  Thread 0 issues the tcgen05.mma instructions and commits them to one
+// A CTA works on tiles of 128 cells; a cell is a row of every M = 128 operand and a lane of tensor memory, and has one
+// thread in inference and four in training.  Thread 0 issues the tcgen05.mma instructions and commits them to one
 // mbarrier; every wait on it is bounded and a timeout ends the CTA's work with an error code.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -24,6 +24,47 @@ constexpr long long MLP_WAIT_CYCLES = 2000000000LL;  // about one second at the 
 constexpr unsigned FULLMASK = 0xffffffffu;
 
 __device__ __forceinline__ float sigm(float z) { return __fdividef(1.f, 1.f + __expf(-z)); }
+// SiLU of two units at a time.  Its cost is the special-function unit, a quarter of the lanes: an exponential and a
+// reciprocal a unit.  Two units share the reciprocal of the product of their denominators (1.5 such operations a unit instead
+// of 2), and additions and scalings go two to an instruction.  The exponents are held below 2^60 so that the product stays
+// finite: z / (1 + exp(-z)) below z = -41 is then z 2^-60, below any rounding of the sums it enters.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 r;
+    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;\n}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 r;
+    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mul.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;\n}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float ex2_fast(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rcp_fast(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+constexpr float LOG2E = 1.4426950408889634f;
+// z and the denominators 1 + exp(-z) of two units, and the reciprocal of the product of the denominators
+struct Silu2 {
+    float2 z, d;
+    float r;
+};
+__device__ __forceinline__ Silu2 silu2(float2 zin, float2 b) {
+    Silu2 s;
+    s.z = add2(zin, b);
+    const float2 t = mul2(s.z, make_float2(-LOG2E, -LOG2E));
+    s.d = add2(make_float2(ex2_fast(fminf(t.x, 60.f)), ex2_fast(fminf(t.y, 60.f))), make_float2(1.f, 1.f));
+    s.r = rcp_fast(s.d.x * s.d.y);
+    return s;
+}
+
 __device__ __forceinline__ uint32_t bf16_bits(float x) {
     return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(x));
 }
@@ -40,31 +81,37 @@ __device__ __forceinline__ void store_bf16(uint8_t* op, int row, int k, int K, f
     *reinterpret_cast<uint16_t*>(op + tc::kmajor_offset(row, k, K)) = (uint16_t)bf16_bits(x);
 }
 
-// 64 FP32 columns [col, col + 64) of this thread's lane
-__device__ __forceinline__ void tmem_ld64(uint32_t base, int warp, int col, float* v) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) tc::tmem_ld16(tc::tmem_addr(base, 32 * warp, col + 16 * j), v + 16 * j);
-    tc::tmem_wait_ld();
-}
+// 32 FP32 columns [col, col + 32) of this thread's lane
 __device__ __forceinline__ void tmem_ld32(uint32_t base, int warp, int col, float* v) {
     tc::tmem_ld16(tc::tmem_addr(base, 32 * warp, col), v);
     tc::tmem_ld16(tc::tmem_addr(base, 32 * warp, col + 16), v + 16);
     tc::tmem_wait_ld();
 }
 
-// Stages W1 (BF16, K padded to 16) and W2 (BF16) as B operands, and the FP32 vectors.
-__device__ void stage_weights(const float* P, uint8_t* sW1, uint8_t* sW2, uint8_t* sW2T, float* sb1, float* sb2,
-                              float* sw3, float* sb3) {
-    for (int e = threadIdx.x; e < MLP_H * 16; e += blockDim.x) {
-        const int n = e >> 4, k = e & 15;
-        store_bf16(sW1, n, k, 16, k < MLP_IN ? P[MLP_OFF_W1 + n * MLP_IN + k] : 0.f);
+// Stages W1 and W2 (BF16) as B operands, W2 transposed where asked for, and the FP32 vectors: 8 elements along K a store, and
+// 8 consecutive lanes write 128 consecutive bytes.
+__device__ __forceinline__ void stage_weights(const float* __restrict__ P, uint8_t* sW1, uint8_t* sW2, uint8_t* sW2T, float* sb1,
+                                              float* sb2, float* sw3, float* sb3) {
+    uint32_t b[8];
+    for (int e = threadIdx.x; e < MLP_H * MLP_IN / 8; e += blockDim.x) {
+        const int n = (e & 7) + 8 * (e >> 4), k0 = 8 * ((e >> 3) & 1);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) b[i] = bf16_bits(P[MLP_OFF_W1 + n * MLP_IN + k0 + i]);
+        store_row8(sW1, n, k0, MLP_IN, b);
     }
-    for (int e = threadIdx.x; e < MLP_H * MLP_H; e += blockDim.x) {
-        const int n = e >> 6, k = e & 63;
-        const float w = P[MLP_OFF_W2 + n * MLP_H + k];
-        store_bf16(sW2, n, k, 64, w);
-        if (sW2T) store_bf16(sW2T, k, n, 64, w);  // B of dH1 = dZ2 W2: row = input unit, K = output unit
+    for (int e = threadIdx.x; e < MLP_H * MLP_H / 8; e += blockDim.x) {
+        const int n = (e & 7) + 8 * (e >> 6), k0 = 8 * ((e >> 3) & 7);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) b[i] = bf16_bits(P[MLP_OFF_W2 + n * MLP_H + k0 + i]);
+        store_row8(sW2, n, k0, MLP_H, b);
     }
+    if (sW2T)  // B of dH1 = dZ2 W2: row = input unit, K = output unit
+        for (int e = threadIdx.x; e < MLP_H * MLP_H / 8; e += blockDim.x) {
+            const int k = e & 63, n0 = 8 * (e >> 6);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) b[i] = bf16_bits(P[MLP_OFF_W2 + (n0 + i) * MLP_H + k]);
+            store_row8(sW2T, k, n0, MLP_H, b);
+        }
     if (threadIdx.x < MLP_H) {
         sb1[threadIdx.x] = P[MLP_OFF_B1 + threadIdx.x];
         sb2[threadIdx.x] = P[MLP_OFF_B2 + threadIdx.x];
@@ -150,10 +197,13 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
 // The layer-1 operand A1 lives in the first 8 KB of the layer-2 operand A2 (A2 is written only after the layer-1 MMA
 // has completed, and A1 only after the layer-2 MMA has), and D2 takes D1's tensor-memory columns (the layer-2 MMA is
 // issued after every thread has read D1): 45 KB of shared memory and 64 columns per CTA, five CTAs per SM.
+// Bound by the special-function unit (192 operations a cell, 174 us for 4 194 304 cells) and by issue: with a reciprocal a
+// unit, single additions and the library exponential's range handling that took 400 us, now 256 (GB300).
 constexpr int INF_W1 = 0, INF_W2 = 2048, INF_A2 = 10240, INF_A1 = INF_A2, INF_F = INF_A2 + 32768;
+constexpr int INF_CTAS = 5;
 constexpr int INF_SMEM = INF_F + 4 * 64 * 4 + 64 + 1024;
 
-__global__ void __launch_bounds__(MLP_THREADS, 5) mlp_infer_kernel(MlpInferArgs A) {
+__global__ void __launch_bounds__(MLP_THREADS, INF_CTAS) mlp_infer_kernel(MlpInferArgs A) {
     extern __shared__ uint8_t smraw[];
     uint8_t* sm = align1024(smraw);
     uint8_t *sW1 = sm + INF_W1, *sW2 = sm + INF_W2, *sA1 = sm + INF_A1, *sA2 = sm + INF_A2;
@@ -211,10 +261,16 @@ __global__ void __launch_bounds__(MLP_THREADS, 5) mlp_infer_kernel(MlpInferArgs 
         for (int half = 0; half < 2; ++half) {
             float z[32];
             tmem_ld32(D1, warp, 32 * half, z);
+            const float4* b4 = reinterpret_cast<const float4*>(sb1 + 32 * half);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const float zz = z[j] + sb1[32 * half + j];
-                z[j] = zz * sigm(zz);
+            for (int j = 0; j < 32; j += 4) {
+                const float4 b = b4[j >> 2];
+                const Silu2 p = silu2(make_float2(z[j], z[j + 1]), make_float2(b.x, b.y));
+                const Silu2 q = silu2(make_float2(z[j + 2], z[j + 3]), make_float2(b.z, b.w));
+                z[j] = (p.z.x * p.d.y) * p.r;
+                z[j + 1] = (p.z.y * p.d.x) * p.r;
+                z[j + 2] = (q.z.x * q.d.y) * q.r;
+                z[j + 3] = (q.z.y * q.d.x) * q.r;
             }
             store_a2<4>(sA2, tid, z, 4 * half);
         }
@@ -232,10 +288,16 @@ __global__ void __launch_bounds__(MLP_THREADS, 5) mlp_infer_kernel(MlpInferArgs 
         for (int half = 0; half < 2; ++half) {
             float z[32];
             tmem_ld32(D2, warp, 32 * half, z);
+            const float4* b4 = reinterpret_cast<const float4*>(sb2 + 32 * half);
+            const float4* w4 = reinterpret_cast<const float4*>(sw3 + 32 * half);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const float zz = z[j] + sb2[32 * half + j];
-                o += sw3[32 * half + j] * (zz * sigm(zz));
+            for (int j = 0; j < 32; j += 4) {
+                const float4 b = b4[j >> 2], w = w4[j >> 2];
+                const Silu2 p = silu2(make_float2(z[j], z[j + 1]), make_float2(b.x, b.y));
+                const Silu2 q = silu2(make_float2(z[j + 2], z[j + 3]), make_float2(b.z, b.w));
+                const float2 np = mul2(p.z, make_float2(w.x, w.y)), nq = mul2(q.z, make_float2(w.z, w.w));
+                o = __fmaf_rn(__fmaf_rn(np.y, p.d.x, np.x * p.d.y), p.r, o);
+                o = __fmaf_rn(__fmaf_rn(nq.y, q.d.x, nq.x * q.d.y), q.r, o);
             }
         }
         const float a = sigm(prior_t + o);
@@ -252,43 +314,61 @@ __global__ void __launch_bounds__(MLP_THREADS, 5) mlp_infer_kernel(MlpInferArgs 
 }
 
 // ---- training: forward + backward of one batch, weight gradients accumulated in tensor memory -------------------------
-// Shared memory (bytes): B operands W1 (64x16), W2 (64x64), W2^T (64x64); A operands of layer 1 (128x32) and layer 2
-// (128x128); GA = [dZ2^T ; dZ1^T] (128 x 128 cells) and GB = [H1 | X] (80 x 128 cells), the operands of the weight
-// gradient product D_acc += GA GB^T (rows 0..63, cols 0..63: dW2; rows 64..127, cols 64..74: dW1); DZ2 (128 x 64),
-// the A operand of dH1 = dZ2 W2.  Tensor memory: D1 [0,64), D2 [64,128), D3 = dH1 [128,192), D_acc [256,336).
-constexpr int TR_W1 = 0, TR_W2 = 2048, TR_W2T = 10240, TR_A1 = 18432, TR_A2 = 26624, TR_GA = 59392, TR_GB = 92160,
-              TR_DZ2 = 112640, TR_F = 129024;
-constexpr int TR_RED = TR_F;                       // [4 warps][3][64] float
-constexpr int TR_ACC = TR_RED + 4 * 3 * 64 * 4;   // [3][64] float + 2 scalars
-constexpr int TR_PAR = TR_ACC + 3 * 64 * 4 + 64;  // b1, b2, w3, b3
-constexpr int TR_BAR = TR_PAR + 4 * 64 * 4;
+// Four threads a cell: thread t has row t & 127 of the tile and 16 of the 64 units, t >> 7 saying which (a warp reads only its
+// own quarter of the tensor-memory lanes, and warps 4 apart share one).
+// Shared memory (bytes): B operands W1 (64x16), W2 (64x64), W2^T (64x64); A2 (128x128), the A operand of layer 2, and after
+// it GA = [dZ2^T ; dZ1^T] (128 x 128 cells); GB = [H1 | X] (80 x 128 cells); GA and GB are the operands of the weight
+// gradient product D_acc += GA GB^T (rows 0..63, cols 0..63: dW2; rows 64..127, cols 64..79: dW1); A1 (128x32), the A operand
+// of layer 1, and after it DZ2 (128 x 64), the A operand of dH1 = dZ2 W2.  Tensor memory: D1 [0,64), D2 and then
+// D3 = dH1 [64,128), D_acc [128,208).  92 KB and 256 columns a CTA, two CTAs per SM.
+//
+// Bound by latency: five dependent products a tile with barriers between them.  One thread a cell and one CTA per SM took
+// 66 us for 32 768 cells (two tiles after one another on most SMs, 64 units a thread); this takes 21 (GB300).
+constexpr int TR_THREADS = 4 * MLP_TILE, TR_CTAS = 2;
+constexpr int TR_W1 = 0, TR_W2 = 2048, TR_W2T = 10240, TR_A2 = 18432, TR_GA = TR_A2, TR_GB = 51200, TR_DZ2 = 71680,
+              TR_A1 = TR_DZ2, TR_F = 88064;
+constexpr int TR_RED = TR_F;                       // [4 row quarters][3][64] float
+constexpr int TR_ACC = TR_RED + 4 * 3 * 64 * 4;    // [3][64] float + 2 scalars
+constexpr int TR_PAR = TR_ACC + 3 * 64 * 4 + 64;   // b1, b2, w3, b3
+constexpr int TR_OUT = TR_PAR + 4 * 64 * 4;        // [4][128] float: the units' shares of the output
+constexpr int TR_BAR = TR_OUT + 4 * 128 * 4;
 constexpr int TR_SMEM = TR_BAR + 64 + 1024;
 
-// Reduce-scatter of 64 values over the warp: afterwards lane l holds the warp sums of entries 2l and 2l+1 in v[0..1].
+// Sum over the warp of 16 values: lane l holds the sum of value l >> 1 afterwards.
 template <int HALF>
 __device__ __forceinline__ void rs_stage(float* v, int lane) {
-    const bool up = (lane & (HALF / 2)) != 0;
+    const bool up = (lane & (2 * HALF)) != 0;
 #pragma unroll
     for (int i = 0; i < HALF; ++i) {
         const float send = up ? v[i] : v[i + HALF];
         const float keep = up ? v[i + HALF] : v[i];
-        v[i] = keep + __shfl_xor_sync(FULLMASK, send, HALF / 2);
+        v[i] = keep + __shfl_xor_sync(FULLMASK, send, 2 * HALF);
     }
 }
-__device__ __forceinline__ void reduce_scatter64(float* v, int lane) {
-    rs_stage<32>(v, lane);
-    rs_stage<16>(v, lane);
+__device__ __forceinline__ float reduce_scatter16(float* v, int lane) {
     rs_stage<8>(v, lane);
     rs_stage<4>(v, lane);
     rs_stage<2>(v, lane);
+    rs_stage<1>(v, lane);
+    return v[0] + __shfl_xor_sync(FULLMASK, v[0], 1);
 }
 __device__ __forceinline__ float warp_sum(float x) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(FULLMASK, x, o);
     return x;
 }
+// 16 gradient entries of consecutive parameters (a multiple of 4 from the start)
+__device__ __forceinline__ void add_grad16(float* g, const float* v) {
+    if ((reinterpret_cast<uintptr_t>(g) & 15) == 0) {
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) atomicAdd(reinterpret_cast<float4*>(g + i), make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]));
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) atomicAdd(g + i, v[i]);
+    }
+}
 
-__global__ void __launch_bounds__(MLP_THREADS, 1) mlp_grad_kernel(MlpGradArgs A) {
+__global__ void __launch_bounds__(TR_THREADS, TR_CTAS) mlp_grad_kernel(MlpGradArgs A) {
     extern __shared__ uint8_t smraw[];
     uint8_t* sm = align1024(smraw);
     uint8_t *sW1 = sm + TR_W1, *sW2 = sm + TR_W2, *sW2T = sm + TR_W2T, *sA1 = sm + TR_A1, *sA2 = sm + TR_A2,
@@ -297,42 +377,49 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_grad_kernel(MlpGradArgs A)
     float* acc = reinterpret_cast<float*>(sm + TR_ACC);
     float* sb1 = reinterpret_cast<float*>(sm + TR_PAR);
     float *sb2 = sb1 + 64, *sw3 = sb2 + 64, *sb3 = sw3 + 64;
+    float* sout = reinterpret_cast<float*>(sm + TR_OUT);
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm + TR_BAR);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int row = tid & 127, rq = warp & 3, c0 = 16 * (tid >> 7);  // cell of the tile, its row quarter, first unit
 
     stage_weights(A.params, sW1, sW2, sW2T, sb1, sb2, sw3, sb3);
-    for (int e = tid; e < 3 * 64 + 2; e += MLP_THREADS) acc[e] = 0.f;
-    // GB rows 64 + MLP_IN .. 79 (padding of the input block, when there are fewer than 16 inputs) stay zero
-    for (int e = tid; e < (16 - MLP_IN) * 128; e += MLP_THREADS) store_bf16(sGB, 64 + MLP_IN + e / 128, e % 128, 128, 0.f);
+    for (int e = tid; e < 3 * 64 + 2; e += TR_THREADS) acc[e] = 0.f;
     if (tid == 0) {
         tc::mbar_init(bar, 1);
         tc::fence_mbar_init();
     }
     if (warp == 0) {
-        tc::tmem_alloc(tslot, 512);
+        tc::tmem_alloc(tslot, 256);
         tc::tmem_relinquish();
     }
     tc::fence_smem_async();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    const uint32_t tbase = *tslot, D1 = tbase, D2 = tbase + 64, D3 = tbase + 128, DACC = tbase + 256;
+    const uint32_t tbase = *tslot, D1 = tbase, D2 = tbase + 64, D3 = D2, DACC = tbase + 128;
     const int64_t ntiles = (A.n + MLP_TILE - 1) / MLP_TILE;
     uint32_t phase = 0;
     int ntile_done = 0;
     bool alive = true;
     for (int64_t t = blockIdx.x; t < ntiles && alive; t += gridDim.x) {
-        const int64_t c = t * MLP_TILE + tid;
+        const int64_t c = t * MLP_TILE + row;
         const bool valid = c < A.n;
-        float x[MLP_IN];
+        {  // this thread's 4 inputs of the cell: hi and lo halves into A1, hi into GB
+            const int f0 = c0 >> 2;
+            float x[4];
 #pragma unroll
-        for (int f = 0; f < MLP_IN; ++f) x[f] = valid ? A.feat[f * A.stride + c] : 0.f;
+            for (int i = 0; i < 4; ++i) x[i] = valid ? A.feat[(f0 + i) * A.stride + c] : 0.f;
+            uint2 h, l;
+            split2(x[0], x[1], h.x, l.x);
+            split2(x[2], x[3], h.y, l.y);
+            *reinterpret_cast<uint2*>(sA1 + tc::kmajor_offset(row, f0, 32)) = h;
+            *reinterpret_cast<uint2*>(sA1 + tc::kmajor_offset(row, 16 + f0, 32)) = l;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) store_bf16(sGB, 64 + f0 + i, row, 128, x[i]);
+        }
         const float prior = valid ? A.feat[MLP_IN * A.stride + c] : 0.f;
         const float y = valid ? A.label[c] : 0.f;
-        store_a1(sA1, tid, x);
-#pragma unroll
-        for (int f = 0; f < MLP_IN; ++f) store_bf16(sGB, 64 + f, tid, 128, x[f]);
         tc::fence_smem_async();
         __syncthreads();
         if (tid == 0) {
@@ -341,15 +428,18 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_grad_kernel(MlpGradArgs A)
             tc::mma_commit(bar);
         }
         if (!(alive = cta_wait(bar, phase, A.error))) break;
-        float v[64];
-        tmem_ld64(D1, warp, 0, v);
+        float v[16], w[16];
+        tc::tmem_ld16(tc::tmem_addr(D1, 32 * rq, c0), v);
+        tc::tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 64; ++j) {
-            const float zz = v[j] + sb1[j];
-            v[j] = zz * sigm(zz);
-            store_bf16(sGB, j, tid, 128, v[j]);
+        for (int j = 0; j < 16; j += 2) {
+            const Silu2 p = silu2(make_float2(v[j], v[j + 1]), make_float2(sb1[c0 + j], sb1[c0 + j + 1]));
+            v[j] = (p.z.x * p.d.y) * p.r;
+            v[j + 1] = (p.z.y * p.d.x) * p.r;
+            store_bf16(sGB, c0 + j, row, 128, v[j]);
+            store_bf16(sGB, c0 + j + 1, row, 128, v[j + 1]);
         }
-        store_a2(sA2, tid, v);
+        store_a2<2>(sA2, row, v, c0 >> 3);
         tc::fence_before_sync();
         tc::fence_smem_async();
         __syncthreads();
@@ -359,46 +449,43 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_grad_kernel(MlpGradArgs A)
             tc::mma_commit(bar);
         }
         if (!(alive = cta_wait(bar, phase, A.error))) break;
-        // output layer, loss and the backward pass down to dZ2
-        tmem_ld64(D2, warp, 0, v);
-        float o = *sb3;
+        // output layer, loss and the backward pass down to dZ2: w = h2, v = dh2/dz2
+        tc::tmem_ld16(tc::tmem_addr(D2, 32 * rq, c0), v);
+        tc::tmem_wait_ld();
+        float o = 0.f;
 #pragma unroll
-        for (int j = 0; j < 64; ++j) {
-            const float zz = v[j] + sb2[j];
-            o += sw3[j] * (zz * sigm(zz));
+        for (int j = 0; j < 16; j += 2) {
+            const Silu2 p = silu2(make_float2(v[j], v[j + 1]), make_float2(sb2[c0 + j], sb2[c0 + j + 1]));
+            const float s0 = p.d.y * p.r, s1 = p.d.x * p.r;
+            w[j] = p.z.x * s0;
+            w[j + 1] = p.z.y * s1;
+            o += sw3[c0 + j] * w[j];
+            o += sw3[c0 + j + 1] * w[j + 1];
+            v[j] = s0 * (1.f + p.z.x * (1.f - s0));
+            v[j + 1] = s1 * (1.f + p.z.y * (1.f - s1));
         }
+        sout[(c0 >> 4) * 128 + row] = o;
+        __syncthreads();
+        o = *sb3 + ((sout[row] + sout[128 + row]) + (sout[256 + row] + sout[384 + row]));
         const float a = sigm(prior + o);
         const float d = valid ? a - y : 0.f;
         const float dz3 = A.scale * d * a * (1.f - a);
-        float w[64];
 #pragma unroll
-        for (int j = 0; j < 64; ++j) {
-            const float zz = v[j] + sb2[j];
-            const float s = sigm(zz);
-            w[j] = dz3 * (zz * s);                                 // dw3 contribution
-            v[j] = dz3 * sw3[j] * (s * (1.f + zz * (1.f - s)));    // dZ2
+        for (int j = 0; j < 16; ++j) {
+            w[j] *= dz3;                  // dw3 contribution
+            v[j] *= dz3 * sw3[c0 + j];    // dZ2
         }
         {
             uint32_t b[8];
 #pragma unroll
-            for (int g = 0; g < 8; ++g) {
+            for (int g = 0; g < 2; ++g) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) b[i] = bf16_bits(v[8 * g + i]);
-                store_row8(sDZ2, tid, 8 * g, 64, b);
+                for (int i = 0; i < 8; ++i) {
+                    b[i] = bf16_bits(v[8 * g + i]);
+                    *reinterpret_cast<uint16_t*>(sGA + tc::kmajor_offset(c0 + 8 * g + i, row, 128)) = (uint16_t)b[i];
+                }
+                store_row8(sDZ2, row, c0 + 8 * g, 64, b);
             }
-#pragma unroll
-            for (int j = 0; j < 64; ++j) store_bf16(sGA, j, tid, 128, v[j]);
-        }
-        reduce_scatter64(w, lane);
-        red[(warp * 3 + 0) * 64 + 2 * lane] = w[0];
-        red[(warp * 3 + 0) * 64 + 2 * lane + 1] = w[1];
-        reduce_scatter64(v, lane);
-        red[(warp * 3 + 1) * 64 + 2 * lane] = v[0];
-        red[(warp * 3 + 1) * 64 + 2 * lane + 1] = v[1];
-        const float s_dz3 = warp_sum(dz3), s_loss = warp_sum(d * d);
-        if (lane == 0) {
-            atomicAdd(&acc[192], s_dz3);
-            atomicAdd(&acc[193], s_loss);
         }
         tc::fence_before_sync();
         tc::fence_smem_async();
@@ -413,28 +500,37 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_grad_kernel(MlpGradArgs A)
                              tc::sdesc(tc::smem_u32(sW2T) + 256 * s, 128, 1024), id, s > 0);
             tc::mma_commit(bar);
         }
-        if (!(alive = cta_wait(bar, phase, A.error))) break;
-        tmem_ld64(D3, warp, 0, v);   // dH1
-        tmem_ld64(D1, warp, 0, w);   // z1 - b1
-#pragma unroll
-        for (int j = 0; j < 64; ++j) {
-            const float zz = w[j] + sb1[j];
-            const float s = sigm(zz);
-            v[j] *= s * (1.f + zz * (1.f - s));   // dZ1
-            store_bf16(sGA, 64 + j, tid, 128, v[j]);
+        // the sums over the cells, while the product runs
+        {
+            const float sw = reduce_scatter16(w, lane), sz = reduce_scatter16(v, lane);
+            if (!(lane & 1)) {
+                red[(rq * 3 + 0) * 64 + c0 + (lane >> 1)] = sw;
+                red[(rq * 3 + 1) * 64 + c0 + (lane >> 1)] = sz;
+            }
+            if (c0 == 0) {
+                const float s_dz3 = warp_sum(dz3), s_loss = warp_sum(d * d);
+                if (lane == 0) {
+                    atomicAdd(&acc[192], s_dz3);
+                    atomicAdd(&acc[193], s_loss);
+                }
+            }
         }
-        reduce_scatter64(v, lane);
-        red[(warp * 3 + 2) * 64 + 2 * lane] = v[0];
-        red[(warp * 3 + 2) * 64 + 2 * lane + 1] = v[1];
+        if (!(alive = cta_wait(bar, phase, A.error))) break;
+        tc::tmem_ld16(tc::tmem_addr(D3, 32 * rq, c0), v);   // dH1
+        tc::tmem_ld16(tc::tmem_addr(D1, 32 * rq, c0), w);   // z1 - b1
+        tc::tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 16; j += 2) {
+            const Silu2 p = silu2(make_float2(w[j], w[j + 1]), make_float2(sb1[c0 + j], sb1[c0 + j + 1]));
+            const float s0 = p.d.y * p.r, s1 = p.d.x * p.r;
+            v[j] *= s0 * (1.f + p.z.x * (1.f - s0));   // dZ1
+            v[j + 1] *= s1 * (1.f + p.z.y * (1.f - s1));
+            store_bf16(sGA, 64 + c0 + j, row, 128, v[j]);
+            store_bf16(sGA, 64 + c0 + j + 1, row, 128, v[j + 1]);
+        }
         tc::fence_before_sync();
         tc::fence_smem_async();
         __syncthreads();
-        if (tid < 64) {
-#pragma unroll
-            for (int q = 0; q < 3; ++q)
-                acc[q * 64 + tid] += red[(0 * 3 + q) * 64 + tid] + red[(1 * 3 + q) * 64 + tid] +
-                                     red[(2 * 3 + q) * 64 + tid] + red[(3 * 3 + q) * 64 + tid];
-        }
         if (tid == 0) {
             // D_acc += [dZ2^T ; dZ1^T] [H1 | X]^T over the 128 cells of the tile
             tc::fence_after_sync();
@@ -445,21 +541,29 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_grad_kernel(MlpGradArgs A)
                              tc::sdesc(tc::smem_u32(sGB) + 256 * s, 128, 2048), id, (ntile_done > 0 || s > 0) ? 1u : 0u);
             tc::mma_commit(bar);
         }
+        {
+            const float sz = reduce_scatter16(v, lane);
+            if (!(lane & 1)) red[(rq * 3 + 2) * 64 + c0 + (lane >> 1)] = sz;
+        }
         if (!(alive = cta_wait(bar, phase, A.error))) break;
+        // all threads have written their sums (cta_wait is a barrier); the next writes to red come after more barriers
+        if (tid < 3 * 64) {
+            const int q = tid >> 6, u = tid & 63;
+            acc[tid] += (red[(0 * 3 + q) * 64 + u] + red[(1 * 3 + q) * 64 + u]) + (red[(2 * 3 + q) * 64 + u] + red[(3 * 3 + q) * 64 + u]);
+        }
         ++ntile_done;
     }
     __syncthreads();
     if (alive && ntile_done > 0) {
-        float v[64];
-        if (warp < 2) {
-            tmem_ld64(DACC, warp, 0, v);
-#pragma unroll
-            for (int i = 0; i < 64; ++i) atomicAdd(&A.grad[MLP_OFF_W2 + tid * 64 + i], v[i]);
-        } else {
-            tc::tmem_ld16(tc::tmem_addr(DACC, 32 * warp, 64), v);
+        float v[16];
+        if (rq < 2) {
+            tc::tmem_ld16(tc::tmem_addr(DACC, 32 * rq, c0), v);
             tc::tmem_wait_ld();
-#pragma unroll
-            for (int f = 0; f < MLP_IN; ++f) atomicAdd(&A.grad[MLP_OFF_W1 + (tid - 64) * MLP_IN + f], v[f]);
+            add_grad16(A.grad + MLP_OFF_W2 + row * 64 + c0, v);
+        } else if (c0 == 0) {
+            tc::tmem_ld16(tc::tmem_addr(DACC, 32 * rq, 64), v);
+            tc::tmem_wait_ld();
+            add_grad16(A.grad + MLP_OFF_W1 + (row - 64) * MLP_IN, v);
         }
         if (tid < 64) {
             atomicAdd(&A.grad[MLP_OFF_W3 + tid], acc[tid]);
@@ -473,7 +577,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_grad_kernel(MlpGradArgs A)
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tbase, 512);
+    if (warp == 0) tc::tmem_dealloc(tbase, 256);
 }
 
 __global__ void mlp_adam_kernel(float* p, const float* g, float* m, float* v, float c1, float c2, float lr) {
@@ -688,14 +792,18 @@ void launch_mlp_infer(const MlpInferArgs& a, int grid, cudaStream_t st) {
 
 void launch_mlp_grad(const MlpGradArgs& a, int grid, cudaStream_t st) {
     mlp_prepare();
-    mlp_grad_kernel<<<grid, MLP_THREADS, TR_SMEM, st>>>(a);
+    mlp_grad_kernel<<<grid, TR_THREADS, TR_SMEM, st>>>(a);
 }
 
-__device__ int32_t g_mlp_error;
-
+// the kernels' error word, in page-locked host memory: written only when a wait ran out, read after the stream is
+// synchronised (a device word cost a copy on every call)
 static int32_t* error_ptr() {
-    static int32_t* p = nullptr;
-    if (!p) cudaGetSymbolAddress((void**)&p, g_mlp_error);
+    static int32_t* const p = [] {
+        int32_t* q = nullptr;
+        if (cudaHostAlloc((void**)&q, sizeof(int32_t), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) return q;
+        *q = 0;
+        return q;
+    }();
     return p;
 }
 
@@ -704,14 +812,9 @@ static int finish(cudaStream_t st) {
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return SDFIBM_ERR_CUDA;
-    int32_t dev_err = 0;
-    if (cudaMemcpyFromSymbol(&dev_err, g_mlp_error, sizeof(int32_t)) != cudaSuccess) return SDFIBM_ERR_CUDA;
-    if (dev_err) {
-        const int32_t zero = 0;
-        cudaMemcpyToSymbol(g_mlp_error, &zero, sizeof(int32_t));
-        return SDFIBM_ERR_TIMEOUT;
-    }
-    return SDFIBM_OK;
+    int32_t* err = error_ptr();
+    if (!err) return SDFIBM_ERR_CUDA;
+    return __atomic_exchange_n(err, 0, __ATOMIC_ACQ_REL) ? SDFIBM_ERR_TIMEOUT : SDFIBM_OK;
 }
 
 }  // namespace sdfibm_dev
@@ -756,9 +859,10 @@ int sdfibm_mlp_forward(const float* params_dev, const float* feat_dev, int64_t s
     a.n = n;
     a.out = out_dev;
     a.error = error_ptr();
+    if (!a.error) return SDFIBM_ERR_CUDA;
     cudaStream_t st = (cudaStream_t)stream;
     const int64_t ntiles = (n + MLP_TILE - 1) / MLP_TILE;
-    launch_mlp_infer(a, (int)std::min<int64_t>(ntiles, 4 * mlp_sm_count()), st);
+    launch_mlp_infer(a, (int)std::min<int64_t>(ntiles, INF_CTAS * mlp_sm_count()), st);
     return finish(st);
 }
 
@@ -774,8 +878,9 @@ static int loss_grad_async(const float* params_dev, const float* feat_dev, const
     a.scale = 2.0f / (float)n;
     a.grad = grad_dev;
     a.error = error_ptr();
+    if (!a.error) return SDFIBM_ERR_CUDA;
     const int64_t ntiles = (n + MLP_TILE - 1) / MLP_TILE;
-    launch_mlp_grad(a, (int)std::min<int64_t>(ntiles, mlp_sm_count()), st);
+    launch_mlp_grad(a, (int)std::min<int64_t>(ntiles, TR_CTAS * mlp_sm_count()), st);
     return SDFIBM_OK;
 }
 
