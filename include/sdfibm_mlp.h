@@ -73,7 +73,7 @@ int sdfibm_mlp_forward(const float* params_dev, const float* feat_dev, int64_t s
                        void* stream);
 
 /* Gradient of loss = mean over the n cells of (a - label)^2.  grad_dev: FP32 [SDFIBM_MLP_NPARAM + 1], overwritten:
- * the gradient, then the sum of (a - label)^2. */
+ * the gradient, then the sum of (a - label)^2; device or page-locked host memory. */
 int sdfibm_mlp_loss_grad(const float* params_dev, const float* feat_dev, const float* label_dev, int64_t stride,
                          int64_t n, float* grad_dev, void* stream);
 

@@ -1103,11 +1103,12 @@ __global__ void finalize_kernel(float* __restrict__ As, float* __restrict__ Ts, 
     }
 }
 
-// forces and counters into page-locked host memory (read after the stream is synchronised): one launch instead of two copies
-__global__ void export_ft_kernel(const double* __restrict__ ft, int64_t n, const Counters* __restrict__ cnt,
-                                 double* __restrict__ h_ft, Counters* __restrict__ h_cnt) {
+// n doubles (forces, solid states) and the counters into page-locked host memory, read after the stream is synchronised: one
+// launch instead of two copies
+__global__ void export_host_kernel(const double* __restrict__ src, int64_t n, const Counters* __restrict__ cnt,
+                                   double* __restrict__ dst, Counters* __restrict__ h_cnt) {
     const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t e = t0; e < n; e += nt) h_ft[e] = ft[e];
+    for (int64_t e = t0; e < n; e += nt) dst[e] = src[e];
     const uint32_t* a = reinterpret_cast<const uint32_t*>(cnt);
     uint32_t* b = reinterpret_cast<uint32_t*>(h_cnt);
     if (t0 < (int64_t)(sizeof(Counters) / 4)) b[t0] = a[t0];

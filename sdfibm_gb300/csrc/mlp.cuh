@@ -305,6 +305,12 @@ struct MlpInferArgs {
     int32_t* error;          // set to SDFIBM_MLP_ERR_TIMEOUT when an MMA completion is not seen in time
 };
 
+// sums of a gradient call (zero between calls)
+struct MlpGradAcc {
+    float sum[(MLP_NPARAM + 4) & ~3];
+    unsigned done;  // CTAs that have added theirs
+};
+
 struct MlpGradArgs {
     const float* params;
     const float* feat;       // [MLP_NFEAT][stride]
@@ -312,7 +318,8 @@ struct MlpGradArgs {
     int64_t stride;
     int64_t n;               // cells of this batch
     float scale;             // 2 / (cells in the batch): d loss / d a = scale * (a - y)
-    float* grad;             // FP32 [MLP_NPARAM + 1], accumulated with atomics; the last entry sums (a - y)^2
+    float* grad;             // FP32 [MLP_NPARAM + 1], device or page-locked; the last entry is the sum of (a - y)^2
+    MlpGradAcc* acc;
     int32_t* error;
 };
 

@@ -70,10 +70,10 @@ def forward(torch, params, feat):
 def loss_grad(torch, params, feat, label):
     """(mean loss, gradient [4993]) of loss = mean((a - label)^2) over the cells."""
     n = feat.shape[1]
-    g = torch.empty(abi.MLP_NPARAM + 1, dtype=torch.float32, device="cuda")
+    g = torch.empty(abi.MLP_NPARAM + 1, dtype=torch.float32, pin_memory=True)  # written by the GPU, no copy
     _check(load().sdfibm_mlp_loss_grad(_ptr(params), _ptr(feat), _ptr(label), feat.stride(0), n, _ptr(g),
                                        _stream(torch)), "sdfibm_mlp_loss_grad")
-    g = g.cpu().numpy()
+    g = g.numpy()
     return float(g[-1]) / n, g[:-1].copy()
 
 
