@@ -224,7 +224,7 @@ struct ClassifyArgs {
     int64_t* fref_index;  // index into alpha
     Recheck* rq;          // deferred SUBSAMPLE rechecks (nullptr: re-evaluate in place)
     int64_t rq_cap;
-    float* rg_phi;        // REF-GEO: [8][feat_cap] vertex distances of the listed cut cells (nullptr: fraction in place)
+    float* rg_phi;        // REF-GEO: [8][feat_cap] vertex distances of the listed cut cells
     // LEARNED: solids whose bounding radius spans fewer cells (SolidPlan::radius_cells) list their cut cells from the
     // back of the list (positions feat_cap - 1 - i, n_small of them): the band sends them to the fallback whole
     float rho_min;
