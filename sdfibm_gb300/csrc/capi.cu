@@ -34,13 +34,7 @@ __global__ void refgeo_cells_kernel(MeshK m, const SolidK* sk, const SolidPlan* 
                                     float* alpha);
 __global__ void recheck_kernel(MeshK m, const SolidK* sk, const sdfibm_solid_state* st, const SolidPlan* plan,
                                const Recheck* rq, int64_t cap, Counters* cnt, float* alpha);
-__global__ void connect_kernel(MeshK m, const SolidK* sk, SolidPlan* plan, const uint8_t* scratch, uint32_t* gbitmaps,
-                               int32_t* in_cell, int32_t* in_solid, int32_t* cut_cell, int32_t* cut_solid,
-                               int64_t cap_in, int64_t cap_cut, Counters* cnt, const int32_t* solids);
-__global__ void connect_small_kernel(MeshK m, const SolidK* sk, SolidPlan* plan, const uint8_t* scratch,
-                                     int32_t* in_cell, int32_t* in_solid, int32_t* cut_cell, int32_t* cut_solid,
-                                     int64_t cap_in, int64_t cap_cut, Counters* cnt, const int32_t* solids,
-                                     int nsolids);
+__global__ void connect_kernel(ConnectArgs A);
 
 __global__ void scan_reset_kernel(const int32_t* in_cell, const int32_t* cut_cell, Counters* cnt, int64_t N,
                                   const uint32_t* sbits, uint32_t* shent, int64_t shent_cap, const int32_t* prev_in_cell,
@@ -141,8 +135,8 @@ struct sdfibm_ctx {
     int64_t gbitmap_words = 0;
     int connect_smem_bytes = 0;
     // flood-fill work: solids with small bbox bitmaps (one warp each) and the others (one CTA each)
-    int32_t *d_small = nullptr, *d_big = nullptr;
-    int n_small = 0, n_big = 0;
+    int32_t* d_by_size = nullptr;  // solids of connect_kernel, the largest bitmaps first
+    int n_small = 0, n_mid = 0, n_big = 0;
     // SUBSAMPLE points whose FP32 test was undecided, re-evaluated in FP64 on full warps by recheck_kernel
     Recheck* d_rq = nullptr;
     int64_t rq_cap = 0;
@@ -417,7 +411,13 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
 
     // static per-solid records
     ctx->hk.resize(nsolids);
-    std::vector<int32_t> small_solids, big_solids;
+    std::vector<int32_t> small_solids, mid_solids, big_solids;
+    // connect_kernel: words of a solid's bitmaps up to which it goes to a warp and to CON_MID threads.  A solid is done soonest
+    // by a CTA, most solids a second are done with few threads each: 100 circles of 200 words take 16 us as CTAs, 25 in groups
+    // of 128 and 43 as warps; 16 384 solids in 512^3 0.26 ms with warps up to 256 words, 0.28 up to 128, 0.38 all as CTAs;
+    // 1800 solids 29 us with warps up to 128 words, 31 up to 256.
+    const int t_small = nsolids >= 64 * ctx->num_sms ? CON_SMALL_WORDS : (nsolids >= 4 * ctx->num_sms ? 128 : 32);
+    const int t_mid = nsolids >= 4 * ctx->num_sms ? CON_MID_WORDS : 0;
     int64_t scratch = 0, gwords = 0, bbox_total = 0;
     int64_t tiles = 0;
     int max_smem_words = 0;
@@ -473,17 +473,16 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
         bbox_total += std::min<int64_t>(cells, N);
         // connect_kernel: four bitmaps (candidates, reached, inside, centre inside) of ext[1] * ext[2] rows
         const int64_t words = 4 * (int64_t)k.ext[1] * k.ext[2] * ((k.ext[0] + 31) / 32);
-        if (words / 4 <= (nsolids >= 8 * ctx->num_sms ? 256 : 32)) {
-            // a warp per solid (connect_small_kernel): small bitmaps, and medium ones when there are solids enough to fill
-            // the GPU that way (100 circles of 200 words: 65 us as warps, under 19 us as CTAs)
-            small_solids.push_back(s);
-        } else if (words * 4 > SMEM_CAP_BYTES) {
-            k.bitmap_global = 1;
-            k.bitmap_off = gwords;
-            gwords += words;
-            big_solids.push_back(s);
-        } else {
-            max_smem_words = std::max<int>(max_smem_words, (int)words);
+        if (words / 4 <= t_small) small_solids.push_back(s);
+        else if (words / 4 <= t_mid) mid_solids.push_back(s);
+        else {
+            if (words * 4 > SMEM_CAP_BYTES) {
+                k.bitmap_global = 1;
+                k.bitmap_off = gwords;
+                gwords += words;
+            } else {
+                max_smem_words = std::max<int>(max_smem_words, (int)words);
+            }
             big_solids.push_back(s);
         }
         k.motion_type = d.motion_type;
@@ -500,7 +499,10 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
         return (int64_t)ka.ext[0] * ka.ext[1] * ka.ext[2] > (int64_t)kb.ext[0] * kb.ext[1] * kb.ext[2];
     };
     std::stable_sort(big_solids.begin(), big_solids.end(), larger);
+    std::stable_sort(mid_solids.begin(), mid_solids.end(), larger);
     std::stable_sort(small_solids.begin(), small_solids.end(), larger);
+    if (!mid_solids.empty()) max_smem_words = std::max(max_smem_words, 4 * 4 * CON_MID_WORDS);
+    if (!small_solids.empty()) max_smem_words = std::max(max_smem_words, 16 * 4 * CON_SMALL_WORDS);
     if (tiles >= ((int64_t)1 << 31)) { ctx->err = "too many bbox tiles"; return bail(SDFIBM_ERR_CAPACITY); }
     ctx->total_tiles = (int)tiles;
     ctx->chunks_cap = tiles;
@@ -508,7 +510,11 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
     ctx->gbitmap_words = gwords;
     ctx->connect_smem_bytes = max_smem_words * 4;
     ctx->n_small = (int)small_solids.size();
+    ctx->n_mid = (int)mid_solids.size();
     ctx->n_big = (int)big_solids.size();
+    std::vector<int32_t> by_size(big_solids);
+    by_size.insert(by_size.end(), mid_solids.begin(), mid_solids.end());
+    by_size.insert(by_size.end(), small_solids.begin(), small_solids.end());
     ctx->rq_cap = ctx->opt.recheck_cap > 0 ? (int64_t)ctx->opt.recheck_cap
                                             : std::min<int64_t>(std::max<int64_t>(scratch / 8, 1 << 20), 1 << 25);
     ctx->ovf_cap = std::max<int64_t>(ctx->rq_cap / 16, std::min<int64_t>(scratch, 1 << 16));
@@ -631,7 +637,7 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
         dalloc(&ctx->d_cbits, (size_t)(ctx->mesh.ncells + 255) / 256) ||
         dalloc(&ctx->d_sbits, (size_t)(ctx->mesh.ncells + 255) / 256) || dalloc(&ctx->d_shent, (size_t)ctx->shent_cap) ||
         dalloc(&ctx->d_centres, (size_t)mesh->nx + mesh->ny + mesh->nz) ||
-        dalloc(&ctx->d_small, small_solids.size()) || dalloc(&ctx->d_big, big_solids.size()) ||
+        dalloc(&ctx->d_by_size, by_size.size()) ||
         dalloc(&ctx->d_rq, (size_t)ctx->rq_cap) || dalloc(&ctx->d_ovf, (size_t)ctx->ovf_cap) ||
         (cell_list &&
          (dalloc(&ctx->d_fref_solid, (size_t)ctx->feat_cap) || dalloc(&ctx->d_fref_index, (size_t)ctx->feat_cap))) ||
@@ -676,8 +682,7 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
     };
     if (up(c->d_sk, c->hk.data(), sizeof(SolidK) * nsolids) || up(c->d_st, st.data(), sizeof(sdfibm_solid_state) * nsolids) ||
         up(c->d_chunks, chunks.data(), sizeof(int2) * chunks.size()) ||
-        up(c->d_small, small_solids.data(), sizeof(int32_t) * small_solids.size()) ||
-        up(c->d_big, big_solids.data(), sizeof(int32_t) * big_solids.size()) ||
+        up(c->d_by_size, by_size.data(), sizeof(int32_t) * by_size.size()) ||
         cudaMemset(c->d_cnt, 0, sizeof(Counters)) != cudaSuccess ||
         cudaMemset(c->d_sh_keys, 0xff, sizeof(int32_t) * ((size_t)c->sh_mask + 1)) != cudaSuccess ||
         cudaMemset(c->d_sh_vals, 0, sizeof(double) * 5 * ((size_t)c->sh_mask + 1)) != cudaSuccess ||
@@ -823,14 +828,12 @@ static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float
             CK(cudaEventRecord(ctx->ev_fork, st));
             CK(cudaStreamWaitEvent(sb, ctx->ev_fork, 0));
         }
-        if (ctx->n_small > 0)
-            connect_small_kernel<<<(ctx->n_small + 7) / 8, 256, 0, sb>>>(
-                ctx->mesh, ctx->d_sk, ctx->d_plan, ctx->d_scratch, ctx->in_cell(), ctx->in_solid(), ctx->cut_cell(),
-                ctx->cut_solid(), ctx->cap, ctx->cap, ctx->d_cnt, ctx->d_small, ctx->n_small);
-        if (ctx->n_big > 0)
-            connect_kernel<<<ctx->n_big, 512, ctx->connect_smem_bytes, sb>>>(
-                ctx->mesh, ctx->d_sk, ctx->d_plan, ctx->d_scratch, ctx->d_gbitmaps, ctx->in_cell(), ctx->in_solid(),
-                ctx->cut_cell(), ctx->cut_solid(), ctx->cap, ctx->cap, ctx->d_cnt, ctx->d_big);
+        ConnectArgs ca{};
+        ca.m = ctx->mesh; ca.sk = ctx->d_sk; ca.plan = ctx->d_plan; ca.scratch = ctx->d_scratch; ca.gbitmaps = ctx->d_gbitmaps;
+        ca.in_cell = ctx->in_cell(); ca.in_solid = ctx->in_solid(); ca.cut_cell = ctx->cut_cell();
+        ca.cut_solid = ctx->cut_solid(); ca.cap_in = ca.cap_cut = ctx->cap; ca.cnt = ctx->d_cnt; ca.solids = ctx->d_by_size;
+        ca.n_big = ctx->n_big; ca.n_mid = ctx->n_mid; ca.n_small = ctx->n_small;
+        connect_kernel<<<ctx->n_big + (ctx->n_mid + 3) / 4 + (ctx->n_small + 15) / 16, 512, ctx->connect_smem_bytes, sb>>>(ca);
         mark(ctx, "connect_kernel");
         claim_kernel<<<ctx->num_sms * 8, 256, 0, sb>>>(ctx->in_cell(), ctx->in_solid(), ctx->cut_cell(),
                                                         ctx->cut_solid(), Ct, ctx->d_cnt, N, ctx->d_cbits,
@@ -1713,7 +1716,7 @@ void sdfibm_cuda_destroy(sdfibm_ctx* ctx) {
     for (void* p : dev)
         if (p) cudaFree(p);
     if (ctx->d_step) cudaFree(ctx->d_step);
-    if (ctx->d_small) cudaFree(ctx->d_small);
+    if (ctx->d_by_size) cudaFree(ctx->d_by_size);
     if (ctx->d_rq) cudaFree(ctx->d_rq);
     if (ctx->d_ovf) cudaFree(ctx->d_ovf);
     if (ctx->d_dirty) cudaFree(ctx->d_dirty);
@@ -1744,7 +1747,6 @@ void sdfibm_cuda_destroy(sdfibm_ctx* ctx) {
     if (ctx->ev_tpre) cudaEventDestroy(ctx->ev_tpre);
     if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
     if (ctx->side_st) cudaStreamDestroy(ctx->side_st);
-    if (ctx->d_big) cudaFree(ctx->d_big);
     for (auto& g : ctx->igraph)
         if (g.valid) cudaGraphExecDestroy(g.exec);
     if (ctx->egraph.valid) cudaGraphExecDestroy(ctx->egraph.exec);

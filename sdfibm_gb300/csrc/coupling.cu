@@ -258,44 +258,56 @@ __global__ void __launch_bounds__(96) plan_kernel(PrepArgs A) {
 // below CT_KEY_BASE -- zero, or the decoded Ct a previous call left -- is an unclaimed cell.
 // One atomicMax claims the cell (any previous value is below every claim word); seeing another claim of this call
 // in its return value, the claimer raises the word to the larger claim with CT_SHARED set.
-__device__ inline bool claim_cell(int32_t* Ct, int32_t cell, int32_t s, int type) {
-    uint32_t* C = reinterpret_cast<uint32_t*>(Ct) + cell;
-    const uint32_t key = CT_KEY_BASE | ((uint32_t)s << 2) | (uint32_t)type;
-    const uint32_t old = atomicMax(C, key);
-    if (old < CT_KEY_BASE) return false;
-    atomicMax(C, max(key, old & ~CT_SHARED) | CT_SHARED);
-    return true;
-}
 
 // set bit (c >> 3) of a chunk bitmap (one bit per 8 consecutive cells)
-__device__ inline void mark_chunk(uint32_t* bits, int64_t c) {
-    uint32_t* w = bits + (c >> 8);
-    const uint32_t b = 1u << ((c >> 3) & 31);
-    if (!(*w & b)) atomicOr(w, b);
-}
+__device__ inline void mark_chunk(uint32_t* bits, int64_t c) { atomicOr(bits + (c >> 8), 1u << ((c >> 3) & 31)); }
 
 // claim pass over this call's lists; marks the chunks of the claimed cells in cbits and, for a cell claimed more than
-// once, in sbits (every claimer after the first sees an earlier claim, so each shared cell's chunk is marked)
-__global__ void claim_kernel(const int32_t* __restrict__ in_cell, const int32_t* __restrict__ in_solid,
-                             const int32_t* __restrict__ cut_cell, const int32_t* __restrict__ cut_solid,
-                             int32_t* __restrict__ Ct, Counters* cnt, int64_t N, uint32_t* __restrict__ cbits,
-                             uint32_t* __restrict__ sbits) {
-    const int n_in = clamp_len(cnt->n_inside, cnt->list_cap), n_cut = clamp_len(cnt->n_cut, cnt->list_cap);
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)n_in + n_cut;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const bool cut = e >= n_in;
-        const int64_t ee = cut ? e - n_in : e;
-        const int32_t c = cut ? cut_cell[ee] : in_cell[ee];
-        const int32_t sw = cut ? cut_solid[ee] : in_solid[ee];
-        if (c < 0 || c >= N) continue;
-        const bool shared = claim_cell(Ct, c, sw & LIST_SOLID_MASK, list_type(sw));
-        if (cbits) {
-            mark_chunk(cbits, c);
-            if (shared) {
-                mark_chunk(sbits, c);
-                atomicAdd(&cnt->shared_marks, 1);
+// once, in sbits (every claimer after the first sees an earlier claim, so each shared cell's chunk is marked).
+// Bound by the latency of the claims (a returning atomic on a line in memory), so a thread has four in flight; neighbours in
+// the lists are neighbours on the mesh, so the first lane of a run marks its chunk.  0.150 -> 0.099 ms at 512^3 and 16 384
+// solids, 0.030 -> 0.018 at 256^3 and 4096 (GB300).
+constexpr int CLAIM_BATCH = 4;
+__global__ void __launch_bounds__(256) claim_kernel(const int32_t* __restrict__ in_cell, const int32_t* __restrict__ in_solid,
+                                                    const int32_t* __restrict__ cut_cell, const int32_t* __restrict__ cut_solid,
+                                                    int32_t* __restrict__ Ct, Counters* cnt, int64_t N,
+                                                    uint32_t* __restrict__ cbits, uint32_t* __restrict__ sbits) {
+    const int64_t n_in = clamp_len(cnt->n_inside, cnt->list_cap), n = n_in + clamp_len(cnt->n_cut, cnt->list_cap);
+    const int lane = threadIdx.x & 31;
+    const int64_t step = (int64_t)gridDim.x * blockDim.x * CLAIM_BATCH;
+    // whole warps: a warp's entries of a batch are consecutive
+    for (int64_t e0 = (int64_t)blockIdx.x * blockDim.x * CLAIM_BATCH + threadIdx.x; e0 - lane < n; e0 += step) {
+        int32_t c[CLAIM_BATCH];
+        uint32_t key[CLAIM_BATCH], old[CLAIM_BATCH];
+#pragma unroll
+        for (int u = 0; u < CLAIM_BATCH; ++u) {
+            const int64_t e = e0 + u * (int64_t)blockDim.x;
+            c[u] = -1;
+            key[u] = 0u;
+            if (e < n) {
+                const bool cut = e >= n_in;
+                const int64_t ee = cut ? e - n_in : e;
+                c[u] = cut ? cut_cell[ee] : in_cell[ee];
+                const int32_t sw = cut ? cut_solid[ee] : in_solid[ee];
+                key[u] = CT_KEY_BASE | ((uint32_t)(sw & LIST_SOLID_MASK) << 2) | (uint32_t)list_type(sw);
+                if (c[u] >= N) c[u] = -1;
             }
         }
+#pragma unroll
+        for (int u = 0; u < CLAIM_BATCH; ++u)
+            old[u] = c[u] >= 0 ? atomicMax(reinterpret_cast<uint32_t*>(Ct) + c[u], key[u]) : 0u;
+#pragma unroll
+        for (int u = 0; u < CLAIM_BATCH; ++u) {
+            const int32_t chunk = c[u] >> 3, before = __shfl_up_sync(0xffffffffu, chunk, 1);
+            if (c[u] >= 0 && (lane == 0 || before != chunk)) mark_chunk(cbits, c[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < CLAIM_BATCH; ++u)
+            if (old[u] >= CT_KEY_BASE) {  // claimed before in this call
+                atomicMax(reinterpret_cast<uint32_t*>(Ct) + c[u], max(key[u], old[u] & ~CT_SHARED) | CT_SHARED);
+                mark_chunk(sbits, c[u]);
+                atomicAdd(&cnt->shared_marks, 1);
+            }
     }
 }
 
@@ -306,7 +318,10 @@ __device__ inline int32_t decode_claim(uint32_t w) {
 }
 
 // ---- connect: the connected set of the seed, bit-parallel --------------------------------------------------------------------------------
-constexpr int CON_THREADS = 512;
+constexpr int CON_THREADS = 512;       // a CTA: one solid, or CON_MID_GROUPS groups of CON_MID with a solid each, or 16 warps
+constexpr int CON_MID = 128;
+constexpr int CON_MID_GROUPS = CON_THREADS / CON_MID;
+constexpr int CON_WARPS = CON_THREADS / 32;
 
 // fill upward (towards higher bits) inside runs of c starting from seeds s (s subset of c)
 __device__ inline uint32_t fill_up(uint32_t c, uint32_t s) { return (((c + s) ^ c) & c) | s; }
@@ -337,17 +352,17 @@ __device__ inline int64_t seed_bit(const SolidPlan& pl, const ActiveBox& b) {
     return x + (int64_t)b.n[0] * (y + (int64_t)b.n[1] * z);
 }
 
-// The reached cells of one solid by a group of NT threads (a CTA, or a warp): bitmaps of the active box, rows along x of W
-// words, C (an inside vertex), I (all inside) and T (centre inside) from the class bytes, then the connected set of the
-// seed, then the lists in ascending label order.
+// The reached cells of one solid by a group of NT threads (a warp, CON_MID threads or a CTA):
+// bitmaps of the active box, rows along x of W words, C (an inside vertex), I (all inside) and T (centre inside) from the class
+// bytes, then the connected set of the seed, then the lists in ascending label order.
 //
 // Nearly every set is connected, and that can be seen in one parallel pass: every row of candidates is one run, every
 // non-empty row but the first of its layer shares a column with the row before it, and every non-empty layer but the
 // first has such a pair with the layer below.  Then C is the answer.  Only sets that fail this (plates thinner than a
-// cell, concave shapes) are flooded from the seed, in sweeps that carry serial chains along y and z.  Bound by latency and
-// by the launch's tail (one CTA per solid, the largest first).  Measured (GB300): 0.69 -> 0.45 ms at 512^3 and 16 384 solids,
-// 0.18 -> 0.11 at 256^3 and 4096, 0.69 -> 0.02 for the four walls of a 1024^2 box (which the plan's vertex box reduces to
-// the cells beside the walls).
+// cell, concave shapes) are flooded from the seed, in sweeps that carry serial chains along y and z.  Bound by issue and
+// by the largest solids, which a launch cannot end without.  Measured (GB300): bitmaps by a byte a lane and a ballot, lists by a
+// word at a time, 0.52 ms at 512^3 and 16 384 solids and 0.16 at 256^3 and 4096; 16 bytes a lane, and lists by a lane a cell,
+// 0.26 and 0.059.
 __device__ inline FastDiv device_fastdiv(uint32_t d) {  // make_fastdiv for d < 2^31
     const uint32_t l = d <= 1 ? 0 : 32 - __clz(d - 1);
     return FastDiv{((1ull << (32 + l)) + d - 1) / d, 32 + l, d};
@@ -358,20 +373,209 @@ struct ConnectShared {
     FastDiv div_sy, div_w;   // by the rows per layer and by the words per row
     int cnt[16][2];          // reached cells of each warp's words
 };
+// barrier of a solid's group: a warp, CON_MID threads (each group its own hardware barrier), or the CTA
 template <int NT>
 __device__ __forceinline__ void group_sync() {
     if (NT == 32) __syncwarp();
-    else __syncthreads();
+    else if (NT == CON_THREADS) __syncthreads();
+    else asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / NT), "n"(NT) : "memory");
 }
 template <int NT>
-__device__ __forceinline__ void connect_body(const MeshK& m, const SolidK& k, SolidPlan& pl, const uint8_t* cls, int s,
-                                             uint32_t* bitmaps, ConnectShared& sh, uint32_t* layers, int max_layers,
-                                             int tid, int32_t* in_cell, int32_t* in_solid, int32_t* cut_cell,
-                                             int32_t* cut_solid, int64_t cap_in, int64_t cap_cut, Counters* cnt) {
+__device__ __forceinline__ bool group_any(bool p) {
+    if (NT == 32) return __any_sync(0xffffffffu, p);
+    if (NT == CON_THREADS) return __syncthreads_or(p) != 0;
+    uint32_t r;
+    asm volatile(
+        "{\n .reg .pred a, b;\n setp.ne.u32 a, %1, 0;\n barrier.cta.red.or.pred b, %2, %3, a;\n selp.u32 %0, 1, 0, b;\n}"
+        : "=r"(r)
+        : "r"((uint32_t)p), "r"(1 + (int)threadIdx.x / NT), "n"(NT)
+        : "memory");
+    return r != 0;
+}
+
+// rows of the active box, W words each
+struct ConnectRows {
+    int sx, sy, W, rows;
+    FastDiv dsy, dw;
+};
+// bits 0 and 1 of 16 class bytes as two 16-bit masks
+__device__ __forceinline__ void class_bits(uint4 v, uint32_t& b0, uint32_t& b1) {
+    const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+    b0 = b1 = 0u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {  // the product gathers the bytes' low bits in bits 28..31
+        b0 |= (((x[i] & 0x01010101u) * 0x10204080u) >> 28) << (4 * i);
+        b1 |= ((((x[i] >> 1) & 0x01010101u) * 0x10204080u) >> 28) << (4 * i);
+    }
+}
+// bitmaps of the rows: a thread per word, which reads the up to 32 class bytes as the aligned 16-byte pieces they lie in (the
+// bytes around them, other rows' or stale, are shifted and masked away; a solid's bytes begin and end with whole pieces)
+template <int NT>
+__device__ __forceinline__ void connect_bitmaps(const SolidK& k, const uint8_t* cls, const int* off, const ConnectRows& q, uint32_t* C,
+                                                uint32_t* I, uint32_t* T, int tid) {
+    const int nwords = q.rows * q.W;
+    for (int w = tid; w < nwords; w += NT) {
+        const int r = q.W == 1 ? w : (int)fdiv((uint32_t)w, q.dw), x = (w - r * q.W) << 5;
+        const int kk = (int)fdiv((uint32_t)r, q.dsy), jj = r - kk * q.sy, n = min(32, q.sx - x);
+        const uint8_t* p = cls + off[0] + x + (int64_t)k.ext[0] * ((jj + off[1]) + (int64_t)k.ext[1] * (kk + off[2]));
+        const int sh = (int)((uintptr_t)p & 15);
+        const uint4* p4 = reinterpret_cast<const uint4*>(p - sh);
+        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+        const uint4 v0 = p4[0], v1 = sh + n > 16 ? p4[1] : zero, v2 = sh + n > 32 ? p4[2] : zero;
+        uint32_t l0, l1, m0, m1, h0, h1;
+        class_bits(v0, l0, l1);
+        class_bits(v1, m0, m1);
+        class_bits(v2, h0, h1);
+        const uint32_t msk = n == 32 ? 0xffffffffu : (1u << n) - 1u;
+        const uint32_t b0 = __funnelshift_r(l0 | (m0 << 16), h0, sh) & msk, b1 = __funnelshift_r(l1 | (m1 << 16), h1, sh) & msk;
+        C[w] = b0 | b1;   // classes: 1 all inside, 2 centre inside, 3 cut
+        I[w] = b0 & ~b1;
+        T[w] = b1 & ~b0;
+    }
+}
+// what the rows say of the set's connectivity, into sh.bad, sh.starts and the layer bitmaps
+template <int NT>
+__device__ __forceinline__ void connect_proof(const ConnectRows& q, const uint32_t* C, ConnectShared& sh, uint32_t* layers, int lw,
+                                              int tid) {
     const unsigned FULL = 0xffffffffu;
-    const int lane = tid & 31, wid = tid >> 5;
+    int bad = 0, starts = 0;
+    for (int r = tid; r < q.rows; r += NT) {
+        const uint32_t* c = C + r * q.W;
+        const int kk = (int)fdiv((uint32_t)r, q.dsy), jj = r - kk * q.sy;
+        int first = -1, last = -1, pop = 0;
+        uint32_t along = 0, below = 0;
+        for (int w = 0; w < q.W; ++w) {
+            const uint32_t x = c[w];
+            if (!x) continue;
+            pop += __popc(x);
+            if (first < 0) first = (w << 5) + __ffs(x) - 1;
+            last = (w << 5) + 31 - __clz(x);
+            if (jj > 0) along |= x & c[w - q.W];
+            if (kk > 0) below |= x & c[w - q.W * q.sy];
+        }
+        if (pop == 0) continue;
+        if (last - first + 1 != pop) ++bad;
+        if (!along) ++starts;
+        atomicOr(layers + (kk >> 5), 1u << (kk & 31));
+        if (below) atomicOr(layers + lw + (kk >> 5), 1u << (kk & 31));
+    }
+    bad = __reduce_add_sync(FULL, bad);
+    starts = __reduce_add_sync(FULL, starts);
+    if ((tid & 31) == 0) {
+        if (bad) atomicAdd(&sh.bad, bad);
+        if (starts) atomicAdd(&sh.starts, starts);
+    }
+}
+// the words [w0, w1) of warp tid / 32
+template <int NT>
+__device__ __forceinline__ void connect_share(int nwords, int tid, int& w0, int& w1) {
     constexpr int NW = NT / 32;
-    const ActiveBox b = active_box(m, k, pl);
+    const int per = (((nwords + NW - 1) / NW) + 31) & ~31;
+    w0 = min(nwords, (tid >> 5) * per);
+    w1 = min(nwords, w0 + per);
+}
+// reached cells: sh.cnt of every warp, then the sums before this warp and of the group
+template <int NT>
+__device__ __forceinline__ void connect_count(const uint32_t* C, const uint32_t* I, int nwords, ConnectShared& sh, int tid) {
+    const unsigned FULL = 0xffffffffu;
+    int w0, w1, nin = 0, ncut = 0;
+    connect_share<NT>(nwords, tid, w0, w1);
+    for (int w = w0 + (tid & 31); w < w1; w += 32) {
+        const uint32_t bits = C[w], in = I[w];
+        nin += __popc(bits & in);
+        ncut += __popc(bits & ~in);
+    }
+    nin = __reduce_add_sync(FULL, nin);
+    ncut = __reduce_add_sync(FULL, ncut);
+    if ((tid & 31) == 0) { sh.cnt[tid >> 5][0] = nin; sh.cnt[tid >> 5][1] = ncut; }
+}
+template <int NT>
+__device__ __forceinline__ void connect_sums(const ConnectShared& sh, int tid, int& before_in, int& before_cut, int& tot_in,
+                                             int& tot_cut) {
+    before_in = before_cut = tot_in = tot_cut = 0;
+#pragma unroll
+    for (int i = 0; i < NT / 32; ++i) {
+        const int a = sh.cnt[i][0], c = sh.cnt[i][1];
+        if (i < (tid >> 5)) { before_in += a; before_cut += c; }
+        tot_in += a;
+        tot_cut += c;
+    }
+}
+// position of the r-th set bit (r < popc(m))
+__device__ __forceinline__ int nth_bit(uint32_t m, int r) {
+    int p = 0;
+#pragma unroll
+    for (int h = 16; h > 0; h >>= 1) {
+        const int c = __popc((m >> p) & ((1u << h) - 1u));
+        if (r >= c) { r -= c; p += h; }
+    }
+    return p;
+}
+// the lists of the rows from pin and pcut on: 32 words at a time, a lane per listed cell, which finds its word in the prefix
+// sums and its bit in the word
+template <int NT>
+__device__ __forceinline__ void connect_emit(const ConnectArgs& A, int s, const int* c0, const ConnectRows& q, const uint32_t* C,
+                                             const uint32_t* I, const uint32_t* T, int64_t pin, int64_t pcut, int tid) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = tid & 31;
+    int w0, w1;
+    connect_share<NT>(q.rows * q.W, tid, w0, w1);
+    for (int wb = w0; wb < w1; wb += 32) {
+        const int w = wb + lane;
+        uint32_t bits = 0, in = 0, ci = 0;
+        int label = 0;
+        if (w < w1) {
+            bits = C[w]; in = I[w]; ci = T[w];
+            const int r = (int)fdiv((uint32_t)w, q.dw), kk = (int)fdiv((uint32_t)r, q.dsy), jj = r - kk * q.sy;
+            label = (c0[0] + ((w - r * q.W) << 5)) + A.m.nx * ((c0[1] + jj) + A.m.ny * (c0[2] + kk));
+        }
+        const uint32_t mi = bits & in, mc = bits & ~in;
+        const int a = __popc(mi), c = __popc(mc);
+        int xa = a, xc = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int ya = __shfl_up_sync(FULL, xa, o), yc = __shfl_up_sync(FULL, xc, o);
+            if (lane >= o) { xa += ya; xc += yc; }
+        }
+        const int na = __shfl_sync(FULL, xa, 31), nc = __shfl_sync(FULL, xc, 31);
+        for (int t = lane; t - lane < na; t += 32) {
+            int src = 0;
+#pragma unroll
+            for (int h = 16; h > 0; h >>= 1)
+                if (__shfl_sync(FULL, xa, src + h - 1) <= t) src += h;
+            const uint32_t m = __shfl_sync(FULL, mi, src);
+            const int r = t - __shfl_sync(FULL, xa - a, src), l = __shfl_sync(FULL, label, src);
+            if (t < na) {
+                A.in_cell[pin + t] = l + nth_bit(m, r);
+                A.in_solid[pin + t] = list_word(s, 1);
+            }
+        }
+        for (int t = lane; t - lane < nc; t += 32) {
+            int src = 0;
+#pragma unroll
+            for (int h = 16; h > 0; h >>= 1)
+                if (__shfl_sync(FULL, xc, src + h - 1) <= t) src += h;
+            const uint32_t m = __shfl_sync(FULL, mc, src), tt = __shfl_sync(FULL, ci, src);
+            const int r = t - __shfl_sync(FULL, xc - c, src), l = __shfl_sync(FULL, label, src);
+            if (t < nc) {
+                const int p = nth_bit(m, r);
+                A.cut_cell[pcut + t] = l + p;
+                A.cut_solid[pcut + t] = list_word(s, ((tt >> p) & 1u) ? 2 : 3);
+            }
+        }
+        pin += na;
+        pcut += nc;
+    }
+}
+
+constexpr int CON_MAX_LAYERS = 2048;
+template <int NT>
+__device__ __forceinline__ void connect_body(const ConnectArgs& A, const SolidK& k, int s, uint32_t* bitmaps, ConnectShared& sh,
+                                             uint32_t* layers, int max_layers, int tid) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = tid & 31;
+    SolidPlan& pl = A.plan[s];
+    const ActiveBox b = active_box(A.m, k, pl);
     const int sx = b.n[0], sy = b.n[1], sz = b.n[2];
     if (tid == 0) {
         sh.first = ~0u;
@@ -390,76 +594,17 @@ __device__ __forceinline__ void connect_body(const MeshK& m, const SolidK& k, So
         return;
     }
     const int W = (sx + 31) >> 5, rows = sy * sz, nwords = rows * W;
+    const ConnectRows q{sx, sy, W, rows, sh.div_sy, sh.div_w};
     uint32_t* C = bitmaps;
     uint32_t* I = C + nwords;
     uint32_t* T = I + nwords;
     uint32_t* R = T + nwords;
-    const FastDiv dsy = sh.div_sy, dw = sh.div_w;
-    const int ox = b.c0[0] - pl.lo[0], oy = b.c0[1] - pl.lo[1], oz = b.c0[2] - pl.lo[2];
-    auto row_bytes = [&](int row) {
-        const int kk = (int)fdiv((uint32_t)row, dsy), jj = row - kk * sy;
-        return cls + ox + (int64_t)k.ext[0] * ((jj + oy) + (int64_t)k.ext[1] * (kk + oz));
-    };
-    // bitmaps: coalesced byte loads and ballots, several loads in flight; narrow boxes take two or four rows at once
-    {
-        constexpr int GW = 8;
-        const int lg = sx <= 8 ? 3 : (sx <= 16 ? 4 : 5), rpl = 32 >> lg;
-        const int sub = lane >> lg, col = lane & ((1 << lg) - 1);
-        const uint32_t msk = lg == 5 ? FULL : (1u << (1 << lg)) - 1u;
-        const int units = W == 1 ? (rows + rpl - 1) / rpl : nwords;  // loads
-        for (int u0 = wid * GW; u0 < units; u0 += NW * GW) {
-            uint8_t v[GW];
-#pragma unroll
-            for (int u = 0; u < GW; ++u) {
-                int row, x;
-                if (W == 1) { row = (u0 + u) * rpl + sub; x = col; }
-                else { row = (int)fdiv((uint32_t)(u0 + u), dw); x = ((u0 + u - row * W) << 5) + lane; }
-                v[u] = (u0 + u < units && row < rows && x < sx) ? row_bytes(row)[x] : (uint8_t)0;
-            }
-#pragma unroll
-            for (int u = 0; u < GW; ++u) {
-                const uint32_t bc = __ballot_sync(FULL, v[u] != 0), bi = __ballot_sync(FULL, v[u] == 1),
-                               bt = __ballot_sync(FULL, v[u] == 2);
-                const int w = W == 1 ? (u0 + u) * rpl + lane : u0 + u;
-                if (u0 + u < units && lane < (W == 1 ? rpl : 1) && w < nwords) {
-                    const int sft = W == 1 ? lane << lg : 0;
-                    C[w] = (bc >> sft) & msk;
-                    I[w] = (bi >> sft) & msk;
-                    T[w] = (bt >> sft) & msk;
-                }
-            }
-        }
-    }
+    const int off[3] = {b.c0[0] - pl.lo[0], b.c0[1] - pl.lo[1], b.c0[2] - pl.lo[2]};
+    connect_bitmaps<NT>(k, A.scratch + k.scratch_off, off, q, C, I, T, tid);
     group_sync<NT>();
     bool connected = false;
     if (proof) {
-        int bad = 0, starts = 0;
-        for (int row = tid; row < rows; row += NT) {
-            const uint32_t* c = C + row * W;
-            const int kk = (int)fdiv((uint32_t)row, dsy), jj = row - kk * sy;
-            int first = -1, last = -1, pop = 0;
-            uint32_t along = 0, below = 0;
-            for (int w = 0; w < W; ++w) {
-                const uint32_t x = c[w];
-                if (!x) continue;
-                pop += __popc(x);
-                if (first < 0) first = (w << 5) + __ffs(x) - 1;
-                last = (w << 5) + 31 - __clz(x);
-                if (jj > 0) along |= x & c[w - W];
-                if (kk > 0) below |= x & c[w - W * sy];
-            }
-            if (pop == 0) continue;
-            if (last - first + 1 != pop) ++bad;
-            if (!along) ++starts;
-            atomicOr(layers + (kk >> 5), 1u << (kk & 31));
-            if (below) atomicOr(layers + lw + (kk >> 5), 1u << (kk & 31));
-        }
-        bad = __reduce_add_sync(FULL, bad);
-        starts = __reduce_add_sync(FULL, starts);
-        if (lane == 0) {
-            if (bad) atomicAdd(&sh.bad, bad);
-            if (starts) atomicAdd(&sh.starts, starts);
-        }
+        connect_proof<NT>(q, C, sh, layers, lw, tid);
         group_sync<NT>();
         int nl = 0, links = 0;
         for (int i = 0; i < lw; ++i) {
@@ -540,126 +685,61 @@ __device__ __forceinline__ void connect_body(const MeshK& m, const SolidK& k, So
                 }
                 group_sync<NT>();
             }
-            changed = NT == 32 ? __any_sync(FULL, changed) : __syncthreads_or(changed);
-            if (!changed) break;
+            if (!group_any<NT>(changed != 0)) break;
             if (round >= max_rounds) {
-                if (tid == 0) set_error(cnt, DERR_FLOOD_LIMIT);
+                if (tid == 0) set_error(A.cnt, DERR_FLOOD_LIMIT);
                 break;
             }
         }
         C = R;
     }
-    // the lists: warp w takes the words [w0, w1), a lane counting a word, then a lane storing a cell
-    const int per = (((nwords + NW - 1) / NW) + 31) & ~31;
-    const int w0 = min(nwords, wid * per), w1 = min(nwords, w0 + per);
-    int nin = 0, ncut = 0;
-    for (int w = w0 + lane; w < w1; w += 32) {
-        const uint32_t bits = C[w], in = I[w];
-        nin += __popc(bits & in);
-        ncut += __popc(bits & ~in);
-    }
-    nin = __reduce_add_sync(FULL, nin);
-    ncut = __reduce_add_sync(FULL, ncut);
-    if (lane == 0) { sh.cnt[wid][0] = nin; sh.cnt[wid][1] = ncut; }
+    connect_count<NT>(C, I, nwords, sh, tid);
     group_sync<NT>();
-    int before_in = 0, before_cut = 0, tot_in = 0, tot_cut = 0;
-#pragma unroll
-    for (int i = 0; i < NW; ++i) {
-        const int a = sh.cnt[i][0], c = sh.cnt[i][1];
-        if (i < wid) { before_in += a; before_cut += c; }
-        tot_in += a;
-        tot_cut += c;
-    }
+    int before_in, before_cut, tot_in, tot_cut;
+    connect_sums<NT>(sh, tid, before_in, before_cut, tot_in, tot_cut);
     if (tid == 0) {
-        sh.base_in = atomicAdd(&cnt->n_inside, tot_in);
-        sh.base_cut = atomicAdd(&cnt->n_cut, tot_cut);
+        sh.base_in = atomicAdd(&A.cnt->n_inside, tot_in);
+        sh.base_cut = atomicAdd(&A.cnt->n_cut, tot_cut);
         pl.n_inside = tot_in;
         pl.n_cut = tot_cut;
     }
     group_sync<NT>();
-    if ((int64_t)sh.base_in + tot_in > cap_in || (int64_t)sh.base_cut + tot_cut > cap_cut) {
-        if (tid == 0) set_error(cnt, DERR_CAPACITY);
+    if ((int64_t)sh.base_in + tot_in > A.cap_in || (int64_t)sh.base_cut + tot_cut > A.cap_cut) {
+        if (tid == 0) set_error(A.cnt, DERR_CAPACITY);
         return;
     }
-    int64_t pin = (int64_t)sh.base_in + before_in, pcut = (int64_t)sh.base_cut + before_cut;
-    const uint32_t below = (1u << lane) - 1u;
-    for (int wb = w0; wb < w1; wb += 32) {
-        const int w = wb + lane;
-        uint32_t bits = 0, in = 0, ci = 0;
-        int label = 0;
-        if (w < w1) {
-            bits = C[w]; in = I[w]; ci = T[w];
-            const int row = (int)fdiv((uint32_t)w, dw), kk = (int)fdiv((uint32_t)row, dsy), jj = row - kk * sy;
-            label = (b.c0[0] + ((w - row * W) << 5)) + m.nx * ((b.c0[1] + jj) + m.ny * (b.c0[2] + kk));
-        }
-        const int a = __popc(bits & in), c = __popc(bits & ~in);
-        int xa = a, xc = c;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int ya = __shfl_up_sync(FULL, xa, o), yc = __shfl_up_sync(FULL, xc, o);
-            if (lane >= o) { xa += ya; xc += yc; }
-        }
-        uint32_t some = __ballot_sync(FULL, bits != 0);
-        while (some) {
-            const int src = __ffs(some) - 1;
-            some &= some - 1;
-            const uint32_t bb = __shfl_sync(FULL, bits, src), ii = __shfl_sync(FULL, in, src), tt = __shfl_sync(FULL, ci, src);
-            const int cell = __shfl_sync(FULL, label, src) + lane, oi = __shfl_sync(FULL, xa - a, src),
-                      oc = __shfl_sync(FULL, xc - c, src);
-            if ((bb >> lane) & 1u) {
-                if ((ii >> lane) & 1u) {
-                    const int64_t p = pin + oi + __popc(bb & ii & below);
-                    in_cell[p] = cell;
-                    in_solid[p] = list_word(s, 1);
-                } else {
-                    const int64_t p = pcut + oc + __popc(bb & ~ii & below);
-                    cut_cell[p] = cell;
-                    cut_solid[p] = list_word(s, ((tt >> lane) & 1u) ? 2 : 3);
-                }
-            }
-        }
-        pin += __shfl_sync(FULL, xa, 31);
-        pcut += __shfl_sync(FULL, xc, 31);
-    }
+    connect_emit<NT>(A, s, b.c0, q, C, I, T, (int64_t)sh.base_in + before_in, (int64_t)sh.base_cut + before_cut, tid);
 }
 
-// a CTA per solid; bitmaps in shared memory, or in global memory above a size (bitmap_global)
-constexpr int CON_MAX_LAYERS = 2048;
-__global__ void __launch_bounds__(CON_THREADS, 2) connect_kernel(MeshK m, const SolidK* __restrict__ sk,
-                                                              SolidPlan* __restrict__ plan,
-                                                              const uint8_t* __restrict__ scratch,
-                                                              uint32_t* __restrict__ gbitmaps,
-                                                              int32_t* __restrict__ in_cell, int32_t* __restrict__ in_solid,
-                                                              int32_t* __restrict__ cut_cell, int32_t* __restrict__ cut_solid,
-                                                              int64_t cap_in, int64_t cap_cut, Counters* cnt,
-                                                              const int32_t* __restrict__ solids) {
+// Solids in order of size, the largest first: n_big of them a CTA each (bitmaps in shared memory, or in global memory above a
+// size: bitmap_global), then n_mid of them CON_MID threads each, then the others a warp each; one launch, so that the smaller
+// ones fill the SMs while the last of the larger ones end.  (A cluster of 8 CTAs for the largest ones gained nothing: 0.053
+// against 0.059 ms at 256^3, 0.29 against 0.28 at 512^3.)
+__global__ void __launch_bounds__(CON_THREADS, 2) connect_kernel(ConnectArgs A) {
     extern __shared__ uint32_t dsm[];
-    __shared__ ConnectShared sh;
-    __shared__ uint32_t layers[2 * (CON_MAX_LAYERS / 32)];
-    const int s = solids ? solids[blockIdx.x] : blockIdx.x;
-    const SolidK& k = sk[s];
-    connect_body<CON_THREADS>(m, k, plan[s], scratch + k.scratch_off, s, k.bitmap_global ? gbitmaps + k.bitmap_off : dsm, sh,
-                              layers, CON_MAX_LAYERS, threadIdx.x, in_cell, in_solid, cut_cell, cut_solid, cap_in, cap_cut,
-                              cnt);
-}
-
-// a warp per solid for the solids whose bbox bitmap has at most CON_SMALL_WORDS words
-constexpr int CON_SMALL_WORDS = 256;
-constexpr int CON_SMALL_WARPS = 8;
-__global__ void __launch_bounds__(CON_SMALL_WARPS * 32) connect_small_kernel(
-    MeshK m, const SolidK* __restrict__ sk, SolidPlan* __restrict__ plan, const uint8_t* __restrict__ scratch,
-    int32_t* __restrict__ in_cell, int32_t* __restrict__ in_solid, int32_t* __restrict__ cut_cell,
-    int32_t* __restrict__ cut_solid, int64_t cap_in, int64_t cap_cut, Counters* cnt, const int32_t* __restrict__ solids,
-    int nsolids) {
-    __shared__ uint32_t s_bits[CON_SMALL_WARPS][4 * CON_SMALL_WORDS];
-    __shared__ ConnectShared sh[CON_SMALL_WARPS];
-    __shared__ uint32_t layers[CON_SMALL_WARPS][2 * (CON_SMALL_WORDS / 32)];
-    const int wid = threadIdx.x >> 5, item = blockIdx.x * CON_SMALL_WARPS + wid;
-    if (item >= nsolids) return;
-    const int s = solids[item];
-    const SolidK& k = sk[s];
-    connect_body<32>(m, k, plan[s], scratch + k.scratch_off, s, s_bits[wid], sh[wid], layers[wid], CON_SMALL_WORDS,
-                     threadIdx.x & 31, in_cell, in_solid, cut_cell, cut_solid, cap_in, cap_cut, cnt);
+    __shared__ ConnectShared sh[CON_WARPS];
+    __shared__ uint32_t layers[CON_WARPS * 2 * (CON_SMALL_WORDS / 32)];
+    static_assert(CON_WARPS * 2 * (CON_SMALL_WORDS / 32) >= 2 * (CON_MAX_LAYERS / 32) &&
+                      CON_WARPS * (CON_SMALL_WORDS / 32) >= CON_MID_GROUPS * (CON_MID_WORDS / 32), "layer bitmaps");
+    const int mid_ctas = (A.n_mid + CON_MID_GROUPS - 1) / CON_MID_GROUPS, tid = threadIdx.x;
+    const int b = (int)blockIdx.x - A.n_big;
+    if (b < 0) {
+        const int s = A.solids ? A.solids[blockIdx.x] : (int)blockIdx.x;
+        const SolidK& k = A.sk[s];
+        connect_body<CON_THREADS>(A, k, s, k.bitmap_global ? A.gbitmaps + k.bitmap_off : dsm, sh[0], layers, CON_MAX_LAYERS, tid);
+    } else if (b < mid_ctas) {
+        const int g = tid / CON_MID, item = b * CON_MID_GROUPS + g;
+        if (item >= A.n_mid) return;
+        const int s = A.solids[A.n_big + item];
+        connect_body<CON_MID>(A, A.sk[s], s, dsm + g * 4 * CON_MID_WORDS, sh[g], layers + g * 2 * (CON_MID_WORDS / 32), CON_MID_WORDS,
+                              tid % CON_MID);
+    } else {
+        const int g = tid >> 5, item = (b - mid_ctas) * CON_WARPS + g;
+        if (item >= A.n_small) return;
+        const int s = A.solids[A.n_big + A.n_mid + item];
+        connect_body<32>(A, A.sk[s], s, dsm + g * 4 * CON_SMALL_WORDS, sh[g], layers + g * 2 * (CON_SMALL_WORDS / 32),
+                         CON_SMALL_WORDS, tid & 31);
+    }
 }
 
 // ---- shared cells -----------------------------------------------------------------------------------------------------
@@ -820,28 +900,52 @@ __global__ void scan_reset_kernel(const int32_t* __restrict__ in_cell, const int
                                   int64_t shent_cap, const int32_t* __restrict__ prev_in_cell,
                                   const int32_t* __restrict__ prev_cut_cell, float* As, float* Fs, float* Ts, int32_t* Ct,
                                   const uint32_t* __restrict__ cbits) {
+    constexpr int B = 4;  // entries of a thread in flight: bound by their latency
     const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
     if (cnt->shared_marks != 0) {
         const int64_t n_in = clamp_len(cnt->n_inside, cnt->list_cap), n_cut = clamp_len(cnt->n_cut, cnt->list_cap);
-        for (int64_t e = t0; e < n_in + n_cut; e += nt) {
-            const int32_t c = e < n_in ? in_cell[e] : cut_cell[e - n_in];
-            if (c < 0 || c >= N) continue;
-            if (!((sbits[c >> 8] >> ((c >> 3) & 31)) & 1u)) continue;  // no cell of this chunk is shared
-            if (!(reinterpret_cast<const uint32_t*>(Ct)[c] & CT_SHARED)) continue;
-            const int32_t slot = atomicAdd(&cnt->n_shent, 1);
-            if (slot < shent_cap) shent[slot] = (uint32_t)e;
-            else set_error(cnt, DERR_SHARED_TABLE);
+        for (int64_t e0 = t0; e0 < n_in + n_cut; e0 += B * nt) {
+            int32_t c[B];
+            uint32_t w[B];
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                const int64_t e = e0 + u * nt;
+                c[u] = e >= n_in + n_cut ? -1 : (e < n_in ? in_cell[e] : cut_cell[e - n_in]);
+                if (c[u] >= N) c[u] = -1;
+            }
+#pragma unroll
+            for (int u = 0; u < B; ++u) w[u] = c[u] >= 0 ? sbits[c[u] >> 8] : 0u;
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                if (!((w[u] >> ((c[u] >> 3) & 31)) & 1u)) continue;  // no cell of this chunk is shared
+                if (!(reinterpret_cast<const uint32_t*>(Ct)[c[u]] & CT_SHARED)) continue;
+                const int32_t slot = atomicAdd(&cnt->n_shent, 1);
+                if (slot < shent_cap) shent[slot] = (uint32_t)(e0 + u * nt);
+                else set_error(cnt, DERR_SHARED_TABLE);
+            }
         }
     }
     if (prev_in_cell) {
         const int64_t n_in = clamp_len(cnt->prev_n_inside, cnt->list_cap), n_cut = clamp_len(cnt->prev_n_cut, cnt->list_cap);
-        for (int64_t e = t0; e < n_in + n_cut; e += nt) {
-            const int64_t c = e < n_in ? prev_in_cell[e] : prev_cut_cell[e - n_in];
-            if (c < 0 || c >= N) continue;
-            if ((cbits[c >> 8] >> ((c >> 3) & 31)) & 1u) continue;  // written by the chunked coupling
-            if (reinterpret_cast<const uint32_t*>(Ct)[c] >= CT_KEY_BASE) continue;
-            As[c] = 0.f; Ts[c] = 0.f; Ct[c] = 0;
-            Fs[c] = 0.f; Fs[N + c] = 0.f; Fs[2 * N + c] = 0.f;
+        for (int64_t e0 = t0; e0 < n_in + n_cut; e0 += B * nt) {
+            int32_t cc[B];
+            uint32_t w[B];
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                const int64_t e = e0 + u * nt;
+                cc[u] = e >= n_in + n_cut ? -1 : (e < n_in ? prev_in_cell[e] : prev_cut_cell[e - n_in]);
+                if (cc[u] >= N) cc[u] = -1;
+            }
+#pragma unroll
+            for (int u = 0; u < B; ++u) w[u] = cc[u] >= 0 ? cbits[cc[u] >> 8] : ~0u;
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                const int64_t c = cc[u];
+                if ((w[u] >> ((c >> 3) & 31)) & 1u) continue;  // written by the chunked coupling
+                if (reinterpret_cast<const uint32_t*>(Ct)[c] >= CT_KEY_BASE) continue;
+                As[c] = 0.f; Ts[c] = 0.f; Ct[c] = 0;
+                Fs[c] = 0.f; Fs[N + c] = 0.f; Fs[2 * N + c] = 0.f;
+            }
         }
     }
 }

@@ -142,6 +142,22 @@ inline StepParams step_params(double time, double dt, int nsub, double rho_V) {
     return StepParams{time, dt, dt / nsub, 1.0 / dt, rho_V / dt};
 }
 
+// connect_kernel.  Words of a bitmap (rows along x of the bbox) up to which a solid goes to a warp or to CON_MID threads.
+constexpr int CON_SMALL_WORDS = 256;
+constexpr int CON_MID_WORDS = 512;
+struct ConnectArgs {
+    MeshK m;
+    const SolidK* sk;
+    SolidPlan* plan;
+    const uint8_t* scratch;   // class bytes
+    uint32_t* gbitmaps;
+    int32_t *in_cell, *in_solid, *cut_cell, *cut_solid;
+    int64_t cap_in, cap_cut;
+    Counters* cnt;
+    const int32_t* solids;    // n_big + n_mid + n_small, the largest first (nullptr: 0, 1, ...)
+    int n_big, n_mid, n_small;
+};
+
 // plan_kernel: the head of an interact
 struct PrepArgs {
     MeshK m;

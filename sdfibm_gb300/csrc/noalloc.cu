@@ -35,9 +35,7 @@ __global__ void plan_kernel(PrepArgs A);
 int classify_kind(int shape_type, bool flat);
 void launch_classify(const ClassifyArgs& A, bool flat, int grid, cudaStream_t st);
 int classify_occupancy(int method, bool flat);
-__global__ void connect_kernel(MeshK m, const SolidK* sk, SolidPlan* plan, const uint8_t* scratch, uint32_t* gbitmaps,
-                               int32_t* in_cell, int32_t* in_solid, int32_t* cut_cell, int32_t* cut_solid,
-                               int64_t cap_in, int64_t cap_cut, Counters* cnt, const int32_t* solids);
+__global__ void connect_kernel(ConnectArgs A);
 }  // namespace sdfibm_dev
 
 using namespace sdfibm_dev;
@@ -306,10 +304,12 @@ extern "C" int sdfibm_cuda_touched_noalloc(const sdfibm_mesh_desc* mesh, const s
     CA.any_first = kind == 0 && m.nz > 2 ? nchunks : 0;
     CA.any_grid = grid;
     launch_classify(CA, m.nz <= 2, grid, st);
-    connect_kernel<<<1, 512, 0, st>>>(m, d_sk, d_plan, b + OFF_CLS, reinterpret_cast<uint32_t*>(b + OFF_BITMAP),
-                                      reinterpret_cast<int32_t*>(b + OFF_IN_CELL), reinterpret_cast<int32_t*>(b + OFF_IN_SOLID),
-                                      reinterpret_cast<int32_t*>(b + OFF_CUT_CELL), reinterpret_cast<int32_t*>(b + OFF_CUT_SOLID),
-                                      NA_MAX_BBOX_CELLS, NA_MAX_BBOX_CELLS, d_cnt, nullptr);
+    ConnectArgs ca{};
+    ca.m = m; ca.sk = d_sk; ca.plan = d_plan; ca.scratch = b + OFF_CLS; ca.gbitmaps = reinterpret_cast<uint32_t*>(b + OFF_BITMAP);
+    ca.in_cell = reinterpret_cast<int32_t*>(b + OFF_IN_CELL); ca.in_solid = reinterpret_cast<int32_t*>(b + OFF_IN_SOLID);
+    ca.cut_cell = reinterpret_cast<int32_t*>(b + OFF_CUT_CELL); ca.cut_solid = reinterpret_cast<int32_t*>(b + OFF_CUT_SOLID);
+    ca.cap_in = ca.cap_cut = NA_MAX_BBOX_CELLS; ca.cnt = d_cnt; ca.n_big = 1;
+    connect_kernel<<<1, 512, 0, st>>>(ca);
     noalloc_order_kernel<<<1, 1024, 0, st>>>(cells, types, capacity, n_device);
     return cudaGetLastError() == cudaSuccess ? SDFIBM_OK : SDFIBM_ERR_CUDA;
 }
