@@ -264,11 +264,13 @@ struct sdfibm_ctx {
     Poly* poly = nullptr;
 };
 
-// Most solids of the one-launch evolve.  Each CTA (one per SM) tests its solids' pairs a warp at a time, so its sub-step grows
-// with the solids per SM, where the launch-per-stage path keeps its launches' cost: 20 sub-steps of free spheres took (one
-// launch / launch per stage) 0.19 / 0.88 ms at 2000 solids, 0.55 / 1.13 at 8000, 1.83 / 1.45 at 16 384, 4.75 / 2.45 at
-// 38 000.  More plane-like solids than EV_MAX_PLANES (each tests every sphere) take the launches too.
-static int evolve_limit(int num_sms) { return 64 * num_sms; }
+// Most solids of the one-launch evolve.  Each CTA (one per SM) tests its solids' pairs a warp at a time, and where solids cross
+// half the skin in a sub-step against all others, while the launch-per-stage path keeps its launches' cost and its grid.  20
+// sub-steps of free spheres took (one launch / launch per stage, us): 192 / 1049 at 1800 solids, 206 / 898 at 3000, 281 / 996
+// at 4500, 521 / 1222 at 9700; with one solid in a hundred that fast 489 / 943 at 3000, 1837 / 1011 at 4500, and with all of
+// them 940 / 1053 and 2110 / 1153.  The line lies where the one launch is the faster one at any speed.  More plane-like solids
+// than EV_MAX_PLANES (each tests every sphere) take the launches too.
+static int evolve_limit(int num_sms) { return 20 * num_sms; }
 constexpr int EV_MAX_PLANES = 64;
 
 // event bracketing of each launch when timing is on: mark(ctx, name) after a launch records its end

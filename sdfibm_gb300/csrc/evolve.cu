@@ -5,7 +5,7 @@
 // src/libcollision/ugrid.cpp:5-77, collision.cpp:7-57).
 //
 // Without collisions every solid is independent, so one thread runs all sub-steps of one solid in a single launch.
-// With collisions up to 64 solids per SM run all sub-steps in one cooperative launch (evolve_contacts_kernel); for more, each
+// With collisions up to 20 solids per SM run all sub-steps in one cooperative launch (evolve_contacts_kernel); for more, each
 // sub-step is: forces + grid hash, counting sort of solid ids by grid cell, pair forces (each solid sums its own side of
 // every pair: no atomics, the pair law is evaluated once per side), move.
 #include <cstdint>
@@ -488,15 +488,19 @@ __global__ void collide_kernel(const SolidK* __restrict__ sk, sdfibm_solid_state
 // launch and memory latency.  Here CTA b keeps solids [b per, (b + 1) per): a thread per solid holds its state in
 // registers over all sub-steps, the other warps test its pairs meanwhile, and one grid barrier a sub-step publishes the
 // new positions (two buffers).  The pairs come from lists built once, by testing all solids in FP32, of the solids nearer
-// than the contact distance plus a skin.  A solid that has moved half the skin is hot from then on: it tests every solid, the others test
-// the hot ones beside their lists (a solid that left its stable step size does not make everybody search again); past
-// EV_HOT of them every CTA builds its lists again.  Pairs go through the FP32 screen, the reference's 27-cell rule on the UGrid keys and the FP64 contact law, as in collide_kernel, so the contacts are
-// the same.  The rotation half of a move needs no pair and runs in warps of its own beside the barrier and the pairs.  Plane-like solids (law 0) test every sphere, spheres every plane: for up to EV_MAX_PLANES.
+// than the contact distance plus a skin.  A solid that has moved half the skin is hot from then on: it tests every solid, the
+// others test the hot ones beside their lists (a solid that left its stable step size does not make everybody search again);
+// past EV_HOT of them every CTA lists its pairs in every sub-step, without a skin.  Pairs go through the FP32 screen, the
+// reference's 27-cell rule on the UGrid keys and the FP64 contact law, as in collide_kernel, so the contacts are the same.
+// The rotation half of a move needs no pair and runs in warps of its own beside the barrier and the pairs.  Plane-like solids
+// (law 0) test every sphere, spheres every plane: for up to EV_MAX_PLANES.
 // Bound by latency: 9 us a sub-step (barrier, two dependent L2 reads, the FP64 chains of a contact and a move).  Measured
-// (GB300): 104 solids 1.26 -> 0.20 ms, 1800 solids 1.4 -> 0.19 ms.
+// (GB300), 20 sub-steps: 104 solids 1.26 -> 0.20 ms, 1800 solids 1.05 -> 0.19 ms, all of them crossing the skin in every
+// sub-step 1.18 -> 0.61 ms (2.6 with room for 256 hot ones and one record a lane in flight).
 constexpr int EV_THREADS = 256, EV_WARPS = EV_THREADS / 32;
 constexpr int EV_LIST = 128;              // listed neighbours of a solid; more: it tests every solid every sub-step
-constexpr int EV_HOT = 256;               // solids beyond half the skin before the lists are made again
+constexpr int EV_HOT = 32;                // solids beyond half the skin before the lists are made in every sub-step
+constexpr int EV_BATCH = 4;               // records of a lane in flight when a warp tests many solids
 int evolve_contacts_threads() { return EV_THREADS; }
 int evolve_contacts_list() { return EV_LIST; }
 int evolve_contacts_hot() { return EV_HOT; }
@@ -670,7 +674,7 @@ __global__ void __launch_bounds__(EV_THREADS, 1) evolve_contacts_kernel(const So
     __shared__ int32_t s_cq[EV_WARPS][32], s_ce[EV_WARPS][32], s_cn[EV_WARPS];
     __shared__ int32_t s_n[EV_THREADS];   // listed neighbours, -1: more than the list holds
     __shared__ int s_hot[EV_THREADS];
-    __shared__ int s_ok, s_move, s_build;
+    __shared__ int s_ok, s_move, s_build, s_storm;
     const unsigned FULL = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int s0 = blockIdx.x * per, own = min(per, S - s0);  // >= 1
@@ -756,7 +760,7 @@ __global__ void __launch_bounds__(EV_THREADS, 1) evolve_contacts_kernel(const So
             move_rotation(sk[s], q, om, torque, time, dt, om_new, q_new);
         }
     };
-    if (tid == 0) { s_build = 1; s_move = 0; }
+    if (tid == 0) { s_build = 1; s_move = 0; s_storm = 0; }
     __syncthreads();
     if (tid == 0) ev_arrive(w);
     for (int it = 0; it < nsub; ++it) {
@@ -768,7 +772,8 @@ __global__ void __launch_bounds__(EV_THREADS, 1) evolve_contacts_kernel(const So
         if (wid >= cw0) {
             if (tid == 32 * cw0) {
                 s_ok = ev_wait(w, gridDim.x * arrive) ? 1 : 0;
-                if (it > 0) s_build = __ldcg(&w.ctrl->rebuild[(it - 1) & 1]) == it;
+                if (it > 0 && !s_storm) s_storm = __ldcg(&w.ctrl->rebuild[(it - 1) & 1]) == it;
+                s_build = it == 0 || s_storm;
             }
             ev_bar(bar, 32 * ncw);
             if (s_ok && s_build) {  // lists of the CTA's solids, four of them per pass over the records
@@ -780,17 +785,26 @@ __global__ void __launch_bounds__(EV_THREADS, 1) evolve_contacts_kernel(const So
                         a[u] = i0 + u < own ? __ldcg(rec + s0 + i0 + u) : make_float4(0.f, 0.f, 0.f, NAN);
                         n[u] = 0;
                     }
-                    for (int q0 = 0; q0 < S; q0 += 32) {
-                        const int qq = q0 + lane;
-                        const float4 b = qq < S ? __ldcg(rec + qq) : make_float4(0.f, 0.f, 0.f, NAN);
+                    const float reach = s_storm ? 0.f : skin;
+                    for (int q0 = 0; q0 < S; q0 += 32 * EV_BATCH) {
+                        float4 b[EV_BATCH];
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            const bool hit = ev_sphere_near(a[u], b, skin) && qq != s0 + i0 + u;
-                            const unsigned bal = __ballot_sync(FULL, hit);
-                            if (bal) {
-                                const int to = n[u] + __popc(bal & ((1u << lane) - 1u));
-                                if (hit && to < EV_LIST) w.list[(int64_t)(s0 + i0 + u) * EV_LIST + to] = qq;
-                                n[u] += __popc(bal);
+                        for (int v = 0; v < EV_BATCH; ++v) {
+                            const int qq = q0 + 32 * v + lane;
+                            b[v] = qq < S ? __ldcg(rec + qq) : make_float4(0.f, 0.f, 0.f, NAN);
+                        }
+#pragma unroll
+                        for (int v = 0; v < EV_BATCH; ++v) {
+                            const int qq = q0 + 32 * v + lane;
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                const bool hit = ev_sphere_near(a[u], b[v], reach) && qq != s0 + i0 + u;
+                                const unsigned bal = __ballot_sync(FULL, hit);
+                                if (bal) {
+                                    const int to = n[u] + __popc(bal & ((1u << lane) - 1u));
+                                    if (hit && to < EV_LIST) w.list[(int64_t)(s0 + i0 + u) * EV_LIST + to] = qq;
+                                    n[u] += __popc(bal);
+                                }
                             }
                         }
                     }
@@ -803,7 +817,7 @@ __global__ void __launch_bounds__(EV_THREADS, 1) evolve_contacts_kernel(const So
             }
             // pair forces, a warp per solid; entries of the hot list hold the step they count from (a CTA ahead of this one
             // may add to it meanwhile)
-            const int nhot = s_ok ? min(__ldcg(&w.ctrl->nhot), EV_HOT) : 0;
+            const int nhot = s_ok && !s_storm ? min(__ldcg(&w.ctrl->nhot), EV_HOT) : 0;
             for (int i = wid - cw0; i < (s_ok ? own : 0); i += ncw) {
                 const int p = s0 + i;
                 const int4 kp = __ldcg(key + p);
@@ -814,7 +828,7 @@ __global__ void __launch_bounds__(EV_THREADS, 1) evolve_contacts_kernel(const So
                     if (rp.w == rp.w) {  // a sphere law
                         const int n = s_n[i];
                         const int32_t* list = w.list + (int64_t)p * EV_LIST;
-                        const bool all = n < 0 || s_hot[i];
+                        const bool all = n < 0 || (s_hot[i] && !s_storm);
                         if (lane == 0) s_cn[wid] = 0;
                         __syncwarp();
                         auto near = [&](int qq) {
@@ -831,9 +845,21 @@ __global__ void __launch_bounds__(EV_THREADS, 1) evolve_contacts_kernel(const So
                             const int slot = atomicAdd(&s_cn[wid], 1);
                             if (slot < 32) s_cq[wid][slot] = qq;
                         };
-                        for (int e = lane; e < (all ? S : n); e += 32) {
-                            const int qq = all ? e : list[e];
-                            if (near(qq) && (all || !is_hot(qq))) add(qq);
+                        for (int e0 = lane; e0 < (all ? S : n); e0 += 32 * EV_BATCH) {
+                            int qq[EV_BATCH];
+                            float4 b[EV_BATCH];
+#pragma unroll
+                            for (int v = 0; v < EV_BATCH; ++v) {
+                                const int e = e0 + 32 * v;
+                                qq[v] = e < (all ? S : n) ? (all ? e : list[e]) : p;
+                            }
+#pragma unroll
+                            for (int v = 0; v < EV_BATCH; ++v) b[v] = __ldcg(rec + qq[v]);
+#pragma unroll
+                            for (int v = 0; v < EV_BATCH; ++v)
+                                if (qq[v] != p && ev_sphere_near(rp, b[v], 0.f) && ev_neighbours(kp, __ldcg(key + qq[v])) &&
+                                    (all || !is_hot(qq[v])))
+                                    add(qq[v]);
                         }
                         if (!all)
                             for (int h = lane; h < nhot; h += 32) {
@@ -926,7 +952,7 @@ __global__ void __launch_bounds__(EV_THREADS, 1) evolve_contacts_kernel(const So
                 const D3 d = pos - at;
                 // beyond half the skin, with room.  Off the grid, or not finite, a solid has no sphere pair; back on the grid
                 // it counts from then on
-                if (on && !s_hot[tid] && magSqr(d) > 0.24 * (double)skin * (double)skin) {
+                if (on && !s_storm && !s_hot[tid] && magSqr(d) > 0.24 * (double)skin * (double)skin) {
                     const int slot = atomicAdd(&w.ctrl->nhot, 1);
                     if (slot < EV_HOT) {
                         __stcg(w.hot + slot, make_int2(s, it + 1));
@@ -940,8 +966,8 @@ __global__ void __launch_bounds__(EV_THREADS, 1) evolve_contacts_kernel(const So
         if (last) break;
         __syncthreads();
         if (tid == 0) {
-            // no room among the hot ones: every CTA lists again.  Two slots by step, since a CTA ahead of this one may
-            // already ask for the next step (but not for the one after it)
+            // no room among the hot ones: every CTA lists again, without a skin, from the next sub-step to the last.  Two
+            // slots by step, since a CTA ahead of this one may already ask for the next step (but not for the one after it)
             if (s_move) atomicMax(&w.ctrl->rebuild[it & 1], it + 1);
             s_move = 0;
             ev_arrive(w);
