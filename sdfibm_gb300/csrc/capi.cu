@@ -67,7 +67,7 @@ __global__ void export64_kernel(Counters* cnt, int64_t N, uint32_t* dirty, const
 __global__ void u64_to_planes_kernel(const double* U64, int64_t N, float* U);
 __global__ void fields_to_f64_kernel(int64_t N, const float* As, const float* Fs, const float* Ts, const int32_t* Ct,
                                      double* out);
-__global__ void fix_internal_kernel(MeshK m, const sdfibm_solid_state* st, const int32_t* in_cell,
+__global__ void fix_internal_kernel(MeshK m, const double* centres, const sdfibm_solid_state* st, const int32_t* in_cell,
                                     const int32_t* in_solid, const int32_t* Ct, float* U, const Counters* cnt);
 // evolve.cu
 
@@ -1381,7 +1381,7 @@ int sdfibm_cuda_fix_internal(sdfibm_ctx* ctx, const int32_t* Ct, float* U) {
         CK(cudaGetLastError());
         return SDFIBM_OK;
     }
-    fix_internal_kernel<<<ctx->num_sms * 4, 256, 0, ctx->stream>>>(ctx->mesh, ctx->d_st, ctx->in_cell(),
+    fix_internal_kernel<<<ctx->num_sms * 4, 256, 0, ctx->stream>>>(ctx->mesh, ctx->d_centres, ctx->d_st, ctx->in_cell(),
                                                                     ctx->in_solid(), Ct, U, ctx->d_cnt);
     CK(cudaGetLastError());
     return SDFIBM_OK;

@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(96) plan_kernel(PrepArgs A) {
             cnt->n_inside = 0; cnt->n_cut = 0; cnt->n_shared = 0; cnt->shared_marks = 0;
             cnt->exact_rechecks = 0; cnt->bbox_cells = 0;
             cnt->n_feat = 0; cnt->n_fb = 0; cnt->n_recheck = 0; cnt->n_ovf = 0; cnt->n_shent = 0;
-            cnt->n_inband = 0; cnt->n_small = 0;
+            cnt->n_inband = 0; cnt->n_small = 0; cnt->couple_next = 0;
         }
     }
     const int s = blockIdx.x * 32 + lane;
@@ -822,6 +822,24 @@ __device__ __forceinline__ float ff_u_minus_us(float U, float u0h, float u0l, fl
     return __fadd_rn(d, __fsub_rn(g, lo));
 }
 
+// Conversions between the formats on the integer pipes: the FP64 pipe, which the exact forcing keeps busy, takes 64 issue slots
+// for one.  Zeros and normal values (the others go to the instruction); double to float rounds to nearest even.
+__device__ __forceinline__ double wide(float x) {
+    const uint32_t b = __float_as_uint(x), m = b & 0x7fffffffu;
+    double r = __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + 0x38000000u)), (int)(b << 29));
+    if (m == 0u) r = __hiloint2double((int)b, 0);
+    else if (m - 0x00800000u >= 0x7f000000u) r = (double)x;
+    return r;
+}
+__device__ __forceinline__ float narrow(double x) {
+    const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x), m = hi & 0x7fffffffu;
+    const uint64_t v = ((uint64_t)m << 32) | lo, r = v + 0x0fffffffu + ((lo >> 29) & 1u);
+    uint32_t b = (uint32_t)(r >> 29) + 0x40000000u;
+    if ((m | lo) == 0u) b = 0u;
+    else if (m - 0x38100000u >= 0x0fd00000u) return (float)x;  // outside 2^-126 .. 2^127
+    return __uint_as_float(b | (hi & 0x80000000u));
+}
+
 // Per-cell forcing of solid s on cell c with fluid velocity U (pcHydrodynamicInteraction, solidcloud.cpp:384-390):
 // alpha, the FP32 Fs and the cell's contributions to the force/torque sums (:411-421), FP64 in f6 (exact mode) or
 // FP32 in g6.
@@ -843,18 +861,22 @@ __device__ __forceinline__ float cell_forcing(const CoupleArgs& A, int64_t c, in
         if (alpha < 0.f) alpha = __fdiv_rn(-alpha - 1.f, (float)A.count_samples);
     }
     if (EXACT) {
-        // the reference's FP64 sequence
+        // FP64; the cross products as fused multiply-adds: 24 operations a cell for 43 as written out with conversions
         const sdfibm_solid_state& st = A.st[s];
-        const D3 x = state_pos(st);
         // mesh_C from its per-axis tables: the FP64 pipe also converts the indices, twelve of its instructions a cell
-        const D3 cc{A.centres[i], A.centres[m.nx + j], A.centres[m.nx + m.ny + k]};
-        const D3 vel{st.vel[0], st.vel[1], st.vel[2]}, om{st.omega[0], st.omega[1], st.omega[2]};
-        const D3 uf{(double)Ux, (double)Uy, (double)Uz};
-        const D3 us = vel + cross(om, cc - x);
-        const D3 f_ = (double)alpha * (uf - us);
-        const D3 t_ = cross(cc - x, f_);
-        f6[0] = f_.x; f6[1] = f_.y; f6[2] = f_.z; f6[3] = t_.x; f6[4] = t_.y; f6[5] = t_.z;
-        fs[0] = (float)(f_.x * dtINV); fs[1] = (float)(f_.y * dtINV); fs[2] = (float)(f_.z * dtINV);
+        const double dx = A.centres[i] - st.pos[0], dy = A.centres[m.nx + j] - st.pos[1],
+                     dz = A.centres[m.nx + m.ny + k] - st.pos[2];
+        const double ox = st.omega[0], oy = st.omega[1], oz = st.omega[2];
+        double fx = __fma_rn(oz, dy, __fma_rn(-oy, dz, wide(Ux) - st.vel[0]));
+        double fy = __fma_rn(ox, dz, __fma_rn(-oz, dx, wide(Uy) - st.vel[1]));
+        double fz = __fma_rn(oy, dx, __fma_rn(-ox, dy, wide(Uz) - st.vel[2]));
+        if (alpha != 1.f) {
+            const double al = wide(alpha);
+            fx *= al; fy *= al; fz *= al;
+        }
+        f6[0] = fx; f6[1] = fy; f6[2] = fz;
+        f6[3] = __fma_rn(dy, fz, -(dz * fy)); f6[4] = __fma_rn(dz, fx, -(dx * fz)); f6[5] = __fma_rn(dx, fy, -(dy * fx));
+        fs[0] = narrow(fx * dtINV); fs[1] = narrow(fy * dtINV); fs[2] = narrow(fz * dtINV);
     } else {
         // U - us in two-float arithmetic (the difference can cancel; about 2^-46 of the magnitudes, against 2^-24 of
         // the difference for the FP32 rounding that follows), FP32 after it.  The cell offsets from the seed are
@@ -975,8 +997,8 @@ __device__ __noinline__ void couple_shared(const CoupleArgs& A, int64_t n) {
 }
 
 // Chunked coupling.  The claim pass marks in cbits every chunk of 8 consecutive cells that holds a claimed cell (and
-// in sbits the chunks of cells claimed more than once).  This kernel runs over the marked chunks, a warp per 64 bits of the bitmap
-// (in the order given below), four chunks at a time with 8 lanes each, and writes the four fields of every
+// in sbits the chunks of cells claimed more than once).  This kernel runs over the marked chunks, a warp per 64 bits of the
+// bitmap, four chunks at a time with 8 lanes each, and writes the four fields of every
 // cell of a marked chunk: zero for an unclaimed cell (a cell that no solid touches, or one the previous call touched:
 // the sparse reset inside these chunks), zero As / Ts / Fs and the claim word kept in Ct for a shared cell
 // (finalize_kernel writes its sums and decodes its Ct), and for a cell claimed once the forcing of its solid.  The
@@ -988,10 +1010,23 @@ __device__ __noinline__ void couple_shared(const CoupleArgs& A, int64_t n) {
 // visits the same chunks).
 constexpr int CPL_WARPS = CPL_THREADS / 32;
 
+// Force and torque sums of the FP64 forcing: the warp's contributions go through shared memory, and lane (g, r) of 5 x 6 adds
+// component r of the cells 7 g .. 7 g + 6, seven additions a batch, keeping the sum of a run of cells of one solid (over
+// batches too) until another solid follows.
+struct FtSum {
+    double acc;
+    int solid;
+};
+constexpr int FT_GROUPS = 5, FT_CELLS = 7, FT_STRIDE = 33;
+__device__ __forceinline__ void ft_flush(const CoupleArgs& A, FtSum& q, int r) {
+    if (q.solid >= 0) atomicAdd(A.ftacc + 6 * q.solid + r, q.acc);
+    q.acc = 0.0;
+}
+
 // forcing of the first `count` queued cells (lane l takes entry l), written to the fields, F/T summed per solid
 template <bool EXACT>
-__device__ __forceinline__ void couple_queued(const CoupleArgs& A, const int32_t* qc, const uint32_t* qk, int count,
-                                              float dtINV32, double dtINV) {
+__device__ __forceinline__ void couple_queued(const CoupleArgs& A, const int32_t* qc, const uint32_t* qk, double* sv, FtSum& ft,
+                                              int count, float dtINV32, double dtINV) {
     const int lane = threadIdx.x & 31;
     const int64_t N = A.m.ncells;
     int s = -1;
@@ -1012,37 +1047,53 @@ __device__ __forceinline__ void couple_queued(const CoupleArgs& A, const int32_t
         A.Fs[2 * N + c] = fs[2];
         A.Ct[c] = type == 1 ? s + 4 : type;
     }
+    if (EXACT) {
+#pragma unroll
+        for (int r = 0; r < 6; ++r) sv[r * FT_STRIDE + lane] = f6[r];
+        __syncwarp();
+        const int g = lane / 6, r = lane - 6 * g;
+        if (g < FT_GROUPS) {
+            double v[FT_CELLS];
+            int who[FT_CELLS];
+#pragma unroll
+            for (int i = 0; i < FT_CELLS; ++i) {
+                const int e = min(FT_CELLS * g + i, 31);
+                v[i] = sv[r * FT_STRIDE + e];
+                who[i] = FT_CELLS * g + i < count ? (int)((qk[e] - CT_KEY_BASE) >> 2) : -1;
+            }
+#pragma unroll
+            for (int i = 0; i < FT_CELLS; ++i) {
+                if (who[i] < 0) break;
+                if (who[i] != ft.solid) {
+                    ft_flush(A, ft, r);
+                    ft.solid = who[i];
+                }
+                ft.acc += v[i];
+            }
+        }
+        return;
+    }
     uint32_t pend = __ballot_sync(0xffffffffu, s >= 0);
     while (pend) {
         const int sl = __shfl_sync(0xffffffffu, s, __ffs(pend) - 1);
         const bool mine = s == sl;
         pend &= ~__ballot_sync(0xffffffffu, mine);
-        double v;
-        if (EXACT) {
-            double t[8];
+        float t[8];
 #pragma unroll
-            for (int r = 0; r < 8; ++r) t[r] = mine ? f6[r] : 0.0;
-            v = warp_total4(reduce_scatter8(t, lane));
-        } else {
-            float t[8];
-#pragma unroll
-            for (int r = 0; r < 8; ++r) t[r] = mine ? g6[r] : 0.f;
-            v = warp_total4((double)reduce_scatter8(t, lane));
-        }
+        for (int r = 0; r < 8; ++r) t[r] = mine ? g6[r] : 0.f;
+        const double v = warp_total4((double)reduce_scatter8(t, lane));
         const int slot = lane >> 2;
         if ((lane & 3) == 0 && slot < 6) atomicAdd(A.ftacc + 6 * sl + slot, v);
     }
 }
 
-// Order of the marked chunks.  Memory order for the FP32 forcing, whose time goes to memory latency.  The FP64 forcing is
-// bound by the FP64 pipe (1/64 of the FP32 rate), where every distinct solid of a batch costs a reduction of nine additions:
-// there an item is 64 consecutive cells (a byte of the bitmap) on each of 8 rows, whose distance is the row length in whole
-// bytes, its chunks taken column by column, so that a batch of 32 queued cells covers about 8 x 8 cells of one or two solids
-// instead of a row's five (the mesh rows need not be multiples of 64 cells: any partition of the bytes gives the same fields).
-// Measured (GB300): FP64 at 256^3 and 4096 solids, 2.2 M cells, 0.51 -> 0.34 ms (0.37 and 0.35 with 2 and 4 rows, 0.46 in
-// memory order); FP32 at 512^3, 10.5 M cells, 0.56 ms in memory order and 0.62 with 4 rows.
+// The FP32 forcing is bound by memory latency.  The FP64 forcing is bound by the FP64 pipe (1/64 of the FP32 rate): 24
+// operations a cell and 7 a batch of 32 for the sums; its items are taken as warps get free, since their cells differ much in
+// number.  Measured (GB300): FP64 at 256^3 and 4096 solids, 2.2 M cells, 0.34 -> 0.20 ms (the earlier form: 43 operations a
+// cell and conversions on the same pipe, a reduction of nine additions for every distinct solid of a batch, about 3; chunks
+// in patches of 64 x 8 cells paid then, now they take 0.21); FP32 at 512^3, 10.5 M cells, 0.56 ms.
 template <bool EXACT>
-__global__ void __launch_bounds__(CPL_THREADS) couple_chunks_kernel(CoupleArgs A) {
+__global__ void __launch_bounds__(CPL_THREADS, 4) couple_chunks_kernel(CoupleArgs A) {
     __shared__ int32_t s_qc[CPL_WARPS][64];   // per warp: queued cells claimed once, and their claim words
     __shared__ uint32_t s_qk[CPL_WARPS][64];
     const unsigned FULL = 0xffffffffu;
@@ -1050,79 +1101,82 @@ __global__ void __launch_bounds__(CPL_THREADS) couple_chunks_kernel(CoupleArgs A
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, grp = lane >> 3, sub = lane & 7;
     int32_t* qc = s_qc[wib];
     uint32_t* qk = s_qk[wib];
-    const int64_t nbytes = (N + 63) >> 6;
-    const int rs = max(1, (A.m.nx + 32) >> 6);  // row length in bytes
-    const int64_t items = EXACT ? (nbytes + 8 * rs - 1) / (8 * rs) * rs : (nbytes + 7) >> 3;
+    __shared__ double s_ft[EXACT ? CPL_WARPS : 1][6 * FT_STRIDE];
+    double* sv = s_ft[EXACT ? wib : 0];
+    FtSum ft{0.0, -1};
+    const int64_t words = (N + 255) >> 8, items = (words + 1) >> 1;
     const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
     const double dtINV = A.step->dtINV;
     const float dtINV32 = (float)dtINV;
     const uint32_t* C = reinterpret_cast<const uint32_t*>(A.Ct);
-    const uint8_t* marks = reinterpret_cast<const uint8_t*>(A.cbits);
     const int64_t n_shared = min((int64_t)A.cnt->n_shent, A.shent_cap);
     if (n_shared > 0) couple_shared<EXACT>(A, n_shared);
     int nq = 0;  // warp-uniform
-    for (int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < items; t += nw) {
-        int64_t b0;        // first byte
-        uint64_t rem = 0;  // EXACT: bit 8 chunk + row; else bit = chunk
-        if (EXACT) {
-            const int64_t blk = t / rs;
-            b0 = blk * 8 * rs + (t - blk * rs);
-            unsigned byte = 0;
-            if (lane < 8 && b0 + (int64_t)lane * rs < nbytes) byte = marks[b0 + (int64_t)lane * rs];
-            if (!__any_sync(FULL, byte != 0)) continue;
-#pragma unroll
-            for (int bit = 0; bit < 8; ++bit) rem |= (uint64_t)__ballot_sync(FULL, (byte >> bit) & 1u) << (8 * bit);
-        } else {
-            b0 = t * 8;
-            rem = A.cbits[2 * t];
-            if (b0 + 4 < nbytes) rem |= (uint64_t)A.cbits[2 * t + 1] << 32;
+    // tickets of up to 32 items, about five tickets a warp; the items of a ticket lie far apart (a solid's cells spread over the
+    // warps) and their marks are read by a lane each.  FP64: the next ticket is asked for while this one is done.
+    const int64_t run = max((int64_t)1, min((int64_t)32, items / (5 * nw))), tickets = (items + run - 1) / run;
+    for (int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < tickets;) {
+        const int64_t first = t;
+        int asked = 0;
+        if (EXACT && lane == 0) asked = atomicAdd(&A.cnt->couple_next, 1);
+        uint64_t marks = 0;
+        const int64_t w = 2 * (first + lane * tickets);
+        if (w < words) {
+            marks = A.cbits[w];
+            if (w + 1 < words) marks |= (uint64_t)A.cbits[w + 1] << 32;
         }
-        auto cell_of = [&](uint64_t left) {  // this lane's cell of the next four chunks of `left`, -1: none
-            for (int q = 0; q < grp; ++q) left &= left - 1;
-            const int at = __ffsll((long long)left) - 1;
-            if (at < 0) return (int64_t)-1;
-            const int64_t c = EXACT ? ((b0 + (int64_t)(at & 7) * rs) << 6) + (at & ~7) + sub : (b0 << 6) + (at << 3) + sub;
-            return c < N ? c : (int64_t)-1;
-        };
-        int64_t c = cell_of(rem);
-        uint32_t claim = c >= 0 ? C[c] : 0u;
-        while (rem) {  // warp-uniform: four marked chunks per pass, the claims of the next pass loaded ahead
+        for (unsigned some = __ballot_sync(FULL, marks != 0); some; some &= some - 1) {
+            const int64_t cur = first + (__ffs(some) - 1) * tickets;
+            uint64_t rem = __shfl_sync(FULL, marks, __ffs(some) - 1);  // bit: chunk
+            auto cell_of = [&](uint64_t left) {  // this lane's cell of the next four chunks of `left`, -1: none
+                for (int q = 0; q < grp; ++q) left &= left - 1;
+                const int at = __ffsll((long long)left) - 1;
+                if (at < 0) return (int64_t)-1;
+                const int64_t c = (cur << 9) + (at << 3) + sub;
+                return c < N ? c : (int64_t)-1;
+            };
+            int64_t c = cell_of(rem);
+            uint32_t claim = c >= 0 ? C[c] : 0u;
+            while (rem) {  // warp-uniform: four marked chunks per pass, the claims of the next pass loaded ahead
 #pragma unroll
-            for (int q = 0; q < 4; ++q) rem &= rem - 1;
-            const int64_t c_next = cell_of(rem);
-            const uint32_t claim_next = c_next >= 0 ? C[c_next] : 0u;
-            const bool single = claim >= CT_KEY_BASE && !(claim & CT_SHARED);
-            if (c >= 0 && !single) {
-                A.As[c] = 0.f;
-                A.Ts[c] = 0.f;
-                A.Fs[c] = 0.f;
-                A.Fs[N + c] = 0.f;
-                A.Fs[2 * N + c] = 0.f;
-                A.Ct[c] = (claim & CT_SHARED) ? (int32_t)claim : 0;
-            }
-            const uint32_t m = __ballot_sync(FULL, single);
-            if (single) {
-                const int pos = nq + __popc(m & ((1u << lane) - 1u));
-                qc[pos] = (int32_t)c;
-                qk[pos] = claim;
-            }
-            nq += __popc(m);
-            __syncwarp();
-            if (nq >= 32) {
-                couple_queued<EXACT>(A, qc, qk, 32, dtINV32, dtINV);
-                __syncwarp();
-                if (lane < nq - 32) {
-                    qc[lane] = qc[32 + lane];
-                    qk[lane] = qk[32 + lane];
+                for (int q = 0; q < 4; ++q) rem &= rem - 1;
+                const int64_t c_next = cell_of(rem);
+                const uint32_t claim_next = c_next >= 0 ? C[c_next] : 0u;
+                const bool single = claim >= CT_KEY_BASE && !(claim & CT_SHARED);
+                if (c >= 0 && !single) {
+                    A.As[c] = 0.f;
+                    A.Ts[c] = 0.f;
+                    A.Fs[c] = 0.f;
+                    A.Fs[N + c] = 0.f;
+                    A.Fs[2 * N + c] = 0.f;
+                    A.Ct[c] = (claim & CT_SHARED) ? (int32_t)claim : 0;
                 }
-                nq -= 32;
+                const uint32_t m = __ballot_sync(FULL, single);
+                if (single) {
+                    const int pos = nq + __popc(m & ((1u << lane) - 1u));
+                    qc[pos] = (int32_t)c;
+                    qk[pos] = claim;
+                }
+                nq += __popc(m);
                 __syncwarp();
+                if (nq >= 32) {
+                    couple_queued<EXACT>(A, qc, qk, sv, ft, 32, dtINV32, dtINV);
+                    __syncwarp();
+                    if (lane < nq - 32) {
+                        qc[lane] = qc[32 + lane];
+                        qk[lane] = qk[32 + lane];
+                    }
+                    nq -= 32;
+                    __syncwarp();
+                }
+                c = c_next;
+                claim = claim_next;
             }
-            c = c_next;
-            claim = claim_next;
         }
+        t = nw + (EXACT ? (int64_t)__shfl_sync(FULL, asked, 0) : t);
     }
-    if (nq > 0) couple_queued<EXACT>(A, qc, qk, nq, dtINV32, dtINV);
+    if (nq > 0) couple_queued<EXACT>(A, qc, qk, sv, ft, nq, dtINV32, dtINV);
+    if (EXACT && lane < 6 * FT_GROUPS) ft_flush(A, ft, lane % 6);
 }
 void launch_couple_chunks(const CoupleArgs& A, bool exact, int grid, cudaStream_t st) {
     if (exact) couple_chunks_kernel<true><<<grid, CPL_THREADS, 0, st>>>(A);
@@ -1146,28 +1200,76 @@ __global__ void centres_kernel(MeshK m, double* __restrict__ out) {
 // Forcing applied to a GPU-resident fluid (main.cpp:70-77, its cell fields): U = U - Fs dt and T = (1 - As) T + Ts,
 // in FP64 and rounded once to the FP32 fields, over the chunks the last interact marked in cbits.  Every other cell
 // has As = Fs = Ts = 0 there and keeps its values, as in the dense update.  With cbits == nullptr (unstructured
-// meshes) every cell is visited.  A warp per bitmap word, each store instruction covering 32 consecutive cells.
-__global__ void apply_forcing_kernel(int64_t N, const uint32_t* __restrict__ cbits, double dt,
-                                     const float* __restrict__ As, const float* __restrict__ Fs,
-                                     const float* __restrict__ Ts, float* __restrict__ U, float* __restrict__ T) {
+// meshes) every cell is visited.  A warp reads its words, a lane each, and queues the cells of the marked chunks that change (a
+// cell without force and solid keeps U and T), 32 consecutive cells at a time; they are updated on full warps.
+// Bound by the FP64 pipe: 6 operations a cell.  Early steps of 1800 solids at 256 x 288 x 224 166 -> 87 us (15 operations,
+// with the conversions, for every cell of a marked chunk, 13 of 32 lanes active), 100 circles at 1024^2 31 -> 25 (GB300).
+constexpr int APPLY_THREADS = 256;
+__device__ __forceinline__ void apply_queued(int64_t N, const int32_t* q, int count, double dt, const float* __restrict__ As,
+                                             const float* __restrict__ Fs, const float* __restrict__ Ts, float* __restrict__ U,
+                                             float* __restrict__ T) {
     const int lane = threadIdx.x & 31;
+    if (lane >= count) return;
+    const int64_t c = q[lane];
+    float f[3], u[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) { f[a] = Fs[a * N + c]; u[a] = U[a * N + c]; }
+    // separate roundings, as the solver's own field operations (no contraction into FMAs)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) U[a * N + c] = narrow(__dsub_rn(wide(u[a]), __dmul_rn(wide(f[a]), dt)));
+    if (T) T[c] = narrow(__dadd_rn(__dmul_rn(__dsub_rn(1.0, wide(As[c])), wide(T[c])), wide(Ts[c])));
+}
+__global__ void __launch_bounds__(APPLY_THREADS) apply_forcing_kernel(int64_t N, const uint32_t* __restrict__ cbits, double dt,
+                                                                      const float* __restrict__ As, const float* __restrict__ Fs,
+                                                                      const float* __restrict__ Ts, float* __restrict__ U,
+                                                                      float* __restrict__ T) {
+    __shared__ int32_t s_q[APPLY_THREADS / 32][64];
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    int32_t* q = s_q[threadIdx.x >> 5];
     const int64_t words = (N + 255) >> 8;
     const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < words; w += nw) {
-        const uint32_t word = cbits ? cbits[w] : 0xffffffffu;
-        if (!word) continue;
+    const int64_t run = max((int64_t)1, min((int64_t)32, words / (8 * nw)));
+    const int64_t tickets = (words + run - 1) / run;  // of up to 32 words, far apart
+    const bool finite = fabs(dt) < INFINITY;          // else every cell changes
+    int nq = 0;                                       // warp-uniform
+    for (int64_t t0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t0 < tickets; t0 += nw) {
+        const int64_t w0 = t0 + lane * tickets;
+        const uint32_t marks = w0 >= words ? 0u : (cbits ? cbits[w0] : 0xffffffffu);
+        for (unsigned some = __ballot_sync(FULL, marks != 0u); some; some &= some - 1) {
+            const int src = __ffs(some) - 1;
+            const int64_t w = t0 + src * tickets;
+            const uint32_t word = __shfl_sync(FULL, marks, src);
+            unsigned change = 0;  // bit t: this lane's cell of 32 t .. 32 t + 31
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            const int idx = 32 * t + lane;
-            const int64_t c = (w << 8) + idx;
-            if (((word >> (idx >> 3)) & 1u) && c < N) {
-                // separate roundings, as the solver's own field operations (no contraction into FMAs)
-                for (int a = 0; a < 3; ++a)
-                    U[a * N + c] = (float)__dsub_rn((double)U[a * N + c], __dmul_rn((double)Fs[a * N + c], dt));
-                if (T) T[c] = (float)__dadd_rn(__dmul_rn(__dsub_rn(1.0, (double)As[c]), (double)T[c]), (double)Ts[c]);
+            for (int t = 0; t < 8; ++t) {
+                const int idx = 32 * t + lane;
+                const int64_t c = (w << 8) + idx;
+                if (((word >> (idx >> 3)) & 1u) && c < N &&
+                    (!finite || Fs[c] != 0.f || Fs[N + c] != 0.f || Fs[2 * N + c] != 0.f || (T && (As[c] != 0.f || Ts[c] != 0.f))))
+                    change |= 1u << t;
+            }
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+                const bool on = (change >> t) & 1u;
+                const unsigned m = __ballot_sync(FULL, on);
+                if (!m) continue;
+                if (on) q[nq + __popc(m & ((1u << lane) - 1u))] = (int32_t)((w << 8) + 32 * t + lane);
+                nq += __popc(m);
+                __syncwarp();
+                if (nq >= 32) {
+                    apply_queued(N, q, 32, dt, As, Fs, Ts, U, T);
+                    __syncwarp();
+                    nq -= 32;
+                    const int32_t keep = q[32 + lane];
+                    __syncwarp();
+                    if (lane < nq) q[lane] = keep;
+                    __syncwarp();
+                }
             }
         }
     }
+    if (nq > 0) apply_queued(N, q, nq, dt, As, Fs, Ts, U, T);
 }
 
 // ---- finalize: cells shared by several solids, forces ------------------------------------------------------------------
@@ -1387,8 +1489,10 @@ __global__ void fields_to_f64_kernel(int64_t N, const float* __restrict__ As, co
     }
 }
 
-// SolidCloud::fixInternal over the ALL_INSIDE list: U = rigid velocity of the solid that owns the cell
-__global__ void fix_internal_kernel(MeshK m, const sdfibm_solid_state* __restrict__ st,
+// SolidCloud::fixInternal over the ALL_INSIDE list: U = rigid velocity of the solid that owns the cell.  Bound by the FP64 pipe:
+// 12 operations a cell (30 with the centres and the roundings computed on it).
+// 36 -> 18 us in the same steps, 21 -> 10 for the circles (GB300).
+__global__ void fix_internal_kernel(MeshK m, const double* __restrict__ centres, const sdfibm_solid_state* __restrict__ st,
                                     const int32_t* __restrict__ in_cell, const int32_t* __restrict__ in_solid,
                                     const int32_t* __restrict__ Ct, float* __restrict__ U, const Counters* cnt) {
     const int n_in = clamp_len(cnt->n_inside, cnt->list_cap);
@@ -1401,9 +1505,11 @@ __global__ void fix_internal_kernel(MeshK m, const sdfibm_solid_state* __restric
         int i, j, k;
         cell_ijk(m, c, i, j, k);
         const sdfibm_solid_state& x = st[s];
-        const D3 vel{x.vel[0], x.vel[1], x.vel[2]}, om{x.omega[0], x.omega[1], x.omega[2]};
-        const D3 u = vel + cross(om, mesh_C(m, i, j, k) - state_pos(x));
-        U[c] = (float)u.x; U[N + c] = (float)u.y; U[2 * N + c] = (float)u.z;
+        const double dx = centres[i] - x.pos[0], dy = centres[m.nx + j] - x.pos[1], dz = centres[m.nx + m.ny + k] - x.pos[2];
+        const double ox = x.omega[0], oy = x.omega[1], oz = x.omega[2];
+        U[c] = narrow(__fma_rn(oy, dz, __fma_rn(-oz, dy, x.vel[0])));
+        U[N + c] = narrow(__fma_rn(oz, dx, __fma_rn(-ox, dz, x.vel[1])));
+        U[2 * N + c] = narrow(__fma_rn(ox, dy, __fma_rn(-oy, dx, x.vel[2])));
     }
 }
 

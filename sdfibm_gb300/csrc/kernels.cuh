@@ -111,6 +111,7 @@ struct Counters {
     int32_t n_fb;             // LEARNED: of those, cells outside the model's band (SUBSAMPLE fallback)
     int32_t n_recheck;        // SUBSAMPLE points left to recheck_kernel this call
     int32_t n_ovf;            // LEARNED: fallback cells whose points overflowed the recheck list (recount_kernel)
+    int32_t couple_next;      // next 64 chunks of couple_chunks_kernel (FP64 forcing)
     int32_t n_shent;          // list entries on cells several solids claimed (scan_reset_kernel)
     int32_t n_inband;         // LEARNED: listed cut cells inside the band, compacted for the network
     int32_t n_small;          // LEARNED: cut cells of solids under rho_min, listed from the back (fallback)
