@@ -442,24 +442,79 @@ __device__ inline int block_log2(int n, bool flat) {
     return 0;
 }
 
-// Run counting for the convex shapes (3-D): the inside samples of a lattice column (a, b) are one run, since the
-// exact inside function q is convex along the column's line.  Along the column the local coordinates are
-// w + c d (c the sample index), so the quadric is the polynomial A c^2 + 2 B c + C and the box the maximum of three
-// |w + c d| - k.  The run's ends come from their FP32 roots (any error there only costs time); the polynomial values
-// at a few samples, within Egh of q there, then decide the whole column:
-//   run [c1, c2] found: c1 and c2 inside, c1 - 1 and c2 + 1 outside (or off the column).  Every sample between the
-//     ends is inside (q there is at most its value at the ends) and every sample past c2 + 1 outside (q grows past a
-//     rise from an inside to an outside sample), and likewise before c1 - 1;
-//   no sample in the interval: the samples cv and cv + 1 around the closest approach outside, with q certified to
-//     rise from cv to cv - 1 and from cv + 1 to cv + 2 (computed rise of at least 2 Egh); every sample past them is
-//     then outside.  For the box, a slab that holds neither end of the column (on the same side) settles it first.
-// A column that does not verify (a value within Egh of zero, a run end off by one, a flat approach) is walked sample
-// by sample with the coordinates, bound and deferral of subsample_count.  The count is therefore the exhaustive
+// Run counting for the convex shapes (3-D): the inside samples of a lattice column (a, b) are one run.  Along the column the
+// local coordinates are w + c d (c the sample index), so the inside function q is the quadric polynomial A c^2 + 2 B c + C or
+// the box maximum of three |w + c d| - k.  Two intervals of c decide the column: I, where q <= -E, holds certain samples only,
+// and P, where q <= E, all possible ones (E >= every rounding between the real q of the reference's sample and the interval's
+// ends).  If both hold the same samples, that is the column's count, and it is 0 if P holds none; else the column is walked
+// sample by sample with the coordinates, bound and deferral of subsample_count.  The count is therefore the exhaustive
 // lattice count.
 //
-// Egh: the polynomial's value differs from the walk's coordinates-then-shape evaluation by the roundings of w, d,
-// the coefficients and the Horner steps, each a few units of roundoff of the magnitudes sum k X^2 + k3 (quadric) or
-// max |X| + max k (box) over the cell; the caller adds 64 (quadric) or 32 (box) units of roundoff of those sums to Eg.
+// E.  Quadric, M = sum k X^2 + k3 over the cell: w, d and the coefficients give the polynomial's value to a few units of
+// roundoff u of M.  An end is (-B -+ s) / A with s = sqrt(B^2 - A (C -+ E)); B^2 <= A M and s^2 <= A M, so B^2 - A C is
+// good to 3 u A M and the ends to an error that changes q by at most 16 u M (2^-22 for the approximate root included);
+// sample_frame adds 128 u M to Eg.  Box, m = max |X| + max k: the ends err by a few u m; sample_frame adds 64 u m, and a slab
+// the column hardly moves against (|d| < E / 4 n) takes that d, which shifts a coordinate by E / 4: 1.3 E in all.
+struct RunFrame {
+    float kdx, kdy, kdz, A, minvA, AE;               // quadric (minvA: -1 / A)
+    float ix, iy, iz, px, py, pz, cx, cy, cz;        // box: -1 / d, half widths of P and of I
+    float last;                                      // n - 1
+};
+template <int T>
+__device__ __forceinline__ RunFrame run_frame(const SampleFrame& f, float Egh, int n, float invn) {
+    RunFrame r;
+    r.last = (float)(n - 1);
+    const float dx = f.szx * invn, dy = f.szy * invn, dz = f.szz * invn;
+    if (T == SS_QUADRIC) {
+        r.kdx = f.k0 * dx; r.kdy = f.k1 * dy; r.kdz = f.k2 * dz;
+        r.A = __fmaf_rn(dx, r.kdx, __fmaf_rn(dy, r.kdy, dz * r.kdz));
+        r.minvA = -__frcp_rn(r.A);
+        // a leading coefficient that is no normal number: no column is decided (E = NaN)
+        r.AE = r.A > 1e-36f ? r.A * Egh : NAN;
+    } else {
+        const float least = 0.25f * Egh * invn, E = 1.3f * Egh;
+        const float ix = __frcp_rn(fabsf(dx) < least ? least : dx), iy = __frcp_rn(fabsf(dy) < least ? least : dy),
+                    iz = __frcp_rn(fabsf(dz) < least ? least : dz);
+        r.ix = -ix; r.iy = -iy; r.iz = -iz;
+        r.px = (f.k0 + E) * fabsf(ix); r.py = (f.k1 + E) * fabsf(iy); r.pz = (f.k2 + E) * fabsf(iz);
+        r.cx = (f.k0 - E) * fabsf(ix); r.cy = (f.k1 - E) * fabsf(iy); r.cz = (f.k2 - E) * fabsf(iz);
+    }
+    return r;
+}
+__device__ __forceinline__ float sqrt_fast(float x) {
+    float y;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// inside samples of the column whose sample c has the local coordinates w + c d, or -1: to be walked (as is whatever is not a
+// number here)
+template <int T>
+__device__ __forceinline__ float run_column(const SampleFrame& f, const RunFrame& r, float wx, float wy, float wz) {
+    float p1, p2, c1, c2;  // P and I
+    bool none, some = true;  // P is empty, I is not
+    if (T == SS_QUADRIC) {
+        const float B = __fmaf_rn(wx, r.kdx, __fmaf_rn(wy, r.kdy, wz * r.kdz));
+        const float C = __fmaf_rn(wx * wx, f.k0, __fmaf_rn(wy * wy, f.k1, __fmaf_rn(wz * wz, f.k2, -f.k3)));
+        const float disc = __fmaf_rn(B, B, r.A * -C), dp = disc + r.AE, dc = disc - r.AE;
+        const float mid = B * r.minvA, sp = sqrt_fast(dp), sc = sqrt_fast(dc);  // NaN below zero
+        p1 = __fmaf_rn(sp, r.minvA, mid); p2 = __fmaf_rn(-sp, r.minvA, mid);
+        c1 = __fmaf_rn(sc, r.minvA, mid); c2 = __fmaf_rn(-sc, r.minvA, mid);
+        none = dp <= 0.f;
+    } else {
+        const float mx = wx * r.ix, my = wy * r.iy, mz = wz * r.iz;
+        p1 = fmaxf(fmaxf(mx - r.px, my - r.py), mz - r.pz); p2 = fminf(fminf(mx + r.px, my + r.py), mz + r.pz);
+        c1 = fmaxf(fmaxf(mx - r.cx, my - r.cy), mz - r.cz); c2 = fminf(fminf(mx + r.cx, my + r.cy), mz + r.cz);
+        none = p1 > p2;
+        some = mx + my + mz == mx + my + mz;
+    }
+    some = some && c1 <= c2;
+    // the first and the last sample of each in the column, plus 3 2^22 (the sum's last place is 1: its directed rounding is
+    // the ceiling or the floor); an end beyond the column's is the column's, however uncertain it is
+    const float R = 12582912.f;
+    const float pa = __fadd_ru(fmaxf(p1, 0.f), R), pb = __fadd_rd(fminf(p2, r.last), R), cnt = pb - pa + 1.f;
+    const bool same = pa == __fadd_ru(fmaxf(c1, 0.f), R) && pb == __fadd_rd(fminf(c2, r.last), R);
+    return none || cnt <= 0.f ? 0.f : (same && some ? cnt : -1.f);
+}
 template <int T, bool DEFER_ONLY>
 __device__ __forceinline__ int subsample_runs_body(const MeshK& m, const ShapeK& sh, const SampleFrame& f, float Egh,
                                                    int64_t i, int64_t j, int64_t k, int n, const D3& x, const Q4& q,
@@ -469,15 +524,8 @@ __device__ __forceinline__ int subsample_runs_body(const MeshK& m, const ShapeK&
     const int lane = threadIdx.x & 31;
     uint16_t* walk_list = s_walk[(threadIdx.x >> 5) & 7];
     // correctly rounded reciprocals (the same values as 1.0f / x, without the division sequence)
-    const float inv2n = __frcp_rn((float)(2 * n)), nf = (float)n, invn = __frcp_rn(nf);
-    const float rise = 2.0001f * Egh;
-    // per-sample step along the column and the per-cell parts of the polynomial
-    const float dx = f.szx * invn, dy = f.szy * invn, dz = f.szz * invn;
-    const float kdx = f.k0 * dx, kdy = f.k1 * dy, kdz = f.k2 * dz;
-    const float A = __fmaf_rn(dx, kdx, __fmaf_rn(dy, kdy, dz * kdz));
-    const float invA = __frcp_rn(A);
-    const float idx_ = __frcp_rn(dx), idy = __frcp_rn(dy), idz = __frcp_rn(dz);
-    const float kx0 = f.k0 * idx_, ky0 = f.k1 * idy, kz0 = f.k2 * idz;
+    const float inv2n = __frcp_rn((float)(2 * n)), invn = __frcp_rn((float)n);
+    const RunFrame rf = run_frame<T>(f, Egh, n, invn);
     auto column_base = [&](int col, int& ia, int& ib, float& bx, float& by, float& bz) {
         ib = __float2int_rz(((float)col + 0.5f) * invn);
         ia = col - ib * n;
@@ -501,76 +549,15 @@ __device__ __forceinline__ int subsample_runs_body(const MeshK& m, const ShapeK&
 #pragma unroll 1
     for (int base = 0; base < n * n; base += 32) {
         const int col = base + lane;
-        int res = 0;
+        float res = 0.f;
         int ia = 0, ib = 0;
         float bx = 0.f, by = 0.f, bz = 0.f;
         if (col < n * n) {
             column_base(col, ia, ib, bx, by, bz);
             // coordinates of sample c: w + c d
-            const float wx = __fmaf_rn(f.szx, inv2n, bx), wy = __fmaf_rn(f.szy, inv2n, by),
-                        wz = __fmaf_rn(f.szz, inv2n, bz);
-            float B2 = 0.f, C = 0.f;
-            float cl, cr;
-            if (T == SS_QUADRIC) {
-                const float B = __fmaf_rn(wx, kdx, __fmaf_rn(wy, kdy, wz * kdz));
-                C = __fmaf_rn(wx * wx, f.k0, __fmaf_rn(wy * wy, f.k1, (wz * wz) * f.k2)) - f.k3;
-                B2 = 2.f * B;
-                const float disc = __fmaf_rn(B, B, -A * C);
-                const float sq = disc > 0.f ? disc * rsqrtf(disc) : 0.f;  // approximate: only locates the run
-                cl = (-B - sq) * invA;
-                cr = disc > 0.f ? (-B + sq) * invA : cl - 1.f;  // empty: cl marks the closest approach
-            } else {
-                const float lx = __fmaf_rn(-wx, idx_, -kx0), rx = __fmaf_rn(-wx, idx_, kx0);
-                const float ly = __fmaf_rn(-wy, idy, -ky0), ry = __fmaf_rn(-wy, idy, ky0);
-                const float lz = __fmaf_rn(-wz, idz, -kz0), rz = __fmaf_rn(-wz, idz, kz0);
-                cl = fmaxf(fmaxf(fminf(lx, rx), fminf(ly, ry)), fminf(lz, rz));
-                cr = fminf(fminf(fmaxf(lx, rx), fmaxf(ly, ry)), fmaxf(lz, rz));
-            }
-            auto g_at = [&](int c3) {
-                const float c = (float)c3;
-                if (T == SS_QUADRIC) return __fmaf_rn(__fmaf_rn(A, c, B2), c, C);
-                return fmaxf(fmaxf(fabsf(__fmaf_rn(c, dx, wx)) - f.k0, fabsf(__fmaf_rn(c, dy, wy)) - f.k1),
-                             fabsf(__fmaf_rn(c, dz, wz)) - f.k2);
-            };
-            // clamped before the conversions (inf / NaN safe)
-            const float ul = fminf(fmaxf(cl, -2.f), nf + 1.f), ur = fminf(fmaxf(cr, -2.f), nf + 1.f);
-            const int c1 = max((int)ceilf(ul), 0), c2 = min((int)floorf(ur), n - 1);
-            // inside: g < -Egh, outside: g > Egh (band() of the walk, as plain comparisons)
-            res = -1;
-            if (cl <= cr && c1 <= c2) {
-                bool ok = g_at(c1) < -Egh && (c2 == c1 || g_at(c2) < -Egh);
-                if (ok && c1 > 0) ok = g_at(c1 - 1) > Egh;
-                if (ok && c2 < n - 1) ok = g_at(c2 + 1) > Egh;
-                if (ok) res = c2 - c1 + 1;
-            } else {
-                // the pair cv, cv + 1 around the closest approach: both outside, q rising from cv to cv - 1 and
-                // from cv + 1 to cv + 2 (a pair rather than one sample: with the approach halfway between two
-                // samples, the rise from the nearer one to the other would be about zero)
-                float um = (T == SS_QUADRIC && !(cl <= cr)) ? ul : 0.5f * (ul + ur);
-                bool separated = false;
-                if (T == SS_BOX) {
-                    // a slab whose coordinate is beyond it at both ends of the column, on the same side, holds no
-                    // sample (the coordinate is linear along the column; computed within Egh of q at the ends)
-                    const float last = nf - 1.f;
-                    auto beyond = [&](float w0, float d0, float k0) {
-                        const float x1 = __fmaf_rn(last, d0, w0);
-                        return (w0 > 0.f) == (x1 > 0.f) && fabsf(w0) - k0 > Egh && fabsf(x1) - k0 > Egh;
-                    };
-                    separated = beyond(wx, dx, f.k0) || beyond(wy, dy, f.k1) || beyond(wz, dz, f.k2);
-                }
-                if (separated) {
-                    res = 0;
-                } else {
-                    const int cv = min(max(__float2int_rd(fminf(fmaxf(um, 0.f), nf - 2.f)), 0), n - 2);
-                    const float g0 = g_at(cv), g1 = g_at(cv + 1);
-                    bool ok = g0 > Egh && g1 > Egh;
-                    if (ok && cv >= 1) ok = g_at(cv - 1) - g0 >= rise;
-                    if (ok && cv + 2 <= n - 1) ok = g_at(cv + 2) - g1 >= rise;
-                    if (ok) res = 0;
-                }
-            }
+            res = run_column<T>(f, rf, __fmaf_rn(f.szx, inv2n, bx), __fmaf_rn(f.szy, inv2n, by), __fmaf_rn(f.szz, inv2n, bz));
         }
-        const bool walk = res < 0;
+        const bool walk = res < 0.f;
         const unsigned mask = __ballot_sync(FULL, walk);
         const int pos = nwalk + __popc(mask & ((1u << lane) - 1u));
         nwalk += __popc(mask);
@@ -581,7 +568,7 @@ __device__ __forceinline__ int subsample_runs_body(const MeshK& m, const ShapeK&
                 for (int c3 = 0; c3 < n; ++c3) cnt += walk_sample(ia, ib, c3, bx, by, bz);
             }
         } else {
-            cnt += res;
+            cnt += (int)res;
         }
     }
     __syncwarp();
@@ -609,18 +596,14 @@ __device__ __noinline__ int subsample_runs(const MeshK& m, const ShapeK& sh, con
     return subsample_runs_body<T, DEFER_ONLY>(m, sh, f, Egh, i, j, k, n, x, q, rechecks, df);
 }
 
-// Inside count of the cell's n^3 (n^2 on one-layer meshes) lattice; with a Defer the undecided points are not counted
-// here but appended to the recheck list.  DEFER_ONLY: x, q and (i, j, k) only feed the FP64 path, which it lacks.
-template <bool DEFER_ONLY>
-static __device__ __forceinline__ int subsample_warp_body(const MeshK& m, const ShapeK& sh, const float* M,
-                                                          const TileFrame& tf, int a0, int b0, int c0, const D3& x,
-                                                          const Q4& q, int64_t i, int64_t j, int64_t k, int n,
-                                                          unsigned long long* rechecks, const Defer* df) {
+// The frame of a cell's lattice (cell (a0, b0, c0) of the tile) and its bounds: Ep of the coordinates with the offset, Egh of the
+// columns' intervals (E above).
+__device__ __forceinline__ int sample_frame(const MeshK& m, const ShapeK& sh, const float* M, const TileFrame& tf, int a0, int b0,
+                                            int c0, SampleFrame& f, float& Ep, float& Egh) {
     const float u = U32;
     const float hx = m.h32[0], hy = m.h32[1], hz = m.h32[2];
     const float ox = (float)a0 * hx, oy = (float)b0 * hy, oz = (float)c0 * hz;  // cell corner within the tile
     const float dx = tf.bx + ox, dy = tf.by + oy, dz = tf.bz + oz;
-    SampleFrame f;
     f.px = __fmaf_rn(M[0], dx, __fmaf_rn(M[1], dy, M[2] * dz));
     f.py = __fmaf_rn(M[3], dx, __fmaf_rn(M[4], dy, M[5] * dz));
     f.pz = __fmaf_rn(M[6], dx, __fmaf_rn(M[7], dy, M[8] * dz));
@@ -641,8 +624,10 @@ static __device__ __forceinline__ int subsample_warp_body(const MeshK& m, const 
         kind = SS_QUADRIC;
     else if (type == SDFIBM_SHAPE_RECTANGLE || type == SDFIBM_SHAPE_BOX)
         kind = SS_BOX;
-    float Ep = f.E;
-    if (kind != SS_GENERIC) {
+    Ep = f.E;
+    Egh = 0.f;
+    if (kind == SS_GENERIC) return kind;
+    {
         // sample = (corner + com) + steps: one more rounding of the corner, the conversion of com to FP32, and the
         // stepping FMAs now run at magnitudes up to |com| larger (the ellipsoid ignores com, as the reference does)
         const bool use_com = type != SDFIBM_SHAPE_ELLIPSOID;
@@ -663,10 +648,6 @@ static __device__ __forceinline__ int subsample_warp_body(const MeshK& m, const 
     const float mx = fabsf(f.px) + fabsf(f.sxx) + fabsf(f.syx) + fabsf(f.szx) + Ep;
     const float my = fabsf(f.py) + fabsf(f.sxy) + fabsf(f.syy) + fabsf(f.szy) + Ep;
     const float mz = fabsf(f.pz) + fabsf(f.sxz) + fabsf(f.syz) + fabsf(f.szz) + Ep;
-    // 3-D convex shapes count runs along columns from 5 samples per axis; out of line (the classify pass), lattices
-    // of 16 and more skip 4 x 4 x 4 blocks instead
-    const bool use_runs = !m.twod && !prism && n >= 5 && (DEFER_ONLY || n < 16);
-    int cnt;
     if (kind == SS_QUADRIC) {
         switch (type) {
             case SDFIBM_SHAPE_CIRCLE:
@@ -676,7 +657,32 @@ static __device__ __forceinline__ int subsample_warp_body(const MeshK& m, const 
         }
         f.Eg = (2.f * (mx * f.k0 + my * f.k1 + mz * f.k2) + Ep * (f.k0 + f.k1 + f.k2)) * Ep +
                10.f * u * (mx * mx * f.k0 + my * my * f.k1 + mz * mz * f.k2 + f.k3);
-        const float Egh = f.Eg + 64.f * u * (mx * mx * f.k0 + my * my * f.k1 + mz * mz * f.k2 + f.k3);
+        Egh = f.Eg + 128.f * u * (mx * mx * f.k0 + my * my * f.k1 + mz * mz * f.k2 + f.k3);
+    } else {
+        f.k0 = a[0]; f.k1 = a[1];
+        f.k2 = prism ? INFINITY : a[2];  // the rectangle has no z extent
+        f.k3 = 0.f;
+        f.Eg = Ep + 2.f * u * (fmaxf(mx, fmaxf(my, prism ? 0.f : mz)) + fmaxf(a[0], fmaxf(a[1], prism ? 0.f : a[2])));
+        Egh = f.Eg + 64.f * u * (fmaxf(mx, fmaxf(my, mz)) + fmaxf(a[0], fmaxf(a[1], a[2])));
+    }
+    return kind;
+}
+
+// Inside count of the cell's n^3 (n^2 on one-layer meshes) lattice; with a Defer the undecided points are not counted
+// here but appended to the recheck list.  DEFER_ONLY: x, q and (i, j, k) only feed the FP64 path, which it lacks.
+template <bool DEFER_ONLY>
+static __device__ __forceinline__ int subsample_warp_body(const MeshK& m, const ShapeK& sh, const float* M,
+                                                          const TileFrame& tf, int a0, int b0, int c0, const D3& x,
+                                                          const Q4& q, int64_t i, int64_t j, int64_t k, int n,
+                                                          unsigned long long* rechecks, const Defer* df) {
+    SampleFrame f;
+    float Ep, Egh;
+    const int kind = sample_frame(m, sh, M, tf, a0, b0, c0, f, Ep, Egh);
+    // 3-D convex shapes count runs along columns from 5 samples per axis; out of line (the classify pass), lattices
+    // of 16 and more skip 4 x 4 x 4 blocks instead
+    const bool use_runs = !m.twod && !sh.prism && n >= 5 && (DEFER_ONLY || n < 16);
+    int cnt;
+    if (kind == SS_QUADRIC) {
         const int lb = block_log2(n, m.twod != 0);
         if (use_runs && DEFER_ONLY)
             cnt = subsample_runs_body<SS_QUADRIC, true>(m, sh, f, Egh, i, j, k, n, x, q, rechecks, df);
@@ -687,10 +693,6 @@ static __device__ __forceinline__ int subsample_warp_body(const MeshK& m, const 
         else
             cnt = subsample_count<SS_QUADRIC, DEFER_ONLY>(m, sh, f, i, j, k, n, x, q, rechecks, df);
     } else if (kind == SS_BOX) {
-        f.k0 = a[0]; f.k1 = a[1];
-        f.k2 = prism ? INFINITY : a[2];  // the rectangle has no z extent
-        f.Eg = Ep + 2.f * u * (fmaxf(mx, fmaxf(my, prism ? 0.f : mz)) + fmaxf(a[0], fmaxf(a[1], prism ? 0.f : a[2])));
-        const float Egh = f.Eg + 32.f * u * (fmaxf(mx, fmaxf(my, mz)) + fmaxf(a[0], fmaxf(a[1], a[2])));
         const int lb = block_log2(n, m.twod != 0);
         if (use_runs && DEFER_ONLY)
             cnt = subsample_runs_body<SS_BOX, true>(m, sh, f, Egh, i, j, k, n, x, q, rechecks, df);
@@ -1586,25 +1588,28 @@ __device__ __forceinline__ void classify_body(const ClassifyArgs& A) {
     }
 }
 
-// SUBSAMPLE count of one listed cell (bbox index idx of solid s) from the cell's own FP32 frame, built as the classify
-// pass builds a tile's: the solid's rounded base plus a whole number of cells.
+// FP32 frame of the listed cell idx of a solid, built as the classify pass builds a tile's: the solid's rounded base plus a
+// whole number of cells; the cell's place in the bbox
+__device__ __forceinline__ int3 cell_frame(const FallbackArgs& A, const SolidK& k, const SolidPlan& pl, int64_t idx, TileFrame& tf) {
+    const uint32_t local = (uint32_t)(idx - k.scratch_off);  // < bbox cells of one solid (< 2^31)
+    const int row = (int)fdiv(local, k.div_e0), lc = (int)fdiv(local, k.div_e01);
+    const int la = (int)local - row * k.ext[0], lb = row - lc * k.ext[1];
+    const float sbx = pl.base32[0], sby = pl.base32[1], sbz = pl.base32[2];
+    const float ofx = (float)la * A.m.h32[0], ofy = (float)lb * A.m.h32[1], ofz = (float)lc * A.m.h32[2];
+    tf.bx = sbx + ofx; tf.by = sby + ofy; tf.bz = sbz + ofz;
+    tf.babs = fabsf(sbx) + fabsf(sby) + fabsf(sbz) + 2.f * (fabsf(ofx) + fabsf(ofy) + fabsf(ofz)) +
+              fabsf(tf.bx) + fabsf(tf.by) + fabsf(tf.bz);
+    tf.e64 = pl.e64;
+    return make_int3(la, lb, lc);
+}
+// SUBSAMPLE count of one listed cell (bbox index idx of solid s) by a warp
 template <bool DEFER_ONLY>
 __device__ __forceinline__ int count_listed_cell(const FallbackArgs& A, int s, int64_t idx, unsigned long long* rechecks,
                                                  const Defer* df) {
     const SolidK& k = A.sk[s];
     const SolidPlan& pl = A.plan[s];
-    const uint32_t local = (uint32_t)(idx - k.scratch_off);  // < bbox cells of one solid (< 2^31)
-    const int row = (int)fdiv(local, k.div_e0), lc = (int)fdiv(local, k.div_e01);
-    const int la = (int)local - row * k.ext[0], lb = row - lc * k.ext[1];
     TileFrame tf;
-    {
-        const float sbx = pl.base32[0], sby = pl.base32[1], sbz = pl.base32[2];
-        const float ofx = (float)la * A.m.h32[0], ofy = (float)lb * A.m.h32[1], ofz = (float)lc * A.m.h32[2];
-        tf.bx = sbx + ofx; tf.by = sby + ofy; tf.bz = sbz + ofz;
-        tf.babs = fabsf(sbx) + fabsf(sby) + fabsf(sbz) + 2.f * (fabsf(ofx) + fabsf(ofy) + fabsf(ofz)) +
-                  fabsf(tf.bx) + fabsf(tf.by) + fabsf(tf.bz);
-        tf.e64 = pl.e64;
-    }
+    const int3 at = cell_frame(A, k, pl, idx, tf);
     float M[9];
 #pragma unroll
     for (int r = 0; r < 9; ++r) M[r] = pl.M[r];
@@ -1614,15 +1619,104 @@ __device__ __forceinline__ int count_listed_cell(const FallbackArgs& A, int s, i
     }
     const Q4 q = state_quat(A.st[s]);
     const D3 x = state_pos(A.st[s]);
-    return subsample_warp(A.m, k.shape, M, tf, 0, 0, 0, x, q, pl.lo[0] + la, pl.lo[1] + lb, pl.lo[2] + lc, A.n,
+    return subsample_warp(A.m, k.shape, M, tf, 0, 0, 0, x, q, pl.lo[0] + at.x, pl.lo[1] + at.y, pl.lo[2] + at.z, A.n,
                           rechecks, df);
 }
 
-// SUBSAMPLE of listed cells, one warp per cell: the cut cells of the classify pass (SUBSAMPLE, fb_list == nullptr)
+// The same of 32 listed cells at once, a lane each: all lanes do the same column of their own cells, so nothing of a cell's
+// frame is computed 32 times and no lane is without a column.  Columns left to the walk are listed and their samples spread
+// over the lanes, which take the frame of the sample's cell from its lane.  Lanes with `mine` have cells of kind T.
+constexpr int WALK_CAP = 96;
+constexpr int SUB_WINDOW = 256;  // cells of a warp sorted by kind
+struct ThreadWalk {
+    uint32_t list[WALK_CAP];  // lane of the cell | column << 5
+    int32_t inside[32];       // walked samples found inside, per lane
+    int32_t overflow[32];
+};
+template <int T>
+__device__ __forceinline__ int thread_runs(const FallbackArgs& A, const ShapeK& sh, const SampleFrame& f, float Egh, bool mine,
+                                           int s, int64_t idx, ThreadWalk& tw, unsigned long long* rechecks) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, n = A.n;
+    const float inv2n = __frcp_rn((float)(2 * n)), invn = __frcp_rn((float)n);
+    const RunFrame rf = run_frame<T>(f, Egh, n, invn);
+    float cnt = 0.f;
+    int nwalk = 0;
+    auto flush = [&]() {
+        __syncwarp();
+        for (int e0 = 0; e0 < nwalk * n; e0 += 32) {
+            const int e = min(e0 + lane, nwalk * n - 1), w = __float2int_rz(((float)e + 0.5f) * invn), c3 = e - w * n;
+            const uint32_t it = tw.list[w];
+            const int from = (int)(it & 31u), col = (int)(it >> 5), ib = __float2int_rz(((float)col + 0.5f) * invn), ia = col - ib * n;
+            SampleFrame g;
+            auto of = [&](float v) { return __shfl_sync(FULL, v, from); };
+            g.px = of(f.px); g.py = of(f.py); g.pz = of(f.pz);
+            g.sxx = of(f.sxx); g.sxy = of(f.sxy); g.sxz = of(f.sxz);
+            g.syx = of(f.syx); g.syy = of(f.syy); g.syz = of(f.syz);
+            g.szx = of(f.szx); g.szy = of(f.szy); g.szz = of(f.szz);
+            g.k0 = of(f.k0); g.k1 = of(f.k1); g.k2 = of(f.k2); g.k3 = of(f.k3);
+            g.Eg = of(f.Eg);
+            const int so = __shfl_sync(FULL, s, from);
+            const int64_t io = __shfl_sync(FULL, idx, from);
+            const float ta = (float)(2 * ia + 1) * inv2n, tb = (float)(2 * ib + 1) * inv2n, tc = (float)(2 * c3 + 1) * inv2n;
+            const float bx = __fmaf_rn(tb, g.syx, __fmaf_rn(ta, g.sxx, g.px)), by = __fmaf_rn(tb, g.syy, __fmaf_rn(ta, g.sxy, g.py)),
+                        bz = __fmaf_rn(tb, g.syz, __fmaf_rn(ta, g.sxz, g.pz));
+            if (e0 + lane < nwalk * n) {
+                int r = band(sample_g<T>(g, __fmaf_rn(tc, g.szx, bx), __fmaf_rn(tc, g.szy, by), __fmaf_rn(tc, g.szz, bz)), g.Eg);
+                if (r == 2) {
+                    ++*rechecks;
+                    const Defer df{A.rq, A.rq_cap, &A.cnt->n_recheck, io, so, &tw.overflow[from]};
+                    r = undecided_sample<true>(&df, sh, A.m, 0, 0, 0, ia, ib, c3, n, D3{0, 0, 0}, Q4{1, D3{0, 0, 0}});
+                }
+                if (r) atomicAdd(&tw.inside[from], r);
+            }
+        }
+        nwalk = 0;
+        __syncwarp();
+    };
+    // coordinates of a column's sample 0
+    const float qx = __fmaf_rn(f.szx, inv2n, f.px), qy = __fmaf_rn(f.szy, inv2n, f.py), qz = __fmaf_rn(f.szz, inv2n, f.pz);
+    float oa = 1.f;  // 2 ia + 1, exact
+#pragma unroll 1
+    for (int ia = 0; ia < n; ++ia, oa += 2.f) {
+        const float ta = oa * inv2n;
+        const float ux = __fmaf_rn(ta, f.sxx, qx), uy = __fmaf_rn(ta, f.sxy, qy), uz = __fmaf_rn(ta, f.sxz, qz);
+        float ob = 1.f;
+        for (int ib0 = 0; ib0 < n; ib0 += 32) {
+            uint32_t walk = 0;  // columns ib0 + bit of this row
+            const int m = min(32, n - ib0);
+#pragma unroll 2
+            for (int b = 0; b < m; ++b, ob += 2.f) {
+                const float tb = ob * inv2n;
+                const float res = run_column<T>(f, rf, __fmaf_rn(tb, f.syx, ux), __fmaf_rn(tb, f.syy, uy), __fmaf_rn(tb, f.syz, uz));
+                if (res < 0.f) walk |= 1u << b;
+                cnt += fmaxf(res, 0.f);
+            }
+            if (!mine) walk = 0;
+            while (__any_sync(FULL, walk != 0)) {
+                const unsigned mask = __ballot_sync(FULL, walk != 0);
+                if (walk) {
+                    tw.list[nwalk + __popc(mask & ((1u << lane) - 1u))] = (uint32_t)lane | (uint32_t)(ia + (ib0 + __ffs(walk) - 1) * n) << 5;
+                    walk &= walk - 1;
+                }
+                nwalk += __popc(mask);
+                if (nwalk > WALK_CAP - 32) flush();
+            }
+        }
+    }
+    flush();
+    return (int)cnt;
+}
+
+// SUBSAMPLE of listed cells: the cut cells of the classify pass (SUBSAMPLE, fb_list == nullptr)
 // or the cells outside the network's band (LEARNED fallback).  Undecided points always go to the recheck list (this
 // kernel holds no FP64 path, which keeps its register count and so its occupancy); a cell some of whose points found
 // the list full is listed for recount_kernel.
-__global__ void __launch_bounds__(256, 4) subsample_cells_kernel(FallbackArgs A) {
+// 3-D convex shapes on lattices of 5 samples and more are done a lane per cell from A.lane_min cells on, everything else a
+// warp per cell.  Bound by issue.  Measured (GB300): 1.32 M cells of 10^3 samples, 1.32 -> 0.33 ms (a warp per cell with four
+// evaluations of q to verify each column's run: 984 instructions a cell, now 226); 1.2 M cells of 16^3, 2.11 -> 0.75 ms.  A warp
+// per cell took 32 cells each however few there were: 1092 cells 98 -> 12 us.
+__global__ void __launch_bounds__(256, 3) subsample_cells_kernel(FallbackArgs A) {
     __shared__ int32_t s_overflow[8];
     const int lane = threadIdx.x & 31;
     int32_t* overflow = s_overflow + ((threadIdx.x >> 5) & 7);
@@ -1635,37 +1729,110 @@ __global__ void __launch_bounds__(256, 4) subsample_cells_kernel(FallbackArgs A)
     const int64_t nfb = A.fb_list ? min(n_fb + n_back, A.cap) : min((int64_t)A.cnt->n_feat, A.cap);
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     unsigned long long rechecks = 0;
+    __shared__ ThreadWalk tw[8];
+    __shared__ uint8_t s_order[8][SUB_WINDOW];
+    const bool lanes = nfb >= A.lane_min && A.n >= 5 && !A.m.twod;
     if (lane == 0) *overflow = 0;
     __syncwarp();
-    // each warp takes 32 consecutive list entries: the 32 lanes load their (solid, index) pairs at once, then the
-    // warp counts the cells one after the other
-    for (int64_t base = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; base < nfb; base += warps * 32) {
-        int s_l = 0;
-        int64_t idx_l = 0;
-        if (base + lane < nfb) {
-            const int64_t q = base + lane;
-            const int64_t slot = !A.fb_list ? q : (q < n_fb ? (int64_t)A.fb_list[q] : A.cap - 1 - (q - n_fb));
-            s_l = A.fref_solid[slot];
-            idx_l = A.fref_index[slot];
-        }
-        const int batch = (int)min((int64_t)32, nfb - base);
-        for (int t = 0; t < batch; ++t) {
-            const int s = __shfl_sync(0xffffffffu, s_l, t);
-            const int64_t idx = __shfl_sync(0xffffffffu, idx_l, t);
-            const Defer df{A.rq, A.rq_cap, &A.cnt->n_recheck, idx, s, overflow};
-            const int cnt = count_listed_cell<true>(A, s, idx, &rechecks, &df);
-            __syncwarp();
-            if (lane == 0) {
-                A.alpha[idx] = -1.f - (float)cnt;
-                if (*(volatile int32_t*)overflow) {
-                    *overflow = 0;
-                    const int slot = atomicAdd(&A.cnt->n_ovf, 1);
-                    if (slot < A.ovf_cap) A.ovf[slot] = Recheck{idx, s, 0u};
-                    else set_error(A.cnt, DERR_CAPACITY);
+    auto entry = [&](int64_t q, int& s, int64_t& idx) {  // q-th listed cell
+        const int64_t slot = !A.fb_list ? q : (q < n_fb ? (int64_t)A.fb_list[q] : A.cap - 1 - (q - n_fb));
+        s = A.fref_solid[slot];
+        idx = A.fref_index[slot];
+    };
+    // each warp takes consecutive list entries, as many as give every warp some: a lane per cell, up to SUB_WINDOW of them,
+    // sorted by kind so that the lanes of a batch are alike, else up to 32, one after the other
+    const int64_t share = (nfb + warps - 1) / warps;
+    const int window = lanes ? (int)min((int64_t)SUB_WINDOW, (share + 31) & ~(int64_t)31) : (int)min((int64_t)32, share);
+    for (int64_t base = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * window; base < nfb; base += warps * window) {
+        const int count = (int)min((int64_t)window, nfb - base);
+        int rest = count, first = 0;  // entries left to the warp loop: order[first ..] (lanes), else all
+        uint8_t* order = s_order[(threadIdx.x >> 5) & 7];
+        if (lanes) {
+            // order: quadrics from the front, then boxes, then the others
+            int n_kind[3] = {0, 0, 0};
+            unsigned kinds = 0;  // two bits a batch
+            for (int t = 0; t < count; t += 32) {
+                int kind = 3, s = 0;
+                int64_t idx = 0;
+                if (t + lane < count) {
+                    entry(base + t + lane, s, idx);
+                    const ShapeK& sh = A.sk[s].shape;
+                    kind = sh.prism ? 2 : (sh.type == SDFIBM_SHAPE_SPHERE || sh.type == SDFIBM_SHAPE_ELLIPSOID ? 0
+                                                                      : (sh.type == SDFIBM_SHAPE_BOX ? 1 : 2));
+                }
+                kinds |= (unsigned)kind << (t >> 4);
+#pragma unroll
+                for (int v = 0; v < 3; ++v) n_kind[v] += __popc(__ballot_sync(0xffffffffu, kind == v));
+            }
+            int at[3] = {0, n_kind[0], n_kind[0] + n_kind[1]};
+            for (int t = 0; t < count; t += 32) {
+                const int kind = (kinds >> (t >> 4)) & 3;
+#pragma unroll
+                for (int v = 0; v < 3; ++v) {
+                    const unsigned m = __ballot_sync(0xffffffffu, kind == v);
+                    if (kind == v) order[at[v] + __popc(m & ((1u << lane) - 1u))] = (uint8_t)(t + lane);
+                    at[v] += __popc(m);
                 }
             }
             __syncwarp();
+            ThreadWalk& w = tw[(threadIdx.x >> 5) & 7];
+            first = n_kind[0] + n_kind[1];
+            rest = count - first;
+            for (int v = 0; v < 2; ++v) {
+                const int lo = v == 0 ? 0 : n_kind[0], hi = lo + n_kind[v];
+                for (int e0 = lo; e0 < hi; e0 += 32) {
+                    const bool mine = e0 + lane < hi;
+                    int s = 0;
+                    int64_t idx = 0;
+                    if (mine) entry(base + order[e0 + lane], s, idx);
+                    const SolidK& k = A.sk[s];
+                    SampleFrame f{};
+                    float Egh = 0.f;
+                    if (mine) {
+                        TileFrame tf;
+                        cell_frame(A, k, A.plan[s], idx, tf);
+                        float Ep;
+                        sample_frame(A.m, k.shape, A.plan[s].M, tf, 0, 0, 0, f, Ep, Egh);
+                    }
+                    w.inside[lane] = 0;
+                    w.overflow[lane] = 0;
+                    const int cnt = v == 0 ? thread_runs<SS_QUADRIC>(A, k.shape, f, Egh, mine, s, idx, w, &rechecks)
+                                           : thread_runs<SS_BOX>(A, k.shape, f, Egh, mine, s, idx, w, &rechecks);
+                    if (mine) {
+                        A.alpha[idx] = -1.f - (float)(cnt + w.inside[lane]);
+                        if (w.overflow[lane]) {
+                            const int slot = atomicAdd(&A.cnt->n_ovf, 1);
+                            if (slot < A.ovf_cap) A.ovf[slot] = Recheck{idx, s, 0u};
+                            else set_error(A.cnt, DERR_CAPACITY);
+                        }
+                    }
+                    __syncwarp();
+                }
+            }
         }
+        for (int t0 = 0; t0 < rest; t0 += 32) {
+            int s_l = 0;
+            int64_t idx_l = 0;
+            if (t0 + lane < rest) entry(base + (lanes ? order[first + t0 + lane] : t0 + lane), s_l, idx_l);
+            for (int t = 0; t < min(32, rest - t0); ++t) {
+                const int s = __shfl_sync(0xffffffffu, s_l, t);
+                const int64_t idx = __shfl_sync(0xffffffffu, idx_l, t);
+                const Defer df{A.rq, A.rq_cap, &A.cnt->n_recheck, idx, s, overflow};
+                const int cnt = count_listed_cell<true>(A, s, idx, &rechecks, &df);
+                __syncwarp();
+                if (lane == 0) {
+                    A.alpha[idx] = -1.f - (float)cnt;
+                    if (*(volatile int32_t*)overflow) {
+                        *overflow = 0;
+                        const int slot = atomicAdd(&A.cnt->n_ovf, 1);
+                        if (slot < A.ovf_cap) A.ovf[slot] = Recheck{idx, s, 0u};
+                        else set_error(A.cnt, DERR_CAPACITY);
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        __syncwarp();
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) rechecks += __shfl_xor_sync(0xffffffffu, rechecks, o);

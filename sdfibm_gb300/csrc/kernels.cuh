@@ -262,6 +262,7 @@ struct FallbackArgs {
     float* alpha;
     Counters* cnt;
     int n;                     // samples per axis
+    int64_t lane_min;          // cells from which a lane counts a cell (else a warp)
     Recheck* rq;
     int64_t rq_cap;
     Recheck* ovf;              // cells to recount (idx, solid), see recount_kernel
