@@ -29,9 +29,9 @@ __global__ void subsample_cells_kernel(FallbackArgs A);
 __global__ void recount_kernel(FallbackArgs A);
 __global__ void learned_stencil_kernel(StencilArgs A);
 int stencil_block();
-__global__ void refgeo_cells_kernel(MeshK m, const SolidK* sk, const SolidPlan* plan, const int32_t* fref_solid,
-                                    const int64_t* fref_index, const float* rg_phi, int64_t cap, const Counters* cnt,
-                                    float* alpha);
+void launch_refgeo_cells(const MeshK& m, const SolidK* sk, const sdfibm_solid_state* st, const SolidPlan* plan,
+                         const int32_t* fref_solid, const int64_t* fref_index, const float* rg_phi, int64_t cap,
+                         const Counters* cnt, float* alpha, int grid, cudaStream_t stream);
 __global__ void recheck_kernel(MeshK m, const SolidK* sk, const sdfibm_solid_state* st, const SolidPlan* plan,
                                const Recheck* rq, int64_t cap, Counters* cnt, float* alpha);
 __global__ void connect_kernel(ConnectArgs A);
@@ -858,10 +858,8 @@ static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float
             ++launches;
         }
         if (refgeo) {
-            refgeo_cells_kernel<<<ctx->refgeo_grid, 256, 0, st>>>(ctx->mesh, ctx->d_sk, ctx->d_plan,
-                                                                   ctx->d_fref_solid, ctx->d_fref_index,
-                                                                   ctx->d_rg_phi, ctx->feat_cap, ctx->d_cnt,
-                                                                   ctx->d_alpha);
+            launch_refgeo_cells(ctx->mesh, ctx->d_sk, ctx->d_st, ctx->d_plan, ctx->d_fref_solid, ctx->d_fref_index,
+                                ctx->d_rg_phi, ctx->feat_cap, ctx->d_cnt, ctx->d_alpha, ctx->refgeo_grid, st);
             mark(ctx, "refgeo_cells_kernel");
             ++launches;
         }

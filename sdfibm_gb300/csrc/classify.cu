@@ -815,26 +815,23 @@ __device__ __forceinline__ FF ff_scale(FF x, float n) {  // n: a small integer, 
 }
 __device__ __forceinline__ FF ff_abs(FF x) { return x.hi < 0.f ? FF{-x.hi, -x.lo} : x; }
 
-// Solid::phi of bbox vertex (da, db, dc) as sdf_mixed computes it (the same FP32 formula after the cancelling
-// differences), the local point from the plan's two-float map; err bounds the difference to the exact value with a
-// factor of 4 to spare over the operations' roundoff (2^-44 of the magnitudes).
-__device__ inline float sdf_ff(const ShapeK& s, const SolidPlan& pl, float da, float db, float dc, float& err) {
-    FF P[3];
-    float ml = 0.f;
+// component r of the local point of bbox vertex (da, db, dc) from the plan's two-float map; mag: the sum of the magnitudes
+__device__ __forceinline__ FF ff_local(const SolidPlan& pl, int r, float da, float db, float dc, float& mag) {
     const float f3[3] = {da, db, dc};
+    FF v{pl.lmap_hi[r], pl.lmap_lo[r]};
+    mag = fabsf(pl.lmap_hi[r]);
 #pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        FF v{pl.lmap_hi[r], pl.lmap_lo[r]};
-        float mag = fabsf(pl.lmap_hi[r]);
-#pragma unroll
-        for (int t = 0; t < 3; ++t) {
-            const int i = 3 + 3 * t + r;
-            v = ff_add(v, ff_scale(FF{pl.lmap_hi[i], pl.lmap_lo[i]}, f3[t]));
-            mag += fabsf(f3[t] * pl.lmap_hi[i]);
-        }
-        P[r] = v;
-        ml = fmaxf(ml, mag);
+    for (int t = 0; t < 3; ++t) {
+        const int i = 3 + 3 * t + r;
+        v = ff_add(v, ff_scale(FF{pl.lmap_hi[i], pl.lmap_lo[i]}, f3[t]));
+        mag += fabsf(f3[t] * pl.lmap_hi[i]);
     }
+    return v;
+}
+// Solid::phi at local point P as sdf_mixed computes it (the same FP32 formula after the cancelling differences); err bounds
+// the difference to the exact value with a factor of 4 to spare over the operations' roundoff (2^-44 of the magnitudes, ml those
+// of the local point).
+__device__ inline float sdf_ff_at(const ShapeK& s, const FF (&P)[3], float ml, float& err) {
     const float U44 = 5.6843418860808015e-14f;  // 2^-44
     const float* a = s.p32;
     if (s.type == SDFIBM_SHAPE_ELLIPSOID) {  // the reference's ellipsoid ignores com
@@ -852,7 +849,8 @@ __device__ inline float sdf_ff(const ShapeK& s, const SolidPlan& pl, float da, f
     float qm = 0.f;
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
-        q[r] = ff_add(P[r], FF{s.com32[r], s.com_lo[r]});
+        q[r] = P[r];
+        if (s.com32[r] != 0.f) q[r] = ff_add(P[r], FF{s.com32[r], s.com_lo[r]});  // (adding zero changes nothing)
         qm = fmaxf(qm, fabsf(q[r].hi));
     }
     const float mag = ml + fabsf(s.com32[0]) + fabsf(s.com32[1]) + fabsf(s.com32[2]) + qm;
@@ -873,6 +871,18 @@ __device__ inline float sdf_ff(const ShapeK& s, const SolidPlan& pl, float da, f
     err = 4.f * U44 * (mag + a[0] + a[1] + a[2]);
     const float dxp = fmaxf(0.f, d[0]), dyp = fmaxf(0.f, d[1]), dzp = fmaxf(0.f, d[2]);
     return sqrtf(dxp * dxp + dyp * dyp + dzp * dzp) + fminf(0.f, fmaxf(d[2], fmaxf(d[0], d[1])));
+}
+
+__device__ inline float sdf_ff(const ShapeK& s, const SolidPlan& pl, float da, float db, float dc, float& err) {
+    FF P[3];
+    float ml = 0.f;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        float mag;
+        P[r] = ff_local(pl, r, da, db, dc, mag);
+        ml = fmaxf(ml, mag);
+    }
+    return sdf_ff_at(s, P, ml, err);
 }
 
 __device__ inline float filter_mixed(const ShapeK& s, float phi, bool* exact_needed) {
@@ -1151,8 +1161,8 @@ __device__ __forceinline__ void classify_any(const ClassifyArgs& A, const int2 c
 // meshes circles, ellipses, rectangles and half spaces that turn about z.  One error bound covers every vertex of the solid's bounding box,
 // so a vertex costs a few multiply-adds and two comparisons; a tile's answers are ballots, and cells are read off them with
 // shifts.  Tiles are culled 32 at a time, a lane each.  Bound by instruction issue.  Measured against a test per vertex with
-// its own bound (GB300, 512^3, 16 384 solids): LEARNED 1.13 -> 0.43 ms, REF-GEO (half of it now the vertex distances)
-// 1.63 -> 0.92 ms.
+// its own bound (GB300, 512^3, 16 384 solids): LEARNED 1.13 -> 0.43 ms, REF-GEO 1.63 -> 0.44 (0.92 while it computed the
+// vertex distances too, which refgeo_cells_kernel does now).
 //
 // The bound.  A local coordinate is M (b + v h) + com from FP32 roundings of the base b (bbox corner minus centre), M, h and
 // com, added in a chain of at most 12 roundings of partial sums no larger than A = max|M| (|b|_1 + sum_a ext_a h_a) + |com|_1:
@@ -1242,22 +1252,13 @@ static __device__ __noinline__ bool fast_exact(const MeshK& m, const SolidK& k, 
     return in != 0;
 }
 
-// vertex distances of a tile for REF-GEO (see classify_any): u-th needed vertex v = (a, b, c) of the tile at (x0, y0, z0)
-static __device__ __forceinline__ float fast_phi(const MeshK& m, const SolidK& k, const SolidPlan& pl,
-                                                 const sdfibm_solid_state& st, bool prism, int da, int db, int dc) {
+// vertex distance for REF-GEO of a 2-D shape (see classify_any) at bbox vertex (da, db, dc)
+static __device__ __forceinline__ float flat_phi(const MeshK& m, const SolidK& k, const SolidPlan& pl, const sdfibm_solid_state& st,
+                                                 int da, int db, int dc) {
     const ShapeK& sh = k.shape;
-    bool exact = false;
-    float ph;
-    if (sh.type == SDFIBM_SHAPE_PLANE) {  // unfiltered, FP64
-        exact = true;
-        ph = 0.f;
-    } else if (!prism) {
-        float err;
-        ph = sdf_ff(sh, pl, (float)da, (float)db, (float)dc, err);
-        const float aph = fabsf(ph);
-        exact = fabsf(aph - 1e-8f) <= 1e-14f + err;  // the filter's decision is not certain
-        if (aph < 1e-8f) ph = -1e-8f;
-    } else {
+    bool exact = sh.type == SDFIBM_SHAPE_PLANE;  // unfiltered, FP64
+    float ph = 0.f;
+    if (!exact) {
         const double* L = pl.lmap;
         const double a = da, b = db, c = dc;
         const D3 plc{L[0] + a * L[3] + b * L[6] + c * L[9], L[1] + a * L[4] + b * L[7] + c * L[10],
@@ -1276,9 +1277,9 @@ __device__ __forceinline__ void classify_fast(const ClassifyArgs& A, const int2 
                                               unsigned& valid_cells) {
     constexpr int TX = FLAT ? 8 : 4, TY = TX, TZ = FLAT ? 2 : 4;
     constexpr int V = TX + 1, NPASS = FLAT ? 4 : 2, NL = FLAT ? 3 : 5;  // passes over the cells, ballots of vertices
-    constexpr int NVERT = FLAT ? V * V : V * V * V;
-    __shared__ float s_phi[CLS_WARPS][METHOD == SDFIBM_FRACTION_REFGEO ? NVERT : 1];
-    __shared__ uint8_t s_list[CLS_WARPS][METHOD == SDFIBM_FRACTION_REFGEO ? NVERT : 1];
+    constexpr int NVERT = METHOD == SDFIBM_FRACTION_REFGEO && FLAT ? V * V : 1;
+    __shared__ float s_phi[CLS_WARPS][NVERT];
+    __shared__ uint8_t s_list[CLS_WARPS][NVERT];
     const unsigned FULL = 0xffffffffu;
     const MeshK& m = A.m;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1454,48 +1455,33 @@ __device__ __forceinline__ void classify_fast(const ClassifyArgs& A, const int2 
                 if (box) out[cell_offset(x, y, z, p)] = cls[p];
             }
             if (METHOD < 0 || ncut == 0) continue;
-            if (METHOD == SDFIBM_FRACTION_REFGEO) {
-                // Solid::phi once per vertex next to a cut cell, the needed vertices compacted
+            if (METHOD == SDFIBM_FRACTION_REFGEO && FLAT) {
+                // Solid::phi once per vertex next to a cut cell, the needed vertices compacted: rows of cut cells (any
+                // layer, any pass), widened to their vertices.  (In 3-D refgeo_cells_kernel computes them.)
                 uint8_t* list = s_list[w];
                 int n = 0;
-                if (FLAT) {
-                    // rows of cut cells (any layer, any pass), widened to their vertices
-                    unsigned need_row = 0;  // lane r < 9: vertex row r
+                unsigned need_row = 0;  // lane r < 9: vertex row r
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const unsigned c2 = cut_b[h] | cut_b[h + 2];
+                for (int h = 0; h < 2; ++h) {
+                    const unsigned c2 = cut_b[h] | cut_b[(h + 2) % NPASS];
 #pragma unroll
-                        for (int r = 0; r < 4; ++r) {
-                            const unsigned row = (c2 >> (8 * r)) & 0xffu, wide = row | (row << 1);
-                            if (lane == 4 * h + r || lane == 4 * h + r + 1) need_row |= wide;
-                        }
+                    for (int r = 0; r < 4; ++r) {
+                        const unsigned row = (c2 >> (8 * r)) & 0xffu, wide = row | (row << 1);
+                        if (lane == 4 * h + r || lane == 4 * h + r + 1) need_row |= wide;
                     }
+                }
 #pragma unroll
-                    for (int l = 0; l < NL; ++l) {
-                        const unsigned row = __shfl_sync(FULL, need_row, min(vb + 3 * l, 8));
-                        const bool need = lane < 27 && ((row >> va) & 1u);
-                        const unsigned bal = __ballot_sync(FULL, need);
-                        if (need) list[n + __popc(bal & below)] = (uint8_t)(lane + 27 * l);
-                        n += __popc(bal);
-                    }
-                } else {
-                    unsigned prev = 0;
-#pragma unroll
-                    for (int l = 0; l < NL; ++l) {
-                        unsigned wide = l < 4 ? cutm[l < 4 ? l : 0] : 0u;
-                        wide |= wide << 1;
-                        wide |= wide << 5;
-                        const unsigned need = wide | prev;
-                        if ((need >> lane) & 1u) list[n + __popc(need & below)] = (uint8_t)(lane + 25 * l);
-                        n += __popc(need);
-                        prev = wide;
-                    }
+                for (int l = 0; l < NL; ++l) {
+                    const unsigned row = __shfl_sync(FULL, need_row, min(vb + 3 * l, 8));
+                    const bool need = lane < 27 && ((row >> va) & 1u);
+                    const unsigned bal = __ballot_sync(FULL, need);
+                    if (need) list[n + __popc(bal & below)] = (uint8_t)(lane + 27 * l);
+                    n += __popc(bal);
                 }
                 __syncwarp();
                 for (int u = lane; u < n; u += 32) {
                     const int v = list[u];
-                    const int a = v % V, b = FLAT ? v / V : (v / V) % V, c = FLAT ? 0 : v / (V * V);
-                    s_phi[w][v] = fast_phi(m, k, pl, st, FLAT, x * TX + a, y * TY + b, z * TZ + c);
+                    s_phi[w][v] = flat_phi(m, k, pl, st, x * TX + v % V, y * TY + v / V, z * TZ);
                 }
                 __syncwarp();
             }
@@ -1509,13 +1495,11 @@ __device__ __forceinline__ void classify_fast(const ClassifyArgs& A, const int2 
                     const int64_t at = (int64_t)base + __popc(cut_b[p] & below);
                     const int64_t slot = back ? A.feat_cap - 1 - at : at;
                     if (slot >= 0 && slot < A.feat_cap) {
-                        if (METHOD == SDFIBM_FRACTION_REFGEO) {
-                            const int b = FLAT ? cb + 4 * (p & 1) : cb, c = FLAT ? 0 : (lane >> 4) + 2 * p;
-                            const int v0 = ca + V * (b + V * c);
-                            constexpr int up = FLAT ? 0 : V * V;  // flat: the layers' distances are the same
-                            const int vo[8] = {0, 1, V, V + 1, up, up + 1, up + V, up + V + 1};
+                        if (METHOD == SDFIBM_FRACTION_REFGEO && FLAT) {  // the layers' distances are the same
+                            const int v0 = ca + V * (cb + 4 * (p & 1));
+                            const int vo[4] = {0, 1, V, V + 1};
 #pragma unroll
-                            for (int q = 0; q < 8; ++q) A.rg_phi[q * A.feat_cap + slot] = s_phi[w][v0 + vo[q]];
+                            for (int q = 0; q < 8; ++q) A.rg_phi[q * A.feat_cap + slot] = s_phi[w][v0 + vo[q & 3]];
                         }
                         A.fref_solid[slot] = s;
                         A.fref_index[slot] = k.scratch_off + cell_offset(x, y, z, p);
@@ -1858,14 +1842,21 @@ __global__ void __launch_bounds__(256) recount_kernel(FallbackArgs A) {
 
 // REF-GEO fraction of the listed cut cells, one thread per cell (GeometricTools::calcCellVolume on the cell's vertex
 // distances, see refgeo32): the tile pass lists the cells, so every lane here has a cell.  Cells at the mesh boundary, whose
-// face lists differ, take refgeo32; the others refgeo_inner.  Bound by issue: 0.54 -> 0.23 ms at 512^3 and
-// 16 384 solids, 0.12 -> 0.065 at 256^3 and 4096, 18 -> 8 us for one cylinder, where the chain of one cell counts (GB300).
-__global__ void __launch_bounds__(256) refgeo_cells_kernel(MeshK m, const SolidK* __restrict__ sk,
+// face lists differ, take refgeo32; the others refgeo_inner.  In 3-D (!FLAT) the distances of the shapes of
+// classify_fast are computed here, eight a cell, rather than once a vertex in the classify pass: that pass then fits its
+// instruction cache and this one runs beside the connected sets.  Bound by issue.  Measured (GB300), with the classify pass:
+// 512^3 and 16 384 solids 0.92 + 0.54 ms with table-driven fractions, 0.92 + 0.23 unrolled, 0.44 + 0.68 with the distances here
+// (the interact 2.06 -> 2.00); 256^3 and 4096 0.23 + 0.12, 0.23 + 0.065, 0.12 + 0.16 (0.64 -> 0.62); one cylinder 18 -> 8 us,
+// where the chain of one cell counts.
+template <bool FLAT>
+__global__ void __launch_bounds__(256, FLAT ? 4 : 3) refgeo_cells_kernel(MeshK m, const SolidK* __restrict__ sk,
+                                                           const sdfibm_solid_state* __restrict__ st,
                                                            const SolidPlan* __restrict__ plan,
                                                            const int32_t* __restrict__ fref_solid,
                                                            const int64_t* __restrict__ fref_index,
                                                            const float* __restrict__ rg_phi, int64_t cap,
                                                            const Counters* cnt, float* __restrict__ alpha) {
+    __shared__ float s_ph[FLAT ? 1 : 8][256];
     const int64_t n = min((int64_t)cnt->n_feat, cap);
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
         const int s = fref_solid[e];
@@ -1876,8 +1867,45 @@ __global__ void __launch_bounds__(256) refgeo_cells_kernel(MeshK m, const SolidK
         const int row = (int)fdiv(local, k.div_e0), lc = (int)fdiv(local, k.div_e01);
         const int la = (int)local - row * k.ext[0], lb = row - lc * k.ext[1];
         float ph[8];
+        const int type = k.shape.type;
+        if (!FLAT && (type == SDFIBM_SHAPE_SPHERE || type == SDFIBM_SHAPE_ELLIPSOID || type == SDFIBM_SHAPE_BOX)) {
+            // the shapes of classify_fast: the local points of the corners by three sums of pairs each
+            FF P[3];
+            float ml = 0.f;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) ph[q] = rg_phi[q * cap + e];
+            for (int r = 0; r < 3; ++r) {
+                float mag;
+                P[r] = ff_local(pl, r, (float)la, (float)lb, (float)lc, mag);
+                ml = fmaxf(ml, mag + fabsf(pl.lmap_hi[3 + r]) + fabsf(pl.lmap_hi[6 + r]) + fabsf(pl.lmap_hi[9 + r]));
+            }
+            auto step = [&](const FF (&from)[3], FF (&to)[3], int axis) {
+#pragma unroll
+                for (int r = 0; r < 3; ++r)
+                    to[r] = ff_add(from[r], FF{pl.lmap_hi[3 + 3 * axis + r], pl.lmap_lo[3 + 3 * axis + r]});
+            };
+#pragma unroll 1
+            for (int q = 0; q < 8; q += 2) {  // rows along x: (y, z) = (0, 0), (1, 0), (0, 1), (1, 1)
+                FF A0[3] = {P[0], P[1], P[2]}, B[3];
+                if (q & 2) step(A0, A0, 1);
+                if (q & 4) step(A0, A0, 2);
+                step(A0, B, 0);
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    float err, p = sdf_ff_at(k.shape, u ? B : A0, ml, err);
+                    const float ap = fabsf(p);
+                    if (ap < 1e-8f) p = -1e-8f;
+                    if (fabsf(ap - 1e-8f) <= 1e-14f + err)  // the filter's decision is not certain
+                        p = exact_phi_point(k.shape, m, (int64_t)pl.lo[0] + la + u, (int64_t)pl.lo[1] + lb + ((q >> 1) & 1),
+                                            (int64_t)pl.lo[2] + lc + (q >> 2), state_pos(st[s]), state_quat(st[s]));
+                    s_ph[FLAT ? 0 : q + u][threadIdx.x] = p;
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) ph[q] = s_ph[FLAT ? 0 : q][threadIdx.x];
+        } else {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) ph[q] = rg_phi[q * cap + e];
+        }
         const int I = pl.lo[0] + la, J = pl.lo[1] + lb, K = pl.lo[2] + lc;
         float apz = 0.f, apz1 = 0.f;
         if (m.twod) {
@@ -1896,6 +1924,14 @@ __global__ void __launch_bounds__(256) refgeo_cells_kernel(MeshK m, const SolidK
         }
         alpha[idx] = a;
     }
+}
+
+void launch_refgeo_cells(const MeshK& m, const SolidK* sk, const sdfibm_solid_state* st, const SolidPlan* plan,
+                         const int32_t* fref_solid, const int64_t* fref_index, const float* rg_phi, int64_t cap, const Counters* cnt,
+                         float* alpha, int grid, cudaStream_t stream) {
+    if (m.nz <= 2)
+        refgeo_cells_kernel<true><<<grid, 256, 0, stream>>>(m, sk, st, plan, fref_solid, fref_index, rg_phi, cap, cnt, alpha);
+    else refgeo_cells_kernel<false><<<grid, 256, 0, stream>>>(m, sk, st, plan, fref_solid, fref_index, rg_phi, cap, cnt, alpha);
 }
 
 // The deferred SUBSAMPLE points: one per thread, the reference's FP64 point and inside test, an inside point lowers the
@@ -1923,7 +1959,7 @@ __global__ void __launch_bounds__(256) recheck_kernel(MeshK m, const SolidK* __r
 // only), so each kernel carries only its own path, and one per set of shapes.  CTAs per SM: as many as their registers allow
 // without spilling much.
 template <bool FLAT, int METHOD>
-__global__ void __launch_bounds__(CLS_WARPS * 32, METHOD == SDFIBM_FRACTION_REFGEO ? 3 : 4) classify_kernel(ClassifyArgs A) {
+__global__ void __launch_bounds__(CLS_WARPS * 32, METHOD == SDFIBM_FRACTION_REFGEO && FLAT ? 3 : 4) classify_kernel(ClassifyArgs A) {
     classify_body<FLAT, METHOD, true>(A);
 }
 template <bool FLAT, int METHOD>
