@@ -799,31 +799,20 @@ static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float
     if (S > 0) {
         ClassifyArgs CA{};
         CA.m = ctx->mesh; CA.sk = ctx->d_sk; CA.st = ctx->d_st; CA.plan = ctx->d_plan; CA.chunks = ctx->d_chunks;
-        CA.total_chunks = ctx->total_chunks; CA.cls = ctx->d_scratch; CA.alpha = ctx->d_alpha; CA.cnt = ctx->d_cnt;
+        CA.total_chunks = ctx->total_chunks; CA.cls = ctx->d_scratch; CA.cnt = ctx->d_cnt;
         CA.chunk_tiles = ctx->chunk_tiles;
         CA.fast_chunks = ctx->fast_chunks;
         CA.any_first = ctx->mesh.nz <= 2 ? 0 : ctx->fast_chunks;
         CA.any_grid = std::min(2 * ctx->num_sms, (ctx->total_chunks - CA.any_first + 7) / 8);
-        CA.method = ctx->opt.fraction_method; CA.subsample_n = ctx->opt.subsample_n;
+        CA.method = ctx->opt.fraction_method;
         const bool learned = ctx->opt.fraction_method == SDFIBM_FRACTION_LEARNED;
         const bool subsample = ctx->opt.fraction_method == SDFIBM_FRACTION_SUBSAMPLE;
         const bool refgeo = ctx->opt.fraction_method == SDFIBM_FRACTION_REFGEO;
-        if (refgeo) {
-            // cut cells and their vertex distances listed by the classify pass, fractions by refgeo_cells_kernel
-            CA.feat_cap = ctx->feat_cap; CA.fref_solid = ctx->d_fref_solid; CA.fref_index = ctx->d_fref_index;
-            CA.rg_phi = ctx->d_rg_phi;
-        }
-        if (subsample) {
-            // cut cells listed by the classify pass, sampled by subsample_cells_kernel
-            CA.rq = ctx->d_rq; CA.rq_cap = ctx->rq_cap;
-            CA.feat_cap = ctx->feat_cap; CA.fref_solid = ctx->d_fref_solid; CA.fref_index = ctx->d_fref_index;
-        }
-        if (learned) {
-            // cut cells listed by the classify pass; learned_stencil_kernel computes the model's inputs (the cells of
-            // solids under rho_min cells, listed from the back, go to the fallback whole)
-            CA.feat_cap = ctx->feat_cap; CA.fref_solid = ctx->d_fref_solid; CA.fref_index = ctx->d_fref_index;
-            CA.rho_min = ctx->rho_min;
-        }
+        // the cut cells, listed by the classify pass for the fraction kernels (LEARNED: those of solids under rho_min cells
+        // from the back, they go to the fallback whole; REF-GEO: with their vertex distances for all but the 3-D shapes)
+        CA.feat_cap = ctx->feat_cap; CA.fref_solid = ctx->d_fref_solid; CA.fref_index = ctx->d_fref_index;
+        CA.rg_phi = ctx->d_rg_phi;
+        CA.rho_min = ctx->rho_min;
         launch_classify(CA, ctx->mesh.nz <= 2, std::min(ctx->classify_grid, (ctx->fast_chunks + 7) / 8), st);
         mark(ctx, "classify_kernel");
         // the component pass needs only the class bytes and the seeds: on the side stream, beside the fraction

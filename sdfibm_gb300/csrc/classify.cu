@@ -7,17 +7,18 @@
 //      (CellEnumerator::_next, src/cellenumerator.cpp:6-34): 0 no inside vertex, 1 all inside, 2 centre inside,
 //      3 centre outside;
 //   3. lists every cut candidate (class 2/3) for the fraction kernels:
-//      REF-GEO   with the signed distances of its 8 vertices (two-float for 3-D spheres, ellipsoids and boxes, FP64
-//                numerators elsewhere, see sdf_ff / sdf_mixed); refgeo_cells_kernel then runs
-//                GeometricTools::calcCellVolume (src/geometrictools.cpp:13-116) in FP32 in cell-local coordinates
-//                (vertices on {0,1}^3, every term a product of non-negative factors), a thread per cell;
+//      REF-GEO   as (solid, fraction index), with the signed distances of its 8 vertices in FP64 numerators (sdf_mixed) for
+//                all shapes but 3-D spheres, ellipsoids and boxes; refgeo_cells_kernel computes those (two-float, sdf_ff_at)
+//                and runs GeometricTools::calcCellVolume (src/geometrictools.cpp:13-116) in FP32 in cell-local
+//                coordinates (vertices on {0,1}^3, every term a product of non-negative factors), a thread per cell;
 //      SUBSAMPLE as (solid, fraction index); subsample_cells_kernel counts the n^3 (2-D: n^2) midpoint lattice of
-//                each listed cell, a warp per cell, with the same exact inside test as the vertices (run counting
-//                along lattice columns for the convex shapes), undecided points rechecked in FP64 by recheck_kernel;
+//                each listed cell, a lane per cell (a warp for few cells), with the same exact inside test as the vertices
+//                (run counting along lattice columns for the convex shapes), undecided points rechecked in FP64 by
+//                recheck_kernel;
 //      LEARNED   as (solid, fraction index); learned_stencil_kernel (stencil.cu) computes the network's inputs and
 //                band, the cells outside the band go to subsample_cells_kernel.
-// The allocation-free entry point computes the fractions inside the tile pass instead.  Candidates that the flood
-// fill later leaves out simply have their alpha ignored.
+// The allocation-free entry point wants the classes only.  Candidates that the flood fill later leaves out simply have their
+// alpha ignored.
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -716,11 +717,6 @@ static __device__ __noinline__ int subsample_warp(const MeshK& m, const ShapeK& 
     return subsample_warp_body<false>(m, sh, M, tf, a0, b0, c0, x, q, i, j, k, n, rechecks, df);
 }
 
-// the fraction of a complete count (cnt and n^3 are exact in FP32: one correct rounding)
-__device__ inline float count_fraction(const MeshK& m, int cnt, int n) {
-    return __fdiv_rn((float)cnt, (float)(n * n * (m.twod ? 1 : n)));
-}
-
 // ---- signed distance for REF-GEO: FP64 where it decides, FP32 where it only scales ------------------------------------
 // The geometry consumes phi in FP32, so phi needs ~1e-7 relative accuracy and the reference's exact sign and filter
 // (|phi| < 1e-8 -> -1e-8).  The local point and every cancelling difference (|p|^2 - r^2, |x| - a, ...) are FP64; the
@@ -984,7 +980,6 @@ __device__ __forceinline__ void classify_any(const ClassifyArgs& A, const int2 c
         const int32_t vlo0 = pl.vlo[0], vlo1 = pl.vlo[1], vlo2 = pl.vlo[2];
         const int32_t vhi0 = pl.vhi[0], vhi1 = pl.vhi[1], vhi2 = pl.vhi[2];
         uint8_t* out = A.cls + k.scratch_off;
-        float* alpha = A.alpha + k.scratch_off;
         const float sb[3] = {pl.base32[0], pl.base32[1], pl.base32[2]};
         for (int t = ch.y; t < t_end; ++t) {
             const int tx = t % k.ntile[0], ty = (t / k.ntile[0]) % k.ntile[1], tz = t / (k.ntile[0] * k.ntile[1]);
@@ -1134,23 +1129,11 @@ __device__ __forceinline__ void classify_any(const ClassifyArgs& A, const int2 c
                 // the cut cells and their vertex distances are listed; refgeo_cells_kernel computes the fractions
                 write_refgeo_list<TX, TY, TZ>(A, cutlist, ncut, vphi, s, k.scratch_off + local_index(0, 0, 0), k.ext[0],
                                               k.ext[1]);
-            } else if (A.fref_index) {
+            } else if (METHOD >= 0) {
                 // SUBSAMPLE and LEARNED: the cut cells are listed; subsample_cells_kernel samples them (LEARNED:
                 // learned_stencil_kernel computes the model's inputs, a thread per cell), a warp per cell
                 write_cut_list<TX, TY, TZ>(A, cutlist, ncut, s, k.scratch_off + local_index(0, 0, 0), k.ext[0],
                                            k.ext[1]);
-            } else if (METHOD == SDFIBM_FRACTION_SUBSAMPLE) {
-                // SUBSAMPLE without a cell list (allocation-free entry): the warp shares the samples of one cut cell
-                // (LEARNED always lists its cut cells, so its classify pass carries no sampling code)
-                for (int u = 0; u < ncut; ++u) {
-                    const int e = cutlist[u];
-                    const int a = e % TX, b = (e / TX) % TY, c = e / (TX * TY);
-                    const int64_t li = local_index(a, b, c);
-                    const Defer df{A.rq, A.rq_cap, &A.cnt->n_recheck, k.scratch_off + li, s, nullptr};
-                    const int cnt = subsample_warp(m, sh, M, tf, a, b, c, x, q, I0 + a, J0 + b, K0 + c,
-                                                   A.subsample_n, &rechecks, A.rq ? &df : nullptr);
-                    if (lane == 0) alpha[li] = A.rq ? -1.f - (float)cnt : count_fraction(m, cnt, A.subsample_n);
-                }
             }
             __syncwarp();
         }

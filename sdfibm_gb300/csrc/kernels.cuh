@@ -129,8 +129,8 @@ struct Recheck {
     uint32_t sample;
 };
 
-// Time-step parameters the kernels read from device memory; plan_kernel and set_step_kernel write them at the head of a call, so a
-// captured graph replays with new values after one kernel-node update.
+// Time-step parameters the kernels read from device memory; plan_kernel and set_step_kernel write them at the head of a
+// call, so a captured graph replays with new values after one kernel-node update.
 struct StepParams {
     double time;
     double dt;
@@ -231,17 +231,13 @@ struct ClassifyArgs {
     int any_first;       // first chunk classify_any_kernel looks at
     int any_grid;        // its CTAs
     uint8_t* cls;      // class byte per bbox cell
-    float* alpha;      // solid fraction per bbox cell (cut candidates only)
     Counters* cnt;
     int method;        // sdfibm_fraction_method, or -1: classification only
-    int subsample_n;
-    // SUBSAMPLE, LEARNED, REF-GEO: the list of cut cells (solid, index into alpha), feat_cap entries
+    // SUBSAMPLE, LEARNED, REF-GEO: the list of cut cells (solid, index into the fraction scratch), feat_cap entries
     int64_t feat_cap;
     int32_t* fref_solid;
-    int64_t* fref_index;  // index into alpha
-    Recheck* rq;          // deferred SUBSAMPLE rechecks (nullptr: re-evaluate in place)
-    int64_t rq_cap;
-    float* rg_phi;        // REF-GEO: [8][feat_cap] vertex distances of the listed cut cells
+    int64_t* fref_index;
+    float* rg_phi;        // REF-GEO: [8][feat_cap] vertex distances of the listed cut cells (not of the 3-D shapes of classify_fast)
     // LEARNED: solids whose bounding radius spans fewer cells (SolidPlan::radius_cells) list their cut cells from the
     // back of the list (positions feat_cap - 1 - i, n_small of them): the band sends them to the fallback whole
     float rho_min;
