@@ -824,10 +824,10 @@ __device__ __forceinline__ FF ff_local(const SolidPlan& pl, int r, float da, flo
     }
     return v;
 }
-// Solid::phi at local point P as sdf_mixed computes it (the same FP32 formula after the cancelling differences); err bounds
-// the difference to the exact value with a factor of 4 to spare over the operations' roundoff (2^-44 of the magnitudes, ml those
-// of the local point).
-__device__ inline float sdf_ff_at(const ShapeK& s, const FF (&P)[3], float ml, float& err) {
+// Solid::phi at local point P as sdf_mixed computes it (the same FP32 formula after the cancelling differences); err / den
+// bounds the difference to the exact value with a factor of 4 to spare over the operations' roundoff (2^-44 of the magnitudes,
+// ml those of the local point).
+__device__ inline float sdf_ff_at(const ShapeK& s, const FF (&P)[3], float ml, float& err, float& den) {
     const float U44 = 5.6843418860808015e-14f;  // 2^-44
     const float* a = s.p32;
     if (s.type == SDFIBM_SHAPE_ELLIPSOID) {  // the reference's ellipsoid ignores com
@@ -835,10 +835,10 @@ __device__ inline float sdf_ff_at(const ShapeK& s, const FF (&P)[3], float ml, f
         const FF yb = ff_mul(ff_mul(P[1], P[1]), FF{a[4], s.p_lo[4]});
         const FF zc = ff_mul(ff_mul(P[2], P[2]), FF{a[5], s.p_lo[5]});
         const FF sum = ff_add(ff_add(ff_add(xa, yb), zc), FF{-1.f, 0.f});
-        const float den = sqrtf(xa.hi * a[3] + yb.hi * a[4] + zc.hi * a[5]);
+        den = sqrtf(xa.hi * a[3] + yb.hi * a[4] + zc.hi * a[5]);
         const float am = fmaxf(a[3], fmaxf(a[4], a[5]));
         const float pm = fmaxf(fabsf(P[0].hi), fmaxf(fabsf(P[1].hi), fabsf(P[2].hi)));
-        err = 4.f * U44 * (xa.hi + yb.hi + zc.hi + 1.f + 6.f * am * pm * (ml + pm)) / den;
+        err = 4.f * U44 * (xa.hi + yb.hi + zc.hi + 1.f + 6.f * am * pm * (ml + pm));
         return (0.5f * __fadd_rn(sum.hi, sum.lo)) / den;
     }
     FF q[3];
@@ -853,8 +853,8 @@ __device__ inline float sdf_ff_at(const ShapeK& s, const FF (&P)[3], float ml, f
     if (s.type == SDFIBM_SHAPE_SPHERE) {
         const FF qq = ff_add(ff_add(ff_mul(q[0], q[0]), ff_mul(q[1], q[1])), ff_mul(q[2], q[2]));
         const FF num = ff_add(qq, FF{-a[1], -s.p_lo[1]});
-        const float den = sqrtf(qq.hi) + a[0];
-        err = 4.f * U44 * (qq.hi + a[1] + 6.f * qm * mag) / den;
+        den = sqrtf(qq.hi) + a[0];
+        err = 4.f * U44 * (qq.hi + a[1] + 6.f * qm * mag);
         return __fadd_rn(num.hi, num.lo) / den;
     }
     // box
@@ -865,11 +865,19 @@ __device__ inline float sdf_ff_at(const ShapeK& s, const FF (&P)[3], float ml, f
         d[r] = __fadd_rn(t.hi, t.lo);
     }
     err = 4.f * U44 * (mag + a[0] + a[1] + a[2]);
+    den = 1.f;
     const float dxp = fmaxf(0.f, d[0]), dyp = fmaxf(0.f, d[1]), dzp = fmaxf(0.f, d[2]);
     return sqrtf(dxp * dxp + dyp * dyp + dzp * dzp) + fminf(0.f, fmaxf(d[2], fmaxf(d[0], d[1])));
 }
 
-__device__ inline float sdf_ff(const ShapeK& s, const SolidPlan& pl, float da, float db, float dc, float& err) {
+// the filter of sdf.h:147-150 on such a value; false: its decision is not certain
+__device__ __forceinline__ bool ff_filter(float& phi, float err, float den) {
+    const float a = fabsf(phi);
+    if (a < 1e-8f) phi = -1e-8f;
+    return !((fabsf(a - 1e-8f) - 1e-14f) * den <= err);
+}
+__device__ inline float sdf_ff(const ShapeK& s, const SolidPlan& pl, float da, float db, float dc, float& err,
+                               float& den) {
     FF P[3];
     float ml = 0.f;
 #pragma unroll
@@ -878,7 +886,7 @@ __device__ inline float sdf_ff(const ShapeK& s, const SolidPlan& pl, float da, f
         P[r] = ff_local(pl, r, da, db, dc, mag);
         ml = fmaxf(ml, mag);
     }
-    return sdf_ff_at(s, P, ml, err);
+    return sdf_ff_at(s, P, ml, err, den);
 }
 
 __device__ inline float filter_mixed(const ShapeK& s, float phi, bool* exact_needed) {
@@ -1109,11 +1117,9 @@ __device__ __forceinline__ void classify_any(const ClassifyArgs& A, const int2 c
                     bool exact = false;
                     float ph;
                     if (ff_shape) {
-                        float err;
-                        ph = sdf_ff(sh, pl, (float)(tx * TX + a), (float)(ty * TY + b), (float)(tz * TZ + c), err);
-                        const float aph = fabsf(ph);
-                        exact = fabsf(aph - 1e-8f) <= 1e-14f + err;  // the filter's decision is not certain
-                        if (aph < 1e-8f) ph = -1e-8f;
+                        float err, den;
+                        ph = sdf_ff(sh, pl, (float)(tx * TX + a), (float)(ty * TY + b), (float)(tz * TZ + c), err, den);
+                        exact = !ff_filter(ph, err, den);
                     } else {
                         const double da = (double)(tx * TX + a), db = (double)(ty * TY + b),
                                      dc = (double)(tz * TZ + c);
@@ -1828,8 +1834,8 @@ __global__ void __launch_bounds__(256) recount_kernel(FallbackArgs A) {
 // face lists differ, take refgeo32; the others refgeo_inner.  In 3-D (!FLAT) the distances of the shapes of
 // classify_fast are computed here, eight a cell, rather than once a vertex in the classify pass: that pass then fits its
 // instruction cache and this one runs beside the connected sets.  Bound by issue.  Measured (GB300), with the classify pass:
-// 512^3 and 16 384 solids 0.92 + 0.54 ms with table-driven fractions, 0.92 + 0.23 unrolled, 0.44 + 0.68 with the distances here
-// (the interact 2.06 -> 2.00); 256^3 and 4096 0.23 + 0.12, 0.23 + 0.065, 0.12 + 0.16 (0.64 -> 0.62); one cylinder 18 -> 8 us,
+// 512^3 and 16 384 solids 0.92 + 0.54 ms with table-driven fractions, 0.92 + 0.23 unrolled, 0.44 + 0.77 with the distances here
+// (the interact 2.09 -> 2.05); 256^3 and 4096 0.23 + 0.12, 0.23 + 0.065, 0.12 + 0.18 (0.65 -> 0.63); one cylinder 18 -> 8 us,
 // where the chain of one cell counts.
 template <bool FLAT>
 __global__ void __launch_bounds__(256, FLAT ? 4 : 3) refgeo_cells_kernel(MeshK m, const SolidK* __restrict__ sk,
@@ -1852,35 +1858,44 @@ __global__ void __launch_bounds__(256, FLAT ? 4 : 3) refgeo_cells_kernel(MeshK m
         float ph[8];
         const int type = k.shape.type;
         if (!FLAT && (type == SDFIBM_SHAPE_SPHERE || type == SDFIBM_SHAPE_ELLIPSOID || type == SDFIBM_SHAPE_BOX)) {
-            // the shapes of classify_fast: the local points of the corners by three sums of pairs each
+            // the shapes of classify_fast: the corners' local points as ff_local computes them, its sums shared (x, then y,
+            // then z)
+            auto step = [&](const FF (&from)[3], const float (&mf)[3], FF (&to)[3], float (&mt)[3], int axis, float n) {
+#pragma unroll
+                for (int r = 0; r < 3; ++r) {
+                    const int i = 3 + 3 * axis + r;
+                    to[r] = ff_add(from[r], ff_scale(FF{pl.lmap_hi[i], pl.lmap_lo[i]}, n));
+                    mt[r] = mf[r] + fabsf(n * pl.lmap_hi[i]);
+                }
+            };
             FF P[3];
-            float ml = 0.f;
+            float mp[3];
 #pragma unroll
             for (int r = 0; r < 3; ++r) {
-                float mag;
-                P[r] = ff_local(pl, r, (float)la, (float)lb, (float)lc, mag);
-                ml = fmaxf(ml, mag + fabsf(pl.lmap_hi[3 + r]) + fabsf(pl.lmap_hi[6 + r]) + fabsf(pl.lmap_hi[9 + r]));
+                P[r] = FF{pl.lmap_hi[r], pl.lmap_lo[r]};
+                mp[r] = fabsf(pl.lmap_hi[r]);
             }
-            auto step = [&](const FF (&from)[3], FF (&to)[3], int axis) {
-#pragma unroll
-                for (int r = 0; r < 3; ++r)
-                    to[r] = ff_add(from[r], FF{pl.lmap_hi[3 + 3 * axis + r], pl.lmap_lo[3 + 3 * axis + r]});
-            };
 #pragma unroll 1
-            for (int q = 0; q < 8; q += 2) {  // rows along x: (y, z) = (0, 0), (1, 0), (0, 1), (1, 1)
-                FF A0[3] = {P[0], P[1], P[2]}, B[3];
-                if (q & 2) step(A0, A0, 1);
-                if (q & 4) step(A0, A0, 2);
-                step(A0, B, 0);
+            for (int a = 0; a < 2; ++a) {
+                FF X[3];
+                float mx[3];
+                step(P, mp, X, mx, 0, (float)(la + a));
+#pragma unroll 1
+                for (int b = 0; b < 2; ++b) {
+                    FF Y[3];
+                    float my[3];
+                    step(X, mx, Y, my, 1, (float)(lb + b));
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    float err, p = sdf_ff_at(k.shape, u ? B : A0, ml, err);
-                    const float ap = fabsf(p);
-                    if (ap < 1e-8f) p = -1e-8f;
-                    if (fabsf(ap - 1e-8f) <= 1e-14f + err)  // the filter's decision is not certain
-                        p = exact_phi_point(k.shape, m, (int64_t)pl.lo[0] + la + u, (int64_t)pl.lo[1] + lb + ((q >> 1) & 1),
-                                            (int64_t)pl.lo[2] + lc + (q >> 2), state_pos(st[s]), state_quat(st[s]));
-                    s_ph[FLAT ? 0 : q + u][threadIdx.x] = p;
+                    for (int c = 0; c < 2; ++c) {
+                        FF Z[3];
+                        float mz[3], err, den;
+                        step(Y, my, Z, mz, 2, (float)(lc + c));
+                        float p = sdf_ff_at(k.shape, Z, fmaxf(fmaxf(mz[0], mz[1]), mz[2]), err, den);
+                        if (!ff_filter(p, err, den))
+                            p = exact_phi_point(k.shape, m, (int64_t)pl.lo[0] + la + a, (int64_t)pl.lo[1] + lb + b,
+                                                (int64_t)pl.lo[2] + lc + c, state_pos(st[s]), state_quat(st[s]));
+                        s_ph[FLAT ? 0 : a + 2 * b + 4 * c][threadIdx.x] = p;
+                    }
                 }
             }
 #pragma unroll
