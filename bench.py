@@ -37,7 +37,7 @@ ALG_BYTES = {
     "couple_chunks_kernel": ("coupling_cells", 32.0),  # U read 12, As/Ts/Fs written 20
     "claim_kernel": ("coupling_cells", 4.0),       # Ct written
     "finalize_kernel": ("coupling_cells", 8.0),    # Ct and As rewritten for the cells that need it
-    "reset_kernel": ("coupling_cells", 24.0),      # previous cells zeroed
+    "scan_reset_kernel": ("coupling_cells", 24.0),  # previous cells zeroed
     "classify_kernel": ("bbox_cells", 1.0),        # one class byte per bbox cell (+ the cut-cell outputs below)
     "connect_kernel": ("bbox_cells", 1.0),         # class bytes read once
     "mlp_infer_kernel": ("network_cells", 80.0),   # 16 inputs + prior + destination read, fraction written
@@ -47,19 +47,19 @@ ALG_BYTES = {
 # 256^3 / 2048-solid learned workload (the full-size workload's distribution at half scale per axis);
 # profiles/<kernel>_poly3d_256_learned.md and profiles/launches_poly3d_256_learned.md record the captures
 NCU_BYTES_PER_UNIT = {
-    "couple_chunks_kernel": 121.3,  # 161.6 MB for 1,332,670 coupling cells: whole 32-byte sectors of the marked chunks
-    "classify_kernel": 0.84,        # 3.6 MB for 4,282,843 bbox cells left after the box test
-    "subsample_cells_kernel": 52.5,  # 8.1 MB for 154,364 sampled cells
-    "learned_stencil_kernel": 11.8,  # 9.0 MB for 760,774 listed cut cells
+    "couple_chunks_kernel": 124.6,  # 166.1 MB for 1,332,670 coupling cells: whole 32-byte sectors of the marked chunks
+    "classify_kernel": 2.55,        # 10.9 MB for 4,282,843 bbox cells left after the box test
+    "subsample_cells_kernel": 42.1,  # 6.5 MB for 154,364 sampled cells
+    "learned_stencil_kernel": 12.4,  # 9.4 MB for 760,774 listed cut cells
 }
 # Warp instructions per unit (ncu smsp__inst_executed.sum of one launch / its units), per (kernel, method); the
 # stencil, sampling and classification kernels are bound by instruction issue, and these counts give their issue
 # roofline
 INST_PER_UNIT = {
-    ("learned_stencil_kernel", "learned"): ("learned_cells", 373.0),  # 283.8 M for 760,774 listed cut cells
-    ("subsample_cells_kernel", "learned"): ("sampled_cells", 1716.3),  # 264.9 M for 154,364 16^3 cells
-    ("classify_kernel", "learned"): ("bbox_cells", 31.08),            # 133.1 M for 4,282,843 bbox cells
-    ("classify_kernel", "refgeo"): ("bbox_cells", 37.82),             # 162.0 M for the same bbox cells
+    ("learned_stencil_kernel", "learned"): ("learned_cells", 374.6),  # 285.0 M for 760,774 listed cut cells
+    ("subsample_cells_kernel", "learned"): ("sampled_cells", 621.6),  # 95.9 M for 154,364 16^3 cells
+    ("classify_kernel", "learned"): ("bbox_cells", 10.71),            # 45.9 M for 4,282,843 bbox cells
+    ("classify_kernel", "refgeo"): ("bbox_cells", 10.54),             # 45.1 M for the same bbox cells
 }
 # FLOPs of the two tensor-core layers per predicted cell: hi and lo BF16 halves of a 16x64 and a 64x64 product
 MLP_FLOPS_PER_CELL = 2 * (2 * 16 * 64) + 2 * (2 * 64 * 64)
