@@ -466,7 +466,7 @@ def main():
     ap.add_argument("--no-e2e", action="store_true")
     ap.add_argument("--no-autotune", action="store_true", help="default launch configuration (no autotuner)")
     ap.add_argument("--exact-forcing", action="store_true",
-                    help="the reference's FP64 forcing sequence per cell (default: FP64 for the rigid-body "
+                    help="FP64 forcing per cell (default: FP64 for the rigid-body "
                          "velocity and U - us, FP32 after it, FP64 force/torque sums)")
     args = ap.parse_args()
     rank = int(os.environ.get("RANK", "0"))

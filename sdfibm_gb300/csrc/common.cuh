@@ -68,13 +68,4 @@ __device__ inline int classify_point(const ShapeK& sh, const float* M, const Til
     return r;
 }
 
-__device__ inline int find_solid(const int32_t* prefix, int S, int item) {
-    int lo = 0, hi = S;  // prefix[lo] <= item < prefix[hi]
-    while (hi - lo > 1) {
-        int mid = (lo + hi) >> 1;
-        if (prefix[mid] <= item) lo = mid; else hi = mid;
-    }
-    return lo;
-}
-
 }  // namespace sdfibm_dev
