@@ -802,8 +802,7 @@ static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float
         CA.total_chunks = ctx->total_chunks; CA.cls = ctx->d_scratch; CA.cnt = ctx->d_cnt;
         CA.chunk_tiles = ctx->chunk_tiles;
         CA.fast_chunks = ctx->fast_chunks;
-        CA.any_first = ctx->mesh.nz <= 2 ? 0 : ctx->fast_chunks;
-        CA.any_grid = std::min(2 * ctx->num_sms, (ctx->total_chunks - CA.any_first + 7) / 8);
+        CA.any_grid = std::min(2 * ctx->num_sms, (any_chunks(CA, ctx->mesh.nz <= 2) + 7) / 8);
         CA.method = ctx->opt.fraction_method;
         const bool learned = ctx->opt.fraction_method == SDFIBM_FRACTION_LEARNED;
         const bool subsample = ctx->opt.fraction_method == SDFIBM_FRACTION_SUBSAMPLE;

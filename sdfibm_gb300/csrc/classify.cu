@@ -1515,36 +1515,40 @@ __device__ __forceinline__ bool fast_shape(const SolidK& k, const sdfibm_solid_s
     return t == SDFIBM_SHAPE_SPHERE || t == SDFIBM_SHAPE_ELLIPSOID || t == SDFIBM_SHAPE_BOX;
 }
 
-// FAST: the chunks classify_fast takes; else the others
+// FAST: the chunks classify_fast takes; else the others.  Chunks are taken one at a time with an atomic; on flat meshes the
+// other kernel first looks at the chunks before fast_chunks, nearly all of which are the first kernel's: 32 together, which
+// lie a grid of warps apart, since those of a tilted solid are neighbours (32 neighbours a warp, all shapes: one tailed circle of
+// 81 items 165 us, now 22; 1500 of them 893, now 152; 300 3-D shapes on two layers 248, now 31; GB300).
 template <bool FLAT, int METHOD, bool FAST>
 __device__ __forceinline__ void classify_body(const ClassifyArgs& A) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     unsigned long long rechecks = 0, valid_cells = 0;
     unsigned rechecks32 = 0, valid32 = 0;
-    int32_t* next = FAST ? &A.cnt->classify_next : &A.cnt->classify_any_next;
-    const int n = FAST ? A.fast_chunks : A.total_chunks;
-    if (FLAT && !FAST) {
-        // nearly every chunk is the other kernel's: 32 looked at together
-        const int nw = gridDim.x * CLS_WARPS;
-        for (int c0 = (blockIdx.x * CLS_WARPS + (threadIdx.x >> 5)) * 32; c0 < n; c0 += nw * 32) {
-            const int2 ch = c0 + lane < n ? A.chunks[c0 + lane] : make_int2(-1, 0);
-            unsigned mine = __ballot_sync(FULL, ch.x >= 0 && !fast_shape<FLAT>(A.sk[max(ch.x, 0)], A.st[max(ch.x, 0)]));
-            while (mine) {
-                const int src = __ffs(mine) - 1;
-                mine &= mine - 1;
-                const int2 c = make_int2(__shfl_sync(FULL, ch.x, src), __shfl_sync(FULL, ch.y, src));
-                classify_any<FLAT ? 8 : 4, FLAT ? 8 : 4, FLAT ? 2 : 4, METHOD>(A, c, rechecks, valid_cells);
-            }
+    const int nw = gridDim.x * CLS_WARPS;
+    int64_t look = FLAT ? blockIdx.x * CLS_WARPS + (threadIdx.x >> 5) : A.fast_chunks;
+    int2 seen = make_int2(-1, 0);  // chunk look + lane * nw
+    unsigned mine = 0;             // of those, the ones to be done here
+    for (;;) {
+        int2 ch;
+        if (!FAST && mine) {
+            const int src = __ffs(mine) - 1;
+            mine &= mine - 1;
+            ch = make_int2(__shfl_sync(FULL, seen.x, src), __shfl_sync(FULL, seen.y, src));
+        } else if (!FAST && look < A.fast_chunks) {
+            const int64_t at = look + lane * (int64_t)nw;
+            look += 32 * (int64_t)nw;
+            seen = at < A.fast_chunks ? A.chunks[at] : make_int2(-1, 0);
+            mine = __ballot_sync(FULL, seen.x >= 0 && !fast_shape<FLAT>(A.sk[max(seen.x, 0)], A.st[max(seen.x, 0)]));
+            continue;
+        } else {
+            int chunk = 0;
+            if (lane == 0) chunk = FAST ? atomicAdd(&A.cnt->classify_next, 1) : atomicAdd(&A.cnt->classify_any_next, 1) + A.fast_chunks;
+            chunk = __shfl_sync(FULL, chunk, 0);
+            if (chunk >= (FAST ? A.fast_chunks : A.total_chunks)) break;
+            ch = A.chunks[chunk];
+            if (FAST && !fast_shape<FLAT>(A.sk[ch.x], A.st[ch.x])) continue;
         }
-    }
-    for (; FAST || !FLAT;) {
-        int chunk = 0;
-        if (lane == 0) chunk = atomicAdd(next, 1) + (FAST ? 0 : A.any_first);
-        chunk = __shfl_sync(FULL, chunk, 0);
-        if (chunk >= n) break;
-        const int2 ch = A.chunks[chunk];
-        if (fast_shape<FLAT>(A.sk[ch.x], A.st[ch.x]) != FAST) continue;
         if (FAST) classify_fast<FLAT, METHOD>(A, ch, rechecks32, valid32);
         else classify_any<FLAT ? 8 : 4, FLAT ? 8 : 4, FLAT ? 2 : 4, METHOD>(A, ch, rechecks, valid_cells);
     }
@@ -1961,15 +1965,14 @@ __global__ void __launch_bounds__(CLS_WARPS * 32, METHOD == SDFIBM_FRACTION_REFG
     classify_body<FLAT, METHOD, true>(A);
 }
 template <bool FLAT, int METHOD>
-__global__ void __launch_bounds__(CLS_WARPS * 32, FLAT ? 1 : 2) classify_any_kernel(ClassifyArgs A) {
+__global__ void __launch_bounds__(CLS_WARPS * 32, 2) classify_any_kernel(ClassifyArgs A) {
     classify_body<FLAT, METHOD, false>(A);
 }
 
 template <bool FLAT, int METHOD>
 static void launch_classify_as(const ClassifyArgs& A, int grid, cudaStream_t st) {
     if (A.fast_chunks > 0) classify_kernel<FLAT, METHOD><<<grid, CLS_WARPS * 32, 0, st>>>(A);
-    if (A.any_first < A.total_chunks)
-        classify_any_kernel<FLAT, METHOD><<<A.any_grid, CLS_WARPS * 32, 0, st>>>(A);
+    if (any_chunks(A, FLAT) > 0) classify_any_kernel<FLAT, METHOD><<<A.any_grid, CLS_WARPS * 32, 0, st>>>(A);
 }
 template <bool FLAT>
 static void launch_classify_flat(const ClassifyArgs& A, int grid, cudaStream_t st) {
@@ -1987,7 +1990,7 @@ void launch_classify(const ClassifyArgs& A, bool flat, int grid, cudaStream_t st
 }
 
 // Shapes whose chunks classify_kernel may take (0) and those it never takes (1): the chunk table holds them in this order.
-// On flat meshes the first kind is decided per call by the orientation, and both kernels look at those chunks.
+// On flat meshes the first kind is decided per call by the orientation, and both kernels look at those chunks (any_chunks).
 int classify_kind(int shape_type, bool flat) {
     if (flat)
         return shape_type == SDFIBM_SHAPE_CIRCLE || shape_type == SDFIBM_SHAPE_ELLIPSE ||

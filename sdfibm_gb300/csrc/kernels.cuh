@@ -228,8 +228,7 @@ struct ClassifyArgs {
     int total_chunks;
     int chunk_tiles;     // tiles per work item
     int fast_chunks;     // leading chunks whose shapes classify_kernel may take
-    int any_first;       // first chunk classify_any_kernel looks at
-    int any_grid;        // its CTAs
+    int any_grid;        // CTAs of classify_any_kernel
     uint8_t* cls;      // class byte per bbox cell
     Counters* cnt;
     int method;        // sdfibm_fraction_method, or -1: classification only
@@ -242,6 +241,8 @@ struct ClassifyArgs {
     // back of the list (positions feat_cap - 1 - i, n_small of them): the band sends them to the fallback whole
     float rho_min;
 };
+// chunks classify_any_kernel looks at: on flat meshes all of them
+inline int any_chunks(const ClassifyArgs& A, bool flat) { return flat ? A.total_chunks : A.total_chunks - A.fast_chunks; }
 
 // SUBSAMPLE of listed cells: every listed cut cell (fb_list == nullptr), or the LEARNED cells left to SUBSAMPLE by
 // the network's confidence band

@@ -301,7 +301,6 @@ extern "C" int sdfibm_cuda_touched_noalloc(const sdfibm_mesh_desc* mesh, const s
     CA.cls = b + OFF_CLS; CA.cnt = d_cnt; CA.method = -1;
     const int kind = classify_kind(solid->shape.type, m.nz <= 2);
     CA.fast_chunks = kind == 0 ? nchunks : 0;
-    CA.any_first = kind == 0 && m.nz > 2 ? nchunks : 0;
     CA.any_grid = grid;
     launch_classify(CA, m.nz <= 2, grid, st);
     ConnectArgs ca{};

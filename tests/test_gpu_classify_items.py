@@ -1,0 +1,72 @@
+"""Work items of the classify pass: on one- and two-layer meshes the solids its first kernel does not take (tailed circles, tilted
+prisms, 3-D shapes) against the oracle, few and many of them, and beside solids that kernel takes; and their tiles go to as many
+warps as there are."""
+import numpy as np
+import pytest
+
+from gpu_helpers import check_interact, run_pair
+from sdfibm_gb300 import abi
+from sdfibm_gb300.cloud import SolidCloud
+from sdfibm_gb300.host import make_shape, make_solid
+from sdfibm_gb300.workloads import Workload
+
+pytestmark = pytest.mark.gpu
+
+
+def _flat(side, kinds, count, nz=1):
+    h = 1.0 / side
+    rng = np.random.default_rng(side + count)
+    per = int(np.ceil(count ** 0.5))
+    solids = []
+    for i in range(count):
+        kind, e = kinds[i % len(kinds)], (0.0, 0.0, float(rng.uniform(0, 360)))
+        at = ((i % per + 0.5) / per, (i // per + 0.5) / per, 0.0)
+        if kind in ("Circle_Tail", "Circle_TwoTail"):
+            s = make_shape(kind, radius=6.3 * h, ratio=1.0, thickness=2.1 * h)
+        elif kind == "tilted":
+            s, e = make_shape("Circle", radius=5.2 * h), (20.0, 15.0, 0.0)
+        elif kind == "Circle":
+            s = make_shape("Circle", radius=5.2 * h)
+        elif kind == "Sphere":
+            s = make_shape("Sphere", radius=4.7 * h)
+        else:
+            s, e = make_shape("Box", radiusa=4 * h, radiusb=3 * h, radiusc=5 * h), tuple(rng.uniform(0, 90, 3))
+        solids.append(make_solid(i, s, 1.4, at, e, vel=rng.normal(0, 0.1, 3), omega=rng.normal(0, 1, 3)))
+    mesh = abi.mesh_desc((side, side, nz), (0.0, 0.0, -0.5 * h * nz), (h, h, h), twod=int(nz == 1 and "tilted" not in kinds
+                                                                                       and "Sphere" not in kinds))
+    return mesh, solids
+
+
+@pytest.mark.parametrize("method", [abi.FRACTION_REFGEO, abi.FRACTION_SUBSAMPLE])
+@pytest.mark.parametrize("kinds,count,nz", [(("Circle_Tail",), 1, 1), (("Circle_Tail", "Circle_TwoTail", "Circle"), 49, 1),
+                                            (("tilted",), 1, 1), (("Circle", "tilted", "Sphere", "Box"), 36, 2)])
+def test_flat_shapes_of_the_second_kernel(cuda_lib, torch_cuda, kinds, count, nz, method):
+    mesh, solids = _flat(160, kinds, count, nz)
+    w = Workload("flat", mesh, solids, abi.options(rho_f=1.0, fraction_method=method, subsample_n=8), 1e-3, (0.1, 0.0, 0.0), 0.05, 5)
+    check_interact(w, run_pair(torch_cuda, w, steps=2))
+
+
+def _classify_us(torch, mesh, solids):
+    cloud = SolidCloud(mesh, solids, abi.options(rho_f=1.0, timing=1))
+    f = cloud.new_fields()
+    U = torch.zeros(3, mesh.nx * mesh.ny * mesh.nz, device="cuda")
+    best = 1e9
+    for _ in range(12):
+        cloud.interact(0.0, 1e-3, U, f, want_ft=False)
+        best = min(best, cloud.kernel_times()["classify_kernel"] * 1e3)
+    items = cloud.stats()["work_items"]
+    cloud.close()
+    return best, items
+
+
+def test_neighbouring_tiles_go_to_different_warps(cuda_lib, torch_cuda):
+    """A tailed circle of some eighty one-tile items takes no longer than one of a few: a warp each (32 neighbours a warp would
+    take several times as long)."""
+    h = 1.0 / 400
+    mesh = abi.mesh_desc((400, 400, 1), (0.0, 0.0, -0.5), (h, h, 1.0), twod=1)
+    few, n_few = _classify_us(torch_cuda, mesh, [make_solid(0, make_shape("Circle_Tail", radius=h, ratio=0.5, thickness=0.5 * h), 1.4,
+                                                            (0.5, 0.5, 0.0))])
+    many, n_many = _classify_us(torch_cuda, mesh, [make_solid(0, make_shape("Circle_Tail", radius=14 * h, ratio=1.0, thickness=4 * h),
+                                                              1.4, (0.5, 0.5, 0.0))])
+    assert n_few <= 9 and n_many >= 64
+    assert many <= 4 * few, (many, few)
