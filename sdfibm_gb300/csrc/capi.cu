@@ -22,7 +22,7 @@
 namespace sdfibm_dev {
 // coupling.cu
 __global__ void plan_kernel(PrepArgs A);
-void launch_classify(const ClassifyArgs& A, bool flat, int grid, cudaStream_t st);
+int launch_classify(const ClassifyArgs& A, bool flat, int grid, cudaStream_t st);
 int classify_occupancy(int method, bool flat);
 int classify_kind(int shape_type, bool flat);
 __global__ void subsample_cells_kernel(FallbackArgs A);
@@ -812,7 +812,7 @@ static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float
         CA.feat_cap = ctx->feat_cap; CA.fref_solid = ctx->d_fref_solid; CA.fref_index = ctx->d_fref_index;
         CA.rg_phi = ctx->d_rg_phi;
         CA.rho_min = ctx->rho_min;
-        launch_classify(CA, ctx->mesh.nz <= 2, std::min(ctx->classify_grid, (ctx->fast_chunks + 7) / 8), st);
+        launches += launch_classify(CA, ctx->mesh.nz <= 2, std::min(ctx->classify_grid, (ctx->fast_chunks + 7) / 8), st);
         mark(ctx, "classify_kernel");
         // the component pass needs only the class bytes and the seeds: on the side stream, beside the fraction
         // kernels below (one stream while timing, so that every kernel has its own events)
@@ -838,7 +838,7 @@ static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float
             ctx->in_cell(), ctx->cut_cell(), ctx->d_cnt, N, ctx->d_sbits, ctx->d_shent, ctx->shent_cap,
             dense ? nullptr : ctx->d_lists[prev][0], ctx->d_lists[prev][2], As, Fs, Ts, Ct, ctx->d_cbits);
         mark(ctx, "scan_reset_kernel");
-        launches += 4;
+        launches += 3;
         if (ctx->u64_dev) {  // interact_host64: U read at the coupling cells from the page-locked FP64 field
             gather_u64_kernel<<<ctx->num_sms * 8, 256, 0, sb>>>(ctx->in_cell(), ctx->cut_cell(), ctx->d_cnt, N,
                                                                  ctx->u64_dev, const_cast<float*>(U));

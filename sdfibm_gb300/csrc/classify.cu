@@ -1970,23 +1970,24 @@ __global__ void __launch_bounds__(CLS_WARPS * 32, 2) classify_any_kernel(Classif
 }
 
 template <bool FLAT, int METHOD>
-static void launch_classify_as(const ClassifyArgs& A, int grid, cudaStream_t st) {
-    if (A.fast_chunks > 0) classify_kernel<FLAT, METHOD><<<grid, CLS_WARPS * 32, 0, st>>>(A);
-    if (any_chunks(A, FLAT) > 0) classify_any_kernel<FLAT, METHOD><<<A.any_grid, CLS_WARPS * 32, 0, st>>>(A);
+static int launch_classify_as(const ClassifyArgs& A, int grid, cudaStream_t st) {
+    const bool fast = A.fast_chunks > 0, any = any_chunks(A, FLAT) > 0;
+    if (fast) classify_kernel<FLAT, METHOD><<<grid, CLS_WARPS * 32, 0, st>>>(A);
+    if (any) classify_any_kernel<FLAT, METHOD><<<A.any_grid, CLS_WARPS * 32, 0, st>>>(A);
+    return (int)fast + (int)any;
 }
 template <bool FLAT>
-static void launch_classify_flat(const ClassifyArgs& A, int grid, cudaStream_t st) {
+static int launch_classify_flat(const ClassifyArgs& A, int grid, cudaStream_t st) {
     switch (A.method) {
-        case SDFIBM_FRACTION_REFGEO: launch_classify_as<FLAT, SDFIBM_FRACTION_REFGEO>(A, grid, st); break;
-        case SDFIBM_FRACTION_SUBSAMPLE: launch_classify_as<FLAT, SDFIBM_FRACTION_SUBSAMPLE>(A, grid, st); break;
-        case SDFIBM_FRACTION_LEARNED: launch_classify_as<FLAT, SDFIBM_FRACTION_LEARNED>(A, grid, st); break;
-        default: launch_classify_as<FLAT, -1>(A, grid, st); break;
+        case SDFIBM_FRACTION_REFGEO: return launch_classify_as<FLAT, SDFIBM_FRACTION_REFGEO>(A, grid, st);
+        case SDFIBM_FRACTION_SUBSAMPLE: return launch_classify_as<FLAT, SDFIBM_FRACTION_SUBSAMPLE>(A, grid, st);
+        case SDFIBM_FRACTION_LEARNED: return launch_classify_as<FLAT, SDFIBM_FRACTION_LEARNED>(A, grid, st);
+        default: return launch_classify_as<FLAT, -1>(A, grid, st);
     }
 }
-// host side: the instantiations for a method and a tile shape
-void launch_classify(const ClassifyArgs& A, bool flat, int grid, cudaStream_t st) {
-    if (flat) launch_classify_flat<true>(A, grid, st);
-    else launch_classify_flat<false>(A, grid, st);
+// host side: the instantiations for a method and a tile shape; the kernels launched
+int launch_classify(const ClassifyArgs& A, bool flat, int grid, cudaStream_t st) {
+    return flat ? launch_classify_flat<true>(A, grid, st) : launch_classify_flat<false>(A, grid, st);
 }
 
 // Shapes whose chunks classify_kernel may take (0) and those it never takes (1): the chunk table holds them in this order.

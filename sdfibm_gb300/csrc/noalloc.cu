@@ -33,7 +33,7 @@
 namespace sdfibm_dev {
 __global__ void plan_kernel(PrepArgs A);
 int classify_kind(int shape_type, bool flat);
-void launch_classify(const ClassifyArgs& A, bool flat, int grid, cudaStream_t st);
+int launch_classify(const ClassifyArgs& A, bool flat, int grid, cudaStream_t st);
 int classify_occupancy(int method, bool flat);
 __global__ void connect_kernel(ConnectArgs A);
 }  // namespace sdfibm_dev

@@ -1,6 +1,6 @@
 """Work items of the classify pass: on one- and two-layer meshes the solids its first kernel does not take (tailed circles, tilted
-prisms, 3-D shapes) against the oracle, few and many of them, and beside solids that kernel takes; and their tiles go to as many
-warps as there are."""
+prisms, 3-D shapes) against the oracle, few and many of them, and beside solids that kernel takes; their tiles go to as many warps
+as there are; and the launches a call reports."""
 import numpy as np
 import pytest
 
@@ -70,3 +70,17 @@ def test_neighbouring_tiles_go_to_different_warps(cuda_lib, torch_cuda):
                                                               1.4, (0.5, 0.5, 0.0))])
     assert n_few <= 9 and n_many >= 64
     assert many <= 4 * few, (many, few)
+
+
+@pytest.mark.parametrize("dims,shapes,classify", [((40, 40, 40), ("Sphere",), 1), ((40, 40, 40), ("Sphere", "Circle"), 2),
+                                                  ((40, 40, 40), ("Circle",), 1), ((40, 40, 1), ("Circle",), 2),
+                                                  ((40, 40, 1), ("Circle", "Circle_Tail"), 2), ((40, 40, 1), ("Circle_Tail",), 1)])
+def test_launches_of_a_call(cuda_lib, torch_cuda, dims, shapes, classify):
+    """plan, connect, claim, scan and reset, fractions, couple, finalize, and the classify kernels that have chunks"""
+    kw = dict(Sphere=dict(radius=3.0), Circle=dict(radius=3.0), Circle_Tail=dict(radius=3.0, ratio=1.0, thickness=1.0))
+    solids = [make_solid(i, make_shape(s, **kw[s]), 1.4, (12.0 + 15 * i, 20.0, 0.5 * dims[2])) for i, s in enumerate(shapes)]
+    cloud = SolidCloud(abi.mesh_desc(dims, (0, 0, 0), (1.0, 1.0, 1.0)), solids, abi.options(rho_f=1.0))
+    U = torch_cuda.zeros(3, dims[0] * dims[1] * dims[2], device="cuda")
+    cloud.interact(0.0, 1e-3, U, cloud.new_fields())
+    assert cloud.stats()["launches"] == 7 + classify
+    cloud.close()
