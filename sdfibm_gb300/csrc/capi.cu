@@ -120,7 +120,8 @@ struct sdfibm_ctx {
     int2* d_chunks = nullptr;  // classify work items: (solid, first tile)
     int total_chunks = 0;
     int fast_chunks = 0;       // leading chunks of the shapes classify_kernel may take
-    int chunk_tiles = CHUNK_TILES;
+    int chunk_tiles = CHUNK_TILES;   // most tiles of a work item
+    int spread_tiles[2] = {INT32_MAX, INT32_MAX};  // and of one of a half space, of another solid (see sdfibm_cuda_create)
     int64_t chunks_cap = 0;    // entries reserved in d_chunks
     int total_tiles = 0;
     uint8_t* d_scratch = nullptr;
@@ -146,6 +147,7 @@ struct sdfibm_ctx {
     // touched-cell lists, double buffered: [cur] is this call's, [cur ^ 1] the previous call's (sparse reset)
     int32_t* d_lists[2][4] = {{nullptr, nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr, nullptr}};
     int cur = 0;
+    int item_tiles(int finite) const { return std::min(chunk_tiles, spread_tiles[finite]); }
     int32_t* in_cell() const { return d_lists[cur][0]; }
     int32_t* in_solid() const { return d_lists[cur][1]; }
     int32_t* cut_cell() const { return d_lists[cur][2]; }
@@ -301,10 +303,11 @@ static int fail(sdfibm_ctx* ctx, int code, const std::string& msg) {
             return fail(ctx, SDFIBM_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));       \
     } while (0)
 
-// classify work items: chunks of up to chunk_tiles consecutive tiles of each solid, the solids grouped by shape type
+// classify work items: chunks of up to wall_tiles (solids of finite size: finite_tiles) consecutive tiles, the solids grouped by shape type
 // (stable): the cut-cell lists then come out grouped by type too, so that the warps of the per-cell kernels mostly
 // run one shape's distance code (the learned stencil: 11 % faster at 256^3 than with the types interleaved)
-static std::vector<int2> make_chunks(const std::vector<SolidK>& hk, int chunk_tiles, bool flat, int* fast_chunks) {
+static std::vector<int2> make_chunks(const std::vector<SolidK>& hk, int wall_tiles, int finite_tiles, bool flat,
+                                     int* fast_chunks) {
     std::vector<int2> chunks;
     *fast_chunks = 0;
     std::vector<size_t> order(hk.size());
@@ -318,7 +321,8 @@ static std::vector<int2> make_chunks(const std::vector<SolidK>& hk, int chunk_ti
     for (size_t s : order) {
         const SolidK& k = hk[s];
         const int nt = k.ntile[0] * k.ntile[1] * k.ntile[2];
-        for (int t0 = 0; t0 < nt; t0 += chunk_tiles) chunks.push_back(make_int2((int)s, t0));
+        const int step = k.infinite ? wall_tiles : finite_tiles;
+        for (int t0 = 0; t0 < nt; t0 += step) chunks.push_back(make_int2((int)s, t0));
         if (classify_kind(k.shape.type, flat) == 0) *fast_chunks = (int)chunks.size();
     }
     return chunks;
@@ -531,18 +535,27 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
         ctx->sh_mask = (int32_t)(t - 1);
         ctx->shent_cap = 2 * t;  // a shared cell has two or more entries
     }
-    // work items of CHUNK_TILES tiles, fewer where they would leave warps of the launch without one (about 24 warps an SM;
-    // half spaces do not count, nearly all of their tiles are skipped): one cylinder's 9 tiles took 36 us in two items and
-    // 12 in nine
-    int64_t finite_tiles = 0;
-    for (const SolidK& k : ctx->hk)
-        if (!k.infinite) finite_tiles += (int64_t)k.ntile[0] * k.ntile[1] * k.ntile[2];
-    ctx->chunk_tiles = (int)std::max<int64_t>(1, std::min<int64_t>(CHUNK_TILES, finite_tiles / (24 * (int64_t)ctx->num_sms)));
+    // work items of CHUNK_TILES tiles, of a solid of finite size fewer where they would leave warps of the launch without one
+    // (about 24 warps an SM): one cylinder's 9 tiles took 36 us in two items and 12 in nine.  Of a half space nearly all tiles
+    // are skipped: what counts of it is a layer of tiles (a row on flat meshes), and its items hold two at least.  A call with
+    // six walls and four spheres, items of one tile / by the rule, us: 10 697 / 5140 at 512^3 (eight), 1697 / 1134 at 256^3
+    // (six), 395 / 367 at 128^3 (two; eight 470); four walls and nine circles at 1024^2 163 / 149 (two; eight 171)
+    int64_t all_finite = 0, faces = 0;
+    for (const SolidK& k : ctx->hk) {
+        const int64_t a = k.ntile[0], b = k.ntile[1], c = k.ntile[2];
+        if (k.infinite) faces += mesh->nz <= 2 ? std::max(a, b) : std::max(a * b, std::max(b * c, a * c));
+        else all_finite += a * b * c;
+    }
+    auto spread = [&](int64_t n, int64_t least) { return (int)std::min<int64_t>(std::max(least, n / (24 * (int64_t)ctx->num_sms)), INT32_MAX); };
+    ctx->chunk_tiles = CHUNK_TILES;
+    ctx->spread_tiles[0] = spread(all_finite + faces, 2);
+    ctx->spread_tiles[1] = spread(all_finite, 1);
     if (ctx->opt.tile_cells > 0) {
         const int cells_per_tile = mesh->nz <= 2 ? 8 * 8 * 2 : 4 * 4 * 4;
         ctx->chunk_tiles = std::max(1, std::min(255, ctx->opt.tile_cells / cells_per_tile));
+        ctx->spread_tiles[0] = ctx->spread_tiles[1] = INT32_MAX;
     }
-    std::vector<int2> chunks = make_chunks(ctx->hk, ctx->chunk_tiles, mesh->nz <= 2, &ctx->fast_chunks);
+    std::vector<int2> chunks = make_chunks(ctx->hk, ctx->item_tiles(0), ctx->item_tiles(1), mesh->nz <= 2, &ctx->fast_chunks);
     ctx->total_chunks = (int)chunks.size();
 
     // collision grid (UGrid(bbox of the mesh, 2*max radiusB))
@@ -800,7 +813,7 @@ static int enqueue_interact(sdfibm_ctx* ctx, double time, double dt, const float
         ClassifyArgs CA{};
         CA.m = ctx->mesh; CA.sk = ctx->d_sk; CA.st = ctx->d_st; CA.plan = ctx->d_plan; CA.chunks = ctx->d_chunks;
         CA.total_chunks = ctx->total_chunks; CA.cls = ctx->d_scratch; CA.cnt = ctx->d_cnt;
-        CA.chunk_tiles = ctx->chunk_tiles;
+        CA.wall_tiles = ctx->item_tiles(0); CA.finite_tiles = ctx->item_tiles(1);
         CA.fast_chunks = ctx->fast_chunks;
         CA.any_grid = std::min(2 * ctx->num_sms, (any_chunks(CA, ctx->mesh.nz <= 2) + 7) / 8);
         CA.method = ctx->opt.fraction_method;
@@ -1507,10 +1520,11 @@ static std::string tune_key(const sdfibm_ctx* ctx) {
 
 static int apply_tuning(sdfibm_ctx* ctx, const Tuning& t) {
     int fast = 0;
-    std::vector<int2> ch = make_chunks(ctx->hk, t.chunk_tiles, ctx->mesh.nz <= 2, &fast);
+    std::vector<int2> ch = make_chunks(ctx->hk, t.chunk_tiles, t.chunk_tiles, ctx->mesh.nz <= 2, &fast);
     if ((int64_t)ch.size() > ctx->chunks_cap) return fail(ctx, SDFIBM_ERR_CAPACITY, "chunk table too small");
     CK(cudaMemcpy(ctx->d_chunks, ch.data(), sizeof(int2) * ch.size(), cudaMemcpyHostToDevice));
     ctx->chunk_tiles = t.chunk_tiles;
+    ctx->spread_tiles[0] = ctx->spread_tiles[1] = INT32_MAX;
     ctx->total_chunks = (int)ch.size();
     ctx->fast_chunks = fast;
     ctx->opt.tile_cells = t.chunk_tiles * (ctx->mesh.nz <= 2 ? 8 * 8 * 2 : 4 * 4 * 4);
@@ -1590,7 +1604,7 @@ int sdfibm_cuda_autotune(sdfibm_ctx* ctx, double dt, const float* U, float* As, 
         Tuning t = best;
         t.chunk_tiles = tc;
         int fast = 0;
-        if ((int64_t)make_chunks(ctx->hk, tc, ctx->mesh.nz <= 2, &fast).size() > ctx->chunks_cap) continue;
+        if ((int64_t)make_chunks(ctx->hk, tc, tc, ctx->mesh.nz <= 2, &fast).size() > ctx->chunks_cap) continue;
         std::map<std::string, float> ms;
         if ((rc = measure(t, ms))) break;
         if (ms.count("classify_kernel") && ms["classify_kernel"] < best_cls) {

@@ -953,7 +953,7 @@ static __device__ __noinline__ void write_cut_list(const ClassifyArgs& A, const 
     }
 }
 
-// ---- the tile kernel: one warp per chunk of up to chunk_tiles tiles of one solid ------------------------------------------
+// ---- the tile kernel: one warp per chunk of consecutive tiles of one solid ------------------------------------------
 constexpr int CLS_WARPS = 8;
 
 // one chunk of any shape: a test per vertex with its own error bound
@@ -978,7 +978,7 @@ __device__ __forceinline__ void classify_any(const ClassifyArgs& A, const int2 c
         const SolidK& k = A.sk[s];
         const SolidPlan& pl = A.plan[s];
         const int ntile_all = k.ntile[0] * k.ntile[1] * k.ntile[2];
-        const int t_end = min(ch.y + A.chunk_tiles, ntile_all);
+        const int t_end = min(ch.y + (k.infinite ? A.wall_tiles : A.finite_tiles), ntile_all);
         const Q4 q = state_quat(A.st[s]);
         const D3 x = state_pos(A.st[s]);
         const ShapeK& sh = k.shape;
@@ -1281,7 +1281,7 @@ __device__ __forceinline__ void classify_fast(const ClassifyArgs& A, const int2 
     const FastFrame f = fast_frame(m, k, pl, FLAT);
     const int e0 = k.ext[0], e1 = k.ext[1], e2 = k.ext[2], lo0 = pl.lo[0], lo1 = pl.lo[1], lo2 = pl.lo[2];
     const int nt0 = k.ntile[0], nt01 = k.ntile[0] * k.ntile[1];
-    const int t_end = min(ch.y + A.chunk_tiles, nt01 * k.ntile[2]);
+    const int t_end = min(ch.y + (k.infinite ? A.wall_tiles : A.finite_tiles), nt01 * k.ntile[2]);
     uint8_t* out = A.cls + k.scratch_off;
     // LEARNED, a solid under rho_min cells: listed from the back, for the fallback
     const bool back = METHOD == SDFIBM_FRACTION_LEARNED && pl.radius_cells < A.rho_min;
@@ -1525,17 +1525,18 @@ __device__ __forceinline__ void classify_body(const ClassifyArgs& A) {
     const int lane = threadIdx.x & 31;
     unsigned long long rechecks = 0, valid_cells = 0;
     unsigned rechecks32 = 0, valid32 = 0;
+    constexpr bool LOOK = FLAT && !FAST;
     const int nw = gridDim.x * CLS_WARPS;
-    int64_t look = FLAT ? blockIdx.x * CLS_WARPS + (threadIdx.x >> 5) : A.fast_chunks;
+    int64_t look = blockIdx.x * CLS_WARPS + (threadIdx.x >> 5);
     int2 seen = make_int2(-1, 0);  // chunk look + lane * nw
     unsigned mine = 0;             // of those, the ones to be done here
     for (;;) {
         int2 ch;
-        if (!FAST && mine) {
+        if (LOOK && mine) {
             const int src = __ffs(mine) - 1;
             mine &= mine - 1;
             ch = make_int2(__shfl_sync(FULL, seen.x, src), __shfl_sync(FULL, seen.y, src));
-        } else if (!FAST && look < A.fast_chunks) {
+        } else if (LOOK && look < A.fast_chunks) {
             const int64_t at = look + lane * (int64_t)nw;
             look += 32 * (int64_t)nw;
             seen = at < A.fast_chunks ? A.chunks[at] : make_int2(-1, 0);

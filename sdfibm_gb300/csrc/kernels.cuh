@@ -216,7 +216,7 @@ constexpr uint32_t CT_KEY_BASE = 1u << 30;
 constexpr uint32_t CT_SHARED = 1u << 31;
 constexpr int SHARED_MAX_PROBES = 64;
 
-// classify work items: up to chunk_tiles consecutive tiles of one solid (default below; the autotuner may change it)
+// classify work items: up to this many consecutive tiles of one solid by default
 constexpr int CHUNK_TILES = 8;
 
 struct ClassifyArgs {
@@ -226,7 +226,8 @@ struct ClassifyArgs {
     SolidPlan* plan;
     const int2* chunks;  // (solid, first tile)
     int total_chunks;
-    int chunk_tiles;     // tiles per work item
+    int wall_tiles;      // tiles per work item of a half space
+    int finite_tiles;    // and of the other solids
     int fast_chunks;     // leading chunks whose shapes classify_kernel may take
     int any_grid;        // CTAs of classify_any_kernel
     uint8_t* cls;      // class byte per bbox cell

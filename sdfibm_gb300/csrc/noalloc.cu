@@ -297,7 +297,7 @@ extern "C" int sdfibm_cuda_touched_noalloc(const sdfibm_mesh_desc* mesh, const s
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int grid = nchunks < 4 * (sms > 0 ? sms : 1) ? nchunks : 4 * (sms > 0 ? sms : 1);
     ClassifyArgs CA{};
-    CA.m = m; CA.sk = d_sk; CA.st = d_st; CA.plan = d_plan; CA.chunks = d_chunks; CA.total_chunks = nchunks; CA.chunk_tiles = CHUNK_TILES;
+    CA.m = m; CA.sk = d_sk; CA.st = d_st; CA.plan = d_plan; CA.chunks = d_chunks; CA.total_chunks = nchunks; CA.wall_tiles = CA.finite_tiles = CHUNK_TILES;
     CA.cls = b + OFF_CLS; CA.cnt = d_cnt; CA.method = -1;
     const int kind = classify_kind(solid->shape.type, m.nz <= 2);
     CA.fast_chunks = kind == 0 ? nchunks : 0;

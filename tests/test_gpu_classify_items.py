@@ -84,3 +84,27 @@ def test_launches_of_a_call(cuda_lib, torch_cuda, dims, shapes, classify):
     cloud.interact(0.0, 1e-3, U, cloud.new_fields())
     assert cloud.stats()["launches"] == 7 + classify
     cloud.close()
+
+
+WALLS = [((0.0, 0.5, 0.5), (0, 0, -90.0)), ((1.0, 0.5, 0.5), (0, 0, 90.0)), ((0.5, 0.0, 0.5), (0, 0, 0.0)),
+         ((0.5, 1.0, 0.5), (0, 0, 180.0)), ((0.5, 0.5, 0.0), (90.0, 0, 0)), ((0.5, 0.5, 1.0), (-90.0, 10.0, 0))]
+
+
+@pytest.mark.parametrize("n,spheres", [((31, 33, 30), 1), ((64, 60, 57), 4), ((96, 40, 1), 2)])
+def test_items_of_half_spaces(cuda_lib, torch_cuda, n, spheres):
+    """Items of two tiles or more for the walls of a cloud of few solids, whose own items are single tiles."""
+    h = 1.0 / max(n)
+    flat = n[2] == 1
+    walls = [w for w in WALLS if not flat or w[1][:2] == (0, 0)]
+    solids = [make_solid(i, make_shape("Plane"), 1.4, tuple(np.array(p) * h * np.array(n)), e) for i, (p, e) in enumerate(walls)]
+    for i in range(spheres):
+        x = (np.array([0.3, 0.4, 0.5]) + 0.25 * (i % 2)) * h * np.array(n)
+        solids.append(make_solid(len(solids), make_shape("Circle" if flat else "Sphere", radius=3.3 * h), 1.4, tuple(x)))
+    mesh = abi.mesh_desc(n, (0.0, 0.0, 0.0), (h, h, h))
+    w = Workload("walls", mesh, solids, abi.options(rho_f=1.0), 1e-3, (0.1, 0.0, 0.0), 0.05, 5)
+    r = run_pair(torch_cuda, w, steps=2)
+    check_interact(w, r)
+    side, layers = (8, 2) if flat else (4, 4)
+    tiles = [-(-d // t) for d, t in zip(n, (side, side, layers))]
+    own = spheres * (4 if flat else 4 ** 3)  # 11 cells a side
+    assert r["gpu"].stats()["work_items"] <= len(walls) * -(-int(np.prod(tiles)) // 2) + own
