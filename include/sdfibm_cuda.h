@@ -146,9 +146,9 @@ typedef struct sdfibm_options {
                                 the caller leaves those fields alone between calls) */
     int32_t exact_forcing;   /* 1: forcing and torque per cell in FP64, solidcloud.cpp:384-417 (default);
                                 0: FP32 forcing with FP64 force/torque sums */
-    int32_t tile_cells;      /* cells per (solid, cell-tile) work item of the classify queue; 0: 8 tiles (512 cells
-                                in 3-D), fewer where that leaves warps without work, or what sdfibm_cuda_autotune
-                                chose */
+    int32_t tile_cells;      /* cells per (solid, cell-tile) work item of the classify queue; 0: up to 8 tiles (512
+                                cells in 3-D) or what sdfibm_cuda_autotune chose, fewer where that leaves warps
+                                without work */
     int32_t timing;          /* 1: record CUDA events around every kernel (sdfibm_cuda_kernel_times) */
     int32_t learned_fallback_n; /* LEARNED: samples per axis of the SUBSAMPLE evaluation of the cells outside the
                                    network's confidence band (0: 16, the lattice the network was trained on) */

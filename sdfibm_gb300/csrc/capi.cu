@@ -121,7 +121,8 @@ struct sdfibm_ctx {
     int total_chunks = 0;
     int fast_chunks = 0;       // leading chunks of the shapes classify_kernel may take
     int chunk_tiles = CHUNK_TILES;   // most tiles of a work item
-    int spread_tiles[2] = {INT32_MAX, INT32_MAX};  // and of one of a half space, of another solid (see sdfibm_cuda_create)
+    int spread_tiles[2] = {1, 1};    // and of one of a half space, of another solid (see sdfibm_cuda_create) ...
+    bool exact_tiles = false;        // ... unless the caller asked for a size
     int64_t chunks_cap = 0;    // entries reserved in d_chunks
     int total_tiles = 0;
     uint8_t* d_scratch = nullptr;
@@ -147,7 +148,7 @@ struct sdfibm_ctx {
     // touched-cell lists, double buffered: [cur] is this call's, [cur ^ 1] the previous call's (sparse reset)
     int32_t* d_lists[2][4] = {{nullptr, nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr, nullptr}};
     int cur = 0;
-    int item_tiles(int finite) const { return std::min(chunk_tiles, spread_tiles[finite]); }
+    int item_tiles(int finite) const { return exact_tiles ? chunk_tiles : std::min(chunk_tiles, spread_tiles[finite]); }
     int32_t* in_cell() const { return d_lists[cur][0]; }
     int32_t* in_solid() const { return d_lists[cur][1]; }
     int32_t* cut_cell() const { return d_lists[cur][2]; }
@@ -553,7 +554,7 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
     if (ctx->opt.tile_cells > 0) {
         const int cells_per_tile = mesh->nz <= 2 ? 8 * 8 * 2 : 4 * 4 * 4;
         ctx->chunk_tiles = std::max(1, std::min(255, ctx->opt.tile_cells / cells_per_tile));
-        ctx->spread_tiles[0] = ctx->spread_tiles[1] = INT32_MAX;
+        ctx->exact_tiles = true;
     }
     std::vector<int2> chunks = make_chunks(ctx->hk, ctx->item_tiles(0), ctx->item_tiles(1), mesh->nz <= 2, &ctx->fast_chunks);
     ctx->total_chunks = (int)chunks.size();
@@ -1520,11 +1521,11 @@ static std::string tune_key(const sdfibm_ctx* ctx) {
 
 static int apply_tuning(sdfibm_ctx* ctx, const Tuning& t) {
     int fast = 0;
-    std::vector<int2> ch = make_chunks(ctx->hk, t.chunk_tiles, t.chunk_tiles, ctx->mesh.nz <= 2, &fast);
+    ctx->chunk_tiles = t.chunk_tiles;  // the largest: a cloud whose items hold fewer (spread_tiles) keeps those
+    ctx->exact_tiles = false;
+    std::vector<int2> ch = make_chunks(ctx->hk, ctx->item_tiles(0), ctx->item_tiles(1), ctx->mesh.nz <= 2, &fast);
     if ((int64_t)ch.size() > ctx->chunks_cap) return fail(ctx, SDFIBM_ERR_CAPACITY, "chunk table too small");
     CK(cudaMemcpy(ctx->d_chunks, ch.data(), sizeof(int2) * ch.size(), cudaMemcpyHostToDevice));
-    ctx->chunk_tiles = t.chunk_tiles;
-    ctx->spread_tiles[0] = ctx->spread_tiles[1] = INT32_MAX;
     ctx->total_chunks = (int)ch.size();
     ctx->fast_chunks = fast;
     ctx->opt.tile_cells = t.chunk_tiles * (ctx->mesh.nz <= 2 ? 8 * 8 * 2 : 4 * 4 * 4);
@@ -1603,8 +1604,6 @@ int sdfibm_cuda_autotune(sdfibm_ctx* ctx, double dt, const float* U, float* As, 
     for (int tc : tiles_cand) {
         Tuning t = best;
         t.chunk_tiles = tc;
-        int fast = 0;
-        if ((int64_t)make_chunks(ctx->hk, tc, tc, ctx->mesh.nz <= 2, &fast).size() > ctx->chunks_cap) continue;
         std::map<std::string, float> ms;
         if ((rc = measure(t, ms))) break;
         if (ms.count("classify_kernel") && ms["classify_kernel"] < best_cls) {

@@ -108,3 +108,21 @@ def test_items_of_half_spaces(cuda_lib, torch_cuda, n, spheres):
     tiles = [-(-d // t) for d, t in zip(n, (side, side, layers))]
     own = spheres * (4 if flat else 4 ** 3)  # 11 cells a side
     assert r["gpu"].stats()["work_items"] <= len(walls) * -(-int(np.prod(tiles)) // 2) + own
+
+
+@pytest.mark.parametrize("dims,shape,items", [((400, 200, 1), dict(radius=5.0), 9), ((48, 48, 48), dict(radius=6.0), 125)])
+def test_tuning_keeps_the_items_of_a_small_cloud(cuda_lib, torch_cuda, dims, shape, items):
+    """One solid's tiles are an item each, with a warp for every one of them, and stay so when the autotuner has chosen."""
+    s = make_shape("Circle" if dims[2] == 1 else "Sphere", **shape)
+    cloud = SolidCloud(abi.mesh_desc(dims, (0, 0, 0), (1.0, 1.0, 1.0)), [make_solid(0, s, 1.4, tuple(0.47 * d for d in dims))],
+                       abi.options(rho_f=1.0))
+    U = torch_cuda.zeros(3, int(np.prod(dims)), device="cuda")
+    f = cloud.new_fields()
+    cloud.interact(0.0, 1e-3, U, f)
+    assert cloud.stats()["work_items"] == items
+    want = {k: v.clone() for k, v in f.items()}
+    assert cloud.autotune(1e-3, U, f) in (2, 4, 8, 16, 32)
+    cloud.interact(0.0, 1e-3, U, f)
+    assert cloud.stats()["work_items"] == items
+    assert all(torch_cuda.equal(want[k], f[k]) for k in f)
+    cloud.close()
