@@ -1513,9 +1513,9 @@ static std::map<std::string, Tuning> g_tune_cache;
 
 static std::string tune_key(const sdfibm_ctx* ctx) {
     char b[256];
-    std::snprintf(b, sizeof(b), "%d.%d.%d/%d/%d.%d.%d/%d/%d/%d", ctx->mesh.nx, ctx->mesh.ny, ctx->mesh.nz, ctx->S,
-                  ctx->opt.fraction_method, ctx->opt.subsample_n, ctx->opt.learned_fallback_n, ctx->total_tiles,
-                  ctx->num_sms, (int)ctx->model_set);
+    std::snprintf(b, sizeof(b), "%d.%d.%d/%d/%d.%d.%d.%d/%d/%d/%d", ctx->mesh.nx, ctx->mesh.ny, ctx->mesh.nz, ctx->S,
+                  ctx->opt.fraction_method, ctx->opt.subsample_n, ctx->opt.learned_fallback_n, (int)(ctx->opt.exact_forcing != 0),
+                  ctx->total_tiles, ctx->num_sms, (int)ctx->model_set);
     return b;
 }
 

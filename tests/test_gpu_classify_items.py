@@ -126,3 +126,17 @@ def test_tuning_keeps_the_items_of_a_small_cloud(cuda_lib, torch_cuda, dims, sha
     assert cloud.stats()["work_items"] == items
     assert all(torch_cuda.equal(want[k], f[k]) for k in f)
     cloud.close()
+
+
+def test_tuning_knows_the_forcing(cuda_lib, torch_cuda):
+    """The FP64 and the FP32 forcing are different kernels: a choice made for one is not taken for the other."""
+    mesh = abi.mesh_desc((44, 43, 41), (0, 0, 0), (1.0, 1.0, 1.0))
+    solids = [make_solid(0, make_shape("Sphere", radius=6.0), 1.4, (21.0, 20.0, 19.0))]
+    U = torch_cuda.zeros(3, 44 * 43 * 41, device="cuda")
+    cached = []
+    for exact in (1, 0, 1, 0):
+        cloud = SolidCloud(mesh, solids, abi.options(rho_f=1.0, exact_forcing=exact))
+        cloud.autotune(1e-3, U, cloud.new_fields())
+        cached.append(cloud.tuning()["from_cache"])
+        cloud.close()
+    assert cached == [0, 0, 1, 1]
