@@ -1444,7 +1444,22 @@ int sdfibm_cuda_touched(sdfibm_ctx* ctx, int32_t solid, int64_t* cells, int8_t* 
         CK(cudaMemcpy(&cnt, P.w.count + solid, sizeof(int32_t), cudaMemcpyDeviceToHost));
         std::vector<int32_t> qc(cnt);
         std::vector<int8_t> qt(cnt);
-        if (cnt) {
+        if (cnt && P.k.uniform_np) {
+            const int64_t o = (int64_t)solid * P.w.words;
+            std::vector<uint32_t> b[3];
+            const uint32_t* src[3] = {P.w.visited + o, P.w.all_in + o, P.w.centre_in + o};
+            for (int i = 0; i < 3; ++i) {
+                b[i].resize(P.w.words);
+                CK(cudaMemcpy(b[i].data(), src[i], sizeof(uint32_t) * P.w.words, cudaMemcpyDeviceToHost));
+            }
+            int32_t at = 0;
+            for (int64_t i = 0; i < P.w.words; ++i)
+                for (uint32_t left = b[0][i] & ~(b[1][i] & b[2][i]); left && at < cnt; left &= left - 1, ++at) {
+                    const uint32_t bit = left & (0u - left);
+                    qc[at] = (int32_t)(32 * i) + __builtin_ctz(left);
+                    qt[at] = b[1][i] & bit ? 1 : (b[2][i] & bit ? 2 : 3);
+                }
+        } else if (cnt) {
             CK(cudaMemcpy(qc.data(), P.w.queue + (int64_t)solid * P.w.qcap, sizeof(int32_t) * cnt,
                           cudaMemcpyDeviceToHost));
             CK(cudaMemcpy(qt.data(), P.w.qtype + (int64_t)solid * P.w.qcap, cnt, cudaMemcpyDeviceToHost));
@@ -1829,19 +1844,22 @@ int sdfibm_cuda_create_polymesh(const double* points, int64_t npoints, const int
     PolyWork& w = P.w;
     w.words = (N + 31) / 32;
     w.qcap = N;
+    w.batches = (N + POLY_BATCH - 1) / POLY_BATCH;
     const bool ok = ok_set && poly_alloc(P, &w.visited, (size_t)(S * w.words)) == cudaSuccess &&
-         poly_alloc(P, &w.queue, (size_t)(S * w.qcap)) == cudaSuccess &&
-         poly_alloc(P, &w.qtype, (size_t)(S * w.qcap)) == cudaSuccess &&
          poly_alloc(P, &w.count, (size_t)S) == cudaSuccess && poly_alloc(P, &w.acc, (size_t)(5 * N)) == cudaSuccess &&
          poly_alloc(P, &w.claim, (size_t)N) == cudaSuccess && poly_alloc(P, &w.nitems, 1) == cudaSuccess &&
-         (!k.uniform_np ||
-          (poly_alloc(P, &w.plan, (size_t)S) == cudaSuccess &&
-           poly_alloc(P, &w.items, (size_t)(S * k.nblocks)) == cudaSuccess &&
-           poly_alloc(P, &w.parent, (size_t)(S * w.qcap)) == cudaSuccess &&
-           poly_alloc(P, &w.clist, (size_t)(S * w.qcap)) == cudaSuccess &&
-           poly_alloc(P, &w.ctype, (size_t)(S * w.qcap)) == cudaSuccess &&
-           poly_alloc(P, &w.ccount, (size_t)S) == cudaSuccess && poly_alloc(P, &w.seed, (size_t)S) == cudaSuccess &&
-           poly_alloc(P, &w.mincand, (size_t)S) == cudaSuccess)) &&
+         (k.uniform_np ? poly_alloc(P, &w.plan, (size_t)S) == cudaSuccess &&
+                             poly_alloc(P, &w.items, (size_t)(S * k.nblocks)) == cudaSuccess &&
+                             poly_alloc(P, &w.parent, (size_t)(S * N)) == cudaSuccess &&
+                             poly_alloc(P, &w.all_in, (size_t)(S * w.words)) == cudaSuccess &&
+                             poly_alloc(P, &w.centre_in, (size_t)(S * w.words)) == cudaSuccess &&
+                             poly_alloc(P, &w.wlist, (size_t)(S * w.words)) == cudaSuccess &&
+                             poly_alloc(P, &w.wstart, (size_t)(S * w.batches)) == cudaSuccess &&
+                             poly_alloc(P, &w.wcount, (size_t)S) == cudaSuccess &&
+                             poly_alloc(P, &w.seed, (size_t)S) == cudaSuccess &&
+                             poly_alloc(P, &w.mincand, (size_t)S) == cudaSuccess
+                       : poly_alloc(P, &w.queue, (size_t)(S * w.qcap)) == cudaSuccess &&
+                             poly_alloc(P, &w.qtype, (size_t)(S * w.qcap)) == cudaSuccess) &&
          cudaMemset(w.count, 0, sizeof(int32_t) * S) == cudaSuccess &&
          // poly_finalize_kernel leaves these as they are here
          cudaMemset(w.acc, 0, sizeof(double) * 5 * N) == cudaSuccess &&

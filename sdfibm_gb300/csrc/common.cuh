@@ -10,6 +10,17 @@ namespace sdfibm_dev {
 
 __device__ inline void set_error(Counters* cnt, int32_t code) { atomicCAS(&cnt->error, 0, code); }
 
+// position of the r-th set bit (r < popc(m))
+__device__ __forceinline__ int nth_bit(uint32_t m, int r) {
+    int p = 0;
+#pragma unroll
+    for (int h = 16; h > 0; h >>= 1) {
+        const int c = __popc((m >> p) & ((1u << h) - 1u));
+        if (r >= c) { r -= c; p += h; }
+    }
+    return p;
+}
+
 // ---- geometry helpers (closed form of the uniform mesh, identical to the oracle's UniformMesh) ----------------------
 __device__ inline double mesh_coord(const MeshK& m, int a, int64_t i) { return m.o[a] + (double)i * m.h[a]; }
 __device__ inline double mesh_centre(const MeshK& m, int a, int64_t i) { return m.o[a] + ((double)i + 0.5) * m.h[a]; }

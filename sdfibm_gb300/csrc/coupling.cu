@@ -501,16 +501,6 @@ __device__ __forceinline__ void connect_sums(const ConnectShared& sh, int tid, i
         tot_cut += c;
     }
 }
-// position of the r-th set bit (r < popc(m))
-__device__ __forceinline__ int nth_bit(uint32_t m, int r) {
-    int p = 0;
-#pragma unroll
-    for (int h = 16; h > 0; h >>= 1) {
-        const int c = __popc((m >> p) & ((1u << h) - 1u));
-        if (r >= c) { r -= c; p += h; }
-    }
-    return p;
-}
 // the lists of the rows from pin and pcut on: 32 words at a time, a lane per listed cell, which finds its word in the prefix
 // sums and its bit in the word
 template <int NT>

@@ -6,7 +6,7 @@
 // with an inside vertex that holds the seed.  Four kernels find it, spread over the whole GPU whatever the solid count:
 //   poly_plan_kernel      the blocks of 128 consecutive cells whose boxes meet each solid's bounding region;
 //   poly_classify_kernel  a warp per 32 cells of those blocks: the inside test of every vertex (FP32 with a rigorous error
-//                         bound, FP64 inside it), a bit and a list entry per cell with an inside vertex; beside it a CTA
+//                         bound, FP64 inside it), a bit per cell with an inside vertex and a list of their words; beside it a CTA
 //                         per solid finds the nearest cell centre (meshSearch::findNearestCell, solidcloud.cpp:363);
 //   poly_link_kernel      union-find over the face neighbours of the listed cells;
 //   poly_couple_kernel    keeps the cells of the seed's set (a seed without an inside vertex: the lowest label's), computes
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(256) poly_plan_kernel(PolyK m, const SolidK* _
         P.kind = sh.type == SDFIBM_SHAPE_PLANE ? 3 : (!sh.prism ? 0 : (q.v.x == 0.0 && q.v.y == 0.0 ? 1 : 2));
         if (blockIdx.y == 0) {
             w.plan[s] = P;
-            w.ccount[s] = 0;
+            w.wcount[s] = 0;
             w.count[s] = 0;
             w.mincand[s] = 0x7fffffff;
             for (int r = 0; r < 6; ++r) ftacc[6 * s + r] = 0.0;
@@ -432,13 +432,16 @@ __global__ void __launch_bounds__(256) poly_classify_kernel(PolyK m, const Solid
         const bool cand = n_in > 0;
         const unsigned bal = __ballot_sync(0xffffffffu, cand);
         if (!bal) continue;
-        int base = 0;
+        const int64_t at = (int64_t)s * w.words;
         if (lane == 0) {
-            w.visited[(int64_t)s * w.words + word] = bal;
-            base = atomicAdd(w.ccount + s, __popc(bal));
+            w.visited[at + word] = bal;
+            // its place in the list, and how many cells lie before it
+            const unsigned long long before = atomicAdd(w.wcount + s, (1ull << 32) | (unsigned)__popc(bal));
+            const int32_t pos = (int32_t)(before >> 32), cells = (int32_t)before, batch = (cells + POLY_BATCH - 1) / POLY_BATCH;
+            w.wlist[at + pos] = make_int2(word, cells);
+            if (batch * POLY_BATCH < cells + __popc(bal)) w.wstart[s * w.batches + batch] = pos;
             atomicMin(w.mincand + s, word * 32 + __ffs(bal) - 1);
         }
-        base = __shfl_sync(0xffffffffu, base, 0);
         // links inside the word: each cell to one listed neighbour of a lower label here, then to that chain's end
         int up = lane;
         if (cand)
@@ -448,8 +451,8 @@ __global__ void __launch_bounds__(256) poly_classify_kernel(PolyK m, const Solid
             }
 #pragma unroll
         for (int k = 0; k < 5; ++k) up = __shfl_sync(0xffffffffu, up, up);
+        int t = 1;
         if (cand) {
-            int8_t t = 1;
             if (n_in < np) {
                 const double* C = m.Cc + 3 * (int64_t)c;
                 const float hx = (float)C[0], hy = (float)C[1], hz = (float)C[2];
@@ -458,10 +461,12 @@ __global__ void __launch_bounds__(256) poly_classify_kernel(PolyK m, const Solid
                 if (in == 2) in = inside64(sh, world2local(poly_vec(m.Cc, c), state_pos(st[s]), state_quat(st[s]))) ? 1 : 0;
                 t = in ? 2 : 3;
             }
-            const int64_t o = (int64_t)s * w.qcap, pos = o + base + __popc(bal & ((1u << lane) - 1u));
-            w.clist[pos] = c;
-            w.ctype[pos] = t;
-            w.parent[o + c] = word * 32 + up;
+            w.parent[(int64_t)s * m.ncells + c] = word * 32 + up;
+        }
+        const unsigned b1 = __ballot_sync(0xffffffffu, cand && t == 1), b2 = __ballot_sync(0xffffffffu, cand && t == 2);
+        if (lane == 0) {
+            w.all_in[at + word] = b1;
+            w.centre_in[at + word] = b2;
         }
     }
 }
@@ -480,29 +485,52 @@ __device__ inline int32_t poly_root(int32_t* parent, int32_t c) {
     return c;
 }
 
-// Union over the face neighbours of the listed cells (each pair from its higher label): the higher root is hung under the
-// lower one by compare-and-swap.  A failed swap means that root has been hung meanwhile, so labels only fall and the loop
-// ends.
+// Union over the face neighbours of the listed words' cells (each pair from its higher label): the higher root is hung under
+// the lower one by compare-and-swap.  A failed swap means that root has been hung meanwhile, so labels only fall and the loop
+// ends.  A CTA takes up to 32 words at a time (fewer where that spreads them over more CTAs), a thread per cell, which finds its
+// word in the prefix sums.
 __global__ void __launch_bounds__(256) poly_link_kernel(PolyK m, PolyWork w) {
-    const int s = blockIdx.x;
-    const int32_t n = w.ccount[s];
-    const int64_t o = (int64_t)s * w.qcap;
-    int32_t* parent = w.parent + o;
+    __shared__ int s_word[32], s_end[32];
+    __shared__ uint32_t s_bits[32];
+    const int s = blockIdx.x, tid = threadIdx.x, n = (int)(w.wcount[s] >> 32);
+    int32_t* parent = w.parent + (int64_t)s * m.ncells;
     const uint32_t* bits = w.visited + (int64_t)s * w.words;
-    for (int32_t e = blockIdx.y * blockDim.x + threadIdx.x; e < n; e += gridDim.y * blockDim.x) {
-        const int32_t c = w.clist[o + e];
-        for (int32_t r = m.cc_off[c]; r < m.cc_off[c + 1]; ++r) {
-            const int32_t nb = m.ccl[r];
-            if (nb >= c || !((bits[nb >> 5] >> (nb & 31)) & 1u)) continue;
-            int32_t a = poly_root(parent, c), b = poly_root(parent, nb);
-            while (a != b) {
-                if (a < b) { const int32_t t = a; a = b; b = t; }
-                const int32_t seen = atomicCAS(parent + a, a, b);
-                if (seen == a) break;
-                a = poly_root(parent, seen);
-                b = poly_root(parent, b);
+    const int take = max(1, min(32, (n + (int)gridDim.y - 1) / (int)gridDim.y));
+    for (int w0 = blockIdx.y * take; w0 < n; w0 += gridDim.y * take) {
+        if (tid < 32) {
+            const bool on = tid < take && w0 + tid < n;
+            const int word = on ? w.wlist[(int64_t)s * w.words + w0 + tid].x : 0;
+            const uint32_t b = on ? bits[word] : 0u;
+            int end = __popc(b);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, end, o);
+                if (tid >= o) end += y;
+            }
+            s_word[tid] = word; s_bits[tid] = b; s_end[tid] = end;
+        }
+        __syncthreads();
+        for (int e = tid; e < s_end[31]; e += blockDim.x) {
+            int i = 0;
+#pragma unroll
+            for (int h = 16; h > 0; h >>= 1)
+                if (s_end[i + h - 1] <= e) i += h;
+            const uint32_t b = s_bits[i];
+            const int32_t c = s_word[i] * 32 + nth_bit(b, e - s_end[i] + __popc(b));
+            for (int32_t r = m.cc_off[c]; r < m.cc_off[c + 1]; ++r) {
+                const int32_t nb = m.ccl[r];
+                if (nb >= c || !((bits[nb >> 5] >> (nb & 31)) & 1u)) continue;
+                int32_t a = poly_root(parent, c), d = poly_root(parent, nb);
+                while (a != d) {
+                    if (a < d) { const int32_t t = a; a = d; d = t; }
+                    const int32_t seen = atomicCAS(parent + a, a, d);
+                    if (seen == a) break;
+                    a = poly_root(parent, seen);
+                    d = poly_root(parent, d);
+                }
             }
         }
+        __syncthreads();
     }
 }
 
@@ -603,12 +631,12 @@ __device__ double poly_cell_volume8(const PolyK& m, int32_t c, const ShapeK& sh,
     return volume;
 }
 
-// Touched cells of one solid (blockIdx.x), POLY_BATCH list entries a CTA: linked, the entries of clist in the seed's set
-// (added to the touched list here); else the touched list itself.  The cut cells of a batch are spread over the CTA's 32
-// groups of 8 lanes, then a lane per cell does the forcing.  Bound by the FP64 pipe (about 2000 operations a cut cell): 174 us
-// for the 140 000-cell mesh's 40 solids, 360 us with a thread per cell; 33 us against 169 us for one cylinder.  The solids
-// run along grid.x, so that the first batches of all of them land on different SMs.
-constexpr int POLY_BATCH = 64;
+// Touched cells of one solid (blockIdx.x), POLY_BATCH of them a CTA: linked, of the cells with an inside vertex in the order of
+// their list of words those in the seed's set (the others are marked); else of the touched list.  The cut cells of a batch are
+// spread over the CTA's 32 groups of 8 lanes, then a lane per cell does the forcing.  Bound by the FP64 pipe (about 2000
+// operations a cut cell): 174 us for the 140 000-cell mesh's 40 solids, 360 us with a thread per cell; 33 us against 169 us for
+// one cylinder.  (Batches of whole words, whose cells differ in number: 186 us.)  The solids run along grid.x, so that the first
+// batches of all of them land on different SMs.
 __global__ void __launch_bounds__(256, 2) poly_couple_kernel(PolyK m, const SolidK* __restrict__ sk,
                                                              const sdfibm_solid_state* __restrict__ st, PolyWork w,
                                                              const float* __restrict__ U, double* __restrict__ ftacc,
@@ -616,17 +644,20 @@ __global__ void __launch_bounds__(256, 2) poly_couple_kernel(PolyK m, const Soli
     __shared__ double s_phi[32][POLY_MAX_CELL_POINTS];
     __shared__ double s_alpha[POLY_BATCH], s_R[9];
     __shared__ int32_t s_cell[POLY_BATCH], s_cut[POLY_BATCH];
+    __shared__ int8_t s_type[POLY_BATCH];
     __shared__ int s_ncut;
     const unsigned FULL = 0xffffffffu;
     const int s = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
-    const int64_t o = (int64_t)s * w.qcap;
-    const int32_t n = linked ? w.ccount[s] : w.count[s];
+    const int64_t o = (int64_t)s * w.qcap, ow = (int64_t)s * w.words;
+    const unsigned long long listed = linked ? w.wcount[s] : 0ull;
+    const int32_t n = linked ? (int32_t)listed : w.count[s], nwords = (int32_t)(listed >> 32);
+    int32_t* parent = w.parent + (int64_t)s * m.ncells;
     if ((int64_t)blockIdx.y * POLY_BATCH >= n) return;
     int32_t home = 0;
     if (tid < POLY_BATCH && linked) {
         const int32_t sd = w.seed[s];
-        const bool on = sd < m.ncells && ((w.visited[(int64_t)s * w.words + (sd >> 5)] >> (sd & 31)) & 1u);
-        home = poly_root(w.parent + o, on ? sd : w.mincand[s]);
+        const bool on = sd < m.ncells && ((w.visited[ow + (sd >> 5)] >> (sd & 31)) & 1u);
+        home = poly_root(parent, on ? sd : w.mincand[s]);
     }
     const ShapeK& sh = sk[s].shape;
     const D3 x = state_pos(st[s]);
@@ -643,23 +674,42 @@ __global__ void __launch_bounds__(256, 2) poly_couple_kernel(PolyK m, const Soli
     for (int64_t b = blockIdx.y; b * POLY_BATCH < n; b += gridDim.y) {
         int32_t c = -1;
         int t = 0;
+        if (linked) {
+            // the words of the batch: at most POLY_BATCH from the one its first cell lies in, by other warps than those that
+            // look for the seed's root meanwhile
+            const int j = tid - POLY_BATCH;
+            const int32_t first = (int32_t)b * POLY_BATCH, at = j >= 0 && j < POLY_BATCH ? w.wstart[s * w.batches + b] + j : nwords;
+            if (at < nwords) {
+                const int2 it = w.wlist[ow + at];
+                if (it.y < first + POLY_BATCH) {
+                    const uint32_t bits = w.visited[ow + it.x], in = w.all_in[ow + it.x], ci = w.centre_in[ow + it.x];
+                    int to = it.y - first;
+                    for (uint32_t left = bits; left; left &= left - 1, ++to) {
+                        const int i = __ffs(left) - 1;
+                        if (to >= 0 && to < POLY_BATCH) {
+                            s_cell[to] = it.x * 32 + i;
+                            s_type[to] = (in >> i) & 1u ? 1 : ((ci >> i) & 1u ? 2 : 3);
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+        }
         if (tid < POLY_BATCH) {  // whole warps
             const int64_t e = b * POLY_BATCH + tid;
             if (e < n) {
-                c = linked ? w.clist[o + e] : w.queue[o + e];
-                t = linked ? w.ctype[o + e] : w.qtype[o + e];
-                if (linked && poly_root(w.parent + o, c) != home) c = -1;
+                c = linked ? s_cell[tid] : w.queue[o + e];
+                t = linked ? s_type[tid] : w.qtype[o + e];
+                if (linked && poly_root(parent, c) != home) {  // left out of the touched cells: both types
+                    atomicOr(w.all_in + ow + (c >> 5), 1u << (c & 31));
+                    atomicOr(w.centre_in + ow + (c >> 5), 1u << (c & 31));
+                    c = -1;
+                }
             }
             const unsigned below = (1u << lane) - 1u;
             if (linked) {
                 const unsigned bal = __ballot_sync(FULL, c >= 0);
-                int base = 0;
-                if (lane == 0 && bal) base = atomicAdd(w.count + s, __popc(bal));
-                base = __shfl_sync(FULL, base, 0) + __popc(bal & below);
-                if (c >= 0) {
-                    w.queue[o + base] = c;
-                    w.qtype[o + base] = (int8_t)t;
-                }
+                if (lane == 0 && bal) atomicAdd(w.count + s, __popc(bal));
             }
             const bool cut = c >= 0 && t != 1;
             const unsigned bal = __ballot_sync(FULL, cut);

@@ -33,6 +33,7 @@ struct PolyK {
     int32_t uniform_np;       // 1: every cell has the same number of points
 };
 constexpr int POLY_BLOCK = 128;  // cells per block: four bitmap words
+constexpr int POLY_BATCH = 64;   // cells a CTA of poly_couple_kernel takes at a time
 
 // Per-call record of a solid (poly_plan_kernel): FP32 map to the local frame and the region its inside points lie in.
 struct PolySolid {
@@ -48,23 +49,28 @@ struct PolySolid {
 };
 
 struct PolyWork {
-    uint32_t* visited;  // [S][words]: cells the search of each solid has reached
+    uint32_t* visited;  // [S][words]: cells the search of each solid has reached; uniform_np: cells with an inside vertex
     int64_t words;
-    int32_t* queue;     // [S][qcap]: touched cells of each solid in search order
-    int8_t* qtype;      // [S][qcap]: their types (1 ALL_INSIDE, 2 CENTER_INSIDE, 3 CENTER_OUTSIDE)
     int32_t* count;     // [S]: touched cells of each solid
-    int64_t qcap;
+    // the breadth-first search
+    int32_t* queue;     // [S][ncells]: touched cells of each solid in search order
+    int8_t* qtype;      // [S][ncells]: their types (1 ALL_INSIDE, 2 CENTER_INSIDE, 3 CENTER_OUTSIDE)
+    int64_t qcap;       // ncells
     double* acc;        // [N][5]: sums over the solids of As, Ts, Fs.x, Fs.y, Fs.z
     int32_t* claim;     // [N]: largest 4 * solid + type over the solids touching the cell (-1: none)
     int32_t* err;       // first device error (DeviceError)
-    // meshes whose cells all have the same point count: cells with an inside vertex and their connected sets
+    // meshes whose cells all have the same point count: cells with an inside vertex and their connected sets.  Lists of words
+    // of the bitmap, not of cells: 4.8 bytes a solid and cell (the search takes 5.1), where lists of cells, their types and the
+    // touched ones beside the forest would take 14
     PolySolid* plan;    // [S]
     int2* items;        // (solid, block) pairs whose boxes meet the solid
     int32_t* nitems;    // their count (left zero by poly_finalize_kernel)
-    int32_t* parent;    // [S][qcap], by cell: union-find forest (parent label <= own label)
-    int32_t* clist;     // [S][qcap]: cells with an inside vertex
-    int8_t* ctype;      // [S][qcap]: their types
-    int32_t* ccount;    // [S]: how many
+    int32_t* parent;    // [S][ncells]: union-find forest (parent label <= own label) of the cells with an inside vertex
+    uint32_t *all_in, *centre_in;  // [S][words]: of those, the cells of type 1 and of type 2 (none: type 3; both: not touched)
+    int2* wlist;        // [S][words]: words of visited that hold such cells, and the number of cells before each
+    int32_t* wstart;    // [S][batches]: place in wlist of the word that holds cell POLY_BATCH * i of the list
+    int64_t batches;
+    unsigned long long* wcount;  // [S]: words << 32 | cells of the list
     int32_t* seed;      // [S]: nearest cell
     int32_t* mincand;   // [S]: lowest label of the cells with an inside vertex
 };
