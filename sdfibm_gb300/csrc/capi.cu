@@ -226,7 +226,7 @@ struct sdfibm_ctx {
     bool model_set = false;
     float* d_feat = nullptr;  // [SDFIBM_MLP_NFEAT][feat_cap]: model inputs and prior of the in-band cut cells
     int64_t* d_mlp_index = nullptr;  // fraction index of each of those cells
-    float* d_rg_phi = nullptr;  // REF-GEO: [8][feat_cap] vertex distances of the listed cut cells
+    float* d_rg_phi = nullptr;  // REF-GEO: [8][feat_cap] vertex distances of the listed cut cells (where any are listed)
     int64_t feat_cap = 0;
     int32_t* d_fref_solid = nullptr;
     int64_t* d_fref_index = nullptr;
@@ -641,6 +641,8 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
     const bool cell_list = ctx->opt.fraction_method == SDFIBM_FRACTION_SUBSAMPLE ||
                            ctx->opt.fraction_method == SDFIBM_FRACTION_REFGEO;
     if (cell_list) ctx->feat_cap = std::max<int64_t>(1, scratch);
+    // the classify pass lists no distances of the 3-D shapes classify_kernel takes (refgeo_cells_kernel computes those)
+    const bool listed_phi = ctx->opt.fraction_method == SDFIBM_FRACTION_REFGEO && (mesh->nz <= 2 || ctx->fast_chunks < ctx->total_chunks);
     if (dalloc(&ctx->d_sk, nsolids) || dalloc(&ctx->d_st, nsolids) || dalloc(&ctx->d_plan, nsolids) ||
         dalloc(&ctx->d_chunks, (size_t)ctx->total_tiles) || dalloc(&ctx->d_scratch, scratch) || dalloc(&ctx->d_alpha, scratch) ||
         dalloc(&ctx->d_gbitmaps, gwords) || dalloc(&ctx->d_lists[0][0], ctx->cap) || dalloc(&ctx->d_lists[0][1], ctx->cap) ||
@@ -657,7 +659,7 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
         dalloc(&ctx->d_rq, (size_t)ctx->rq_cap) || dalloc(&ctx->d_ovf, (size_t)ctx->ovf_cap) ||
         (cell_list &&
          (dalloc(&ctx->d_fref_solid, (size_t)ctx->feat_cap) || dalloc(&ctx->d_fref_index, (size_t)ctx->feat_cap))) ||
-        (ctx->opt.fraction_method == SDFIBM_FRACTION_REFGEO && dalloc(&ctx->d_rg_phi, 8 * (size_t)ctx->feat_cap)) ||
+        (listed_phi && dalloc(&ctx->d_rg_phi, 8 * (size_t)ctx->feat_cap)) ||
         cudaMallocHost((void**)&ctx->h_cnt, sizeof(Counters)) != cudaSuccess ||
         cudaMallocHost((void**)&ctx->h_ft, std::max<size_t>(1, 6 * (size_t)nsolids) * sizeof(double)) != cudaSuccess ||
         (nsolids <= STATES_STAGED && cudaMallocHost((void**)&ctx->h_st, std::max(1, nsolids) * sizeof(sdfibm_solid_state)) != cudaSuccess)) {

@@ -140,3 +140,24 @@ def test_tuning_knows_the_forcing(cuda_lib, torch_cuda):
         cached.append(cloud.tuning()["from_cache"])
         cloud.close()
     assert cached == [0, 0, 1, 1]
+
+
+def test_vertex_distances_are_reserved_where_they_are_listed(cuda_lib, torch_cuda):
+    """REF-GEO in 3-D: 32 bytes a bbox cell for the vertex distances that the classify pass lists, which it does for none of the
+    shapes of its first kernel."""
+    h = 1.0 / 64
+
+    def used(shapes):
+        solids = [make_solid(i, s, 1.4, (0.5, 0.5, 0.5)) for i, s in enumerate(shapes)]
+        torch_cuda.cuda.synchronize()
+        free = torch_cuda.cuda.mem_get_info()[0]
+        cloud = SolidCloud(abi.mesh_desc((64, 64, 64), (0, 0, 0), (h, h, h)), solids, abi.options(rho_f=1.0))
+        torch_cuda.cuda.synchronize()
+        mem = free - torch_cuda.cuda.mem_get_info()[0]
+        cloud.close()
+        return mem
+
+    spheres = [make_shape("Sphere", radius=20 * h)] * 200
+    cells = 200 * 45 ** 3
+    used(spheres[:1])
+    assert used(spheres + [make_shape("Circle", radius=2 * h)]) - used(spheres) >= 30 * cells
