@@ -455,7 +455,8 @@ __device__ inline int block_log2(int n, bool flat) {
 // roundoff u of M.  An end is (-B -+ s) / A with s = sqrt(B^2 - A (C -+ E)); B^2 <= A M and s^2 <= A M, so B^2 - A C is
 // good to 3 u A M and the ends to an error that changes q by at most 16 u M (2^-22 for the approximate root included);
 // sample_frame adds 128 u M to Eg.  Box, m = max |X| + max k: the ends err by a few u m; sample_frame adds 64 u m, and a slab
-// the column hardly moves against (|d| < E / 4 n) takes that d, which shifts a coordinate by E / 4: 1.3 E in all.
+// the column hardly moves against (|d| < E / 4 n) takes that d with its own sign (slab_step), which shifts a coordinate by E / 4
+// at most: 1.3 E in all.
 struct RunFrame {
     float kdx, kdy, kdz, A, minvA, AE;               // quadric (minvA: -1 / A)
     float ix, iy, iz, px, py, pz, cx, cy, cz;        // box: -1 / d, half widths of P and of I
@@ -474,8 +475,7 @@ __device__ __forceinline__ RunFrame run_frame(const SampleFrame& f, float Egh, i
         r.AE = r.A > 1e-36f ? r.A * Egh : NAN;
     } else {
         const float least = 0.25f * Egh * invn, E = 1.3f * Egh;
-        const float ix = __frcp_rn(fabsf(dx) < least ? least : dx), iy = __frcp_rn(fabsf(dy) < least ? least : dy),
-                    iz = __frcp_rn(fabsf(dz) < least ? least : dz);
+        const float ix = __frcp_rn(slab_step(dx, least)), iy = __frcp_rn(slab_step(dy, least)), iz = __frcp_rn(slab_step(dz, least));
         r.ix = -ix; r.iy = -iy; r.iz = -iz;
         r.px = (f.k0 + E) * fabsf(ix); r.py = (f.k1 + E) * fabsf(iy); r.pz = (f.k2 + E) * fabsf(iz);
         r.cx = (f.k0 - E) * fabsf(ix); r.cy = (f.k1 - E) * fabsf(iy); r.cz = (f.k2 - E) * fabsf(iz);

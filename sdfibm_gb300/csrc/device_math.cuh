@@ -223,6 +223,9 @@ __device__ inline double sdf64(const ShapeK& s, const D3& p) {
     return 0.0;
 }
 
+// Step of a lattice column against a slab: at least `least` in magnitude, so that it can be divided by, at most `least` from d.
+__host__ __device__ inline float slab_step(float d, float least) { return fabsf(d) < least ? copysignf(least, d) : d; }
+
 // ---- FP32 classification with error bounds ------------------------------------------------------------------------
 constexpr float U32 = 5.9604645e-8f;  // 2^-24, unit roundoff of FP32
 
