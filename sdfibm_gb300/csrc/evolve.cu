@@ -522,7 +522,7 @@ __device__ inline bool ev_wait(EvolveWork w, unsigned target) {
 __device__ inline void ev_bar(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
 // Position record of a solid for the pair tests: x, y, z and the radius, signed by the contact law (1: positive, 2:
-// negative, others: NaN), so that two records have a sphere law when the product of their radii is positive.
+// negative, zero included, others: NaN), so that two records have a sphere law when their radii have the same sign.
 __device__ inline float4 ev_record(const D3& x, int id, double rB) {
     const float r = (float)rB;
     return make_float4((float)x.x, (float)x.y, (float)x.z, id == 1 ? r : (id == 2 ? -r : NAN));
@@ -553,7 +553,7 @@ __device__ inline bool ev_sphere_near(const float4& a, const float4& b, float sk
     const float mag = fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fabsf(a.z)) + fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fabsf(b.z));
     const float rr = fabsf(a.w) + fabsf(b.w);
     const float reach = rr + skin + 1.52587890625e-5f * (mag + rr);
-    return a.w * b.w > 0.f && dx * dx + dy * dy + dz * dz <= reach * reach;
+    return (__float_as_int(a.w) ^ __float_as_int(b.w)) >= 0 && dx * dx + dy * dy + dz * dz <= reach * reach;
 }
 __device__ inline bool ev_plane_near(const float4& n, const float4& xp, const float4& xs) {
     const float d = n.x * (xs.x - xp.x) + n.y * (xs.y - xp.y) + n.z * (xs.z - xp.z), r = fabsf(xs.w);
