@@ -273,7 +273,7 @@ struct sdfibm_ctx {
 // at 4500, 521 / 1222 at 9700; with one solid in a hundred that fast 489 / 943 at 3000, 1837 / 1011 at 4500, and with all of
 // them 940 / 1053 and 2110 / 1153.  The line lies where the one launch is the faster one at any speed.  More plane-like solids
 // than EV_MAX_PLANES (each tests every sphere) take the launches too.
-static int evolve_limit(int num_sms) { return 20 * num_sms; }
+static int evolve_limit(int num_sms) { return EV_PER_SM * num_sms; }
 constexpr int EV_MAX_PLANES = 64;
 
 // event bracketing of each launch when timing is on: mark(ctx, name) after a launch records its end

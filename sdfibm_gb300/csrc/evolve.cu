@@ -498,6 +498,8 @@ __global__ void collide_kernel(const SolidK* __restrict__ sk, sdfibm_solid_state
 // (GB300), 20 sub-steps: 104 solids 1.26 -> 0.20 ms, 1800 solids 1.05 -> 0.19 ms, all of them crossing the skin in every
 // sub-step 1.18 -> 0.61 ms (2.6 with room for 256 hot ones and one record a lane in flight).
 constexpr int EV_THREADS = 256, EV_WARPS = EV_THREADS / 32;
+constexpr int EV_SOLIDS = 32;             // most solids of a CTA: their rotations take half of its warps
+static_assert(EV_PER_SM <= EV_SOLIDS && EV_SOLIDS * 4 <= EV_THREADS / 2, "solids of a CTA");
 constexpr int EV_LIST = 128;              // listed neighbours of a solid; more: it tests every solid every sub-step
 constexpr int EV_HOT = 32;                // solids beyond half the skin before the lists are made in every sub-step
 constexpr int EV_BATCH = 4;               // records of a lane in flight when a warp tests many solids
@@ -668,27 +670,24 @@ __global__ void __launch_bounds__(EV_THREADS, 1) evolve_contacts_kernel(const So
                                                                         GridK gk, FineGridK fg, int mode,
                                                                         const int32_t* __restrict__ planes, int nplanes,
                                                                         float skin, EvolveWork w, Counters* cnt) {
-    __shared__ double s_f[EV_THREADS][3];
-    __shared__ double s_q[32][4], s_om[32][3], s_T[32][3], s_qn[32][4], s_omn[32][3];  // four lanes a solid
+    __shared__ double s_f[EV_SOLIDS][3];
+    __shared__ double s_q[EV_SOLIDS][4], s_om[EV_SOLIDS][3], s_T[EV_SOLIDS][3], s_qn[EV_SOLIDS][4], s_omn[EV_SOLIDS][3];
     __shared__ double s_fc[EV_WARPS][32][3];
     __shared__ int32_t s_cq[EV_WARPS][32], s_ce[EV_WARPS][32], s_cn[EV_WARPS];
-    __shared__ int32_t s_n[EV_THREADS];   // listed neighbours, -1: more than the list holds
-    __shared__ int s_hot[EV_THREADS];
+    __shared__ int32_t s_n[EV_SOLIDS];   // listed neighbours, -1: more than the list holds
+    __shared__ int s_hot[EV_SOLIDS];
     __shared__ int s_ok, s_move, s_build, s_storm;
     const unsigned FULL = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int s0 = blockIdx.x * per, own = min(per, S - s0);  // >= 1
+    const int s0 = blockIdx.x * per, own = min(per, S - s0);  // 1 .. EV_SOLIDS
     const double time = step->time, dt = step->dt_sub;
     unsigned arrive = 0;
-    // warps 0 .. nrot - 1 do the rotations (four lanes a solid up to 32 solids, else a thread each) while the others wait
-    // for the barrier and test the pairs; with more than 128 solids every warp does both
-    const bool quad = own <= 32;
-    const int nrot = quad ? (own + 7) >> 3 : (own + 31) >> 5;
-    const int cw0 = nrot <= EV_WARPS / 2 ? nrot : 0, ncw = EV_WARPS - cw0, bar = cw0 > 0 ? 1 : 0;
+    // warps 0 .. nrot - 1 do the rotations (four lanes a solid) while the others wait for the barrier and test the pairs
+    const int nrot = (own + 7) >> 3, ncw = EV_WARPS - nrot;
     // this thread's solid
     const int s = s0 + tid;
     const bool mine = tid < own;
-    D3 pos{0, 0, 0}, vel{0, 0, 0}, om{0, 0, 0}, force{0, 0, 0}, torque{0, 0, 0}, at{0, 0, 0};
+    D3 pos{0, 0, 0}, vel{0, 0, 0}, om{0, 0, 0}, force{0, 0, 0}, at{0, 0, 0};
     Q4 q{1, D3{0, 0, 0}};
     int id = -1, plane = -1;
     double rB = 0.0;
@@ -708,10 +707,8 @@ __global__ void __launch_bounds__(EV_THREADS, 1) evolve_contacts_kernel(const So
             __stcg(qo + 2, make_double2(n.x, n.y));
             __stcg(qo + 3, make_double2(n.z, 0.0));
         }
-        if (quad) {
-            s_q[tid][0] = q.w; s_q[tid][1] = q.v.x; s_q[tid][2] = q.v.y; s_q[tid][3] = q.v.z;
-            s_om[tid][0] = om.x; s_om[tid][1] = om.y; s_om[tid][2] = om.z;
-        }
+        s_q[tid][0] = q.w; s_q[tid][1] = q.v.x; s_q[tid][2] = q.v.y; s_q[tid][3] = q.v.z;
+        s_om[tid][0] = om.x; s_om[tid][1] = om.y; s_om[tid][2] = om.z;
         return key.w != 0;
     };
     if (mine) {
@@ -726,12 +723,10 @@ __global__ void __launch_bounds__(EV_THREADS, 1) evolve_contacts_kernel(const So
                 if (planes[i] == s) plane = i;
         publish(0);
     }
-    s_hot[tid] = 0;
+    if (tid < EV_SOLIDS) s_hot[tid] = 0;
     if (blockIdx.x == 0 && tid < EV_HOT) __stcg(w.hot + tid, make_int2(0, 0x7fffffff));
     // the forces that need no pair (clearForceAndTorque, applyForcer, addMidFluidForceAndTorque, addMidEnvironment: the
     // same in every sub-step without a forcer) and the rotation half of the move
-    D3 om_new{0, 0, 0};
-    Q4 q_new{1, D3{0, 0, 0}};
     auto rotate = [&](bool first) {
         if (mine) {
             const SolidK& k = sk[s];
@@ -743,21 +738,16 @@ __global__ void __launch_bounds__(EV_THREADS, 1) evolve_contacts_kernel(const So
                 }
                 pre_forces(k, x, time, rho_f, g);
                 force = ld3(x.force);
-                torque = ld3(x.torque);
-                if (quad) { s_T[tid][0] = torque.x; s_T[tid][1] = torque.y; s_T[tid][2] = torque.z; }
+                s_T[tid][0] = x.torque[0]; s_T[tid][1] = x.torque[1]; s_T[tid][2] = x.torque[2];
             }
         }
-        if (quad) {
-            ev_bar(2, 32 * nrot);
-            const int i = min(tid >> 2, own - 1), r = tid & 3;
-            double o, e;
-            move_rotation4(sk[s0 + i], s_q[i], s_om[i], s_T[i], time, dt, o, e);
-            if ((tid >> 2) < own) {
-                s_qn[i][(r + 1) & 3] = e;
-                if (r < 3) s_omn[i][r] = o;
-            }
-        } else if (mine) {
-            move_rotation(sk[s], q, om, torque, time, dt, om_new, q_new);
+        ev_bar(2, 32 * nrot);
+        const int i = min(tid >> 2, own - 1), r = tid & 3;
+        double o, e;
+        move_rotation4(sk[s0 + i], s_q[i], s_om[i], s_T[i], time, dt, o, e);
+        if ((tid >> 2) < own) {
+            s_qn[i][(r + 1) & 3] = e;
+            if (r < 3) s_omn[i][r] = o;
         }
     };
     if (tid == 0) { s_build = 1; s_move = 0; s_storm = 0; }
@@ -769,15 +759,15 @@ __global__ void __launch_bounds__(EV_THREADS, 1) evolve_contacts_kernel(const So
         const int4* key = w.key + (int64_t)buf * S;
         ++arrive;
         if (wid < nrot) rotate(it == 0);
-        if (wid >= cw0) {
-            if (tid == 32 * cw0) {
+        if (wid >= nrot) {
+            if (tid == 32 * nrot) {
                 s_ok = ev_wait(w, gridDim.x * arrive) ? 1 : 0;
                 if (it > 0 && !s_storm) s_storm = __ldcg(&w.ctrl->rebuild[(it - 1) & 1]) == it;
                 s_build = it == 0 || s_storm;
             }
-            ev_bar(bar, 32 * ncw);
+            ev_bar(1, 32 * ncw);
             if (s_ok && s_build) {  // lists of the CTA's solids, four of them per pass over the records
-                for (int i0 = (wid - cw0) * 4; i0 < own; i0 += ncw * 4) {
+                for (int i0 = (wid - nrot) * 4; i0 < own; i0 += ncw * 4) {
                     float4 a[4];
                     int n[4];
 #pragma unroll
@@ -813,12 +803,12 @@ __global__ void __launch_bounds__(EV_THREADS, 1) evolve_contacts_kernel(const So
                         for (int u = 0; u < 4; ++u)
                             if (i0 + u < own) s_n[i0 + u] = n[u] <= EV_LIST ? n[u] : -1;
                 }
-                ev_bar(bar, 32 * ncw);
+                ev_bar(1, 32 * ncw);
             }
             // pair forces, a warp per solid; entries of the hot list hold the step they count from (a CTA ahead of this one
             // may add to it meanwhile)
             const int nhot = s_ok && !s_storm ? min(__ldcg(&w.ctrl->nhot), EV_HOT) : 0;
-            for (int i = wid - cw0; i < (s_ok ? own : 0); i += ncw) {
+            for (int i = wid - nrot; i < (s_ok ? own : 0); i += ncw) {
                 const int p = s0 + i;
                 const int4 kp = __ldcg(key + p);
                 const float4 rp = __ldcg(rec + p);
@@ -932,13 +922,8 @@ __global__ void __launch_bounds__(EV_THREADS, 1) evolve_contacts_kernel(const So
             if (s_build) at = pos;
             const D3 ft{force.x + s_f[tid][0], force.y + s_f[tid][1], force.z + s_f[tid][2]};
             move_translation(k, ft, time, dt, vel, pos);
-            if (quad) {
-                om = D3{s_omn[tid][0], s_omn[tid][1], s_omn[tid][2]};
-                q = Q4{s_qn[tid][0], D3{s_qn[tid][1], s_qn[tid][2], s_qn[tid][3]}};
-            } else {
-                om = om_new;
-                q = q_new;
-            }
+            om = D3{s_omn[tid][0], s_omn[tid][1], s_omn[tid][2]};
+            q = Q4{s_qn[tid][0], D3{s_qn[tid][1], s_qn[tid][2], s_qn[tid][3]}};
             if (last) {
                 sdfibm_solid_state& x = st[s];
                 st3(x.force, ft);

@@ -314,6 +314,9 @@ struct alignas(16) CollRec {
     float x, y, z, r;  // centre and bounding radius rounded to FP32 (the screen of sphere pairs)
 };
 
+// Most solids per SM of the one-launch evolve (see evolve_limit in capi.cu)
+constexpr int EV_PER_SM = 20;
+
 // Work space of evolve_contacts_kernel: published positions (two buffers), the plane-like solids' normals and
 // orientations, neighbour lists and the grid barrier.
 struct EvolveCtrl {
