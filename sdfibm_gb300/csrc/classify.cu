@@ -1542,6 +1542,8 @@ __device__ __forceinline__ void classify_body(const ClassifyArgs& A) {
             seen = at < A.fast_chunks ? A.chunks[at] : make_int2(-1, 0);
             mine = __ballot_sync(FULL, seen.x >= 0 && !fast_shape<FLAT>(A.sk[max(seen.x, 0)], A.st[max(seen.x, 0)]));
             continue;
+        } else if (LOOK && A.fast_chunks >= A.total_chunks) {
+            break;  // nothing in the queue: no warp asks
         } else {
             int chunk = 0;
             if (lane == 0) chunk = FAST ? atomicAdd(&A.cnt->classify_next, 1) : atomicAdd(&A.cnt->classify_any_next, 1) + A.fast_chunks;
