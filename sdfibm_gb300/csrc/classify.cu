@@ -32,7 +32,10 @@ namespace sdfibm_dev {
 // Vertex slots: 0:(i,j,k) 1:(i+1,j,k) 2:(i,j+1,k) 3:(i+1,j+1,k) 4..7 the same at k+1 (ascending point label); the face
 // vertex orders are the ones the mesh stores (owner's hex-model face for internal faces, the cell's own for boundary
 // faces), which fix the apex of each face.
-__constant__ int8_t c_face_slots[9][4] = {
+struct FaceSlots {
+    int8_t v[9][4];
+};
+constexpr FaceSlots FACE_SLOTS = {{
     {1, 3, 7, 5},  // x-max, owner order (internal +x face and x-max boundary face)
     {2, 6, 7, 3},  // y-max
     {4, 5, 7, 6},  // z-max
@@ -42,7 +45,8 @@ __constant__ int8_t c_face_slots[9][4] = {
     {0, 2, 6, 4},  // -x internal face (owner is the lower neighbour)
     {0, 4, 5, 1},  // -y internal face
     {0, 1, 3, 2},  // -z internal face
-};
+}};
+__constant__ FaceSlots c_face_slots = FACE_SLOTS;  // for runtime indices
 
 __device__ inline float lfrac32(float pa, float pb) {
     if (pa > 0.f && pb > 0.f) return 0.f;
@@ -115,7 +119,7 @@ static __device__ __noinline__ float refgeo32(const MeshK& m, const float* ph, i
     if (m.twod) { ap.v[2] = apz; ap.w[2] = apz1; }
     float vol = 0.f;
     auto acc = [&](int slot, int axis, int plane) {
-        const float eps = face_fraction32(ph, c_face_slots[slot], axis);
+        const float eps = face_fraction32(ph, c_face_slots.v[slot], axis);
         vol += (1.0f / 3.0f) * eps * ap.dist(axis, plane);
     };
     // mesh.cells()[c] order: owned internal (+x,+y,+z), boundary faces by patch, then -z,-y,-x
@@ -137,11 +141,7 @@ static __device__ __noinline__ float refgeo32(const MeshK& m, const float* ph, i
 // The same for a cell whose faces are known (inside the mesh in x and y, and in z too unless the mesh has one layer): operation
 // for operation what refgeo32 does, with every vertex, edge and face at a compile-time place.  refgeo32 keeps its cells' arrays
 // in local memory, as its faces pick from them, and divides twice for every edge.
-__device__ __forceinline__ constexpr int face_vertex(int slot, int q) {  // c_face_slots
-    constexpr int8_t F[9][4] = {{1, 3, 7, 5}, {2, 6, 7, 3}, {4, 5, 7, 6}, {0, 4, 6, 2}, {0, 1, 5, 4},
-                                {0, 2, 3, 1}, {0, 2, 6, 4}, {0, 4, 5, 1}, {0, 1, 3, 2}};
-    return F[slot][q];
-}
+__device__ __forceinline__ constexpr int face_vertex(int slot, int q) { return FACE_SLOTS.v[slot][q]; }
 __device__ __forceinline__ constexpr int edge_axis(int o, int a) { return (o ^ a) == 1 ? 0 : ((o ^ a) == 2 ? 1 : 2); }
 // edge from the lower vertex v along an axis: 4 * axis + the other two bits of v
 __device__ __forceinline__ constexpr int edge_slot(int o, int a) {
@@ -269,7 +269,7 @@ static __device__ __noinline__ float exact_phi_point(const ShapeK& sh, const Mes
     return (float)sdf64(sh, world2local(p, x, q));
 }
 
-// ---- SUBSAMPLE: one warp per cut cell ----------------------------------------------------------------------------------
+// ---- SUBSAMPLE: a warp per cut cell -----------------------------------------------------------------------------------
 // Each lane owns (a,b) columns of the n x n x n midpoint lattice and walks its column in z.  Local coordinates step by
 // three precomputed vectors (the columns of the world->local map times h).  One error bound E covers every sample
 // coordinate of the cell; for the convex shapes the bound of the inside function is also taken once per cell, from
@@ -589,7 +589,7 @@ __device__ __forceinline__ int subsample_runs_body(const MeshK& m, const ShapeK&
     return cnt;
 }
 
-// out of line for the classify pass; the fallback kernel inlines the body (DEFER_ONLY, no FP64 path)
+// out of line for the recount (FP64 path included); subsample_cells_kernel inlines the body (DEFER_ONLY, no FP64 path)
 template <int T, bool DEFER_ONLY>
 __device__ __noinline__ int subsample_runs(const MeshK& m, const ShapeK& sh, const SampleFrame& f, float Egh, int64_t i,
                                            int64_t j, int64_t k, int n, const D3& x, const Q4& q,
@@ -679,8 +679,8 @@ static __device__ __forceinline__ int subsample_warp_body(const MeshK& m, const 
     SampleFrame f;
     float Ep, Egh;
     const int kind = sample_frame(m, sh, M, tf, a0, b0, c0, f, Ep, Egh);
-    // 3-D convex shapes count runs along columns from 5 samples per axis; out of line (the classify pass), lattices
-    // of 16 and more skip 4 x 4 x 4 blocks instead
+    // 3-D convex shapes count runs along columns from 5 samples per axis; in the recount lattices of 16 and more skip
+    // 4 x 4 x 4 blocks instead
     const bool use_runs = !m.twod && !sh.prism && n >= 5 && (DEFER_ONLY || n < 16);
     int cnt;
     if (kind == SS_QUADRIC) {
@@ -709,7 +709,7 @@ static __device__ __forceinline__ int subsample_warp_body(const MeshK& m, const 
     return cnt;
 }
 
-// the out-of-line form of the classify pass and of the recount (FP64 path included)
+// the out-of-line form of the recount (FP64 path included)
 static __device__ __noinline__ int subsample_warp(const MeshK& m, const ShapeK& sh, const float* M, const TileFrame& tf,
                                                   int a0, int b0, int c0, const D3& x, const Q4& q, int64_t i,
                                                   int64_t j, int64_t k, int n, unsigned long long* rechecks,
@@ -721,7 +721,8 @@ static __device__ __noinline__ int subsample_warp(const MeshK& m, const ShapeK& 
 // The geometry consumes phi in FP32, so phi needs ~1e-7 relative accuracy and the reference's exact sign and filter
 // (|phi| < 1e-8 -> -1e-8).  The local point and every cancelling difference (|p|^2 - r^2, |x| - a, ...) are FP64; the
 // square roots and the final division only scale a non-cancelling quantity and run in FP32.  Values within 1e-6 of
-// the filter threshold are recomputed with the reference's full FP64 sequence by the caller.
+// the filter threshold are recomputed with the reference's full FP64 sequence by the caller.  2-D shapes and half spaces: 3-D
+// spheres, ellipsoids and boxes have sdf_ff_at.
 __device__ inline float rect_mixed(double x, double y, double ra, double rb) {
     const double dx = fabs(x) - ra, dy = fabs(y) - rb;
     const double dxp = dmax(0.0, dx), dyp = dmax(0.0, dy);
@@ -736,29 +737,14 @@ static __device__ __noinline__ float sdf_mixed(const ShapeK& s, const D3& p) {
             const double qq = magSqr(q);
             return (float)(qq - a[1]) / (sqrtf((float)qq) + (float)a[0]);
         }
-        case SDFIBM_SHAPE_SPHERE: {
-            const D3 q = com + p;
-            const double qq = magSqr(q);
-            return (float)(qq - a[1]) / (sqrtf((float)qq) + (float)a[0]);
-        }
         case SDFIBM_SHAPE_ELLIPSE: {
             const D3 q = com + p;
             const double xa = q.x * q.x * a[2], yb = q.y * q.y * a[3];
             return (float)(0.5 * (xa + yb - 1.0)) / sqrtf((float)(xa * a[2] + yb * a[3]));
         }
-        case SDFIBM_SHAPE_ELLIPSOID: {
-            const double xa = p.x * p.x * a[3], yb = p.y * p.y * a[4], zc = p.z * p.z * a[5];
-            return (float)(0.5 * (xa + yb + zc - 1.0)) / sqrtf((float)(xa * a[3] + yb * a[4] + zc * a[5]));
-        }
         case SDFIBM_SHAPE_RECTANGLE: {
             const D3 q = com + p;
             return rect_mixed(q.x, q.y, a[0], a[1]);
-        }
-        case SDFIBM_SHAPE_BOX: {
-            const D3 q = com + p;
-            const double dx = fabs(q.x) - a[0], dy = fabs(q.y) - a[1], dz = fabs(q.z) - a[2];
-            const double dxp = dmax(0.0, dx), dyp = dmax(0.0, dy), dzp = dmax(0.0, dz);
-            return sqrtf((float)(dxp * dxp + dyp * dyp + dzp * dzp)) + (float)dmin(0.0, dmax(dz, dmax(dx, dy)));
         }
         case SDFIBM_SHAPE_PLANE: return (float)p.y;
         case SDFIBM_SHAPE_CIRCLE_TAIL: {
@@ -781,7 +767,6 @@ static __device__ __noinline__ float sdf_mixed(const ShapeK& s, const D3& p) {
     return 0.f;
 }
 
-// filter of sdf.h:147-150 applied to the mixed value; *exact_needed set when the value sits on the threshold
 // ---- two-float vertex distances (REF-GEO, 3-D spheres, ellipsoids and boxes) ---------------------------------------
 // Pairs hi + lo with error-free sums and products (Dekker, Knuth), explicit rounding intrinsics so that nothing is
 // contracted or reassociated; each operation errs by a few 2^-48 of its operands' magnitudes.  GB300 issues FP32 at 64
@@ -889,6 +874,7 @@ __device__ inline float sdf_ff(const ShapeK& s, const SolidPlan& pl, float da, f
     return sdf_ff_at(s, P, ml, err, den);
 }
 
+// filter of sdf.h:147-150 applied to a value of sdf_mixed; *exact_needed set when the value sits on the threshold
 __device__ inline float filter_mixed(const ShapeK& s, float phi, bool* exact_needed) {
     if (s.type == SDFIBM_SHAPE_PLANE) return phi;  // the plane's distance is unfiltered and exact
     const float a = fabsf(phi);
@@ -896,9 +882,8 @@ __device__ inline float filter_mixed(const ShapeK& s, float phi, bool* exact_nee
     return a < 1e-8f ? -1e-8f : phi;
 }
 
-// LEARNED: the features of the tile's cut cells (one warp), appended to the network's input buffer with the index of
-// the cell's fraction; out of line to keep the tile loop small.  tile0 = fraction index of the tile's cell (0,0,0).
-// REF-GEO: the tile's cut cells (one warp) appended to the cell list with the distances of their 8 vertices
+// REF-GEO: the tile's cut cells (one warp) appended to the cell list with the distances of their 8 vertices; out of line to keep
+// the tile loop small.  tile0 = fraction index of the tile's cell (0,0,0).
 template <int TX, int TY, int TZ>
 static __device__ __noinline__ void write_refgeo_list(const ClassifyArgs& A, const uint8_t* cutlist, int ncut,
                                                       const float* vphi, int s, int64_t tile0, int ext0, int ext1) {
@@ -927,7 +912,7 @@ static __device__ __noinline__ void write_refgeo_list(const ClassifyArgs& A, con
     }
 }
 
-// SUBSAMPLE: the tile's cut cells (one warp) appended to the cell list as (solid, fraction index)
+// SUBSAMPLE and LEARNED: the tile's cut cells (one warp) appended to the cell list as (solid, fraction index)
 template <int TX, int TY, int TZ>
 static __device__ __noinline__ void write_cut_list(const ClassifyArgs& A, const uint8_t* cutlist, int ncut, int s,
                                                    int64_t tile0, int ext0, int ext1) {
@@ -961,6 +946,7 @@ template <int TX, int TY, int TZ, int METHOD>
 __device__ __forceinline__ void classify_any(const ClassifyArgs& A, const int2 ch, unsigned long long& rechecks,
                                              unsigned long long& valid_cells) {
     constexpr int VX = TX + 1, VY = TY + 1, VZ = TZ + 1, NV = VX * VY * VZ, NC = TX * TY * TZ;
+    constexpr bool FLAT = TZ == 2;  // only there 3-D spheres, ellipsoids and boxes come here
     __shared__ uint8_t s_vin[CLS_WARPS][NV];
     __shared__ uint8_t s_need[CLS_WARPS][NV];
     __shared__ float s_phi[CLS_WARPS][NV];
@@ -1006,7 +992,7 @@ __device__ __forceinline__ void classify_any(const ClassifyArgs& A, const int2 c
                 I0 + cx < vlo0 || I0 > vhi0 || J0 + cy < vlo1 || J0 > vhi1 || K0 + cz < vlo2 || K0 > vhi2)
                 continue;
             bool cull = false;
-            if (pl.cull_box) {
+            if (FLAT && pl.cull_box) {
                 // separating axes of the solid's local box: the tile's centre and half extents seen in the local
                 // frame (FP32 with a relative margin of 1e-4 on both sides of every comparison)
                 const float hx = 0.5f * (float)cx * m.h32[0], hy = 0.5f * (float)cy * m.h32[1],
@@ -1109,7 +1095,7 @@ __device__ __forceinline__ void classify_any(const ClassifyArgs& A, const int2 c
                 __syncwarp();
                 const double* L = pl.lmap;
                 // 3-D spheres, ellipsoids and boxes: two-float distances (FP32 pipe); others: sdf_mixed (FP64)
-                const bool ff_shape = !sh.prism && (sh.type == SDFIBM_SHAPE_SPHERE ||
+                const bool ff_shape = FLAT && !sh.prism && (sh.type == SDFIBM_SHAPE_SPHERE ||
                                                     sh.type == SDFIBM_SHAPE_ELLIPSOID || sh.type == SDFIBM_SHAPE_BOX);
                 for (int u = lane; u < nneed; u += 32) {
                     const int v = vlist[u];
@@ -1384,7 +1370,6 @@ __device__ __forceinline__ void classify_fast(const ClassifyArgs& A, const int2 
             }
             // cells: all and any of the eight vertices, this lane's cells of each pass
             unsigned all_p = 0, any_p = 0;  // bit p: pass p
-            unsigned cutm[FLAT ? 1 : 4];    // 3-D: cut cells of layer c at bit a + 5 b (before the mesh limits)
             if (FLAT) {
                 const int r = lane < 9 ? lane : 0;
                 const unsigned row = ((r < 3 ? bits[0] : (r < 6 ? bits[1] : bits[2])) >> (9 * (r % 3))) & 0x1ffu;
@@ -1396,7 +1381,6 @@ __device__ __forceinline__ void classify_fast(const ClassifyArgs& A, const int2 
                     any_p |= an * (5u << h);
                 }
             } else {
-                constexpr unsigned CM = 0xfu * (1u | 1u << 5 | 1u << 10 | 1u << 15);
                 const int pos = ca + 5 * cb;
                 unsigned al0 = bits[0] & (bits[0] >> 1), an0 = bits[0] | (bits[0] >> 1);
                 al0 &= al0 >> 5;
@@ -1407,7 +1391,6 @@ __device__ __forceinline__ void classify_fast(const ClassifyArgs& A, const int2 
                     al1 &= al1 >> 5;
                     an1 |= an1 >> 5;
                     const unsigned al = al0 & al1, an = an0 | an1;
-                    cutm[c] = an & ~al & CM;
                     if ((lane >> 4) == (c & 1)) {
                         all_p |= ((al >> pos) & 1u) << (c >> 1);
                         any_p |= ((an >> pos) & 1u) << (c >> 1);
