@@ -8,17 +8,19 @@
 //             inside test once per vertex (FP32 with a guard band, FP64 re-check inside the band) and writes one
 //             class byte per cell: 0 no inside vertex, 1 all inside, 2 centre inside, 3 centre outside
 //             (CellEnumerator::_next, cellenumerator.cpp:6-34), and lists the cut cells for the fraction kernels
-//   fraction  (classify.cu) REF-GEO a thread per listed cell; SUBSAMPLE a warp per listed cell; LEARNED the network,
-//             then SUBSAMPLE on the cells outside its band; FP64 rechecks of undecided sample points
-//   connect   on a side stream beside the fraction kernels: one CTA (or warp) per solid, bit-parallel flood fill
-//             from the seed over cells with an inside vertex (the BFS of CellEnumerator::intersect with its seed
-//             fallback, cellenumerator.cpp:47-78), then the reached cells appended to the ALL_INSIDE list or the
-//             cut-cell list in ascending cell order; claim of each touched cell; reset of the cells the previous call
-//             touched and this one does not (sparse form of solidcloud.cpp:438-441)
-//   couple    persistent CTAs over 256-entry chunks of both lists: alpha (1, or the fraction), direct forcing, the
-//             final fields of single-owner cells, warp then FP64-atomic reduction of force and torque per solid
+//   fraction  (classify.cu) REF-GEO a thread per listed cell; SUBSAMPLE a lane per listed cell, a warp where there are few;
+//             LEARNED the network, then SUBSAMPLE on the cells outside its band; FP64 rechecks of undecided sample points
+//   connect   on a side stream beside the fraction kernels: a CTA, 128 threads or a warp per solid; the cells with an inside
+//             vertex as bitmaps, a proof that they hang together or a bit-parallel flood fill from the seed (the BFS of
+//             CellEnumerator::intersect with its seed fallback, cellenumerator.cpp:47-78), then the reached cells appended to
+//             the ALL_INSIDE list or the cut-cell list in ascending cell order
+//   claim     of each touched cell, and marks of the 8-cell chunks they lie in
+//   scan      the list entries on cells of several solids; reset of the cells the previous call touched and this one does not
+//             (sparse form of solidcloud.cpp:438-441)
+//   couple    warps over the marked chunks: alpha (1, or the fraction), direct forcing, the final fields of single-owner
+//             cells, zeros for unclaimed ones, force and torque summed per solid in the warp, then by FP64 atomics
 //   finalize  cells of several solids from the FP64 table: Ct of the last solid (as the serial loop), As = min(As,1)
-//             (checkAlpha); ft: FT = rho_f V / dt * sums
+//             (checkAlpha); FT = rho_f V / dt * sums
 #include <cstdint>
 #include <cuda_runtime.h>
 

@@ -3,8 +3,9 @@
 // Two evaluation paths:
 //  * *64 functions reproduce the reference's FP64 arithmetic operation for operation (OpenFOAM vector /
 //    quaternion algebra, src/libshape/ishape.h:43-52, src/libshape/sdf/sdf.h, the shape headers).  The library is
-//    compiled with -fmad=false, so no multiply-add is fused and every result matches a host FP64 evaluation bit
-//    for bit.
+//    compiled with -fmad=false, so no multiply-add is fused unless the code says so, and their results match a host FP64
+//    evaluation bit for bit.  (The FP64 forcing, fixInternal and the polyMesh distances are not among them: written with
+//    fused multiply-adds or the matrix form of the rotation they differ from it in the last place.)
 //  * *32 functions evaluate the same inside test in FP32 together with a rigorous bound on their error and answer
 //    inside / outside / undecided.  Undecided points (a band of about 1e-6 relative around the surface) are
 //    re-evaluated with the *64 path, so classifications are always identical to the FP64 result while almost all

@@ -26,8 +26,10 @@
 //   poly_finalize_kernel  the fields from the FP64 sums: As = min(sum, 1) (checkAlpha, solidcloud.cpp:564-570), Ct of
 //                         the last solid in the reference's order;
 //   poly_fix_kernel       fixInternal (solidcloud.cpp:288-301) with the mesh's cell centres.
-// Every geometric decision is FP64 with the reference's operation sequence (the library is built with -fmad=false),
-// so touched sets and cell types equal the FP64 oracle's on the same mesh.
+// Which points are inside is decided by the reference's FP64 operation sequence (the library is built with -fmad=false)
+// wherever the FP32 bound leaves it open, and the seed by FP64 distances, so touched sets and cell types equal the FP64
+// oracle's on the same mesh.  The distances that the fractions are made of take the local point from the matrix of the
+// rotation (local_matrix), which differs from the reference's quaternion products in the last place.
 #include <cstdint>
 #include <cuda_runtime.h>
 
