@@ -29,7 +29,7 @@
 // Which points are inside is decided by the reference's FP64 operation sequence (the library is built with -fmad=false)
 // wherever the FP32 bound leaves it open, and the seed by FP64 distances, so touched sets and cell types equal the FP64
 // oracle's on the same mesh.  The distances that the fractions are made of take the local point from the matrix of the
-// rotation (local_matrix), which differs from the reference's quaternion products in the last place.
+// rotation (local_matrix), which differs from the reference's quaternion products in the last place (half spaces: the products).
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -545,6 +545,13 @@ __device__ inline double poly_line_fraction(double pa, double pb) {
     return -pa / (pb - pa);
 }
 
+// Distance of a half space.  It has no filter, and the geometry jumps by SMALL / h where it is zero or next to zero, so it is
+// taken in the reference's own operations; the other shapes' distances within 1e-8 are all -1e-8, and the matrix of the rotation
+// serves.  Out of line: the others have no registers to spare for it.
+static __device__ __noinline__ double poly_plane_phi(const PolyK& m, int32_t p, const sdfibm_solid_state& st) {
+    return world2local(poly_point(m, p), state_pos(st), state_quat(st)).y;
+}
+
 constexpr int POLY_MAX_CELL_POINTS = 64;  // points of a cell whose distances are kept; later ones count as 0
 
 // GeometricTools::calcApex over n points (geometrictools.cpp:25-45); point(i), phi(i)
@@ -569,14 +576,17 @@ __device__ inline D3 poly_apex(int n, const Point& point, const Phi& phi) {
 // and the pyramids are added in face order.  A thread per cell spent 169 us on the serial chain of one cylinder's cut
 // cells (FP64 instructions issue every 16 cycles a warp and wait on each other); 8 lanes cut the chain to one distance
 // and one face.  All lanes of the warp call it (c < 0: a group without a cell).
-__device__ double poly_cell_volume8(const PolyK& m, int32_t c, const ShapeK& sh, const D3& x, const double* R, double* phi) {
+__device__ double poly_cell_volume8(const PolyK& m, int32_t c, const ShapeK& sh, const sdfibm_solid_state& st, const D3& x,
+                                    const double* R, double* phi) {
     const int sub = threadIdx.x & 7;
     const int32_t p0 = c < 0 ? 0 : m.cp_off[c], np = c < 0 ? 0 : m.cp_off[c + 1] - p0;
     const int32_t* cp = m.cp + p0;
     for (int i = sub; i < np && i < POLY_MAX_CELL_POINTS; i += 8) {
         const D3 d = poly_point(m, cp[i]) - x;
-        phi[i] = sdf64(sh, D3{R[0] * d.x + R[1] * d.y + R[2] * d.z, R[3] * d.x + R[4] * d.y + R[5] * d.z,
-                              R[6] * d.x + R[7] * d.y + R[8] * d.z});
+        phi[i] = sh.type == SDFIBM_SHAPE_PLANE
+                     ? poly_plane_phi(m, cp[i], st)
+                     : sdf64(sh, D3{R[0] * d.x + R[1] * d.y + R[2] * d.z, R[3] * d.x + R[4] * d.y + R[5] * d.z,
+                                    R[6] * d.x + R[7] * d.y + R[8] * d.z});
     }
     __syncwarp();
     auto phi_at = [&](int slot) { return slot < POLY_MAX_CELL_POINTS ? phi[slot] : 0.0; };
@@ -727,7 +737,7 @@ __global__ void __launch_bounds__(256, 2) poly_couple_kernel(PolyK m, const Soli
         for (int g0 = 0; g0 + ((tid >> 5) << 2) < ncut; g0 += 32) {  // warp-uniform
             const int g = g0 + (tid >> 3);
             const int32_t cc = g < ncut ? s_cell[s_cut[g]] : -1;
-            const double vol = poly_cell_volume8(m, cc, sh, x, s_R, s_phi[tid >> 3]);
+            const double vol = poly_cell_volume8(m, cc, sh, st[s], x, s_R, s_phi[tid >> 3]);
             if (cc >= 0 && (tid & 7) == 0) s_alpha[s_cut[g]] = vol / m.Vc[cc];
         }
         __syncthreads();
