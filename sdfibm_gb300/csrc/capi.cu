@@ -539,8 +539,8 @@ int sdfibm_cuda_create(const sdfibm_mesh_desc* mesh, const sdfibm_solid_desc* so
     // work items of CHUNK_TILES tiles, of a solid of finite size fewer where they would leave warps of the launch without one
     // (about 24 warps an SM): one cylinder's 9 tiles took 36 us in two items and 12 in nine.  Of a half space nearly all tiles
     // are skipped: what counts of it is a layer of tiles (a row on flat meshes), and its items hold two at least.  A call with
-    // six walls and four spheres, items of one tile / by the rule, us: 10 697 / 5140 at 512^3 (eight), 1697 / 1134 at 256^3
-    // (six), 395 / 367 at 128^3 (two; eight 470); four walls and nine circles at 1024^2 163 / 149 (two; eight 171)
+    // six walls and four spheres, items of one tile / by the rule, us: 10 697 / 4833 at 512^3 (eight), 1697 / 1091 at 256^3
+    // (six), 395 / 361 at 128^3 (two; eight 470); four walls and nine circles at 1024^2 163 / 146 (two; eight 171)
     int64_t all_finite = 0, faces = 0;
     for (const SolidK& k : ctx->hk) {
         const int64_t a = k.ntile[0], b = k.ntile[1], c = k.ntile[2];

@@ -1501,7 +1501,7 @@ __device__ __forceinline__ bool fast_shape(const SolidK& k, const sdfibm_solid_s
 // FAST: the chunks classify_fast takes; else the others.  Chunks are taken one at a time with an atomic; on flat meshes the
 // other kernel first looks at the chunks before fast_chunks, nearly all of which are the first kernel's: 32 together, which
 // lie a grid of warps apart, since those of a tilted solid are neighbours (32 neighbours a warp, all shapes: one tailed circle of
-// 81 items 165 us, now 22; 1500 of them 893, now 152; 300 3-D shapes on two layers 248, now 31; GB300).
+// 81 items 165 us, now 22; 1500 of them 893, now 143; 300 3-D shapes on two layers 248, now 31; GB300).
 template <bool FLAT, int METHOD, bool FAST>
 __device__ __forceinline__ void classify_body(const ClassifyArgs& A) {
     const unsigned FULL = 0xffffffffu;

@@ -15,7 +15,7 @@
 //                         FP64 sums per cell over the solids and per solid over its cells.
 // A breadth-first search by one CTA per solid, after a scan of every cell centre, was bound by its chain of levels (dependent
 // loads, eight FP64 inside tests a cell) on one SM: interact took 2.30 ms for one cylinder on 78 400 graded cells and 2.97 ms
-// for 40 solids on 140 000 hexahedra; it takes 0.100 and 0.313 ms now (GB300).
+// for 40 solids on 140 000 hexahedra; it takes 0.100 and 0.306 ms now (GB300).
 // Other meshes keep the search itself, whose order decides the types:
 //   poly_enum_kernel      one CTA per solid: the seed by a scan of all centres, then a level-synchronous breadth-first
 //                         search with the reference's classification (CellEnumerator, src/cellenumerator.cpp:6-78): a
@@ -646,7 +646,7 @@ __device__ double poly_cell_volume8(const PolyK& m, int32_t c, const ShapeK& sh,
 // Touched cells of one solid (blockIdx.x), POLY_BATCH of them a CTA: linked, of the cells with an inside vertex in the order of
 // their list of words those in the seed's set (the others are marked); else of the touched list.  The cut cells of a batch are
 // spread over the CTA's 32 groups of 8 lanes, then a lane per cell does the forcing.  Bound by the FP64 pipe (about 2000
-// operations a cut cell): 174 us for the 140 000-cell mesh's 40 solids, 360 us with a thread per cell; 33 us against 169 us for
+// operations a cut cell): 172 us for the 140 000-cell mesh's 40 solids, 360 us with a thread per cell; 33 us against 169 us for
 // one cylinder.  (Batches of whole words, whose cells differ in number: 186 us.)  The solids run along grid.x, so that the first
 // batches of all of them land on different SMs.
 __global__ void __launch_bounds__(256, 2) poly_couple_kernel(PolyK m, const SolidK* __restrict__ sk,
