@@ -26,8 +26,10 @@ constexpr unsigned FULLMASK = 0xffffffffu;
 __device__ __forceinline__ float sigm(float z) { return __fdividef(1.f, 1.f + __expf(-z)); }
 // SiLU of two units at a time.  Its cost is the special-function unit, a quarter of the lanes: an exponential and a
 // reciprocal a unit.  Two units share the reciprocal of the product of their denominators (1.5 such operations a unit instead
-// of 2), and additions and scalings go two to an instruction.  The exponents are held below 2^60 so that the product stays
-// finite: z / (1 + exp(-z)) below z = -41 is then z 2^-60, below any rounding of the sums it enters.
+// of 2), and additions and scalings go two to an instruction.  z is held above -60 ln 2, so that the product of two denominators
+// stays finite and a unit beyond it, however far, is -41.6 2^-60: below any rounding of the sums it enters.  (With the exponent
+// alone held there a unit at z = -1e20 gave -87.)  A denominator is multiplied by the reciprocal first, which leaves a number
+// below 1, then by z.
 __device__ __forceinline__ float2 add2(float2 a, float2 b) {
     float2 r;
     asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;\n}"
@@ -50,19 +52,25 @@ __device__ __forceinline__ float rcp_fast(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-constexpr float LOG2E = 1.4426950408889634f;
-// z and the denominators 1 + exp(-z) of two units, and the reciprocal of the product of the denominators
-struct Silu2 {
-    float2 z, d;
+__device__ __forceinline__ float max_nan(float x, float y) {  // NaN if either is
     float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(y));
+    return r;
+}
+constexpr float LOG2E = 1.4426950408889634f;
+constexpr float SILU_LEAST = -41.588830833596715f;  // -60 ln 2
+// z and sigmoid(z) of two units
+struct Silu2 {
+    float2 z, s;
 };
 __device__ __forceinline__ Silu2 silu2(float2 zin, float2 b) {
-    Silu2 s;
-    s.z = add2(zin, b);
-    const float2 t = mul2(s.z, make_float2(-LOG2E, -LOG2E));
-    s.d = add2(make_float2(ex2_fast(fminf(t.x, 60.f)), ex2_fast(fminf(t.y, 60.f))), make_float2(1.f, 1.f));
-    s.r = rcp_fast(s.d.x * s.d.y);
-    return s;
+    Silu2 q;
+    q.z = add2(zin, b);
+    q.z = make_float2(max_nan(q.z.x, SILU_LEAST), max_nan(q.z.y, SILU_LEAST));
+    const float2 t = mul2(q.z, make_float2(-LOG2E, -LOG2E)), d = add2(make_float2(ex2_fast(t.x), ex2_fast(t.y)), make_float2(1.f, 1.f));
+    const float r = rcp_fast(d.x * d.y);
+    q.s = mul2(make_float2(d.y, d.x), make_float2(r, r));
+    return q;
 }
 
 __device__ __forceinline__ uint32_t bf16_bits(float x) {
@@ -198,7 +206,7 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
 // has completed, and A1 only after the layer-2 MMA has), and D2 takes D1's tensor-memory columns (the layer-2 MMA is
 // issued after every thread has read D1): 45 KB of shared memory and 64 columns per CTA, five CTAs per SM.
 // Bound by the special-function unit (192 operations a cell, 174 us for 4 194 304 cells) and by issue: with a reciprocal a
-// unit, single additions and the library exponential's range handling that took 400 us, now 256 (GB300).
+// unit, single additions and the library exponential's range handling that took 400 us, now 253 (GB300).
 constexpr int INF_W1 = 0, INF_W2 = 2048, INF_A2 = 10240, INF_A1 = INF_A2, INF_F = INF_A2 + 32768;
 constexpr int INF_CTAS = 5;
 constexpr int INF_SMEM = INF_F + 4 * 64 * 4 + 64 + 1024;
@@ -267,10 +275,11 @@ __global__ void __launch_bounds__(MLP_THREADS, INF_CTAS) mlp_infer_kernel(MlpInf
                 const float4 b = b4[j >> 2];
                 const Silu2 p = silu2(make_float2(z[j], z[j + 1]), make_float2(b.x, b.y));
                 const Silu2 q = silu2(make_float2(z[j + 2], z[j + 3]), make_float2(b.z, b.w));
-                z[j] = (p.z.x * p.d.y) * p.r;
-                z[j + 1] = (p.z.y * p.d.x) * p.r;
-                z[j + 2] = (q.z.x * q.d.y) * q.r;
-                z[j + 3] = (q.z.y * q.d.x) * q.r;
+                const float2 hp = mul2(p.z, p.s), hq = mul2(q.z, q.s);
+                z[j] = hp.x;
+                z[j + 1] = hp.y;
+                z[j + 2] = hq.x;
+                z[j + 3] = hq.y;
             }
             store_a2<4>(sA2, tid, z, 4 * half);
         }
@@ -296,8 +305,8 @@ __global__ void __launch_bounds__(MLP_THREADS, INF_CTAS) mlp_infer_kernel(MlpInf
                 const Silu2 p = silu2(make_float2(z[j], z[j + 1]), make_float2(b.x, b.y));
                 const Silu2 q = silu2(make_float2(z[j + 2], z[j + 3]), make_float2(b.z, b.w));
                 const float2 np = mul2(p.z, make_float2(w.x, w.y)), nq = mul2(q.z, make_float2(w.z, w.w));
-                o = __fmaf_rn(__fmaf_rn(np.y, p.d.x, np.x * p.d.y), p.r, o);
-                o = __fmaf_rn(__fmaf_rn(nq.y, q.d.x, nq.x * q.d.y), q.r, o);
+                o = __fmaf_rn(np.y, p.s.y, __fmaf_rn(np.x, p.s.x, o));
+                o = __fmaf_rn(nq.y, q.s.y, __fmaf_rn(nq.x, q.s.x, o));
             }
         }
         const float a = sigm(prior_t + o);
@@ -429,8 +438,8 @@ __global__ void __launch_bounds__(TR_THREADS, TR_CTAS) mlp_grad_kernel(MlpGradAr
 #pragma unroll
         for (int j = 0; j < 16; j += 2) {
             const Silu2 p = silu2(make_float2(v[j], v[j + 1]), make_float2(sb1[c0 + j], sb1[c0 + j + 1]));
-            v[j] = (p.z.x * p.d.y) * p.r;
-            v[j + 1] = (p.z.y * p.d.x) * p.r;
+            v[j] = p.z.x * p.s.x;
+            v[j + 1] = p.z.y * p.s.y;
             store_bf16(sGB, c0 + j, row, 128, v[j]);
             store_bf16(sGB, c0 + j + 1, row, 128, v[j + 1]);
         }
@@ -451,7 +460,7 @@ __global__ void __launch_bounds__(TR_THREADS, TR_CTAS) mlp_grad_kernel(MlpGradAr
 #pragma unroll
         for (int j = 0; j < 16; j += 2) {
             const Silu2 p = silu2(make_float2(v[j], v[j + 1]), make_float2(sb2[c0 + j], sb2[c0 + j + 1]));
-            const float s0 = p.d.y * p.r, s1 = p.d.x * p.r;
+            const float s0 = p.s.x, s1 = p.s.y;
             w[j] = p.z.x * s0;
             w[j + 1] = p.z.y * s1;
             o += sw3[c0 + j] * w[j];
@@ -517,7 +526,7 @@ __global__ void __launch_bounds__(TR_THREADS, TR_CTAS) mlp_grad_kernel(MlpGradAr
 #pragma unroll
         for (int j = 0; j < 16; j += 2) {
             const Silu2 p = silu2(make_float2(w[j], w[j + 1]), make_float2(sb1[c0 + j], sb1[c0 + j + 1]));
-            const float s0 = p.d.y * p.r, s1 = p.d.x * p.r;
+            const float s0 = p.s.x, s1 = p.s.y;
             v[j] *= s0 * (1.f + p.z.x * (1.f - s0));   // dZ1
             v[j + 1] *= s1 * (1.f + p.z.y * (1.f - s1));
             store_bf16(sGA, 64 + c0 + j, row, 128, v[j]);
