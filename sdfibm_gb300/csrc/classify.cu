@@ -855,11 +855,12 @@ __device__ inline float sdf_ff_at(const ShapeK& s, const FF (&P)[3], float ml, f
     return sqrtf(dxp * dxp + dyp * dyp + dzp * dzp) + fminf(0.f, fmaxf(d[2], fmaxf(d[0], d[1])));
 }
 
-// the filter of sdf.h:147-150 on such a value; false: its decision is not certain
+// the filter of sdf.h:147-150 on such a value; false: its decision is not certain, as where den is 0 or the value no number (an
+// ellipsoid's distance next to its centre)
 __device__ __forceinline__ bool ff_filter(float& phi, float err, float den) {
     const float a = fabsf(phi);
     if (a < 1e-8f) phi = -1e-8f;
-    return !((fabsf(a - 1e-8f) - 1e-14f) * den <= err);
+    return (fabsf(a - 1e-8f) - 1e-14f) * den > err;
 }
 __device__ inline float sdf_ff(const ShapeK& s, const SolidPlan& pl, float da, float db, float dc, float& err,
                                float& den) {
