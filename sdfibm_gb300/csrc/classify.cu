@@ -875,11 +875,12 @@ __device__ inline float sdf_ff(const ShapeK& s, const SolidPlan& pl, float da, f
     return sdf_ff_at(s, P, ml, err, den);
 }
 
-// filter of sdf.h:147-150 applied to a value of sdf_mixed; *exact_needed set when the value sits on the threshold
+// filter of sdf.h:147-150 applied to a value of sdf_mixed; *exact_needed set when the value sits on the threshold or is no number (an
+// ellipse's next to its axis)
 __device__ inline float filter_mixed(const ShapeK& s, float phi, bool* exact_needed) {
     if (s.type == SDFIBM_SHAPE_PLANE) return phi;  // the plane's distance is unfiltered and exact
     const float a = fabsf(phi);
-    if (fabsf(a - 1e-8f) <= 1e-14f) *exact_needed = true;
+    if (!(fabsf(a - 1e-8f) > 1e-14f && a < INFINITY)) *exact_needed = true;
     return a < 1e-8f ? -1e-8f : phi;
 }
 
