@@ -545,11 +545,12 @@ __device__ inline double poly_line_fraction(double pa, double pb) {
     return -pa / (pb - pa);
 }
 
-// Distance of a half space.  It has no filter, and the geometry jumps by SMALL / h where it is zero or next to zero, so it is
-// taken in the reference's own operations; the other shapes' distances within 1e-8 are all -1e-8, and the matrix of the rotation
-// serves.  Out of line: the others have no registers to spare for it.
-static __device__ __noinline__ double poly_plane_phi(const PolyK& m, int32_t p, const sdfibm_solid_state& st) {
-    return world2local(poly_point(m, p), state_pos(st), state_quat(st)).y;
+// Distance in the reference's own operations.  A half space has no filter, and the geometry jumps by SMALL / h where its distance is
+// zero or next to zero, so it is always taken from here; the other shapes' distances within 1e-8 are all -1e-8, and the matrix of
+// the rotation serves, but for the ellipse and the ellipsoid at their centre, where it can be no number when the reference's is.
+// Out of line: the others have no registers to spare for it.
+static __device__ __noinline__ double poly_exact_phi(const PolyK& m, const ShapeK& sh, int32_t p, const sdfibm_solid_state& st) {
+    return sdf64(sh, world2local(poly_point(m, p), state_pos(st), state_quat(st)));
 }
 
 constexpr int POLY_MAX_CELL_POINTS = 64;  // points of a cell whose distances are kept; later ones count as 0
@@ -583,10 +584,15 @@ __device__ double poly_cell_volume8(const PolyK& m, int32_t c, const ShapeK& sh,
     const int32_t* cp = m.cp + p0;
     for (int i = sub; i < np && i < POLY_MAX_CELL_POINTS; i += 8) {
         const D3 d = poly_point(m, cp[i]) - x;
-        phi[i] = sh.type == SDFIBM_SHAPE_PLANE
-                     ? poly_plane_phi(m, cp[i], st)
-                     : sdf64(sh, D3{R[0] * d.x + R[1] * d.y + R[2] * d.z, R[3] * d.x + R[4] * d.y + R[5] * d.z,
-                                    R[6] * d.x + R[7] * d.y + R[8] * d.z});
+        bool exact = sh.type == SDFIBM_SHAPE_PLANE;
+        double v = 0.0;
+        if (!exact) {
+            v = sdf64(sh, D3{R[0] * d.x + R[1] * d.y + R[2] * d.z, R[3] * d.x + R[4] * d.y + R[5] * d.z,
+                             R[6] * d.x + R[7] * d.y + R[8] * d.z});
+            exact = (__double2hiint(v) & 0x7ff00000) == 0x7ff00000;
+        }
+        if (exact) v = poly_exact_phi(m, sh, cp[i], st);
+        phi[i] = v;
     }
     __syncwarp();
     auto phi_at = [&](int slot) { return slot < POLY_MAX_CELL_POINTS ? phi[slot] : 0.0; };
