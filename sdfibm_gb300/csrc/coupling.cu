@@ -70,7 +70,8 @@ __device__ inline void plan_box(const MeshK& m, const SolidK& k, const Q4& q, co
             if (az < 0.3 && (k.ext[0] < n[0] + 2 || k.ext[1] < n[1] + 2)) err = DERR_BBOX;
             const double zlo = m.o[2], zhi = mesh_coord(m, 2, m.nz);
             const double zspan = dmax(fabs(zhi - cw.z), fabs(zlo - cw.z));
-            const double rxy = (sxy > 0) ? r + (zspan + r * sxy) / dmax(az, 0.3) * sxy : r;
+            // one that lies: no bound, the window spans the mesh
+            const double rxy = az < 0.3 ? INFINITY : (sxy > 0 ? r + (zspan + r * sxy) / az * sxy : r);
             rad[0] = rad[1] = rxy * (1.0 + 1e-9);
         }
         // half extents of the oriented bounding box of the inside region along the world axes; FP32, widened
