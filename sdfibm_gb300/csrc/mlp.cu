@@ -59,17 +59,19 @@ __device__ __forceinline__ float max_nan(float x, float y) {  // NaN if either i
 }
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float SILU_LEAST = -41.588830833596715f;  // -60 ln 2
-// z and sigmoid(z) of two units
+// z and sigmoid(z) of two units.  PAIR: their products two to an instruction (the gradient kernel, at 64 registers, spills more
+// with them)
 struct Silu2 {
     float2 z, s;
 };
+template <bool PAIR>
 __device__ __forceinline__ Silu2 silu2(float2 zin, float2 b) {
     Silu2 q;
     q.z = add2(zin, b);
     q.z = make_float2(max_nan(q.z.x, SILU_LEAST), max_nan(q.z.y, SILU_LEAST));
     const float2 t = mul2(q.z, make_float2(-LOG2E, -LOG2E)), d = add2(make_float2(ex2_fast(t.x), ex2_fast(t.y)), make_float2(1.f, 1.f));
     const float r = rcp_fast(d.x * d.y);
-    q.s = mul2(make_float2(d.y, d.x), make_float2(r, r));
+    q.s = PAIR ? mul2(make_float2(d.y, d.x), make_float2(r, r)) : make_float2(d.y * r, d.x * r);
     return q;
 }
 
@@ -206,7 +208,7 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
 // has completed, and A1 only after the layer-2 MMA has), and D2 takes D1's tensor-memory columns (the layer-2 MMA is
 // issued after every thread has read D1): 45 KB of shared memory and 64 columns per CTA, five CTAs per SM.
 // Bound by the special-function unit (192 operations a cell, 174 us for 4 194 304 cells) and by issue: with a reciprocal a
-// unit, single additions and the library exponential's range handling that took 400 us, now 253 (GB300).
+// unit, single additions and the library exponential's range handling that took 400 us, now 256 (GB300).
 constexpr int INF_W1 = 0, INF_W2 = 2048, INF_A2 = 10240, INF_A1 = INF_A2, INF_F = INF_A2 + 32768;
 constexpr int INF_CTAS = 5;
 constexpr int INF_SMEM = INF_F + 4 * 64 * 4 + 64 + 1024;
@@ -273,8 +275,8 @@ __global__ void __launch_bounds__(MLP_THREADS, INF_CTAS) mlp_infer_kernel(MlpInf
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
                 const float4 b = b4[j >> 2];
-                const Silu2 p = silu2(make_float2(z[j], z[j + 1]), make_float2(b.x, b.y));
-                const Silu2 q = silu2(make_float2(z[j + 2], z[j + 3]), make_float2(b.z, b.w));
+                const Silu2 p = silu2<true>(make_float2(z[j], z[j + 1]), make_float2(b.x, b.y));
+                const Silu2 q = silu2<true>(make_float2(z[j + 2], z[j + 3]), make_float2(b.z, b.w));
                 const float2 hp = mul2(p.z, p.s), hq = mul2(q.z, q.s);
                 z[j] = hp.x;
                 z[j + 1] = hp.y;
@@ -302,8 +304,8 @@ __global__ void __launch_bounds__(MLP_THREADS, INF_CTAS) mlp_infer_kernel(MlpInf
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
                 const float4 b = b4[j >> 2], w = w4[j >> 2];
-                const Silu2 p = silu2(make_float2(z[j], z[j + 1]), make_float2(b.x, b.y));
-                const Silu2 q = silu2(make_float2(z[j + 2], z[j + 3]), make_float2(b.z, b.w));
+                const Silu2 p = silu2<true>(make_float2(z[j], z[j + 1]), make_float2(b.x, b.y));
+                const Silu2 q = silu2<true>(make_float2(z[j + 2], z[j + 3]), make_float2(b.z, b.w));
                 const float2 np = mul2(p.z, make_float2(w.x, w.y)), nq = mul2(q.z, make_float2(w.z, w.w));
                 o = __fmaf_rn(np.y, p.s.y, __fmaf_rn(np.x, p.s.x, o));
                 o = __fmaf_rn(nq.y, q.s.y, __fmaf_rn(nq.x, q.s.x, o));
@@ -437,7 +439,7 @@ __global__ void __launch_bounds__(TR_THREADS, TR_CTAS) mlp_grad_kernel(MlpGradAr
         tc::tmem_wait_ld();
 #pragma unroll
         for (int j = 0; j < 16; j += 2) {
-            const Silu2 p = silu2(make_float2(v[j], v[j + 1]), make_float2(sb1[c0 + j], sb1[c0 + j + 1]));
+            const Silu2 p = silu2<false>(make_float2(v[j], v[j + 1]), make_float2(sb1[c0 + j], sb1[c0 + j + 1]));
             v[j] = p.z.x * p.s.x;
             v[j + 1] = p.z.y * p.s.y;
             store_bf16(sGB, c0 + j, row, 128, v[j]);
@@ -459,7 +461,7 @@ __global__ void __launch_bounds__(TR_THREADS, TR_CTAS) mlp_grad_kernel(MlpGradAr
         float o = 0.f;
 #pragma unroll
         for (int j = 0; j < 16; j += 2) {
-            const Silu2 p = silu2(make_float2(v[j], v[j + 1]), make_float2(sb2[c0 + j], sb2[c0 + j + 1]));
+            const Silu2 p = silu2<false>(make_float2(v[j], v[j + 1]), make_float2(sb2[c0 + j], sb2[c0 + j + 1]));
             const float s0 = p.s.x, s1 = p.s.y;
             w[j] = p.z.x * s0;
             w[j + 1] = p.z.y * s1;
@@ -525,7 +527,7 @@ __global__ void __launch_bounds__(TR_THREADS, TR_CTAS) mlp_grad_kernel(MlpGradAr
         tc::tmem_wait_ld();
 #pragma unroll
         for (int j = 0; j < 16; j += 2) {
-            const Silu2 p = silu2(make_float2(w[j], w[j + 1]), make_float2(sb1[c0 + j], sb1[c0 + j + 1]));
+            const Silu2 p = silu2<false>(make_float2(w[j], w[j + 1]), make_float2(sb1[c0 + j], sb1[c0 + j + 1]));
             const float s0 = p.s.x, s1 = p.s.y;
             v[j] *= s0 * (1.f + p.z.x * (1.f - s0));   // dZ1
             v[j + 1] *= s1 * (1.f + p.z.y * (1.f - s1));
